@@ -194,6 +194,8 @@ struct Context {
   DevBuf<float> dSameVal, dOppVal;
   DevBuf<int16_t> dSamePairs, dOppPairs;
   DevBuf<int64_t> dSameStart, dOppStart;
+  DevBuf<uint32_t> dHbCum;
+  ParentSplit psplit;  // work units of the selection and of the PT generator
   SelectParams sp;
 
   DevBuf<Det2> dets;
@@ -348,7 +350,7 @@ struct Context {
     return IntsView{dI1.p, dI2.p, dDirect.p, dExchange.p, hints.norb, dI1f.p, dI2f.p, dV1.p, dV1f.p};
   }
   HeatBathView hb() const {
-    return HeatBathView{dSameVal.p, dSamePairs.p, dSameStart.p, dOppVal.p, dOppPairs.p, dOppStart.p, dSingles.p};
+    return HeatBathView{dSameVal.p, dSamePairs.p, dSameStart.p, dOppVal.p, dOppPairs.p, dOppStart.p, dSingles.p, dHbCum.p};
   }
   void require_ints() const {
     if (!have_ints) throw Error(kErrState, "no integrals loaded (call shci_read_fcidump first)");
@@ -393,6 +395,7 @@ struct Context {
     upload(dOppPairs, hhb.oppPairs);
     upload(dSameStart, hhb.sameStart);
     upload(dOppStart, hhb.oppStart);
+    upload(dHbCum, hhb.cum);
     SHCI_CUDA(cudaStreamSynchronize(stream));
     have_ints = true;
     ndet = 0;
@@ -497,13 +500,13 @@ struct Context {
     cand.reserve((size_t)cap);
     cap = (int64_t)cand.cap;
     int64_t total = select_candidates(dets.p, cmax_dev, ndet, eps1, ints(), hb(), hints.maxEntry, sp, hash, cand.p,
-                                      cap, counter.p, stream);
+                                      cap, counter.p, psplit, stream);
     if (total > cap) {
       cand.release();
       cand.reserve((size_t)total + total / 8);
       cap = (int64_t)cand.cap;
       total = select_candidates(dets.p, cmax_dev, ndet, eps1, ints(), hb(), hints.maxEntry, sp, hash, cand.p, cap,
-                                counter.p, stream);
+                                counter.p, psplit, stream);
       if (total > cap) throw Error(kErrState, "candidate count changed between passes");
     }
     size_t nnew = 0;
@@ -603,7 +606,7 @@ struct Context {
     psp.ncore = 0;
     psp.nact = 1 << 30;
     pt_last = pt_deterministic(dets.p, ndet, c, E0 - hints.coreE, eps2, ints(), hb(), hints.maxEntry, psp, hash,
-                               pt_max_cand, ptw, prims, stream);
+                               pt_max_cand, ptw, psplit, prims, stream);
     t_pt = now_s() - t0;
     pts_last = PtStochResult();
     return pt_last.e2;
@@ -677,7 +680,7 @@ struct Context {
     psp.ncore = 0;
     psp.nact = 1 << 30;
     pts_last = pt_semistochastic(dets.p, ndet, c, ch, E0 - hints.coreE, eps2, eps2L, nsample, max_iter, target, seed,
-                                 ints(), hb(), hints.maxEntry, psp, hash, ptw, prims, stream);
+                                 ints(), hb(), hints.maxEntry, psp, hash, ptw, psplit, prims, stream);
     pt_last = PtResult();
     pt_last.candidates = pts_last.candidates;
     t_pt = now_s() - t0;

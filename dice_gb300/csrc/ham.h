@@ -154,7 +154,59 @@ struct HeatBathView {
   const int16_t* oppPairs;
   const int64_t* oppStart;
   const double* singles;  // (2n)x(2n)
+  // entries of all same-spin / opposite-spin lists whose |value| has these top
+  // 11 bits (bin = bits >> 20) or larger ones: [same, opp][kHbBins]
+  const uint32_t* cum;
 };
+
+// Work units of the kernels that expand parent determinants by the heat-bath
+// lists (selection, perturbation theory). A parent's work goes with the list
+// entries above its threshold eps / |c|, which spans five orders of magnitude
+// over a space: one warp per parent leaves the GPU waiting for the few warps
+// that hold the largest coefficients. A parent estimated above kSplitEntries
+// entries is cut into nsl[p] slices; `extra` lists its slices 1.. (in no
+// particular order, 0xffffffff = unused), and slice 0 of every parent follows
+// them implicitly: unit u < count is extra[u], then parent u - count.
+struct SplitView {
+  const uint2* extra;
+  const unsigned char* nsl;
+  const uint32_t* count;  // claimed entries of extra (may pass cap)
+  uint32_t cap;
+  unsigned long long* next;  // unit queue
+};
+struct ParentSplit {
+  DevBuf<uint2> extra;
+  DevBuf<unsigned char> nsl;
+  DevBuf<uint32_t> count;
+  DevBuf<unsigned long long> next;
+  uint32_t cap = 0;
+  SplitView view() const { return SplitView{extra.p, nsl.p, count.p, cap, next.p}; }
+  void rewind(cudaStream_t s) { SHCI_CUDA(cudaMemsetAsync(next.p, 0, sizeof(unsigned long long), s)); }
+};
+// Splits n parents (plist[i], or i) with thresholds eps / |c[parent]|; the queue
+// starts at its beginning.
+void split_parents(const Det2* dets, const int32_t* plist, const double* c, size_t n, double eps, double maxEntry,
+                   const HeatBathView& hb, int norb, ParentSplit& ps, cudaStream_t s);
+
+// The next unit for the calling warp; false when the queue is empty. Parent
+// 0xffffffff: an unused entry, to be skipped.
+__device__ __forceinline__ bool next_unit(const SplitView& v, size_t n, uint32_t nextra, uint32_t& parent, int& slice,
+                                          int& slices) {
+  unsigned long long u = 0;
+  if ((threadIdx.x & 31) == 0) u = atomicAdd(v.next, 1ull);
+  u = __shfl_sync(kFull, u, 0);
+  if (u >= (unsigned long long)n + nextra) return false;
+  if (u < nextra) {
+    const uint2 e = v.extra[u];
+    parent = e.x;
+    slice = (int)e.y;
+  } else {
+    parent = (uint32_t)(u - nextra);
+    slice = 0;
+  }
+  slices = parent != 0xffffffffu ? v.nsl[parent] : 1;
+  return true;
+}
 
 constexpr int kMaxRestrict = 4;
 struct SelectParams {
@@ -191,7 +243,7 @@ __device__ __forceinline__ int in_mask(const SelectParams& sp, int r, int p) {
 // cap is written and the caller retries with a larger buffer).
 int64_t select_candidates(const Det2* dets, const double* cmax, size_t n, double eps1, const IntsView& ints,
                           const HeatBathView& hb, double maxEntry, const SelectParams& sp, const DetHash& present,
-                          Det2* out, int64_t cap, int64_t* d_counter, cudaStream_t s);
+                          Det2* out, int64_t cap, int64_t* d_counter, ParentSplit& ps, cudaStream_t s);
 // Time reversal (kernels_select.cu): cMax of the reference's symmetrized
 // basis for every determinant (0 for the non-standard member of a pair), and
 // the new determinants of a selection: the standard members of the
@@ -248,7 +300,7 @@ struct PtWork {
 // max_candidates > 0 caps one partition (default: from free device memory).
 PtResult pt_deterministic(const Det2* dets, size_t n, const double* c, double E0, double eps2, const IntsView& ints,
                           const HeatBathView& hb, double maxEntry, const SelectParams& sp, const DetHash& present,
-                          int64_t max_candidates, PtWork& w, Prims& pr, cudaStream_t s);
+                          int64_t max_candidates, PtWork& w, ParentSplit& ps, Prims& pr, cudaStream_t s);
 
 // ---- reduced density matrices (kernels_rdm.cu) ------------------------------
 // Spatial 2-RDM (out[0, n^4): element (p n + q, r n + s) at (p n + q) n^2 + r n + s)
@@ -270,8 +322,8 @@ struct PtStochResult {
 PtStochResult pt_semistochastic(const Det2* dets, size_t n, const double* c_dev, const std::vector<double>& c_host,
                                 double E0, double eps2, double eps2L, int nsample, int max_iter, double target,
                                 uint64_t seed, const IntsView& ints, const HeatBathView& hb, double maxEntry,
-                                const SelectParams& sp, const DetHash& present, PtWork& w, Prims& pr,
-                                cudaStream_t s);
+                                const SelectParams& sp, const DetHash& present, PtWork& w, ParentSplit& ps,
+                                Prims& pr, cudaStream_t s);
 
 // ---- sigma and Davidson vector kernels (kernels_sigma.cu) -------------------
 // Y[:, c] (column-major, leading dimension ldy) = diag .* X[:, c] + Hoff X[:, c]

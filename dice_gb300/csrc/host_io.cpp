@@ -184,6 +184,18 @@ void build_heatbath(const HostInts& H, HostHeatBath& hb) {
       hb.sameStart.push_back((int64_t)hb.sameVal.size());
       hb.oppStart.push_back((int64_t)hb.oppVal.size());
     }
+  // how many entries are at least as large, by the top bits of |value| (exponent
+  // and three fraction bits): what a threshold costs, without searching the lists
+  hb.cum.assign(2 * kHbBins, 0);
+  for (int w = 0; w < 2; ++w) {
+    uint32_t* c = hb.cum.data() + (size_t)w * kHbBins;
+    for (float v : w ? hb.oppVal : hb.sameVal) {
+      uint32_t u;
+      std::memcpy(&u, &v, sizeof(u));
+      ++c[(u & 0x7fffffffu) >> 20];
+    }
+    for (int b = kHbBins - 2; b >= 0; --b) c[b] += c[b + 1];
+  }
   const int n2 = 2 * n;
   hb.singles.assign((size_t)n2 * n2, 0.0);
   for (int i = 0; i < n2; i++)

@@ -17,11 +17,13 @@ struct HostInts {
   double i2(int i, int j, int k, int l) const;  // spin-orbital accessor
 };
 
+constexpr int kHbBins = 2048;  // bins of |value| by its top 11 bits (exponent, three fraction bits)
 struct HostHeatBath {
   std::vector<float> sameVal, oppVal;
   std::vector<int16_t> samePairs, oppPairs;
   std::vector<int64_t> sameStart, oppStart;
   std::vector<double> singles;
+  std::vector<uint32_t> cum;  // [same, opp][bin]: entries in this bin or a larger one
 };
 
 struct Restriction {

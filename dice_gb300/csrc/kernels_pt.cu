@@ -86,7 +86,7 @@ struct PtArgs {
   const float* exch32;
   const float2* coulff;  // and as float pairs
   const float2* exchff;
-  unsigned long long* next;     // parent queue
+  SplitView split;              // work units
   unsigned long long* counter;  // candidates appended (counts past cap too)
   int64_t cap;
   uint64_t* key0;  // candidate determinant, low word
@@ -322,11 +322,11 @@ __global__ void __launch_bounds__(kPtThreads) k_pt_gen(PtArgs a) {
   const unsigned lt = (1u << lane) - 1u;
   const int n2 = 2 * n;
   const SelectParams& sp = a.sp;
-  while (true) {
-    unsigned long long pp = 0;
-    if (lane == 0) pp = atomicAdd(a.next, 1ull);
-    pp = __shfl_sync(kFull, pp, 0);
-    if (pp >= (unsigned long long)a.n) break;
+  const uint32_t nextra = min(*a.split.count, a.split.cap);
+  uint32_t pp;
+  int slice, slices;
+  while (next_unit(a.split, a.n, nextra, pp, slice, slices)) {
+    if (pp == 0xffffffffu) continue;
     const size_t p = a.plist ? (size_t)a.plist[pp] : (size_t)pp;
     const Det2 d = a.dets[p];
     const double cp = a.c[p];
@@ -483,7 +483,7 @@ __global__ void __launch_bounds__(kPtThreads) k_pt_gen(PtArgs a) {
     // I1 has no alpha-beta block); FP32 screen here, the rest when drained
     const int ncB = nclosed - ncA, nhB = n - ncB;
     const int nsA = ncA * nhA, ns = nsA + ncB * nhB;
-    for (int b0 = 0; b0 < ns; b0 += 32) {
+    for (int b0 = 32 * slice; b0 < ns; b0 += 32 * slices) {
       const int q = b0 + lane;
       bool surv = false;
       int ci = 0, oa = 0;
@@ -512,8 +512,9 @@ __global__ void __launch_bounds__(kPtThreads) k_pt_gen(PtArgs a) {
     // for a float v, (double)|v| < eps exactly when |v| < eps rounded up to float
     const float eps_f = __double2float_ru(eps);
     const int npairs = nclosed * (nclosed - 1) / 2;
-    for (int pb = 0; pb < npairs; pb += 32) {
-      const int q = pb + lane;
+    // this slice's pairs: q = slice, slice + slices, ...
+    for (int pb = slice; pb < npairs; pb += 32 * slices) {
+      const int q = pb + lane * slices;
       int ci = 0, cj = 0;
       int64_t lstart = 0, len = 0;
       bool same = false;
@@ -835,6 +836,7 @@ __global__ void __launch_bounds__(kPtRedThreads) k_pt_reduce_stoch(const uint64_
     const uint64_t d0 = k0[k], d1 = k1[k];
     if (k > 0 && d0 == k0[k - 1] && d1 == k1[k - 1]) continue;
     __int128 s1 = 0, s2 = 0, s1b = 0, s2b = 0;
+    bool flagged = false;
     float2 e = make_float2(INFINITY, 0.0f);
     for (size_t j = k; j < m; ++j) {
       if (j > k && (k0[j] != d0 || k1[j] != d1)) break;
@@ -847,14 +849,18 @@ __global__ void __launch_bounds__(kPtRedThreads) k_pt_reduce_stoch(const uint64_
       if (x.x != 0.0f) {
         s1b += f1;
         s2b += f2;
+        flagged = true;
       }
       const float2 ej = make_float2(x.z, x.w);
       if (ff_less(ej, e)) e = ej;
     }
     const double de = (double)e.x + (double)e.y;  // E_a - E0
-    const double n1 = from_fix(s1), n1b = from_fix(s1b);
+    const double n1 = from_fix(s1);
     eA += (n1 * n1 * f - from_fix(s2)) / de;
-    eB += (n1b * n1b * f - from_fix(s2b)) / de;
+    if (flagged) {  // without a deterministic part nothing is: its FP64 work is half of the kernel's
+      const double n1b = from_fix(s1b);
+      eB += (n1b * n1b * f - from_fix(s2b)) / de;
+    }
     cnt += 1.0;
   }
   __shared__ double r0[kPtRedThreads / 32], r1[kPtRedThreads / 32], r2[kPtRedThreads / 32];
@@ -891,7 +897,7 @@ namespace {
 size_t pt_prepare(PtArgs& a, const Det2* dets, size_t n, const double* c, double E0, double eps2,
                   const IntsView& ints, const HeatBathView& hb, double maxEntry, const SelectParams& sp,
                   const DetHash& present, PtWork& w, cudaStream_t s) {
-  w.next.resize(2);
+  w.next.resize(1);
   w.part.resize(3 * kPtRedBlocks);
   a = PtArgs{};
   a.dets = dets;
@@ -904,8 +910,7 @@ size_t pt_prepare(PtArgs& a, const Det2* dets, size_t n, const double* c, double
   a.sp = sp;
   a.hslots = present.slots.p;
   a.hmask = present.mask;
-  a.next = w.next.p;
-  a.counter = w.next.p + 1;
+  a.counter = w.next.p;
   a.nparts = 1;
   if (w.tables_of != ints.I2 || w.tables_n != ints.norb) {
     const size_t nt = (size_t)ints.norb * ints.norb * ints.norb;
@@ -940,12 +945,14 @@ size_t pt_prepare(PtArgs& a, const Det2* dets, size_t n, const double* c, double
 
 PtResult pt_deterministic(const Det2* dets, size_t n, const double* c, double E0, double eps2, const IntsView& ints,
                           const HeatBathView& hb, double maxEntry, const SelectParams& sp, const DetHash& present,
-                          int64_t max_candidates, PtWork& w, Prims& pr, cudaStream_t s) {
+                          int64_t max_candidates, PtWork& w, ParentSplit& ps, Prims& pr, cudaStream_t s) {
   PtResult res;
   if (n == 0) return res;
   if (!(eps2 >= 0.0)) throw Error(kErrInvalid, "epsilon2 must be >= 0");
   PtArgs a;
+  split_parents(dets, nullptr, c, n, eps2, maxEntry, hb, ints.norb, ps, s);
   const size_t gsmem = pt_prepare(a, dets, n, c, E0, eps2, ints, hb, maxEntry, sp, present, w, s);
+  a.split = ps.view();
 
   // capacity of one partition
   int64_t cap = max_candidates;
@@ -974,11 +981,12 @@ PtResult pt_deterministic(const Det2* dets, size_t n, const double* c, double E0
     a.key0 = w.key0.p;
     a.key1 = w.key1.p;
     a.ne = w.ne.p;
-    SHCI_CUDA(cudaMemsetAsync(w.next.p, 0, 2 * sizeof(unsigned long long), s));
+    SHCI_CUDA(cudaMemsetAsync(w.next.p, 0, sizeof(unsigned long long), s));
+    ps.rewind(s);
     k_pt_gen<<<kPtGenBlocks, kPtThreads, gsmem, s>>>(a);
     SHCI_LAUNCH_CHECK();
     unsigned long long total = 0;
-    SHCI_CUDA(cudaMemcpyAsync(&total, w.next.p + 1, sizeof(total), cudaMemcpyDeviceToHost, s));
+    SHCI_CUDA(cudaMemcpyAsync(&total, w.next.p, sizeof(total), cudaMemcpyDeviceToHost, s));
     SHCI_CUDA(cudaStreamSynchronize(s));
     return (int64_t)total;
   };
@@ -1071,15 +1079,15 @@ static void alias_setup(const std::vector<double>& ci, double cumulative, std::v
 PtStochResult pt_semistochastic(const Det2* dets, size_t n, const double* c_dev, const std::vector<double>& c_host,
                                 double E0, double eps2, double eps2L, int nsample, int max_iter, double target,
                                 uint64_t seed, const IntsView& ints, const HeatBathView& hb, double maxEntry,
-                                const SelectParams& sp, const DetHash& present, PtWork& w, Prims& pr,
-                                cudaStream_t s) {
+                                const SelectParams& sp, const DetHash& present, PtWork& w, ParentSplit& ps,
+                                Prims& pr, cudaStream_t s) {
   PtStochResult res;
   if (n == 0) return res;
   if (!(eps2 >= 0.0)) throw Error(kErrInvalid, "epsilon2 must be >= 0");
   if (nsample < 2) throw Error(kErrInvalid, "sampleN must be at least 2");
   if (max_iter < 1) throw Error(kErrInvalid, "nPTiter must be at least 1");
   if (eps2L < 999) res.e_large = pt_deterministic(dets, n, c_dev, E0, eps2L, ints, hb, maxEntry, sp, present, 0, w,
-                                                  pr, s).e2;
+                                                  ps, pr, s).e2;
   double cumulative = 0.0;
   for (size_t i = 0; i < n; i++) cumulative += fabs(c_host[i]);
   std::vector<int> alias;
@@ -1131,6 +1139,8 @@ PtStochResult pt_semistochastic(const Det2* dets, size_t n, const double* c_dev,
     a.plist = dlist.p;
     a.pw = dw.p;
     a.n = (size_t)distinct;
+    split_parents(dets, dlist.p, c_dev, a.n, eps2, maxEntry, hb, ints.norb, ps, s);
+    a.split = ps.view();
     // generate (twice when the buffers turn out too small)
     int64_t room = std::max<int64_t>((int64_t)w.key0.cap, (int64_t)1 << 20), m = 0;
     for (int pass = 0; pass < 2; ++pass) {
@@ -1143,11 +1153,12 @@ PtStochResult pt_semistochastic(const Det2* dets, size_t n, const double* c_dev,
       a.key1 = w.key1.p;
       a.ne = w.ne.p;
       a.n2p = w.n2p.p;
-      SHCI_CUDA(cudaMemsetAsync(w.next.p, 0, 2 * sizeof(unsigned long long), s));
+      SHCI_CUDA(cudaMemsetAsync(w.next.p, 0, sizeof(unsigned long long), s));
+      ps.rewind(s);
       k_pt_gen<<<kPtGenBlocks, kPtThreads, gsmem, s>>>(a);
       SHCI_LAUNCH_CHECK();
       unsigned long long total = 0;
-      SHCI_CUDA(cudaMemcpyAsync(&total, w.next.p + 1, sizeof(total), cudaMemcpyDeviceToHost, s));
+      SHCI_CUDA(cudaMemcpyAsync(&total, w.next.p, sizeof(total), cudaMemcpyDeviceToHost, s));
       SHCI_CUDA(cudaStreamSynchronize(s));
       m = (int64_t)total;
       if (m <= room) break;

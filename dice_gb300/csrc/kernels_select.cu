@@ -1,4 +1,5 @@
-// Heat-bath selection of new determinants, one warp per parent determinant.
+// Heat-bath selection of new determinants, one warp per parent determinant or
+// slice of one (work units below).
 // Restates SHCIgetdeterminants::getDeterminantsVariationalApprox
 // (SHCI/SHCIgetdeterminants.cpp:586-739) as called from the parent loop of
 // DoVariational (SHCI/SHCIbasics.cpp:969-982) with threshold eps1/|cMax_i|:
@@ -10,9 +11,11 @@
 // (pair, entry) work is flattened across the 32 lanes.
 // Candidates already in the variational space are dropped by a hash lookup
 // (the reference's binary_search over SortedDets); sort + unique follow.
+#include <algorithm>
 #include <cmath>
 
 #include "ham.h"
+#include "host_io.h"
 
 namespace shci {
 
@@ -30,10 +33,66 @@ struct SelArgs {
   Det2* out;
   int64_t cap;
   int64_t* counter;
+  SplitView split;
 };
 
 constexpr int kSelThreads = 256;
 constexpr int kSelWarps = kSelThreads / 32;
+
+// ---- work units -------------------------------------------------------------
+// Thread per parent: entries above its threshold in the lists of its occupied
+// pairs, taken as the mean list of each kind (entries above the threshold over
+// all lists / lists), and one slice per kSplitEntries of them. 2048 entries
+// are 64 rounds of a warp, a few times what a slice's set-up costs.
+constexpr float kSplitEntries = 2048.0f;
+constexpr int kSplitMax = 64;
+__global__ void k_split_parents(const Det2* __restrict__ dets, const int32_t* __restrict__ plist,
+                                const double* __restrict__ c, size_t n, double eps, double maxEntry,
+                                const uint32_t* __restrict__ cum, int norb, uint2* __restrict__ extra, uint32_t cap,
+                                uint32_t* __restrict__ count, unsigned char* __restrict__ nsl) {
+  for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
+    const size_t p = plist ? (size_t)plist[i] : i;
+    const double e = fabs(eps / c[p]);
+    int ns = 1;
+    if (e < INFINITY && !(fabs(maxEntry) < e)) {
+      const Det2 d = dets[p];
+      const uint64_t ev = 0x5555555555555555ull;
+      const float na = (float)(__popcll(d.w0 & ev) + __popcll(d.w1 & ev));
+      const float nb = (float)(__popcll(d.w0 & ~ev) + __popcll(d.w1 & ~ev));
+      const unsigned bin = __float_as_uint(__double2float_rd(e)) >> 20;
+      const float lists = 0.5f * (float)norb * (float)(norb + 1);
+      const float est = ((float)cum[bin] * 0.5f * (na * (na - 1.0f) + nb * (nb - 1.0f)) +
+                         (float)cum[kHbBins + bin] * na * nb) / lists;
+      const int want = 1 + (int)fminf(est / kSplitEntries, (float)(kSplitMax - 1));
+      if (want > 1) {
+        const uint32_t base = atomicAdd(count, (uint32_t)(want - 1));
+        if (base + (uint32_t)(want - 1) <= cap) {
+          for (int k = 1; k < want; ++k) extra[base + k - 1] = make_uint2((uint32_t)i, (uint32_t)k);
+          ns = want;
+        }
+      }
+    }
+    nsl[i] = (unsigned char)ns;
+  }
+}
+void split_parents(const Det2* dets, const int32_t* plist, const double* c, size_t n, double eps, double maxEntry,
+                   const HeatBathView& hb, int norb, ParentSplit& ps, cudaStream_t s) {
+  // room for every parent of a small list to be cut fully; a large list has
+  // enough parents to fill the GPU however few of them are cut
+  const size_t cap = n <= 8192 ? n * kSplitMax : (size_t)8192 * kSplitMax;
+  ps.cap = (uint32_t)cap;
+  ps.extra.reserve(cap);
+  ps.nsl.reserve(n);
+  ps.count.reserve(1);
+  ps.next.reserve(1);
+  SHCI_CUDA(cudaMemsetAsync(ps.extra.p, 0xff, cap * sizeof(uint2), s));
+  SHCI_CUDA(cudaMemsetAsync(ps.count.p, 0, sizeof(uint32_t), s));
+  ps.rewind(s);
+  size_t blocks = std::max<size_t>(1, std::min<size_t>((n + 127) / 128, 152 * 16));
+  k_split_parents<<<(unsigned)blocks, 128, 0, s>>>(dets, plist, c, n, eps, maxEntry, hb.cum, norb, ps.extra.p, ps.cap,
+                                                   ps.count.p, ps.nsl.p);
+  SHCI_LAUNCH_CHECK();
+}
 
 // Warp-aggregated append of one candidate per lane with `emit` set.
 __device__ __forceinline__ void append(const SelArgs& a, bool emit, const Det2& cand) {
@@ -57,20 +116,29 @@ __global__ void __launch_bounds__(kSelThreads) k_select(SelArgs a) {
   unsigned char* closed = s_closed[wib];
   unsigned char* open = s_open[wib];
   const int n2 = 2 * a.ints.norb;
-  const int64_t warps = (int64_t)gridDim.x * kSelWarps;
+  const unsigned lt = (1u << lane) - 1u;
+  const uint32_t nextra = min(*a.split.count, a.split.cap);
   const SelectParams& sp = a.sp;
-  for (int64_t p = (int64_t)blockIdx.x * kSelWarps + wib; p < (int64_t)a.n; p += warps) {
+  uint32_t p;
+  int slice, slices;
+  while (next_unit(a.split, a.n, nextra, p, slice, slices)) {
+    if (p == 0xffffffffu) continue;
     const Det2 d = a.dets[p];
     const double eps = a.eps1 / fabs(a.cmax[p]);
     if (!(eps < INFINITY)) continue;  // |c| = 0: nothing passes any threshold
     __syncwarp();
-    if (lane == 0) {
+    {
       int nc = 0, no = 0;
-      for (int q = 0; q < n2; ++q) {
-        if (det_getocc(d, q))
-          closed[nc++] = (unsigned char)q;
-        else
-          open[no++] = (unsigned char)q;
+      for (int base = 0; base < n2; base += 32) {
+        const int q = base + lane;
+        const bool valid = q < n2, occ = valid && det_getocc(d, q);
+        const unsigned mo = __ballot_sync(kFull, occ), mv = __ballot_sync(kFull, valid && !occ);
+        if (occ)
+          closed[nc + __popc(mo & lt)] = (unsigned char)q;
+        else if (valid)
+          open[no + __popc(mv & lt)] = (unsigned char)q;
+        nc += __popc(mo);
+        no += __popc(mv);
       }
     }
     __syncwarp();
@@ -81,7 +149,7 @@ __global__ void __launch_bounds__(kSelThreads) k_select(SelArgs a) {
 
     // ---- singles
     const int ns = nclosed * nopen;
-    for (int base = 0; base < ns; base += 32) {
+    for (int base = 32 * slice; base < ns; base += 32 * slices) {
       const int q = base + lane;
       bool emit = false;
       Det2 cand = d;
@@ -111,8 +179,9 @@ __global__ void __launch_bounds__(kSelThreads) k_select(SelArgs a) {
     // for a float v, (double)|v| < eps exactly when |v| < eps rounded up to float
     const float eps_f = __double2float_ru(eps);
     const int npairs = nclosed * (nclosed - 1) / 2;
-    for (int pb = 0; pb < npairs; pb += 32) {
-      const int q = pb + lane;
+    // this slice's pairs: q = slice, slice + slices, ...
+    for (int pb = slice; pb < npairs; pb += 32 * slices) {
+      const int q = pb + lane * slices;
       int ci = 0, cj = 0;
       int64_t lstart = 0, len = 0;
       bool same = false;
@@ -435,11 +504,13 @@ int64_t count_present(const Det2* q, size_t n, const DetHash& present, const Det
 
 int64_t select_candidates(const Det2* dets, const double* cmax, size_t n, double eps1, const IntsView& ints,
                           const HeatBathView& hb, double maxEntry, const SelectParams& sp, const DetHash& present,
-                          Det2* out, int64_t cap, int64_t* d_counter, cudaStream_t s) {
+                          Det2* out, int64_t cap, int64_t* d_counter, ParentSplit& ps, cudaStream_t s) {
   SHCI_CUDA(cudaMemsetAsync(d_counter, 0, sizeof(int64_t), s));
-  SelArgs a{dets, cmax, n, eps1, ints, hb, maxEntry, sp, present.slots.p, present.mask, out, cap, d_counter};
-  size_t blocks = (n + kSelWarps - 1) / kSelWarps;
-  if (blocks > 152 * 16) blocks = 152 * 16;
+  split_parents(dets, nullptr, cmax, n, eps1, maxEntry, hb, ints.norb, ps, s);
+  SelArgs a{dets, cmax,   n,  eps1, ints,      hb, maxEntry, sp, present.slots.p, present.mask, out,
+            cap,  d_counter, ps.view()};
+  size_t blocks = n <= 8192 ? 8 * n : n / kSelWarps + 1;  // 64 slices a parent at most
+  if (blocks > 152 * 6) blocks = 152 * 6;
   if (blocks < 1) blocks = 1;
   k_select<<<(unsigned)blocks, kSelThreads, 0, s>>>(a);
   SHCI_LAUNCH_CHECK();
