@@ -6,11 +6,11 @@
 // iteration forms G = V^T W (one fused Gram pass), solves the small symmetric
 // eigenproblem on the host in FP64, forms Ritz vectors X = V Q, HX = W Q and
 // residuals R = HX - lambda X on the device, and appends preconditioned,
-// orthogonalised corrections. An iteration is two CUDA graphs, captured once
-// per basis size and active-root set and replayed after that: (1) Ritz
-// vectors, residuals and their norms; (2) corrections, orthonormalisation,
-// collapse, append, sigma and the next Gram matrix. The host reads back only
-// the small matrices (two synchronisations per iteration). The basis is only rotated on collapse; the
+// orthogonalised corrections. An iteration is (1) one launch: Ritz vectors and
+// residual norms; (2) one CUDA graph, captured once per basis size and
+// active-root set and replayed after that: corrections, orthonormalisation,
+// collapse, append, sigma and the next Gram column. The host reads only the
+// small matrices (two synchronisations per iteration). The basis is only rotated on collapse; the
 // subspace sequence is the reference's (same maxCopies, same collapse to the
 // lowest nroots+2 Ritz vectors, corrections orthogonalised against the whole
 // basis before the collapse). Block mode adds one correction per unconverged
@@ -217,7 +217,7 @@ struct Context {
   size_t ncand = 0;  // candidates of the last shci_select_candidates left in cand
 
   // Davidson workspace
-  DevBuf<double> V, W, Vt, Wt, X, Y, R, D, xb64, yb64, gpart, dG, dQ, dlam, dsmall, ftmp;
+  DevBuf<double> V, W, X, Y, R, D, xb64, yb64, gpart, dG, dQ, dlam, dsmall, ftmp;
   DevBuf<float> xb32;
 
   // alpha <-> beta flip map of the current space (-1 unknown, 0 not closed, 1 closed)
@@ -297,7 +297,8 @@ struct Context {
   double* pin = nullptr;  // pinned staging for the small matrices (kPin doubles)
   static constexpr int kPinQ = 0, kPinLam = 256, kPinAct = 272, kPinRR = 288, kPinG = 544, kPinNrm = 800,
                        kPin = 816;
-  DevBuf<double> dactlam, drr, dnrm;
+  DevBuf<double> dactlam, dnrm, davpart;
+  DevBuf<unsigned> davcount;
 
   void graphs_clear() {
     for (auto& kv : gcache) cudaGraphExecDestroy(kv.second.first);
@@ -875,8 +876,6 @@ struct Context {
     if (nroots > 16) throw Error(kErrInvalid, "at most 16 roots");
     V.reserve(N * mmax);
     W.reserve(N * mmax);
-    Vt.reserve(N * mmax);
-    Wt.reserve(N * mmax);
     X.reserve(N * nroots);
     Y.reserve(N * nroots);
     R.reserve(N * nroots);
@@ -944,10 +943,13 @@ struct Context {
     dQ.reserve(256);
     dlam.reserve(16);
     dactlam.reserve(16);
-    drr.reserve(256);
     dnrm.reserve(16);
     dsmall.reserve(16);
     gpart.reserve(256 * 304 + 2 * 304);
+    davpart.reserve(dav_scratch());
+    davcount.reserve(1);
+    SHCI_CUDA(cudaMemsetAsync(davcount.p, 0, sizeof(unsigned), stream));
+    const DavWork dw{davpart.p, davcount.p};
     if (mode == SHCI_MODE_MIXED) xb32.reserve(N * 4);
     if (mode == SHCI_MODE_FP64) xb64.reserve(N * 4);
     if (mode == SHCI_MODE_DIRECT) {
@@ -970,18 +972,9 @@ struct Context {
       sym_eig(m, hs, lam, Q);
       std::memcpy(pin + kPinQ, Q.data(), (size_t)m * m * sizeof(double));
       std::memcpy(pin + kPinLam, lam.data(), (size_t)nroots * sizeof(double));
-      // graph 1: Ritz vectors, residuals and the residual Gram matrix
-      launch_body(((uint64_t)1 << 60) | (uint64_t)m, [&]() {
-        SHCI_CUDA(cudaMemcpyAsync(dQ.p, pin + kPinQ, (size_t)m * m * sizeof(double), cudaMemcpyHostToDevice, stream));
-        SHCI_CUDA(cudaMemcpyAsync(dlam.p, pin + kPinLam, (size_t)nroots * sizeof(double), cudaMemcpyHostToDevice,
-                                  stream));
-        ts_gemm(V.p, N, m, dQ.p, nroots, N, 1.0, 0.0, X.p, N, stream);
-        ts_gemm(W.p, N, m, dQ.p, nroots, N, 1.0, 0.0, Y.p, N, stream);
-        residual(X.p, Y.p, dlam.p, nroots, N, N, R.p, stream);
-        ts_gram(R.p, N, nroots, R.p, N, nroots, N, drr.p, gpart, stream);
-        SHCI_CUDA(cudaMemcpyAsync(pin + kPinRR, drr.p, (size_t)nroots * nroots * sizeof(double),
-                                  cudaMemcpyDeviceToHost, stream));
-      });
+      // Ritz vectors, residuals and their norms: one launch
+      dav_ritz(V.p, W.p, N, m, pin + kPinQ, pin + kPinLam, nroots, N, X.p, Y.p, record_pairs ? R.p : nullptr, dw,
+               pin + kPinRR, stream);
       SHCI_CUDA(cudaStreamSynchronize(stream));
       if (trace_level() > 0) t_g1 += now_s() - t_loop0, t_loop0 = now_s();
       std::vector<double> rn(nroots);
@@ -1103,6 +1096,17 @@ struct Context {
       // graph 2: corrections, orthonormalisation, collapse, append, sigma, Gram
       sigma_deferred = use_graphs;
       launch_body(((uint64_t)2 << 60) | ((uint64_t)m << 40) | ((uint64_t)keep << 20) | amask, [&]() {
+        if (nact == 1) {
+          const size_t c = (size_t)act[0] * N;
+          dav_correction(V.p, N, m, X.p + c, Y.p + c, pin + kPinAct, diag.p, shiftp, sector != 0 ? flipidx.p : nullptr,
+                         flipsgn.p, (double)sector, N, D.p, dw, dG.p, dG.p + 16, dnrm.p, pin + kPinNrm, stream);
+          if (collapse) dav_collapse(V.p, W.p, N, m, pin + kPinQ, keep, N, stream);
+          dav_append(D.p, N, dnrm.p, V.p + (size_t)m1 * N, stream);
+          apply_sigma(mode, V.p, N, m1, 1, W.p, N, m1);
+          // only the new column of G = V^T W
+          dav_column(V.p, N, m1 + 1, W.p + (size_t)m1 * N, N, dw, pin + kPinG, stream);
+          return;
+        }
         SHCI_CUDA(cudaMemcpyAsync(dactlam.p, pin + kPinAct, (size_t)nact * sizeof(double), cudaMemcpyHostToDevice,
                                   stream));
         for (int a = 0; a < nact; ++a) {
@@ -1128,12 +1132,7 @@ struct Context {
         }
         SHCI_CUDA(cudaMemcpyAsync(pin + kPinNrm, dnrm.p, (size_t)nact * sizeof(double), cudaMemcpyDeviceToHost,
                                   stream));
-        if (collapse) {
-          ts_gemm(V.p, N, m, dQ.p, keep, N, 1.0, 0.0, Vt.p, N, stream);
-          ts_gemm(W.p, N, m, dQ.p, keep, N, 1.0, 0.0, Wt.p, N, stream);
-          SHCI_CUDA(cudaMemcpyAsync(V.p, Vt.p, (size_t)keep * N * sizeof(double), cudaMemcpyDeviceToDevice, stream));
-          SHCI_CUDA(cudaMemcpyAsync(W.p, Wt.p, (size_t)keep * N * sizeof(double), cudaMemcpyDeviceToDevice, stream));
-        }
+        if (collapse) dav_collapse(V.p, W.p, N, m, pin + kPinQ, keep, N, stream);
         SHCI_CUDA(cudaMemcpyAsync(V.p + (size_t)m1 * N, D.p, (size_t)nact * N * sizeof(double),
                                   cudaMemcpyDeviceToDevice, stream));
         apply_sigma(mode, V.p, N, m1, nact, W.p, N, m1);

@@ -370,6 +370,28 @@ void ts_gram(const double* A, size_t lda, int ma, const double* B, size_t ldb, i
 // Y = alpha * A Q + beta * Y, Q (m x k column-major, device).
 void ts_gemm(const double* A, size_t lda, int m, const double* Q, int k, size_t N, double alpha, double beta,
              double* Y, size_t ldy, cudaStream_t s);
+// Passes of the Davidson iteration (see kernels_sigma.cu). part: dav_scratch()
+// doubles, count: one zeroed word; Q, lam, rr, nrm_out and out may be pinned
+// host memory.
+struct DavWork {
+  double* part;
+  unsigned* count;
+};
+size_t dav_scratch();
+// X = V Q, Y = W Q, R = Y - X diag(lam) (R may be null), rr[c (nroots + 1)] = |R_c|^2.
+void dav_ritz(const double* V, const double* W, size_t ld, int m, const double* Q, const double* lam, int nroots,
+              size_t N, double* X, double* Y, double* R, const DavWork& w, double* rr, cudaStream_t s);
+// D = preconditioned residual of one root (shift and flip may be null; p: the
+// flip sector), made orthogonal to the m columns of V by two classical
+// Gram-Schmidt passes; *nrm and *nrm_out = |D|^2. g1, g2: m doubles each.
+void dav_correction(const double* V, size_t ld, int m, const double* X, const double* Y, const double* lam,
+                    const double* diag, const double* shift, const int32_t* flip, const int8_t* sign, double p,
+                    size_t N, double* D, const DavWork& w, double* g1, double* g2, double* nrm, double* nrm_out,
+                    cudaStream_t s);
+void dav_append(const double* c, size_t N, const double* g, double* out, cudaStream_t s);
+void dav_column(const double* V, size_t ld, int m, const double* w, size_t N, const DavWork& wk, double* out,
+                cudaStream_t s);
+void dav_collapse(double* V, double* W, size_t ld, int m, const double* Q, int keep, size_t N, cudaStream_t s);
 // c <- c / sqrt(g[0]) when sqrt(g[0]) > 1e-14 (g: device squared norm)
 void scale_inv_norm(double* c, size_t N, const double* g, cudaStream_t s);
 // R[:, c] = Y[:, c] - lam[c] X[:, c]

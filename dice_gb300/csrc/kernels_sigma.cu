@@ -789,13 +789,25 @@ __global__ void __launch_bounds__(256) k_gram_part(const double* __restrict__ A,
   }
 }
 
-__global__ void k_gram_sum(const double* __restrict__ part, int nblocks, int P, double* __restrict__ G) {
-  int t = threadIdx.x;
-  if (t < P) {
-    double s = 0.0;
-    for (int b = 0; b < nblocks; ++b) s += part[(size_t)b * P + t];
-    G[t] = s;
-  }
+// Sum of the blocks' partials of one value by one warp, lanes over the blocks
+// and a fixed tree: independent of scheduling, and the loads are in flight
+// together (one thread per value adding 304 partials in turn took 18 us).
+__device__ __forceinline__ double sum_partials(const double* part, int nblocks, int P, int p) {
+  const int lane = threadIdx.x & 31;
+  double s = 0.0;
+  for (int b = lane; b < nblocks; b += 32) s += __ldcg(part + (size_t)b * P + p);
+#pragma unroll
+  for (int o = 16; o; o >>= 1) s += __shfl_xor_sync(kFull, s, o);
+  return s;
+}
+// one warp per value, 8 per block: with two FP64 lanes per clock and SM, the
+// warps of one block would wait for one another
+__global__ void __launch_bounds__(256) k_gram_sum(const double* __restrict__ part, int nblocks, int P,
+                                                  double* __restrict__ G) {
+  const int p = blockIdx.x * 8 + (threadIdx.x >> 5);
+  if (p >= P) return;
+  const double s = sum_partials(part, nblocks, P, p);
+  if ((threadIdx.x & 31) == 0) G[p] = s;
 }
 
 void ts_gram(const double* A, size_t lda, int ma, const double* B, size_t ldb, int mb, size_t N, double* G,
@@ -810,7 +822,7 @@ void ts_gram(const double* A, size_t lda, int ma, const double* B, size_t ldb, i
   else
     k_gram_part<<<nb, 256, 0, s>>>(A, lda, ma, B, ldb, mb, N, part.p);
   SHCI_LAUNCH_CHECK();
-  k_gram_sum<<<1, 256, 0, s>>>(part.p, (int)nb, ma * mb, G);
+  k_gram_sum<<<(ma * mb + 7) / 8, 256, 0, s>>>(part.p, (int)nb, ma * mb, G);
   SHCI_LAUNCH_CHECK();
 }
 
@@ -907,6 +919,295 @@ __global__ void k_scale_inv_norm(double* __restrict__ c, size_t N, const double*
 }
 void scale_inv_norm(double* c, size_t N, const double* g, cudaStream_t s) {
   k_scale_inv_norm<<<grid_for(N, 256), 256, 0, s>>>(c, N, g);
+  SHCI_LAUNCH_CHECK();
+}
+
+// ---------------------------------------------------------------------------
+// The Davidson iteration's passes over the basis. The basis is small beside
+// the matrix, so what bounds them at ordinary sizes is the number of launches
+// and, in each, the FP64 pipe (two lanes per clock and SM: a warp-wide add
+// occupies it for 16 clocks), not memory. So every pass does all that one
+// reading of V and W allows, sums are reduced by exchanging halves (M - 1 + 5 -
+// log2 M adds per lane for M sums instead of 5 M), and the last block to
+// finish adds the blocks' partials, in block order, instead of a second launch.
+// 81,233 determinants, basis of at most 5: an iteration's vector work, 25
+// launches and 8 copies, took 180 us (gram sums 92, products 36, Gram parts 27);
+// now 7 launches.
+//
+// The small matrices are read from and written to pinned host memory (Q, the
+// eigenvalues, the norms, the new column of the Rayleigh matrix): a few hundred
+// bytes per pass, without copy nodes between the kernels.
+// ---------------------------------------------------------------------------
+// Sums over the grid of M values per thread; `part` holds gridDim.x * M
+// doubles, *count is 0 before and after. Value p goes to out[p * ostride] and,
+// if given, to dev[p] (p < n).
+template <int M>
+__device__ __forceinline__ void grid_sums(double (&v)[M], int n, double* __restrict__ part,
+                                          unsigned* __restrict__ count, double* out, int ostride, double* dev) {
+  __shared__ double s_w[32][M];
+  __shared__ bool s_last;
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  int idx = 0, o = 16;
+#pragma unroll
+  for (int half = M / 2; half >= 1; half >>= 1, o >>= 1) {
+    const bool up = (lane & o) != 0;
+#pragma unroll
+    for (int k = 0; k < half; ++k) {
+      const double keep = up ? v[k + half] : v[k], send = up ? v[k] : v[k + half];
+      v[k] = keep + __shfl_xor_sync(kFull, send, o);
+    }
+    idx += up ? half : 0;
+  }
+  for (int q = o; q; q >>= 1) v[0] += __shfl_xor_sync(kFull, v[0], q);
+  if ((lane & (2 * o - 1)) == 0) s_w[w][idx] = v[0];
+  __syncthreads();
+  if ((int)threadIdx.x < n) {
+    double s = 0.0;
+    for (int k = 0; k < nw; ++k) s += s_w[k][threadIdx.x];
+    __stcg(part + (size_t)blockIdx.x * n + threadIdx.x, s);
+    __threadfence();
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) s_last = atomicAdd(count, 1u) == gridDim.x - 1;
+  __syncthreads();
+  if (!s_last) return;
+  __threadfence();
+  for (int p = w; p < n; p += nw) {
+    const double s = sum_partials(part, (int)gridDim.x, n, p);
+    if (lane == 0) {
+      if (out) out[p * ostride] = s;
+      if (dev) dev[p] = s;
+    }
+  }
+  if (threadIdx.x == 0) *count = 0u;
+}
+
+constexpr int kDavThreads = 512;
+constexpr unsigned kDavBlocks = 152;
+static unsigned dav_blocks(size_t N) {
+  const size_t b = (N + kDavThreads - 1) / kDavThreads;
+  return (unsigned)(b < 1 ? 1 : (b > kDavBlocks ? kDavBlocks : b));
+}
+size_t dav_scratch() { return (size_t)kDavBlocks * kGramMax; }
+
+// X = V Q, Y = W Q, R = Y - X diag(lam) (written where asked for), |R_c|^2.
+template <int M, int NR>
+__global__ void __launch_bounds__(kDavThreads) k_ritz(const double* __restrict__ V, const double* __restrict__ W,
+                                                      size_t ld, int m, const double* Q, const double* lam, int nroots,
+                                                      size_t N, double* __restrict__ X, double* __restrict__ Y,
+                                                      double* __restrict__ R, double* __restrict__ part,
+                                                      unsigned* __restrict__ count, double* rr) {
+  __shared__ double sQ[kGramMax * kGramMax], sL[kGramMax];
+  for (int e = threadIdx.x; e < m * nroots; e += blockDim.x) sQ[e] = Q[e];
+  for (int e = threadIdx.x; e < nroots; e += blockDim.x) sL[e] = lam[e];
+  __syncthreads();
+  double acc[NR];
+#pragma unroll
+  for (int c = 0; c < NR; ++c) acc[c] = 0.0;
+  for (size_t r = (size_t)blockIdx.x * blockDim.x + threadIdx.x; r < N; r += (size_t)gridDim.x * blockDim.x) {
+    double v[M], w[M];
+#pragma unroll
+    for (int i = 0; i < M; ++i) {
+      v[i] = i < m ? V[(size_t)i * ld + r] : 0.0;
+      w[i] = i < m ? W[(size_t)i * ld + r] : 0.0;
+    }
+#pragma unroll
+    for (int c = 0; c < NR; ++c) {
+      if (c >= nroots) break;
+      double x = 0.0, y = 0.0;
+#pragma unroll
+      for (int i = 0; i < M; ++i)
+        if (i < m) {
+          x += v[i] * sQ[c * m + i];
+          y += w[i] * sQ[c * m + i];
+        }
+      const double t = y - sL[c] * x;
+      X[(size_t)c * ld + r] = x;
+      Y[(size_t)c * ld + r] = y;
+      if (R) R[(size_t)c * ld + r] = t;
+      acc[c] += t * t;
+    }
+  }
+  grid_sums<NR>(acc, nroots, part, count, rr, nroots + 1, nullptr);
+}
+void dav_ritz(const double* V, const double* W, size_t ld, int m, const double* Q, const double* lam, int nroots,
+              size_t N, double* X, double* Y, double* R, const DavWork& w, double* rr, cudaStream_t s) {
+  if (m > kGramMax || nroots > kGramMax) throw Error(kErrInvalid, "tall-skinny product too wide");
+  const unsigned nb = dav_blocks(N);
+#define SHCI_RITZ(M, NR) \
+  k_ritz<M, NR><<<nb, kDavThreads, 0, s>>>(V, W, ld, m, Q, lam, nroots, N, X, Y, R, w.part, w.count, rr)
+  if (m <= 8) {
+    if (nroots == 1) SHCI_RITZ(8, 1); else if (nroots <= 4) SHCI_RITZ(8, 4); else SHCI_RITZ(8, 16);
+  } else {
+    if (nroots == 1) SHCI_RITZ(16, 1); else if (nroots <= 4) SHCI_RITZ(16, 4); else SHCI_RITZ(16, 16);
+  }
+#undef SHCI_RITZ
+  SHCI_LAUNCH_CHECK();
+}
+
+// One preconditioned residual entry (k_residual, then k_precondition or
+// k_precondition_shift).
+__device__ __forceinline__ double corrected(const double* __restrict__ X, const double* __restrict__ Y, double lam,
+                                            const double* __restrict__ diag, const double* __restrict__ shift,
+                                            size_t r) {
+  const double t = Y[r] - lam * X[r];
+  double den = lam - diag[r];
+  if (shift) {
+    const double d2 = den - shift[r];
+    if ((d2 > 0) == (den > 0) && fabs(d2) > 0.2 * fabs(den)) den = d2;
+  }
+  return fabs(den) > 1e-12 ? t / den : t / (den - 1.e-12);
+}
+
+// D = the preconditioned residual of one root (projected into the flip sector
+// p when flip is given), G = V^T D.
+template <int M>
+__global__ void __launch_bounds__(kDavThreads) k_dav_correct(const double* __restrict__ V, size_t ld, int m,
+                                                             const double* __restrict__ X,
+                                                             const double* __restrict__ Y, const double* lam,
+                                                             const double* __restrict__ diag,
+                                                             const double* __restrict__ shift,
+                                                             const int32_t* __restrict__ flip,
+                                                             const int8_t* __restrict__ sign, double p, size_t N,
+                                                             double* __restrict__ D, double* __restrict__ part,
+                                                             unsigned* __restrict__ count, double* __restrict__ G) {
+  __shared__ double sl;
+  if (threadIdx.x == 0) sl = *lam;
+  __syncthreads();
+  const double l = sl;
+  double acc[M];
+#pragma unroll
+  for (int i = 0; i < M; ++i) acc[i] = 0.0;
+  for (size_t r = (size_t)blockIdx.x * blockDim.x + threadIdx.x; r < N; r += (size_t)gridDim.x * blockDim.x) {
+    double d = corrected(X, Y, l, diag, shift, r);
+    if (flip) d = 0.5 * (d + p * (double)sign[r] * corrected(X, Y, l, diag, shift, (size_t)flip[r]));
+    D[r] = d;
+#pragma unroll
+    for (int i = 0; i < M; ++i)
+      if (i < m) acc[i] += V[(size_t)i * ld + r] * d;
+  }
+  grid_sums<M>(acc, m, part, count, nullptr, 0, G);
+}
+// D -= V g, then G = V^T D (kNorm false) or |D|^2 (kNorm true).
+template <int M, bool kNorm>
+__global__ void __launch_bounds__(kDavThreads) k_dav_project(const double* __restrict__ V, size_t ld, int m,
+                                                             const double* __restrict__ g, size_t N,
+                                                             double* __restrict__ D, double* __restrict__ part,
+                                                             unsigned* __restrict__ count, double* __restrict__ G,
+                                                             double* out) {
+  __shared__ double sg[M];
+  if ((int)threadIdx.x < m) sg[threadIdx.x] = g[threadIdx.x];
+  __syncthreads();
+  double acc[kNorm ? 1 : M];
+#pragma unroll
+  for (int i = 0; i < (kNorm ? 1 : M); ++i) acc[i] = 0.0;
+  for (size_t r = (size_t)blockIdx.x * blockDim.x + threadIdx.x; r < N; r += (size_t)gridDim.x * blockDim.x) {
+    double v[M], t = 0.0;
+#pragma unroll
+    for (int i = 0; i < M; ++i) v[i] = i < m ? V[(size_t)i * ld + r] : 0.0;
+#pragma unroll
+    for (int i = 0; i < M; ++i)
+      if (i < m) t += v[i] * sg[i];
+    const double d = D[r] - t;
+    D[r] = d;
+    if constexpr (kNorm) {
+      acc[0] += d * d;
+    } else {
+#pragma unroll
+      for (int i = 0; i < M; ++i)
+        if (i < m) acc[i] += v[i] * d;
+    }
+  }
+  grid_sums<(kNorm ? 1 : M)>(acc, kNorm ? 1 : m, part, count, out, 1, G);
+}
+void dav_correction(const double* V, size_t ld, int m, const double* X, const double* Y, const double* lam,
+                    const double* diag, const double* shift, const int32_t* flip, const int8_t* sign, double p,
+                    size_t N, double* D, const DavWork& w, double* g1, double* g2, double* nrm, double* nrm_out,
+                    cudaStream_t s) {
+  if (m > kGramMax) throw Error(kErrInvalid, "Gram block too wide");
+  const unsigned nb = dav_blocks(N);
+#define SHCI_CORR(M)                                                                                                 \
+  k_dav_correct<M><<<nb, kDavThreads, 0, s>>>(V, ld, m, X, Y, lam, diag, shift, flip, sign, p, N, D, w.part, w.count, \
+                                              g1);                                                                   \
+  SHCI_LAUNCH_CHECK();                                                                                               \
+  k_dav_project<M, false><<<nb, kDavThreads, 0, s>>>(V, ld, m, g1, N, D, w.part, w.count, g2, nullptr);              \
+  SHCI_LAUNCH_CHECK();                                                                                               \
+  k_dav_project<M, true><<<nb, kDavThreads, 0, s>>>(V, ld, m, g2, N, D, w.part, w.count, nrm, nrm_out);              \
+  SHCI_LAUNCH_CHECK()
+  if (m <= 8) {
+    SHCI_CORR(8);
+  } else {
+    SHCI_CORR(16);
+  }
+#undef SHCI_CORR
+}
+
+// out = c / sqrt(g[0]) (unscaled when linearly dependent, for the host to drop)
+__global__ void k_append_unit(const double* __restrict__ c, size_t N, const double* __restrict__ g,
+                              double* __restrict__ out) {
+  const double nrm = sqrt(g[0]);
+  const double sc = nrm > 1e-14 ? 1.0 / nrm : 1.0;
+  for (size_t r = (size_t)blockIdx.x * blockDim.x + threadIdx.x; r < N; r += (size_t)gridDim.x * blockDim.x)
+    out[r] = c[r] * sc;
+}
+void dav_append(const double* c, size_t N, const double* g, double* out, cudaStream_t s) {
+  k_append_unit<<<grid_for(N, 256), 256, 0, s>>>(c, N, g, out);
+  SHCI_LAUNCH_CHECK();
+}
+
+// out[i] = V_i . w for the m columns of V (pinned host memory)
+template <int M>
+__global__ void __launch_bounds__(kDavThreads) k_dav_column(const double* __restrict__ V, size_t ld, int m,
+                                                            const double* __restrict__ w, size_t N,
+                                                            double* __restrict__ part, unsigned* __restrict__ count,
+                                                            double* out) {
+  double acc[M];
+#pragma unroll
+  for (int i = 0; i < M; ++i) acc[i] = 0.0;
+  for (size_t r = (size_t)blockIdx.x * blockDim.x + threadIdx.x; r < N; r += (size_t)gridDim.x * blockDim.x) {
+    const double x = w[r];
+#pragma unroll
+    for (int i = 0; i < M; ++i)
+      if (i < m) acc[i] += V[(size_t)i * ld + r] * x;
+  }
+  grid_sums<M>(acc, m, part, count, out, 1, nullptr);
+}
+void dav_column(const double* V, size_t ld, int m, const double* w, size_t N, const DavWork& wk, double* out,
+                cudaStream_t s) {
+  if (m > kGramMax) throw Error(kErrInvalid, "Gram block too wide");
+  const unsigned nb = dav_blocks(N);
+  if (m <= 8)
+    k_dav_column<8><<<nb, kDavThreads, 0, s>>>(V, ld, m, w, N, wk.part, wk.count, out);
+  else
+    k_dav_column<16><<<nb, kDavThreads, 0, s>>>(V, ld, m, w, N, wk.part, wk.count, out);
+  SHCI_LAUNCH_CHECK();
+}
+
+// V <- V Q, W <- W Q in place (m columns to keep <= m): every thread owns its
+// row, so no second copy of the basis is needed.
+__global__ void __launch_bounds__(256) k_dav_collapse(double* __restrict__ V, double* __restrict__ W, size_t ld, int m,
+                                                      const double* Q, int keep, size_t N) {
+  __shared__ double sQ[kGramMax * kGramMax];
+  for (int e = threadIdx.x; e < m * keep; e += blockDim.x) sQ[e] = Q[e];
+  __syncthreads();
+  for (size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x; t < 2 * N; t += (size_t)gridDim.x * blockDim.x) {
+    double* A = t < N ? V : W;
+    const size_t r = t < N ? t : t - N;
+    double a[kGramMax];
+#pragma unroll
+    for (int i = 0; i < kGramMax; ++i) a[i] = i < m ? A[(size_t)i * ld + r] : 0.0;
+    for (int c = 0; c < keep; ++c) {
+      double x = 0.0;
+#pragma unroll
+      for (int i = 0; i < kGramMax; ++i)
+        if (i < m) x += a[i] * sQ[c * m + i];
+      A[(size_t)c * ld + r] = x;
+    }
+  }
+}
+void dav_collapse(double* V, double* W, size_t ld, int m, const double* Q, int keep, size_t N, cudaStream_t s) {
+  if (m > kGramMax || keep > m) throw Error(kErrInvalid, "tall-skinny product too wide");
+  k_dav_collapse<<<grid_for(2 * N, 256), 256, 0, s>>>(V, W, ld, m, Q, keep, N);
   SHCI_LAUNCH_CHECK();
 }
 

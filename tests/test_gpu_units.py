@@ -1,0 +1,82 @@
+"""Work units of the selection and of the PT generator: parents cut into
+slices (one parent, a few heavy ones, heavy and light ones mixed, more slices
+than the unit list holds) give what the oracle, or the parents taken apart,
+give."""
+import numpy as np
+import pytest
+
+from dice_gb300 import engine as eng
+from dice_gb300 import synthetic
+from dice_gb300.shard import ref_order
+from oracle import oracle as orc
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def mol24(tmp_path_factory):
+    d = tmp_path_factory.mktemp("mol24")
+    synthetic.make_workload("mol24", str(d))
+    e = eng.Engine(0)
+    e.read_fcidump(str(d / "FCIDUMP"))
+    yield e, orc.Oracle(str(d / "FCIDUMP"))
+    e.close()
+
+
+def _spread(x):
+    return sum(((int(x) >> k) & 1) << (2 * k) for k in range(24))
+
+
+def _dets(n, seed, orbs=24):
+    """n distinct determinants of 12 alpha and 12 beta electrons in the lowest `orbs` orbitals."""
+    rng = np.random.default_rng(seed)
+    out = {}
+    while len(out) < n:
+        a, b = (sum(1 << int(o) for o in rng.choice(orbs, 12, replace=False)) for _ in range(2))
+        out[_spread(a) | (_spread(b) << 1)] = None
+    return np.array([(w, 0) for w in out], dtype=np.uint64)
+
+
+# the oracle's walk over the lists in Python-call-free C++ takes about a second for 40 heavy parents
+@pytest.mark.parametrize("n,light", [(1, 0), (2, 1), (33, 20), (40, 0)])
+def test_cut_parents_select_what_the_oracle_selects(mol24, n, light):
+    e, o = mol24
+    dets = _dets(n, 11 * n)
+    c = np.ones(n)
+    c[n - light:] = 1e-6  # below every threshold of the lists: whole parents
+    e.set_selection_params()
+    e.set_dets(dets)
+    got = e.select_candidates(c, 1e-5)
+    ref = o.select(dets, c, 1e-5, dets[ref_order(dets)])
+    assert len(got) == len(ref) > 1000 and np.array_equal(got, ref)
+
+
+@pytest.mark.parametrize("n,light", [(1, 0), (3, 1), (12, 0)])
+def test_cut_parents_give_the_oracles_pt(mol24, n, light):
+    e, o = mol24
+    dets = _dets(n, 5 + n)
+    c = np.full(n, 0.3)
+    c[n - light:] = 1e-5
+    e.set_selection_params()
+    e.set_dets(dets)
+    E0 = float(e.diag().min()) - 30.0
+    e2 = e.pt_deterministic(c, E0, 1e-5)
+    ref, st = o.pt_det(dets, c, E0, 1e-5)
+    got = e.pt_stats()
+    assert (got["candidates"], got["unique"]) == (st["outside"], st["unique"])
+    assert abs(e2 - ref) <= 1e-10 * abs(ref)
+
+
+def test_more_slices_than_the_list_holds(mol24):
+    """15,000 heavy parents claim more slices than the unit list has room for; each quarter of them alone
+    does not. The selected determinants are the union of the quarters'."""
+    e, _ = mol24
+    dets = _dets(15000, 3, orbs=15)
+    e.set_selection_params(0, 15)  # few candidates: the list entries are walked all the same
+    e.set_dets(dets)
+    c = np.ones(len(dets))
+    whole = e.select_candidates(c, 1e-7)
+    parts = [e.select_candidates(np.where(np.arange(len(dets)) % 4 == k, c, 0.0), 1e-7) for k in range(4)]
+    ref = np.unique(np.concatenate(parts), axis=0)
+    e.set_selection_params()
+    assert len(whole) == len(ref) and np.array_equal(np.unique(whole, axis=0), ref)
