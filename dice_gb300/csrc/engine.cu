@@ -217,7 +217,7 @@ struct Context {
   size_t ncand = 0;  // candidates of the last shci_select_candidates left in cand
 
   // Davidson workspace
-  DevBuf<double> V, W, X, Y, R, D, xb64, yb64, gpart, dG, dQ, dlam, dsmall, ftmp;
+  DevBuf<double> V, W, X, Y, R, D, xb64, gpart, dG, dQ, dlam, dsmall, ftmp;
   DevBuf<float> xb32;
 
   // alpha <-> beta flip map of the current space (-1 unknown, 0 not closed, 1 closed)
@@ -715,7 +715,7 @@ struct Context {
       // (selection only appends), so only new rows and columns are built
       const size_t n_old = (ham_mode == mode && !H.block) ? H.N : 0;
       H.drop_compressed();  // stale; rebuilt below (frees its memory before the build)
-      build_ham_csr(helpers, dets.p, ints(), H, mode == SHCI_MODE_FP64, mode == SHCI_MODE_MIXED,
+      build_ham_csr(helpers, ints(), H, mode == SHCI_MODE_FP64, mode == SHCI_MODE_MIXED,
                     mode == SHCI_MODE_MIXED, n_old, prims, stream);
       if (mode == SHCI_MODE_MIXED) compress_csr(H, prims, stream);
       pt.mark("ham compress");
@@ -740,7 +740,7 @@ struct Context {
     }
     ensure_diag();
     ham_ok = false;
-    build_ham_block(helpers, dets.p, ints(), H, mode == SHCI_MODE_FP64, mode == SHCI_MODE_MIXED,
+    build_ham_block(helpers, ints(), H, mode == SHCI_MODE_FP64, mode == SHCI_MODE_MIXED,
                     mode == SHCI_MODE_MIXED, r0, r1, prims, stream);
     if (mode == SHCI_MODE_MIXED) compress_csr(H, prims, stream);
     noalloc_ptr = noalloc_scratch_address();
@@ -780,16 +780,12 @@ struct Context {
         }
       } else if (mode == SHCI_MODE_DIRECT_MIXED) {  // FP32 matrix-free
         xb32.reserve(N * kp);
-        yb64.reserve(N * kp);
-        pack_f32(A, lda, c0 + done, kk, kp, N, xb32.p, stream);
-        sigma_direct32(helpers, dets.p, ints(), diag.p, xb32.p, yb64.p, kp, stream);
-        unpack_f64(yb64.p, kp, kk, N, Yp, ldy, yc0 + done, stream);
+        pack_f32(A, lda, c0 + done, kk, kp, N, xb32.p, stream, helpers.perm.p);
+        sigma_direct32(helpers, ints(), diag.p, xb32.p, kp, kk, Yp + (size_t)(yc0 + done) * ldy, ldy, stream);
       } else {
         xb64.reserve(N * kp);
-        yb64.reserve(N * kp);
-        pack_f64(A, lda, c0 + done, kk, kp, N, xb64.p, stream);
-        sigma_direct(helpers, dets.p, ints(), diag.p, xb64.p, yb64.p, kp, stream);
-        unpack_f64(yb64.p, kp, kk, N, Yp, ldy, yc0 + done, stream);
+        pack_f64(A, lda, c0 + done, kk, kp, N, xb64.p, stream, helpers.perm.p);
+        sigma_direct(helpers, ints(), diag.p, xb64.p, kp, kk, Yp + (size_t)(yc0 + done) * ldy, ldy, stream);
       }
       done += kk;
     }
@@ -950,16 +946,8 @@ struct Context {
     davcount.reserve(1);
     SHCI_CUDA(cudaMemsetAsync(davcount.p, 0, sizeof(unsigned), stream));
     const DavWork dw{davpart.p, davcount.p};
-    if (mode == SHCI_MODE_MIXED) xb32.reserve(N * 4);
-    if (mode == SHCI_MODE_FP64) xb64.reserve(N * 4);
-    if (mode == SHCI_MODE_DIRECT) {
-      xb64.reserve(N * 4);
-      yb64.reserve(N * 4);
-    }
-    if (mode == SHCI_MODE_DIRECT_MIXED) {
-      xb32.reserve(N * 4);
-      yb64.reserve(N * 4);
-    }
+    if (mode == SHCI_MODE_MIXED || mode == SHCI_MODE_DIRECT_MIXED) xb32.reserve(N * 4);
+    if (mode == SHCI_MODE_FP64 || mode == SHCI_MODE_DIRECT) xb64.reserve(N * 4);
     if (sym) ftmp.reserve(N);
     const double* shiftp = (shift_ready && shift.n >= N) ? shift.p : nullptr;
     std::vector<double> G = gram_host(V.p, N, m, W.p, N, m);

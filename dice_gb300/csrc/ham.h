@@ -4,28 +4,29 @@
 
 namespace shci {
 
-// Plain-pointer view passed to kernels.
+// Plain-pointer view passed to kernels. Everything is indexed by storage
+// position: the determinants sorted by (alpha string, beta string).
 struct HelperView {
   size_t N;
-  const uint64_t* astr;  // alpha string of each determinant
-  const uint64_t* bstr;  // beta string of each determinant
-  const uint32_t* aidx;  // determinant -> alpha group
-  const uint32_t* bidx;  // determinant -> beta group
-  const int64_t* aStart;  // alpha group g spans [aStart[g], aStart[g+1])
-  const uint32_t* aDets;  // determinant indices grouped by alpha string (AlphaMajorToDet)
-  const uint64_t* aGroupB;  // beta string of aDets[p] (AlphaMajorToBeta)
+  const ulonglong2* str;  // {alpha, beta} string of each position
+  const uint64_t* bstr;   // beta string of each position
+  const uint32_t* agrp;   // position -> alpha group
+  const uint32_t* bgrp;   // position -> beta group
+  const uint64_t* ua;     // alpha string of each alpha group, ascending
+  const int64_t* aStart;  // alpha group g is the positions [aStart[g], aStart[g+1])
   const int64_t* bStart;
-  const uint32_t* bDets;    // BetaMajorToDet
-  const uint64_t* bGroupA;  // BetaMajorToAlpha
-  const int64_t* aSingStart;  // SinglesFromAlpha as CSR over alpha groups
+  const uint32_t* bPos;    // positions grouped by beta string, ascending in each group
+  const uint64_t* bAlpha;  // alpha string of bPos[q]
+  const int64_t* aSingStart;  // single-excitation neighbours of each alpha group as CSR
   const uint32_t* aSing;
   // the list of alpha group g holds its small groups (a few times n_beta
-  // determinants at most) in [aSingStart[g], aSingMid[g]), then the large ones
+  // determinants at most) in [aSingStart[g], aSingMid[g]), then the large ones,
+  // each part ascending
   const int64_t* aSingMid;
   // partial-string index: one 16-byte entry per (determinant J, occupied
   // beta orbital b of J): {beta string of J without b (low, high word),
-  // alpha group of J | b << 26, J}, sorted by (alpha group, partial string),
-  // so that the entries of one key (alpha group, partial string) are a run
+  // alpha group of J | b << 26, position of J}, sorted by (alpha group, partial
+  // string), so that the entries of one key (alpha group, partial string) are a run
   const uint4* m1ent;
   // per alpha group g, an open-addressing table over the group's distinct
   // partial strings: m1dir[g] = first slot << 6 | log2(slots); a slot is
@@ -41,8 +42,10 @@ struct HelperView {
 struct Helpers {
   size_t N = 0;
   int64_t NA = 0, NB = 0, nsing = 0;
-  DevBuf<uint64_t> astr, bstr, ua, ub, aGroupB, bGroupA;
-  DevBuf<uint32_t> aidx, bidx, aDets, bDets, aSing;
+  DevBuf<uint32_t> perm, spos;  // storage position -> determinant index, and its inverse
+  DevBuf<ulonglong2> str;
+  DevBuf<uint64_t> bstr, ua, bAlpha;
+  DevBuf<uint32_t> agrp, bgrp, bPos, aSing;
   DevBuf<int64_t> aStart, bStart, aSingStart, aSingMid;
   DevBuf<uint4> m1ent;
   DevBuf<uint2> m1tab;
@@ -50,14 +53,14 @@ struct Helpers {
   int64_t nm1 = 0;
   void build(const Det2* dets, size_t n, int norb, Prims& pr, cudaStream_t s);
   HelperView view() const {
-    return HelperView{N,         astr.p,      bstr.p,  aidx.p,  bidx.p,  aStart.p, aDets.p,
-                      aGroupB.p, bStart.p,    bDets.p, bGroupA.p, aSingStart.p, aSing.p, aSingMid.p,
-                      nm1 > 0 ? m1ent.p : nullptr, m1tab.p, m1dir.p};
+    return HelperView{N,        str.p,   bstr.p,  agrp.p,       bgrp.p,  ua.p,       aStart.p, bStart.p,
+                      bPos.p,   bAlpha.p, aSingStart.p, aSing.p, aSingMid.p, nm1 > 0 ? m1ent.p : nullptr,
+                      m1tab.p,  m1dir.p};
   }
   size_t bytes() const {
-    return astr.bytes() + bstr.bytes() + ua.bytes() + ub.bytes() + aGroupB.bytes() + bGroupA.bytes() +
-           aidx.bytes() + bidx.bytes() + aDets.bytes() + bDets.bytes() + aSing.bytes() + aStart.bytes() +
-           bStart.bytes() + aSingStart.bytes() + aSingMid.bytes() + m1ent.bytes() + m1tab.bytes() + m1dir.bytes();
+    return perm.bytes() + spos.bytes() + str.bytes() + bstr.bytes() + ua.bytes() + bAlpha.bytes() + agrp.bytes() +
+           bgrp.bytes() + bPos.bytes() + aSing.bytes() + aStart.bytes() + bStart.bytes() + aSingStart.bytes() +
+           aSingMid.bytes() + m1ent.bytes() + m1tab.bytes() + m1dir.bytes();
   }
 };
 
@@ -133,17 +136,18 @@ void compress_csr(Csr& H, Prims& pr, cudaStream_t s);
 // determinants >= n_old and the new columns of the old rows are computed; the
 // old rows are relabelled to the new storage order (a monotone map, so they
 // stay sorted) and merged with their new columns. Otherwise all rows.
-void build_ham_csr(const Helpers& hp, const Det2* dets, const IntsView& ints, Csr& H, bool want64, bool want32,
+void build_ham_csr(const Helpers& hp, const IntsView& ints, Csr& H, bool want64, bool want32,
                    bool want_lo, size_t n_old, Prims& pr, cudaStream_t s);
 // Builds only the full rows of the determinants [r0, r1) (see Csr::block).
-void build_ham_block(const Helpers& hp, const Det2* dets, const IntsView& ints, Csr& H, bool want64, bool want32,
+void build_ham_block(const Helpers& hp, const IntsView& ints, Csr& H, bool want64, bool want32,
                      bool want_lo, size_t r0, size_t r1, Prims& pr, cudaStream_t s);
 void compute_diag(const Det2* dets, size_t n, const IntsView& ints, double* diag, cudaStream_t s);
-void sigma_direct(const Helpers& hp, const Det2* dets, const IntsView& ints, const double* diag, const double* x,
-                  double* y, int k, cudaStream_t s);
-// FP32 matrix-free sigma: x row-interleaved FP32 [N][k], y FP64 [N][k].
-void sigma_direct32(const Helpers& hp, const Det2* dets, const IntsView& ints, const double* diag, const float* x,
-                    double* y, int k, cudaStream_t s);
+// Matrix-free sigma of k = 1, 2 or 4 vectors: x row-interleaved [N][k] in storage
+// order (packed through hp.perm), FP64 or FP32; y column-major (first kw columns).
+void sigma_direct(const Helpers& hp, const IntsView& ints, const double* diag, const double* x, int k, int kw,
+                  double* y, size_t ldy, cudaStream_t s);
+void sigma_direct32(const Helpers& hp, const IntsView& ints, const double* diag, const float* x, int k, int kw,
+                    double* y, size_t ldy, cudaStream_t s);
 
 // ---- selection (kernels_select.cu) -----------------------------------------
 struct HeatBathView {
@@ -362,7 +366,6 @@ void pack_ff(const double* A, size_t lda, int c0, int k, int kp, size_t N, float
 // out row i = in row perm[i] of a row-interleaved array of `bytes_per_row`
 // (4, 8, 16 or 32) bytes per row.
 void gather_rows(const void* in, size_t bytes_per_row, const uint32_t* perm, size_t N, void* out, cudaStream_t s);
-void unpack_f64(const double* in, int kp, int k, size_t N, double* A, size_t lda, int c0, cudaStream_t s);
 // Tall-skinny products over column-major N x m blocks (deterministic order):
 // G (ma x mb, column-major) = A^T B.
 void ts_gram(const double* A, size_t lda, int ma, const double* B, size_t ldb, int mb, size_t N, double* G,

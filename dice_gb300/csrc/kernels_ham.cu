@@ -6,22 +6,25 @@
 //     (replaces MakeHfromSMHelpers2, SHCI/SHCImakeHamiltonian.cpp:486-715);
 //   * the matrix-free sigma (replaces HmultDirect::operator(), SHCI/Hmult.h:241-381).
 //
-// One warp owns one row I = (A, B). The connected determinants J are found in
-// three parts:
+// One warp enumerates the connections of one row I = (A, B), in four parts:
 //   1. determinants sharing I's alpha string: beta distance 1 or 2 (scan of
 //      the alpha group);
 //   2. determinants whose alpha string As is a single excitation of A and
-//      whose beta string equals B or is one excitation away. Every such J
-//      contains the partial string B - b for some occupied b of B, so it is
-//      found by looking up the keys (As, B - b) in the partial-string index
-//      (a hash table per alpha group As gives each key's run of entries):
-//      |B| probes per group As that return (nearly) only connections,
-//      instead of a scan over every determinant of the group -- except for
-//      groups of at most a few times |B| determinants, which are scanned;
+//      whose beta string equals B or is one excitation away:
+//      2a. groups As of at most a few times |B| determinants are scanned;
+//      2b. in the others every such J contains the partial string B - b for
+//          some occupied b of B, so it is found by looking up the keys
+//          (As, B - b) in the partial-string index (a hash table per alpha
+//          group As gives each key's run of entries): |B| probes per group
+//          that return (nearly) only connections;
 //   3. determinants sharing I's beta string: alpha distance 2 (scan of the
 //      beta group).
 // This visits the same (I, J) set as the reference's five helper-list classes
 // (single alpha, alpha-beta, single beta, double beta, double alpha).
+//
+// The tables are in storage order, the order of the matrix's rows and columns,
+// so a scan's hits are column indices in ascending order: each part is emitted
+// as one ascending run and a row is finished by merging four runs, not sorted.
 #include <algorithm>
 #include <type_traits>
 
@@ -40,18 +43,13 @@ static inline unsigned grid_for(size_t n, int threads, size_t max_blocks = 152 *
 // ---------------------------------------------------------------------------
 // Strings and groups
 // ---------------------------------------------------------------------------
-__global__ void k_strings(const Det2* __restrict__ dets, size_t n, uint64_t* __restrict__ astr,
-                          uint64_t* __restrict__ bstr, uint64_t* __restrict__ akey, uint64_t* __restrict__ bkey,
-                          uint32_t* __restrict__ ia, uint32_t* __restrict__ ib) {
+__global__ void k_strings(const Det2* __restrict__ dets, size_t n, uint64_t* __restrict__ a,
+                          uint64_t* __restrict__ b, uint32_t* __restrict__ idx) {
   for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
-    Det2 d = dets[i];
-    uint64_t a = det_alpha(d), b = det_beta(d);
-    astr[i] = a;
-    bstr[i] = b;
-    akey[i] = a;
-    bkey[i] = b;
-    ia[i] = (uint32_t)i;
-    ib[i] = (uint32_t)i;
+    const Det2 d = dets[i];
+    a[i] = det_alpha(d);
+    b[i] = det_beta(d);
+    idx[i] = (uint32_t)i;
   }
 }
 
@@ -60,22 +58,35 @@ __global__ void k_group_flags(const uint64_t* __restrict__ key, size_t n, int64_
     flag[i] = (i == 0 || key[i] != key[i - 1]) ? 1 : 0;
 }
 
-// seg(p) = inclusive count - 1; writes the unique string, group start, the
-// det -> group map and the partner string of every grouped determinant.
-__global__ void k_group_fill(const uint64_t* __restrict__ key, const uint32_t* __restrict__ perm, size_t n,
+// Groups of equal keys: excl + flag - 1 is an entry's group; writes the group's
+// start and key and the group of every position (entry p is position pos[p],
+// or p).
+__global__ void k_group_fill(const uint64_t* __restrict__ key, const uint32_t* __restrict__ pos, size_t n,
                              const int64_t* __restrict__ flag, const int64_t* __restrict__ excl,
-                             uint64_t* __restrict__ ustr, int64_t* __restrict__ start, uint32_t* __restrict__ idx,
-                             const uint64_t* __restrict__ partner, uint64_t* __restrict__ group_partner) {
+                             uint64_t* __restrict__ ukey, int64_t* __restrict__ start, uint32_t* __restrict__ grp) {
   for (size_t p = (size_t)blockIdx.x * blockDim.x + threadIdx.x; p < n; p += (size_t)gridDim.x * blockDim.x) {
-    int64_t seg = excl[p] + flag[p] - 1;
+    const int64_t seg = excl[p] + flag[p] - 1;
     if (flag[p]) {
-      ustr[seg] = key[p];
+      if (ukey) ukey[seg] = key[p];
       start[seg] = (int64_t)p;
     }
-    uint32_t d = perm[p];
-    idx[d] = (uint32_t)seg;
-    group_partner[p] = partner[d];
+    grp[pos ? pos[p] : (uint32_t)p] = (uint32_t)seg;
   }
+}
+__global__ void k_pair_strings(const uint64_t* __restrict__ a, const uint64_t* __restrict__ b,
+                               const uint32_t* __restrict__ perm, size_t n, ulonglong2* __restrict__ str,
+                               uint32_t* __restrict__ spos, uint64_t* __restrict__ bkey, uint32_t* __restrict__ bpos) {
+  for (size_t p = (size_t)blockIdx.x * blockDim.x + threadIdx.x; p < n; p += (size_t)gridDim.x * blockDim.x) {
+    str[p] = make_ulonglong2(a[p], b[p]);
+    spos[perm[p]] = (uint32_t)p;
+    bkey[p] = b[p];
+    bpos[p] = (uint32_t)p;
+  }
+}
+__global__ void k_gather_alpha(const ulonglong2* __restrict__ str, const uint32_t* __restrict__ pos, size_t n,
+                               uint64_t* __restrict__ out) {
+  for (size_t q = (size_t)blockIdx.x * blockDim.x + threadIdx.x; q < n; q += (size_t)gridDim.x * blockDim.x)
+    out[q] = str[pos[q]].x;
 }
 
 __device__ __forceinline__ int64_t bsearch_u64(const uint64_t* __restrict__ a, int64_t n, uint64_t x) {
@@ -132,29 +143,6 @@ __global__ void k_alpha_singles(const uint64_t* __restrict__ ua, int64_t na, int
 
 __global__ void k_iota_last(int64_t* start, int64_t n_groups, int64_t n_total) { start[n_groups] = n_total; }
 
-static void build_groups(const uint64_t* str_of_det, const uint64_t* partner_of_det, size_t n, DevBuf<uint64_t>& key,
-                         DevBuf<uint32_t>& perm, DevBuf<uint64_t>& ustr, DevBuf<int64_t>& start,
-                         DevBuf<uint32_t>& idx, DevBuf<uint64_t>& gpartner, int64_t& ngroups, Prims& pr,
-                         cudaStream_t s) {
-  sort_u64(key.p, perm.p, n, pr, s);
-  DevBuf<int64_t> flag, excl;
-  flag.resize(n);
-  excl.resize(n);
-  k_group_flags<<<grid_for(n, 256), 256, 0, s>>>(key.p, n, flag.p);
-  SHCI_LAUNCH_CHECK();
-  scan_exclusive_i64(flag.p, excl.p, n, &ngroups, pr, s);
-  ustr.resize(ngroups);
-  start.resize(ngroups + 1);
-  idx.resize(n);
-  gpartner.resize(n);
-  k_group_fill<<<grid_for(n, 256), 256, 0, s>>>(key.p, perm.p, n, flag.p, excl.p, ustr.p, start.p, idx.p,
-                                                 partner_of_det, gpartner.p);
-  SHCI_LAUNCH_CHECK();
-  k_iota_last<<<1, 1, 0, s>>>(start.p, ngroups, (int64_t)n);
-  SHCI_LAUNCH_CHECK();
-  (void)str_of_det;
-}
-
 // Partial-string index entries, sorted by (alpha group, partial beta string):
 // the entries of one key are one run and the runs of one alpha group are
 // contiguous, and so are the slots of the group's hash table, so the probes
@@ -165,12 +153,13 @@ __global__ void k_m1_count(const uint64_t* __restrict__ bstr, size_t n, int64_t*
   for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
     cnt[i] = __popcll(bstr[i]);
 }
-__global__ void k_m1_fill(const uint64_t* __restrict__ bstr, const uint32_t* __restrict__ aidx, size_t n,
+// (index entries refer to their determinant by storage position)
+__global__ void k_m1_fill(const uint64_t* __restrict__ bstr, const uint32_t* __restrict__ agrp, size_t n,
                           const int64_t* __restrict__ off, uint64_t* __restrict__ key, uint32_t* __restrict__ perm,
                           uint4* __restrict__ ent) {
   for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
     const uint64_t B = bstr[i];
-    const uint32_t g = aidx[i];
+    const uint32_t g = agrp[i];
     int64_t q = off[i];
     for (uint64_t r = B; r; r &= r - 1) {
       const int b = __ffsll((long long)r) - 1;
@@ -208,11 +197,25 @@ __device__ __forceinline__ uint32_t m1_fingerprint(uint64_t bm) {
   return (uint32_t)((bm * 0xc2b2ae3d27d4eb4full) >> 38);
 }
 constexpr uint32_t kM1Empty = 0xffffffffu;
+// The entries of one group are contiguous, and the largest group holds a tenth
+// of them: a warp's heads of one group are added at once (400,000 determinants:
+// 640 us with one atomic per head).
 __global__ void k_m1_heads(const uint4* __restrict__ ent, int64_t n, uint32_t* __restrict__ keys_of_group) {
   constexpr uint32_t gmask = (1u << kM1GroupBits) - 1u;
-  for (int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; k < n; k += (int64_t)gridDim.x * blockDim.x) {
-    const uint4 e = ent[k];
-    if (k == 0 || !m1_same_key(e, ent[k - 1])) atomicAdd(keys_of_group + (e.z & gmask), 1u);
+  const int lane = threadIdx.x & 31;
+  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+  for (int64_t base = (int64_t)blockIdx.x * blockDim.x + threadIdx.x - lane; base < n; base += stride) {
+    const int64_t k = base + lane;
+    bool head = false;
+    uint32_t g = 0xffffffffu;
+    if (k < n) {
+      const uint4 e = ent[k];
+      g = e.z & gmask;
+      head = k == 0 || !m1_same_key(e, ent[k - 1]);
+    }
+    const unsigned peers = __match_any_sync(kFull, g);
+    const unsigned heads = __ballot_sync(kFull, head);
+    if (k < n && lane == __ffs(peers) - 1 && (heads & peers)) atomicAdd(keys_of_group + g, (uint32_t)__popc(heads & peers));
   }
 }
 // slots of group g: the power of two >= 2 x its distinct keys, at least 2
@@ -266,38 +269,86 @@ __global__ void k_m1_insert(const uint4* __restrict__ ent, int64_t n, const uint
 #define SHCI_SCAN_FACTOR 4
 #endif
 constexpr int kScanFactor = SHCI_SCAN_FACTOR;
+// One warp per group; each part is put in ascending order by counting (a list
+// has at most n_alpha x (norb - n_alpha) entries, some hundred), so that the
+// hits of a row's scans come in ascending order too.
 __global__ void k_split_singles(const int64_t* __restrict__ sstart, const uint32_t* __restrict__ in,
-                                const int64_t* __restrict__ gstart, const uint64_t* __restrict__ gbeta, int64_t na,
+                                const int64_t* __restrict__ gstart, const uint64_t* __restrict__ bstr, int64_t na,
                                 uint32_t* __restrict__ out, int64_t* __restrict__ mid) {
-  for (int64_t g = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; g < na; g += (int64_t)gridDim.x * blockDim.x) {
+  const int lane = threadIdx.x & 31;
+  const int64_t warps = (int64_t)gridDim.x * (blockDim.x >> 5);
+  for (int64_t g = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; g < na; g += warps) {
     const int64_t s0 = sstart[g], s1 = sstart[g + 1];
-    const int64_t cap = (int64_t)kScanFactor * __popcll(gbeta[gstart[g]]);
-    int64_t w = s0;
-    for (int64_t q = s0; q < s1; ++q) {
-      const uint32_t As = in[q];
-      if (gstart[As + 1] - gstart[As] <= cap) out[w++] = As;
-    }
-    mid[g] = w;
-    for (int64_t q = s0; q < s1; ++q) {
-      const uint32_t As = in[q];
-      if (gstart[As + 1] - gstart[As] > cap) out[w++] = As;
+    const int64_t cap = (int64_t)kScanFactor * __popcll(bstr[gstart[g]]);
+    int64_t nsmall = 0;
+    for (int64_t q = s0 + lane; q < s1; q += 32) nsmall += gstart[in[q] + 1] - gstart[in[q]] <= cap;
+#pragma unroll
+    for (int o = 16; o; o >>= 1) nsmall += __shfl_xor_sync(kFull, nsmall, o);
+    if (lane == 0) mid[g] = s0 + nsmall;
+    for (int64_t q = s0; q < s1; q += 32) {
+      const bool mine = q + lane < s1;
+      const uint32_t me = mine ? in[q + lane] : 0u;
+      const bool small = mine && gstart[me + 1] - gstart[me] <= cap;
+      int rank = 0;
+      for (int64_t t = s0; t < s1; t += 32) {
+        const uint32_t other = t + lane < s1 ? in[t + lane] : 0u;
+        const bool osmall = t + lane < s1 && gstart[other + 1] - gstart[other] <= cap;
+        const unsigned sm = __ballot_sync(kFull, osmall);
+        const int cnt = (int)(s1 - t < 32 ? s1 - t : 32);
+        for (int k = 0; k < cnt; ++k) {
+          const uint32_t v = __shfl_sync(kFull, other, k);
+          rank += (v < me) && (((sm >> k) & 1u) != 0) == small;
+        }
+      }
+      if (mine) out[s0 + (small ? 0 : nsmall) + rank] = me;
     }
   }
 }
 
 void Helpers::build(const Det2* dets, size_t n, int norb, Prims& pr, cudaStream_t s) {
   N = n;
-  astr.resize(n);
+  perm.resize(n);
+  spos.resize(n);
+  str.resize(n);
   bstr.resize(n);
-  DevBuf<uint64_t> akey, bkey;
-  akey.resize(n);
-  bkey.resize(n);
-  aDets.resize(n);
-  bDets.resize(n);
-  k_strings<<<grid_for(n, 256), 256, 0, s>>>(dets, n, astr.p, bstr.p, akey.p, bkey.p, aDets.p, bDets.p);
-  SHCI_LAUNCH_CHECK();
-  build_groups(astr.p, bstr.p, n, akey, aDets, ua, aStart, aidx, aGroupB, NA, pr, s);
-  build_groups(bstr.p, astr.p, n, bkey, bDets, ub, bStart, bidx, bGroupA, NB, pr, s);
+  agrp.resize(n);
+  bgrp.resize(n);
+  bPos.resize(n);
+  bAlpha.resize(n);
+  {
+    DevBuf<uint64_t> a, bkey;
+    DevBuf<int64_t> flag, excl;
+    a.resize(n);
+    bkey.resize(n);
+    flag.resize(n);
+    excl.resize(n);
+    const unsigned g = grid_for(n, 256);
+    k_strings<<<g, 256, 0, s>>>(dets, n, a.p, bstr.p, perm.p);
+    SHCI_LAUNCH_CHECK();
+    sort_u128(bstr.p, a.p, perm.p, n, pr, s);  // by (alpha, beta): the storage order
+    k_pair_strings<<<g, 256, 0, s>>>(a.p, bstr.p, perm.p, n, str.p, spos.p, bkey.p, bPos.p);
+    SHCI_LAUNCH_CHECK();
+    k_group_flags<<<g, 256, 0, s>>>(a.p, n, flag.p);
+    SHCI_LAUNCH_CHECK();
+    scan_exclusive_i64(flag.p, excl.p, n, &NA, pr, s);
+    ua.resize((size_t)NA);
+    aStart.resize((size_t)NA + 1);
+    k_group_fill<<<g, 256, 0, s>>>(a.p, nullptr, n, flag.p, excl.p, ua.p, aStart.p, agrp.p);
+    SHCI_LAUNCH_CHECK();
+    k_iota_last<<<1, 1, 0, s>>>(aStart.p, NA, (int64_t)n);
+    SHCI_LAUNCH_CHECK();
+    sort_u64(bkey.p, bPos.p, n, pr, s);  // by beta string, stable: ascending positions within a group
+    k_group_flags<<<g, 256, 0, s>>>(bkey.p, n, flag.p);
+    SHCI_LAUNCH_CHECK();
+    scan_exclusive_i64(flag.p, excl.p, n, &NB, pr, s);
+    bStart.resize((size_t)NB + 1);
+    k_group_fill<<<g, 256, 0, s>>>(bkey.p, bPos.p, n, flag.p, excl.p, nullptr, bStart.p, bgrp.p);
+    SHCI_LAUNCH_CHECK();
+    k_iota_last<<<1, 1, 0, s>>>(bStart.p, NB, (int64_t)n);
+    SHCI_LAUNCH_CHECK();
+    k_gather_alpha<<<g, 256, 0, s>>>(str.p, bPos.p, n, bAlpha.p);
+    SHCI_LAUNCH_CHECK();
+  }
   // alpha single-excitation lists
   DevBuf<int64_t> cnt;
   cnt.resize(NA);
@@ -317,8 +368,8 @@ void Helpers::build(const Det2* dets, size_t n, int norb, Prims& pr, cudaStream_
     DevBuf<uint32_t> split;
     split.resize(total > 0 ? total : 1);
     aSingMid.resize(NA);
-    k_split_singles<<<grid_for((size_t)NA, 256), 256, 0, s>>>(aSingStart.p, aSing.p, aStart.p, aGroupB.p, NA, split.p,
-                                                              aSingMid.p);
+    k_split_singles<<<grid_for((size_t)NA * 32, 256), 256, 0, s>>>(aSingStart.p, aSing.p, aStart.p, bstr.p, NA,
+                                                                   split.p, aSingMid.p);
     SHCI_LAUNCH_CHECK();
     aSing.swap(split);
   }
@@ -343,7 +394,7 @@ void Helpers::build(const Det2* dets, size_t n, int norb, Prims& pr, cudaStream_
       raw.resize(ne);
       m1ent.resize(ne);
       const unsigned eb = grid_for((size_t)ne, 256);
-      k_m1_fill<<<grid_for(n, 256), 256, 0, s>>>(bstr.p, aidx.p, n, o1.p, key.p, perm.p, raw.p);
+      k_m1_fill<<<grid_for(n, 256), 256, 0, s>>>(bstr.p, agrp.p, n, o1.p, key.p, perm.p, raw.p);
       SHCI_LAUNCH_CHECK();
       sort_u64(key.p, perm.p, (size_t)ne, pr, s);  // by partial string
       k_m1_group_keys<<<eb, 256, 0, s>>>(raw.p, perm.p, ne, key.p);
@@ -377,336 +428,520 @@ void Helpers::build(const Det2* dets, size_t n, int norb, Prims& pr, cudaStream_
 }
 
 // ---------------------------------------------------------------------------
-// Row traversal shared by count, emit and the matrix-free sigma.
-// V::step(hit, J) is called by all 32 lanes together.
+// Row traversal shared by count, emit and the matrix-free sigma. The visitor's
+// v.step(hit, p, cls) is called by all 32 lanes together (p: storage position of
+// a connection), v.end_part(part) after each of the four parts.
 // ---------------------------------------------------------------------------
-template <class V>
-__device__ void visit_row(const HelperView& h, uint32_t I, V& v) {
-  const int lane = threadIdx.x & 31;
-  const uint64_t A = h.astr[I], B = h.bstr[I];
-  const uint32_t ia = h.aidx[I], ib = h.bidx[I];
-  // 1. same alpha string: beta single or double
-  {
-    const int64_t p0 = h.aStart[ia], p1 = h.aStart[ia + 1];
-    for (int64_t base = p0; base < p1; base += 32) {
-      int64_t p = base + lane;
-      bool hit = false;
-      uint32_t J = 0;
-      int d = -1;
-      if (p < p1) {
-        d = __popcll(h.aGroupB[p] ^ B);
-        hit = (d == 2 || d == 4);
-        J = h.aDets[p];
+enum : int { kSingleB = 0, kDoubleBB = 1, kAlpha = 2, kDoubleAA = 3 };  // class of a hit; kAlpha: alpha moved once
+
+// One lane's probe of the index: the run of entries of key (group As, bm).
+__device__ __forceinline__ void probe_index(const HelperView& h, uint32_t As, uint64_t bm, uint32_t& lo, int& len) {
+  const uint64_t d = __ldg(h.m1dir + As);
+  const unsigned lg = (unsigned)(d & 63);
+  const uint32_t mask = (uint32_t)((1ull << lg) - 1);
+  const uint2* tab = h.m1tab + (d >> 6);
+  const uint32_t fp = m1_fingerprint(bm);
+  uint32_t q = (uint32_t)m1_slot(bm, lg);
+  for (uint32_t step = 0; step <= mask; ++step) {
+    const uint2 sl = __ldg(tab + q);
+    if (sl.x == kM1Empty) return;
+    if ((sl.y & ((1u << kM1GroupBits) - 1u)) == fp) {
+      // a fingerprint match is confirmed on the run's first entry
+      const uint2 k0 = __ldg(reinterpret_cast<const uint2*>(h.m1ent + sl.x));
+      if (k0.x == (uint32_t)bm && k0.y == (uint32_t)(bm >> 32)) {
+        lo = sl.x;
+        len = (int)(sl.y >> kM1GroupBits) + 1;
+        return;
       }
-      v.step(hit, J, d == 2);
+    }
+    q = (q + 1) & mask;
+  }
+}
+
+// The k-th set bit of B (k < its population count).
+__device__ __forceinline__ int nth_bit(uint64_t B, int k) {
+  for (int t = 0; t < k; ++t) B &= B - 1;
+  return __ffsll((long long)B) - 1;
+}
+
+// Owner of flat entry f among the lanes' ranges (excl: first flat entry of each
+// lane): the last lane with excl <= f.
+__device__ __forceinline__ int flat_owner(int excl, int f) {
+  int lo = 0;
+#pragma unroll
+  for (int st = 16; st >= 1; st >>= 1) {
+    const int e = __shfl_sync(kFull, excl, lo + st);
+    if (e <= f) lo += st;
+  }
+  return lo;
+}
+__device__ __forceinline__ int warp_incl_sum(int v) {
+  const int lane = threadIdx.x & 31;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int y = __shfl_up_sync(kFull, v, o);
+    if (lane >= o) v += y;
+  }
+  return v;
+}
+
+// Parts 1, 2a and 3: the scans. Each reports its hits in ascending position.
+template <class V>
+__device__ __forceinline__ void scan_same_alpha(const HelperView& h, uint32_t ga, uint64_t B, V& v) {
+  const int lane = threadIdx.x & 31;
+  const uint32_t p1 = (uint32_t)h.aStart[ga + 1];
+  for (uint32_t base = (uint32_t)h.aStart[ga]; base < p1; base += 32) {
+    const uint32_t p = base + lane;
+    int d = -1;
+    if (p < p1) d = __popcll(h.bstr[p] ^ B);
+    v.step(d == 2 || d == 4, p, d == 2 ? kSingleB : kDoubleBB);
+  }
+}
+template <class V>
+__device__ __forceinline__ void scan_small_groups(const HelperView& h, int64_t s0, int64_t smid, uint64_t B, V& v) {
+  const int lane = threadIdx.x & 31;
+  for (int64_t base = s0; base < smid; base += 32) {
+    uint32_t g0 = 0;
+    int len = 0;
+    if (base + lane < smid) {
+      const uint32_t As = h.aSing[base + lane];
+      g0 = (uint32_t)h.aStart[As];
+      len = (int)((uint32_t)h.aStart[As + 1] - g0);
+    }
+    const int incl = warp_incl_sum(len);
+    const int total = __shfl_sync(kFull, incl, 31);
+    const int excl = incl - len;
+    const uint32_t off = g0 - (uint32_t)excl;  // position of flat entry f: off of its owner + f
+    for (int f0 = 0; f0 < total; f0 += 32) {
+      const int f = f0 + lane;
+      const uint32_t p = __shfl_sync(kFull, off, flat_owner(excl, f)) + (uint32_t)f;
+      bool hit = false;
+      if (f < total) hit = __popcll(h.bstr[p] ^ B) <= 2;
+      v.step(hit, p, kAlpha);
     }
   }
-  // 2. alpha single excitation: beta equal (single alpha) or beta single
-  // (alpha-beta double). I's list of groups A_s holds the small groups first
-  // (at most a few times |B| determinants: scanned, one popcount each), then
-  // the large ones (found from the partial-string index, |B| probes each).
-  {
-    const int64_t s0 = h.aSingStart[ia], s1 = h.aSingStart[ia + 1];
-    const bool indexed = h.m1ent != nullptr && B != 0;
-    const int64_t smid = indexed ? h.aSingMid[ia] : s1;
-    // the small groups (every group without the index)
-    for (int64_t base = s0; base < smid; base += 32) {
-      int64_t q = base + lane;
-      int64_t g0 = 0, len = 0;
-      if (q < smid) {
-        uint32_t As = h.aSing[q];
-        g0 = h.aStart[As];
-        len = h.aStart[As + 1] - g0;
-      }
-      int64_t incl = len;
-#pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        int64_t y = __shfl_up_sync(kFull, incl, o);
-        if (lane >= o) incl += y;
-      }
-      const int64_t total = __shfl_sync(kFull, incl, 31);
-      const int64_t excl = incl - len;
-      for (int64_t f0 = 0; f0 < total; f0 += 32) {
-        const int64_t f = f0 + lane;
-        int lo = 0;
-#pragma unroll
-        for (int st = 16; st >= 1; st >>= 1) {
-          int c = lo + st;
-          int64_t e = __shfl_sync(kFull, excl, c < 32 ? c : 31);
-          if (c < 32 && e <= f) lo = c;
-        }
-        int64_t gb = __shfl_sync(kFull, g0, lo);
-        int64_t eo = __shfl_sync(kFull, excl, lo);
-        bool hit = false;
-        uint32_t J = 0;
-        int d = -1;
-        if (f < total) {
-          int64_t p = gb + (f - eo);
-          d = __popcll(h.aGroupB[p] ^ B);
-          hit = (d == 0 || d == 2);
-          J = h.aDets[p];
-        }
-        v.step(hit, J, d == 0);
-      }
+}
+template <class V>
+__device__ __forceinline__ void scan_same_beta(const HelperView& h, uint32_t gb, uint64_t A, V& v) {
+  const int lane = threadIdx.x & 31;
+  const uint32_t q1 = (uint32_t)h.bStart[gb + 1];
+  for (uint32_t base = (uint32_t)h.bStart[gb]; base < q1; base += 32) {
+    const uint32_t q = base + lane;
+    bool hit = false;
+    uint32_t p = 0;
+    if (q < q1) {
+      hit = __popcll(h.bAlpha[q] ^ A) == 4;
+      p = h.bPos[q];
     }
-    if (indexed && smid < s1) {
-      const int nb = __popcll(B);
-      const int64_t nprobe = (s1 - smid) * nb;
-      // Probe t = (excitation sidx, occupied beta orbital `which`): each lane
-      // keeps its pair and steps it by 32 probes a round (no division per
-      // probe), and lane k holds the k-th occupied beta orbital of B for the
-      // others to read (B's orbitals beyond the 32nd, possible only past 32 beta
-      // electrons, are found bit by bit)
-      int occ_k = 0;
-      {
-        uint64_t r = B;
-        for (int k = 0; k < lane && r; ++k) r &= r - 1;
-        occ_k = r ? __ffsll((long long)r) - 1 : 0;
+    v.step(hit, p, kDoubleAA);
+  }
+}
+
+// Part 2b in no particular order: probes t = (group, occupied beta orbital)
+// 32 at a time, each lane stepping its own pair (no division per probe).
+template <class V>
+__device__ __forceinline__ void probe_large_groups(const HelperView& h, int64_t smid, int64_t s1, uint64_t B, V& v) {
+  const int lane = threadIdx.x & 31;
+  const int nb = __popcll(B);
+  const int nprobe = (int)(s1 - smid) * nb;
+  if (nprobe == 0) return;
+  const int occ_k = lane < nb ? nth_bit(B, lane) : 0;  // orbitals beyond the 32nd are found bit by bit
+  const int step_q = 32 / nb, step_r = 32 % nb;
+  int sidx = lane / nb, which = lane % nb;
+  for (int base = 0; base < nprobe; base += 32) {
+    uint32_t lo = 0;
+    int len = 0;  // at most 64: one entry per beta orbital outside the key
+    int bq = __shfl_sync(kFull, occ_k, which & 31);  // the beta orbital removed by this probe
+    if (which >= 32) bq = nth_bit(B, which);
+    const uint32_t tag = (uint32_t)bq | (which == 0 ? 256u : 0u);
+    if (base + lane < nprobe) probe_index(h, h.aSing[smid + sidx], B ^ (1ull << bq), lo, len);
+    which += step_r;
+    sidx += step_q;
+    if (which >= nb) {
+      which -= nb;
+      ++sidx;
+    }
+    // flatten the lanes' matches and verify them 32 at a time
+    const int incl = warp_incl_sum(len);
+    const int total = __shfl_sync(kFull, incl, 31);
+    const int excl = incl - len;
+    const uint32_t off = lo - (uint32_t)excl;
+    for (int f0 = 0; f0 < total; f0 += 32) {
+      const int f = f0 + lane;
+      const int src = flat_owner(excl, f);
+      const uint32_t e = __shfl_sync(kFull, off, src) + (uint32_t)f;
+      const uint32_t tg = __shfl_sync(kFull, tag, src);
+      bool hit = false;
+      uint32_t p = 0;
+      if (f < total) {
+        // the entry holds J and the orbital b' its beta string has beyond
+        // B - b: b' == b means beta equal (found once per occupied b, kept
+        // for the first), otherwise a beta single excitation b -> b'
+        const uint2 en = __ldg(reinterpret_cast<const uint2*>(h.m1ent + e) + 1);
+        p = en.y;
+        hit = (en.x >> kM1GroupBits) != (tg & 255u) || (tg & 256u);
       }
+      v.step(hit, p, kAlpha);
+    }
+  }
+}
+
+template <class V>
+__device__ __forceinline__ void visit_row(const HelperView& h, uint32_t p, uint64_t A, uint64_t B, V& v) {
+  const uint32_t ga = h.agrp[p];
+  scan_same_alpha(h, ga, B, v);
+  const int64_t s0 = h.aSingStart[ga], s1 = h.aSingStart[ga + 1];
+  const int64_t smid = (h.m1ent != nullptr && B != 0) ? h.aSingMid[ga] : s1;
+  scan_small_groups(h, s0, smid, B, v);
+  if (smid < s1) probe_large_groups(h, smid, s1, B, v);
+  scan_same_beta(h, h.bgrp[p], A, v);
+}
+
+struct CountVisitor {
+  int c = 0;
+  __device__ void step(bool hit, uint32_t, int) { c += hit; }
+};
+__device__ __forceinline__ int warp_total(int c) {
+#pragma unroll
+  for (int o = 16; o; o >>= 1) c += __shfl_xor_sync(kFull, c, o);
+  return c;
+}
+
+// Connections of row k (position rows[k], or k) by part, and their sum.
+// The index is only probed: a key's run holds the determinants one beta
+// excitation away, and J with B itself (in every run of its group, to be
+// counted once), which the run of the first probe shows.
+__global__ void __launch_bounds__(256) k_ham_count(HelperView h, const uint32_t* __restrict__ rows, int64_t nr,
+                                                   uint4* __restrict__ parts, int64_t* __restrict__ counts) {
+  const int lane = threadIdx.x & 31;
+  const int64_t warps = (int64_t)gridDim.x * (blockDim.x >> 5);
+  for (int64_t k = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; k < nr; k += warps) {
+    const uint32_t p = rows ? rows[k] : (uint32_t)k;
+    const ulonglong2 I = h.str[p];
+    const uint64_t A = I.x, B = I.y;
+    const uint32_t ga = h.agrp[p];
+    CountVisitor v1, v2, v3;
+    scan_same_alpha(h, ga, B, v1);
+    const int64_t s0 = h.aSingStart[ga], s1 = h.aSingStart[ga + 1];
+    const int64_t smid = (h.m1ent != nullptr && B != 0) ? h.aSingMid[ga] : s1;
+    scan_small_groups(h, s0, smid, B, v2);
+    int c4 = 0;
+    const int nb = __popcll(B);
+    const int nprobe = (int)(s1 - smid) * nb;
+    if (nprobe > 0) {
+      const int occ_k = lane < nb ? nth_bit(B, lane) : 0;
       const int step_q = 32 / nb, step_r = 32 % nb;
-      int64_t sidx = lane / nb;
-      int which = lane % nb;
-      for (int64_t base = 0; base < nprobe; base += 32) {
-        const int64_t t = base + lane;
-        // each lane locates the entries of its key (As, B - b)
-        uint32_t lo = 0;
-        int len = 0;  // at most 64: one entry per beta orbital outside the key
-        int bq = __shfl_sync(kFull, occ_k, which & 31);  // the beta orbital removed by this probe
-        if (which >= 32) {
-          uint64_t r = B;
-          for (int k = 0; k < which; ++k) r &= r - 1;
-          bq = __ffsll((long long)r) - 1;
+      int sidx = lane / nb, which = lane % nb;
+      for (int base = 0; base < nprobe; base += 32) {
+        int bq = __shfl_sync(kFull, occ_k, which & 31);
+        if (which >= 32) bq = nth_bit(B, which);
+        if (base + lane < nprobe) {
+          uint32_t lo = 0;
+          int len = 0;
+          probe_index(h, h.aSing[smid + sidx], B ^ (1ull << bq), lo, len);
+          c4 += len;
+          if (which == 0)
+            for (int e = 0; e < len; ++e)
+              if ((int)(__ldg(reinterpret_cast<const uint32_t*>(h.m1ent + lo + e) + 2) >> kM1GroupBits) == bq) {
+                c4 -= nb - 1;
+                break;
+              }
         }
-        const int64_t my_s = sidx;
-        const bool first_b = which == 0;
         which += step_r;
         sidx += step_q;
         if (which >= nb) {
           which -= nb;
           ++sidx;
         }
-        if (t < nprobe) {
-          const uint32_t As = h.aSing[smid + my_s];
-          const uint64_t Bm = B ^ (1ull << bq);
-          // the slot of Bm in group As's table gives the key's run of entries
-          // (a fingerprint match is confirmed on the run's first entry, the
-          // entry the flattening below reads first); an empty slot means no
-          // determinant of the space has the key
-          const uint64_t d = h.m1dir[As];
-          const unsigned lg = (unsigned)(d & 63);
-          const uint64_t mask = (1ull << lg) - 1;
-          const uint2* tab = h.m1tab + (d >> 6);
-          const uint32_t fp = m1_fingerprint(Bm);
-          uint64_t q = m1_slot(Bm, lg);
-          for (uint64_t step = 0; step <= mask; ++step) {
-            const uint2 sl = tab[q];
-            if (sl.x == kM1Empty) break;
-            if ((sl.y & ((1u << kM1GroupBits) - 1u)) == fp) {
-              const uint2 k0 = *reinterpret_cast<const uint2*>(h.m1ent + sl.x);
-              if (k0.x == (uint32_t)Bm && k0.y == (uint32_t)(Bm >> 32)) {
-                lo = sl.x;
-                len = (sl.y >> kM1GroupBits) + 1;
-                break;
-              }
-            }
-            q = (q + 1) & mask;
-          }
-        }
-        // flatten the lanes' matches and verify them 32 at a time
-        int incl = len;
-  #pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-          const int y = __shfl_up_sync(kFull, incl, o);
-          if (lane >= o) incl += y;
-        }
-        const int total = __shfl_sync(kFull, incl, 31);
-        const int excl = incl - len;
-        for (int f0 = 0; f0 < total; f0 += 32) {
-          const int f = f0 + lane;
-          int src = 0;
-  #pragma unroll
-          for (int st = 16; st >= 1; st >>= 1) {
-            const int c = src + st;
-            const int e = __shfl_sync(kFull, excl, c < 32 ? c : 31);
-            if (c < 32 && e <= f) src = c;
-          }
-          const uint32_t elo = __shfl_sync(kFull, lo, src);
-          const int eo = __shfl_sync(kFull, excl, src);
-          const int wb = __shfl_sync(kFull, bq, src);
-          const bool fb = __shfl_sync(kFull, first_b, src);
-          bool hit = false, single = false;
-          uint32_t J = 0;
-          if (f < total) {
-            // the entry holds J and the orbital b' its beta string has beyond
-            // B - b: b' == b means beta equal (found once per occupied b, kept
-            // for the first), otherwise a beta single excitation b -> b'
-            const uint4 en = h.m1ent[(size_t)elo + (uint32_t)(f - eo)];
-            J = en.w;
-            single = (int)(en.z >> kM1GroupBits) == wb;
-            hit = single ? fb : true;
-          }
-          v.step(hit, J, single);
-        }
       }
     }
-  }
-  // 3. same beta string: alpha double
-  {
-    const int64_t p0 = h.bStart[ib], p1 = h.bStart[ib + 1];
-    for (int64_t base = p0; base < p1; base += 32) {
-      int64_t p = base + lane;
-      bool hit = false;
-      uint32_t J = 0;
-      if (p < p1) {
-        int d = __popcll(h.bGroupA[p] ^ A);
-        hit = (d == 4);
-        J = h.bDets[p];
-      }
-      v.step(hit, J, false);
+    scan_same_beta(h, h.bgrp[p], A, v3);
+    const int n1 = warp_total(v1.c), n2 = warp_total(v2.c), n4 = warp_total(c4), n3 = warp_total(v3.c);
+    if (lane == 0) {
+      parts[k] = make_uint4((uint32_t)n1, (uint32_t)n2, (uint32_t)n4, (uint32_t)n3);
+      counts[k] = (int64_t)n1 + n2 + n4 + n3;
     }
   }
 }
 
-struct CountVisitor {
-  int64_t c = 0;
-  __device__ void step(bool hit, uint32_t, bool) { c += hit; }
-};
-
-// Rows [row0, row0 + nr); counts[slot(I)] = number of off-diagonal
-// connections, where slot(I) = slot[I] when a slot map is given (the storage
-// position of a full build, the local row of a row block), else I - row0.
-// order[k], k < nr: those rows in alpha-major order (rows of one
-// alpha string probe the same index sections; run together, they share them
-// in cache). Output positions stay indexed by the row.
-__global__ void k_ham_count(HelperView h, int64_t row0, int64_t nr, const uint32_t* __restrict__ order,
-                            const uint32_t* __restrict__ slot, int64_t* __restrict__ counts) {
+// Writes the columns of each row as four ascending runs (the parts in the order
+// of k_ham_count). The scans' hits come in ascending order. The index's do
+// not: the hits of 32 / |B| groups are collected in shared memory and ranked
+// by counting (some 25 per collection); groups that hold more hits than fit
+// are scanned instead. Bound by instruction issue and the L2 latency of the
+// probes; no element is evaluated here, so 8 blocks fit an SM.
+constexpr int kCollect = 256;
+__global__ void __launch_bounds__(256) k_ham_emit(HelperView h, const uint32_t* __restrict__ rows, int64_t nr,
+                                                  const int64_t* __restrict__ rowptr, int32_t* __restrict__ col) {
+  __shared__ __align__(16) uint32_t s_buf[8][kCollect];
   const int lane = threadIdx.x & 31;
+  const unsigned lt = (1u << lane) - 1u;
+  uint32_t* buf = s_buf[threadIdx.x >> 5];
   const int64_t warps = (int64_t)gridDim.x * (blockDim.x >> 5);
+  struct Append {
+    int32_t* col;
+    int64_t pos;
+    unsigned lt;
+    __device__ void step(bool hit, uint32_t p, int) {
+      const unsigned m = __ballot_sync(kFull, hit);
+      if (hit) col[pos + __popc(m & lt)] = (int32_t)p;
+      pos += __popc(m);
+    }
+  };
   for (int64_t k = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; k < nr; k += warps) {
-    const int64_t I = order[k];
-    CountVisitor v;
-    visit_row(h, (uint32_t)I, v);
-    int64_t c = v.c;
-#pragma unroll
-    for (int o = 16; o; o >>= 1) c += __shfl_xor_sync(kFull, c, o);
-    if (lane == 0) counts[slot ? (int64_t)slot[I] : I - row0] = c;
+    const uint32_t p = rows ? rows[k] : (uint32_t)k;
+    const ulonglong2 I = h.str[p];
+    const uint64_t A = I.x, B = I.y;
+    const uint32_t ga = h.agrp[p];
+    Append v{col, rowptr[k], lt};
+    scan_same_alpha(h, ga, B, v);
+    const int64_t s0 = h.aSingStart[ga], s1 = h.aSingStart[ga + 1];
+    const int64_t smid = (h.m1ent != nullptr && B != 0) ? h.aSingMid[ga] : s1;
+    scan_small_groups(h, s0, smid, B, v);
+    if (smid < s1) {
+      const int nb = __popcll(B);
+      const int per = nb <= 32 ? 32 / nb : 1;  // groups per collection
+      const int mine = nb <= 32 ? lane / nb : 0, which0 = nb <= 32 ? lane % nb : lane;
+      const int bq0 = which0 < nb ? nth_bit(B, which0) : 0;
+      for (int64_t s = smid; s < s1; s += per) {
+        int n = 0;
+        bool over = false;
+        for (int w = 0; w < nb; w += 32) {  // more than one round only past 32 beta electrons
+          const int which = which0 + w;
+          const int bq = w == 0 ? bq0 : (which < nb ? nth_bit(B, which) : 0);
+          uint32_t lo = 0;
+          int len = 0;
+          if (mine < per && which < nb && s + mine < s1) probe_index(h, h.aSing[s + mine], B ^ (1ull << bq), lo, len);
+          const uint32_t tag = (uint32_t)bq | (which == 0 ? 256u : 0u);
+          const int incl = warp_incl_sum(len);
+          const int total = __shfl_sync(kFull, incl, 31);
+          const int excl = incl - len;
+          const uint32_t off = lo - (uint32_t)excl;
+          for (int f0 = 0; f0 < total && !over; f0 += 32) {
+            const int f = f0 + lane;
+            const int src = flat_owner(excl, f);
+            const uint32_t e = __shfl_sync(kFull, off, src) + (uint32_t)f;
+            const uint32_t tg = __shfl_sync(kFull, tag, src);
+            bool hit = false;
+            uint32_t q = 0;
+            if (f < total) {
+              const uint2 en = __ldg(reinterpret_cast<const uint2*>(h.m1ent + e) + 1);
+              q = en.y;
+              hit = (en.x >> kM1GroupBits) != (tg & 255u) || (tg & 256u);
+            }
+            const unsigned m = __ballot_sync(kFull, hit);
+            over = n + __popc(m) > kCollect;
+            if (hit && !over) buf[n + __popc(m & lt)] = q;
+            if (!over) n += __popc(m);
+          }
+        }
+        if (over) {
+          __syncwarp();
+          scan_small_groups(h, s, s + per < s1 ? s + per : s1, B, v);
+          continue;
+        }
+        const int pad = (4 - (n & 3)) & 3;
+        if (lane < pad) buf[n + lane] = 0xffffffffu;
+        __syncwarp();
+        for (int t = 0; t < n; t += 32) {
+          const uint32_t key = t + lane < n ? buf[t + lane] : 0u;
+          int rank = 0;
+          for (int j = 0; j < n; j += 4) {
+            const uint4 o = *reinterpret_cast<const uint4*>(buf + j);
+            rank += (o.x < key) + (o.y < key) + (o.z < key) + (o.w < key);
+          }
+          if (t + lane < n) col[v.pos + rank] = (int32_t)key;
+        }
+        v.pos += n;
+        __syncwarp();
+      }
+    }
+    scan_same_beta(h, h.bgrp[p], A, v);
   }
 }
 
-// H_IJ with the higher-index determinant as the ket, the element the
-// reference stores in row max(I,J) (SHCI/SHCImakeHamiltonian.cpp:565-580).
-// Kept out of line, taking and returning plain values: the visitors' step()
-// is inlined at every scan site of visit_row, and the Slater-Condon code
-// copied into each caused instruction-cache misses, while an out-of-line
-// member taking the visitor by address kept the visitor's state (queue
-// counts, accumulators, output position) in local memory.
-__device__ __noinline__ double ham_element(const double* I1, const double* I2, const double* V1, int norb, Det2 dI,
-                                           Det2 dJ, bool j_below) {
-  const IntsView iv{I1, I2, nullptr, nullptr, norb, nullptr, nullptr, V1, nullptr};
-  return j_below ? hij_any(iv, dJ, dI) : hij_any(iv, dI, dJ);
-}
-__device__ __noinline__ float ham_element_f32(const float* I1f, const float* I2f, const float* V1f, int norb,
-                                              Det2 dI, Det2 dJ, bool j_below) {
-  const IntsView iv{nullptr, nullptr, nullptr, nullptr, norb, I1f, I2f, nullptr, V1f};
-  return j_below ? hij_any_f32(iv, dJ, dI) : hij_any_f32(iv, dI, dJ);
-}
-
-// Emits (col, value) for one row (elements from ham_element).
+// ---------------------------------------------------------------------------
+// Elements. The values are those of Hij_1Excite / Hij_2Excite
+// (SHCI/Determinants.cpp:406-505): the same integrals and differences, summed
+// in the same order, with the parity of the moves taken on the strings. Which
+// of the two determinants is the ket makes no difference: a double's integrals
+// are symmetric, and a single's sum differs only in where its zero terms
+// stand ((ai|ii) - (ai|ii) for the orbital left behind).
 //
-// Connections found by the scans are queued per warp in shared memory, one
-// queue for single and one for double excitations; whenever a queue holds 32
-// entries all lanes evaluate one Slater-Condon element each, so the FP64 work
-// runs on full warps and singles (an O(n_elec) sum) do not wait on doubles.
-struct EmitVisitor {
-  const Det2* dets;
-  const uint32_t* cmap;  // determinant index -> storage column
-  IntsView ints;
-  Det2 dI;
-  uint32_t I;
-  int64_t pos;
-  int32_t* col;
-  double* v64;
-  float* vhi;
-  float* vlo;
-  uint32_t* qs;  // 64 entries: single excitations
-  uint32_t* qd;  // 64 entries: double excitations
-  int ns, nd;
+// Moving an electron of string S between orbitals lo < hi passes the
+// electrons of S strictly between, and in the interleaved order (alpha of an
+// orbital before beta) the other string O's in [lo, hi) for an alpha electron
+// and in (lo, hi] for a beta one.
+// ---------------------------------------------------------------------------
+__device__ __forceinline__ uint64_t bits_from(int lo, int hi) { return (1ull << hi) - (1ull << lo); }  // [lo, hi)
+template <int kSpin>
+__device__ __forceinline__ uint64_t passed(uint64_t S, uint64_t O, int i, int a) {
+  const int lo = i < a ? i : a, hi = i < a ? a : i;
+  const uint64_t m = bits_from(lo, hi), open = m ^ (1ull << lo);
+  return (S & open) ^ (O & (kSpin ? open ^ (1ull << hi) : m));
+}
+__device__ __forceinline__ int low_bit(uint64_t x) { return __ffsll((long long)x) - 1; }
 
-  __device__ void store(int64_t q, uint32_t J) {
-    const double hv = ham_element(ints.I1, ints.I2, ints.V1, ints.norb, dI, dets[J], J < I);
-    col[q] = (int32_t)cmap[J];
-    if (v64) v64[q] = hv;
-    if (vhi) {
-      const float hi = (float)hv;
+// Integral access in either precision (FP64: __dsub_rn, so never contracted).
+template <bool F32>
+struct Elem;
+template <>
+struct Elem<false> {
+  using T = double;
+  __device__ static T i2(const IntsView& v, int i, int j, int k, int l) { return i2_spatial(v.I2, i, j, k, l); }
+  __device__ static T sub(T a, T b) { return __dsub_rn(a, b); }
+  __device__ static T signed_(T v, unsigned odd) {
+    return __longlong_as_double(__double_as_longlong(v) ^ ((long long)odd << 63));
+  }
+  __device__ static T single(const IntsView& v, const Det2& d, int a, int i) { return hij_single(v, d, a, i); }
+};
+template <>
+struct Elem<true> {
+  using T = float;
+  __device__ static T i2(const IntsView& v, int i, int j, int k, int l) { return i2f_spatial(v.I2f, i, j, k, l); }
+  __device__ static T sub(T a, T b) { return __fsub_rn(a, b); }
+  __device__ static T signed_(T v, unsigned odd) { return __uint_as_float(__float_as_uint(v) ^ (odd << 31)); }
+  __device__ static T single(const IntsView& v, const Det2& d, int a, int i) { return hij_single_f32(v, d, a, i); }
+};
+// alpha and beta moved once each
+template <bool F32>
+__device__ __forceinline__ typename Elem<F32>::T elem_ab(const IntsView& v, uint64_t A, uint64_t B, uint64_t A2,
+                                                         uint64_t B2) {
+  const uint64_t x = A ^ A2, y = B ^ B2;
+  const int i = low_bit(x & A), a = low_bit(x & A2), j = low_bit(y & B), b = low_bit(y & B2);
+  const unsigned odd = __popcll(passed<0>(A, B, i, a) ^ passed<1>(B, A2, j, b)) & 1;
+  return Elem<F32>::signed_(Elem<F32>::i2(v, a, i, b, j), odd);
+}
+// two electrons of one spin moved: S -> S2, the other string O
+template <bool F32, int kSpin>
+__device__ __forceinline__ typename Elem<F32>::T elem_same(const IntsView& v, uint64_t S, uint64_t O, uint64_t S2) {
+  const uint64_t x = S ^ S2, d = x & S, c = x & S2;
+  const int i = low_bit(d), j = low_bit(d & (d - 1)), a = low_bit(c), b = low_bit(c & (c - 1));
+  const uint64_t S1 = S ^ (1ull << i) ^ (1ull << a);
+  const unsigned odd = __popcll(passed<kSpin>(S, O, i, a) ^ passed<kSpin>(S1, O, j, b)) & 1;
+  return Elem<F32>::signed_(Elem<F32>::sub(Elem<F32>::i2(v, a, i, b, j), Elem<F32>::i2(v, a, j, b, i)), odd);
+}
+// one electron moved: S -> S2 of spin sp
+template <bool F32>
+__device__ __noinline__ typename Elem<F32>::T elem_single(const double* I1, const double* V1, const float* I1f,
+                                                          const float* V1f, int norb, uint64_t A, uint64_t B,
+                                                          uint64_t S, uint64_t S2, int sp) {
+  const IntsView v{I1, nullptr, nullptr, nullptr, norb, I1f, nullptr, V1, V1f};
+  const uint64_t x = S ^ S2;
+  return Elem<F32>::single(v, det_from_strings(A, B), 2 * low_bit(x & S2) + sp, 2 * low_bit(x & S) + sp);
+}
+
+// ---------------------------------------------------------------------------
+// Finishing the rows: the four ascending runs of a row are merged and the
+// elements evaluated, a thread per connection. An entry's place is its place
+// in its own run plus the entries of the other runs below it; run 1 (same
+// alpha string) is one range of positions that no other run enters, so only
+// the other two runs are searched. Evaluating here, and not where a connection
+// is found, keeps the walk's registers free of the element code and puts
+// every lane on an element. 405,690 rows, 5.5e8 entries (mol24, mixed, full and
+// new rows): emitting with evaluation 27.9 ms and sorting each row 30.7 ms.
+// ---------------------------------------------------------------------------
+constexpr int kRunCap = 3072;  // entries of a row kept in shared memory
+constexpr int kFinThreads = 128;
+
+__device__ __forceinline__ int run_below(const uint32_t* run, int n, uint32_t c) {  // entries of a run below c
+  int lo = 0, hi = n;
+  while (lo < hi) {
+    const int mid = (lo + hi) >> 1;
+    if (run[mid] < c)
+      lo = mid + 1;
+    else
+      hi = mid;
+  }
+  return lo;
+}
+
+__device__ __forceinline__ void finish_row(const HelperView& h, const IntsView& ints, uint32_t p, const uint4& n,
+                                           const uint32_t* run, int64_t p0, int32_t* __restrict__ col,
+                                           double* __restrict__ v64, float* __restrict__ vhi, float* __restrict__ vlo) {
+  const ulonglong2 I = h.str[p];
+  const uint64_t A = I.x, B = I.y;
+  const int n1 = (int)n.x, n2 = (int)n.y, n3 = (int)n.z, n4 = (int)n.w;
+  const uint32_t *r2 = run + n1, *r3 = r2 + n2, *r4 = r3 + n3;
+  const int len = n1 + n2 + n3 + n4;
+  for (int e = threadIdx.x; e < len; e += blockDim.x) {
+    const uint32_t c = run[e];
+    const ulonglong2 J = h.str[c];
+    int rank;
+    double v;
+    if (e < n1) {
+      rank = e + run_below(r2, n2, c) + run_below(r3, n3, c) + run_below(r4, n4, c);
+      v = __popcll(B ^ J.y) == 4 ? elem_same<false, 1>(ints, B, A, J.y)
+                                 : elem_single<false>(ints.I1, ints.V1, nullptr, nullptr, ints.norb, A, B, B, J.y, 1);
+    } else {
+      rank = n1 > 0 && c > run[0] ? n1 : 0;
+      if (e >= n1 + n2 + n3) {
+        rank += e - (n1 + n2 + n3) + run_below(r2, n2, c) + run_below(r3, n3, c);
+        v = elem_same<false, 0>(ints, A, B, J.x);
+      } else {
+        if (e >= n1 + n2)
+          rank += e - (n1 + n2) + run_below(r2, n2, c) + run_below(r4, n4, c);
+        else
+          rank += e - n1 + run_below(r3, n3, c) + run_below(r4, n4, c);
+        v = J.y == B ? elem_single<false>(ints.I1, ints.V1, nullptr, nullptr, ints.norb, A, B, A, J.x, 0)
+                     : elem_ab<false>(ints, A, B, J.x, J.y);
+      }
+    }
+    const int64_t q = p0 + rank;
+    col[q] = (int32_t)c;
+    if (v64) {
+      v64[q] = v;
+    } else {
+      const float hi = (float)v;
       vhi[q] = hi;
-      if (vlo) vlo[q] = (float)(hv - (double)hi);
+      if (vlo) vlo[q] = (float)(v - (double)hi);
     }
   }
-  // evaluate the first `cnt` (<= 32) entries of queue q, then shift the rest
-  // down
-  __device__ int drain(uint32_t* q, int n, int cnt) {
-    const int lane = threadIdx.x & 31;
-    if (lane < cnt) store(pos + lane, q[lane]);
-    pos += cnt;
-    __syncwarp();
-    const int rest = n - cnt;
-    uint32_t v = lane < rest ? q[cnt + lane] : 0u;
-    __syncwarp();
-    if (lane < rest) q[lane] = v;
-    __syncwarp();
-    return rest;
-  }
-  __device__ void step(bool hit, uint32_t J, bool single) {
-    const int lane = threadIdx.x & 31;
-    const unsigned lt = (1u << lane) - 1u;
-    const unsigned ms = __ballot_sync(kFull, hit && single);
-    const unsigned md = __ballot_sync(kFull, hit && !single);
-    if (hit && single) qs[ns + __popc(ms & lt)] = J;
-    if (hit && !single) qd[nd + __popc(md & lt)] = J;
-    ns += __popc(ms);
-    nd += __popc(md);
-    __syncwarp();
-    if (ns >= 32) ns = drain(qs, ns, 32);
-    if (nd >= 32) nd = drain(qd, nd, 32);
-  }
-  __device__ void flush() {
-    if (ns) ns = drain(qs, ns, ns);
-    if (nd) nd = drain(qd, nd, nd);
-  }
-};
+}
 
-// Rows [row0, row0 + nr) into a CSR whose row pointers are indexed by slot(I)
-// (see k_ham_count); columns are storage positions cmap[J].
-// Resident blocks per SM the emit and the matrix-free sigma are compiled for.
-// Both wait on the latency of index probes and gathers. The emit runs best
-// with 6 (at most 40 registers a thread, a few hundred bytes of spills: mol24
-// H build 0.98 s, 1.02 s with 4 blocks); the matrix-free sigma, whose
-// accumulators stay in registers, with 4 (64 registers, almost no spills:
-// mol36, 4 vectors, FP32 64 ms against 70 ms with 6).
-#ifndef SHCI_EMIT_MIN_BLOCKS
-#define SHCI_EMIT_MIN_BLOCKS 6
-#endif
-#ifndef SHCI_DIRECT_MIN_BLOCKS
-#define SHCI_DIRECT_MIN_BLOCKS 4
-#endif
-__global__ void __launch_bounds__(256, SHCI_EMIT_MIN_BLOCKS) k_ham_emit(HelperView h, int64_t row0, int64_t nr,
-                                                     const uint32_t* __restrict__ order,
-                                                     const uint32_t* __restrict__ slot,
-                                                     const uint32_t* __restrict__ cmap,
-                                                     const Det2* __restrict__ dets, IntsView ints,
-                                                     const int64_t* __restrict__ rowptr, int32_t* __restrict__ col,
-                                                     double* __restrict__ v64, float* __restrict__ vhi,
-                                                     float* __restrict__ vlo) {
-  __shared__ uint32_t s_q[8][2][64];
-  const int wib = threadIdx.x >> 5;
-  const int64_t warps = (int64_t)gridDim.x * (blockDim.x >> 5);
-  for (int64_t k = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; k < nr; k += warps) {
-    const int64_t I = order[k];
-    EmitVisitor v{dets, cmap, ints, dets[I], (uint32_t)I, rowptr[slot ? (int64_t)slot[I] : I - row0], col, v64, vhi,
-                  vlo, s_q[wib][0], s_q[wib][1], 0, 0};
-    visit_row(h, (uint32_t)I, v);
-    v.flush();
+__global__ void __launch_bounds__(kFinThreads) k_ham_finish(HelperView h, IntsView ints,
+                                                            const uint32_t* __restrict__ rows, int64_t nr,
+                                                            const uint4* __restrict__ parts,
+                                                            const int64_t* __restrict__ rowptr,
+                                                            int32_t* __restrict__ col, double* __restrict__ v64,
+                                                            float* __restrict__ vhi, float* __restrict__ vlo) {
+  __shared__ uint32_t run[kRunCap];
+  for (int64_t k = blockIdx.x; k < nr; k += gridDim.x) {
+    const int64_t p0 = rowptr[k];
+    const int len = (int)(rowptr[k + 1] - p0);
+    if (len == 0 || len > kRunCap) continue;  // uniform across the block
+    for (int e = threadIdx.x; e < len; e += blockDim.x) run[e] = (uint32_t)col[p0 + e];
+    __syncthreads();
+    finish_row(h, ints, rows ? rows[k] : (uint32_t)k, parts[k], run, p0, col, v64, vhi, vlo);
+    __syncthreads();
   }
+}
+
+// Rows past kRunCap: listed with their places in a scratch copy of their runs.
+__global__ void k_long_runs(const int64_t* __restrict__ rowptr, int64_t nr, uint2* __restrict__ list, uint32_t cap,
+                            unsigned long long* __restrict__ tot) {
+  for (int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; k < nr; k += (int64_t)gridDim.x * blockDim.x) {
+    const int64_t len = rowptr[k + 1] - rowptr[k];
+    if (len <= kRunCap) continue;
+    const unsigned long long i = atomicAdd(tot, 1ull);
+    const unsigned long long off = atomicAdd(tot + 1, (unsigned long long)((len + 31) / 32));
+    if (i < cap) list[i] = make_uint2((uint32_t)k, (uint32_t)off);
+  }
+}
+__global__ void __launch_bounds__(1024) k_ham_finish_long(HelperView h, IntsView ints,
+                                                          const uint32_t* __restrict__ rows,
+                                                          const uint2* __restrict__ list, uint32_t* scratch,
+                                                          const uint4* __restrict__ parts,
+                                                          const int64_t* __restrict__ rowptr,
+                                                          int32_t* __restrict__ col, double* __restrict__ v64,
+                                                          float* __restrict__ vhi, float* __restrict__ vlo) {
+  const uint2 l = list[blockIdx.x];
+  const int64_t p0 = rowptr[l.x];
+  const int len = (int)(rowptr[l.x + 1] - p0);
+  uint32_t* run = scratch + 32 * (size_t)l.y;
+  for (int e = threadIdx.x; e < len; e += blockDim.x) run[e] = (uint32_t)col[p0 + e];
+  __syncthreads();
+  finish_row(h, ints, rows ? rows[l.x] : l.x, parts[l.x], run, p0, col, v64, vhi, vlo);
 }
 
 __global__ void k_set_last(int64_t* rowptr, int64_t n, int64_t total) { rowptr[n] = total; }
@@ -957,39 +1192,20 @@ static void sort_rows(const int64_t* rowptr, size_t n, const CsrVals& v, cudaStr
   SHCI_CUDA(cudaStreamSynchronize(s));  // the scratch is freed on return
 }
 
-// Count, emit and sort the full rows [row0, N) into (rowptr, vals); returns nnz.
-__global__ void k_order_keys(const uint32_t* __restrict__ aidx, int64_t row0, int64_t nr, uint64_t* __restrict__ key,
-                             uint32_t* __restrict__ val) {
-  for (int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; k < nr; k += (int64_t)gridDim.x * blockDim.x) {
-    key[k] = aidx[row0 + k];
-    val[k] = (uint32_t)(row0 + k);
-  }
-}
-
-// Rows [row0, row1) of the determinant array. slot: storage position of each
-// row (full build), local row of a row block, or null (rows at I - row0);
-// cmap: determinant index -> storage column.
-static int64_t emit_rows(const Helpers& hp, size_t row0, size_t row1, const uint32_t* slot, const uint32_t* cmap,
-                         const Det2* dets, const IntsView& ints, DevBuf<int64_t>& rowptr, DevBuf<int32_t>& col,
-                         DevBuf<double>& v64, DevBuf<float>& vhi, DevBuf<float>& vlo, bool want64, bool want32,
-                         bool want_lo, Prims& pr, cudaStream_t s, PhaseTimer& pt) {
-  const size_t nr = row1 - row0;
+// Full rows of nr positions (rows[k], or all when null) into (rowptr, vals),
+// columns ascending; returns nnz.
+static int64_t emit_rows(const Helpers& hp, const uint32_t* rows, size_t nr, const IntsView& ints,
+                         DevBuf<int64_t>& rowptr, DevBuf<int32_t>& col, DevBuf<double>& v64, DevBuf<float>& vhi,
+                         DevBuf<float>& vlo, bool want64, bool want32, bool want_lo, Prims& pr, cudaStream_t s,
+                         PhaseTimer& pt) {
   HelperView hv = hp.view();
   DevBuf<int64_t> counts;
+  DevBuf<uint4> parts;
   counts.resize(nr > 0 ? nr : 1);
-  // the new rows in alpha-major order (stable: by row within an alpha string)
-  DevBuf<uint32_t> order;
-  order.resize(nr > 0 ? nr : 1);
-  if (nr) {
-    DevBuf<uint64_t> okey;
-    okey.resize(nr);
-    k_order_keys<<<grid_for(nr, 256), 256, 0, s>>>(hp.aidx.p, (int64_t)row0, (int64_t)nr, okey.p, order.p);
-    SHCI_LAUNCH_CHECK();
-    sort_u64(okey.p, order.p, nr, pr, s);
-  }
+  parts.resize(nr > 0 ? nr : 1);
   const unsigned blocks = grid_for(nr * 32, 256, 152 * 16);
   if (nr) {
-    k_ham_count<<<blocks, 256, 0, s>>>(hv, (int64_t)row0, (int64_t)nr, order.p, slot, counts.p);
+    k_ham_count<<<blocks, 256, 0, s>>>(hv, rows, (int64_t)nr, parts.p, counts.p);
     SHCI_LAUNCH_CHECK();
   }
   pt.mark("ham count");
@@ -1003,54 +1219,62 @@ static int64_t emit_rows(const Helpers& hp, size_t row0, size_t row1, const uint
   if (want64) v64.resize(cap); else v64.release();
   if (want32) vhi.resize(cap); else vhi.release();
   if (want32 && want_lo) vlo.resize(cap); else vlo.release();
-  CsrVals v{col.p, want64 ? v64.p : nullptr, want32 ? vhi.p : nullptr, (want32 && want_lo) ? vlo.p : nullptr};
-  if (nr) {
-    k_ham_emit<<<blocks, 256, 0, s>>>(hv, (int64_t)row0, (int64_t)nr, order.p, slot, cmap, dets, ints, rowptr.p,
-                                      v.col, v.v64,
-                                      v.vhi, v.vlo);
+  if (total == 0) return 0;
+  k_ham_emit<<<blocks, 256, 0, s>>>(hv, rows, (int64_t)nr, rowptr.p, col.p);
+  SHCI_LAUNCH_CHECK();
+  pt.mark("ham emit");
+  double* d64 = want64 ? v64.p : nullptr;
+  float* dhi = want32 ? vhi.p : nullptr;
+  float* dlo = want32 && want_lo ? vlo.p : nullptr;
+  // the long rows are listed first, and read from their untouched runs
+  const size_t ncap = (size_t)(total / kRunCap) + 1;
+  DevBuf<uint2> list;
+  DevBuf<unsigned long long> tot;
+  list.resize(ncap);
+  tot.resize(2);
+  SHCI_CUDA(cudaMemsetAsync(tot.p, 0, 2 * sizeof(unsigned long long), s));
+  k_long_runs<<<grid_for(nr, 256), 256, 0, s>>>(rowptr.p, (int64_t)nr, list.p, (uint32_t)ncap, tot.p);
+  SHCI_LAUNCH_CHECK();
+  k_ham_finish<<<(unsigned)std::min<size_t>(nr, 152 * 16), kFinThreads, 0, s>>>(hv, ints, rows, (int64_t)nr, parts.p,
+                                                                               rowptr.p, col.p, d64, dhi, dlo);
+  SHCI_LAUNCH_CHECK();
+  unsigned long long nl[2] = {0, 0};
+  SHCI_CUDA(cudaMemcpyAsync(nl, tot.p, sizeof(nl), cudaMemcpyDeviceToHost, s));
+  SHCI_CUDA(cudaStreamSynchronize(s));
+  if (nl[0] > 0) {
+    DevBuf<uint32_t> scratch;
+    scratch.resize(32 * (size_t)nl[1]);
+    k_ham_finish_long<<<(unsigned)nl[0], 1024, 0, s>>>(hv, ints, rows, list.p, scratch.p, parts.p, rowptr.p, col.p,
+                                                        d64, dhi, dlo);
     SHCI_LAUNCH_CHECK();
   }
-  pt.mark("ham emit");
-  // sort every row by column so that the 32 gathers of one warp instruction in
-  // sigma fall on fewer 32-byte sectors of x
-  sort_rows(rowptr.p, nr, v, s);
-  pt.mark("ham row sort");
+  pt.mark("ham finish");
   return total;
 }
 
-// Storage order: the determinants sorted by (alpha string, beta string);
-// perm[i] = determinant at storage position i, spos = its inverse.
-__global__ void k_storage_keys(const uint64_t* __restrict__ astr, const uint64_t* __restrict__ bstr, size_t n,
-                               uint64_t* __restrict__ k0, uint64_t* __restrict__ k1, uint32_t* __restrict__ v) {
+// Positions of the determinants [r0, r1), ascending: flags, and after their
+// scan the positions themselves (and their determinants).
+__global__ void k_range_flags(const uint32_t* __restrict__ perm, size_t n, uint32_t r0, uint32_t r1,
+                              int64_t* __restrict__ flag) {
   for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
-    k0[i] = bstr[i];
-    k1[i] = astr[i];
-    v[i] = (uint32_t)i;
+    const uint32_t d = perm[i];
+    flag[i] = (d >= r0 && d < r1) ? 1 : 0;
   }
 }
-__global__ void k_invert(const uint32_t* __restrict__ perm, size_t n, uint32_t* __restrict__ inv) {
-  for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
-    inv[perm[i]] = (uint32_t)i;
-}
-static void storage_order(const Helpers& hp, DevBuf<uint32_t>& perm, DevBuf<uint32_t>& spos, Prims& pr,
-                          cudaStream_t s) {
-  const size_t n = hp.N;
-  perm.resize(n > 0 ? n : 1);
-  spos.resize(n > 0 ? n : 1);
-  if (n == 0) return;
-  DevBuf<uint64_t> k0, k1;
-  k0.resize(n);
-  k1.resize(n);
-  k_storage_keys<<<grid_for(n, 256), 256, 0, s>>>(hp.astr.p, hp.bstr.p, n, k0.p, k1.p, perm.p);
-  SHCI_LAUNCH_CHECK();
-  sort_u128(k0.p, k1.p, perm.p, n, pr, s);
-  k_invert<<<grid_for(n, 256), 256, 0, s>>>(perm.p, n, spos.p);
-  SHCI_LAUNCH_CHECK();
-  SHCI_CUDA(cudaStreamSynchronize(s));  // k0, k1 are freed on return
+__global__ void k_range_fill(const uint32_t* __restrict__ perm, size_t n, uint32_t r0, uint32_t r1,
+                             const int64_t* __restrict__ pos, uint32_t* __restrict__ where,
+                             uint32_t* __restrict__ which) {
+  for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
+    const uint32_t d = perm[i];
+    if (d >= r0 && d < r1) {
+      where[pos[i]] = (uint32_t)i;
+      if (which) which[pos[i]] = d;
+    }
+  }
 }
 
 // Incremental build helpers. The rows of the new determinants R >= n_old are
-// emitted in full (row R at R - n_old, columns in the new storage order);
+// emitted in full (in storage order, columns in the new storage order);
 // their entries whose column is an old determinant C < n_old are the new
 // columns of old row C (same value: H_CR is evaluated with R, the higher
 // index, as the ket in both places).
@@ -1078,14 +1302,14 @@ __global__ void k_delta_count(const int64_t* __restrict__ rp_new, size_t nr, con
       if (is_old(old, c)) atomicAdd(&dcnt[c], 1ull);
     }
 }
-// The old row at storage position c receives column spos[n_old + r].
+// The old row at storage position c receives column rows[r].
 __global__ void k_delta_fill(const int64_t* __restrict__ rp_new, size_t nr, CsrVals nv,
-                             const uint32_t* __restrict__ old, const uint32_t* __restrict__ spos, int64_t n_old,
+                             const uint32_t* __restrict__ old, const uint32_t* __restrict__ rows,
                              const int64_t* __restrict__ dptr, unsigned long long* __restrict__ dfill, CsrVals dv) {
   const int lane = threadIdx.x & 31;
   const int64_t warps = (int64_t)gridDim.x * (blockDim.x >> 5);
   for (int64_t r = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; r < (int64_t)nr; r += warps) {
-    const int32_t me = (int32_t)spos[n_old + r];
+    const int32_t me = (int32_t)rows[r];
     for (int64_t p = rp_new[r] + lane; p < rp_new[r + 1]; p += 32) {
       const uint32_t c = (uint32_t)nv.col[p];
       if (!is_old(old, c)) continue;
@@ -1106,14 +1330,15 @@ __global__ void k_relabel(const uint32_t* __restrict__ perm_old, const uint32_t*
 }
 __global__ void k_merged_len(const uint32_t* __restrict__ perm, const uint32_t* __restrict__ spos_old,
                              const int64_t* __restrict__ rp_old, const int64_t* __restrict__ dptr, int64_t n_old,
-                             const int64_t* __restrict__ rp_new, int64_t N, int64_t* __restrict__ len) {
+                             const int64_t* __restrict__ rp_new, const int64_t* __restrict__ slot, int64_t N,
+                             int64_t* __restrict__ len) {
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < N; i += (int64_t)gridDim.x * blockDim.x) {
     const int64_t u = perm[i];
     if (u < n_old) {
       const int64_t o = spos_old[u];
       len[i] = (rp_old[o + 1] - rp_old[o]) + (dptr[i + 1] - dptr[i]);
     } else {
-      len[i] = rp_new[u - n_old + 1] - rp_new[u - n_old];
+      len[i] = rp_new[slot[i] + 1] - rp_new[slot[i]];
     }
   }
 }
@@ -1165,8 +1390,8 @@ __global__ void __launch_bounds__(256) k_merge_rows(const uint32_t* __restrict__
                                                     const int64_t* __restrict__ rp_old, CsrVals ov,
                                                     const uint32_t* __restrict__ rel,
                                                     const int64_t* __restrict__ dptr, CsrVals dv,
-                                                    const int64_t* __restrict__ rp_new, CsrVals nv, int64_t n_old,
-                                                    int64_t N, const int64_t* __restrict__ rp, CsrVals out) {
+                                                    const int64_t* __restrict__ rp_new, CsrVals nv,
+                                                    const int64_t* __restrict__ slot, int64_t n_old, int64_t N, const int64_t* __restrict__ rp, CsrVals out) {
   const int lane = threadIdx.x & 31;
   const int64_t warps = (int64_t)gridDim.x * (blockDim.x >> 5);
   int32_t* __restrict__ ocol = out.col;
@@ -1178,7 +1403,7 @@ __global__ void __launch_bounds__(256) k_merge_rows(const uint32_t* __restrict__
     const int64_t d = rp[i];
     const int64_t u = perm[i];
     if (u >= n_old) {  // a new row: copied
-      const int64_t a0 = rp_new[u - n_old], la = rp_new[u - n_old + 1] - a0;
+      const int64_t a0 = rp_new[slot[i]], la = rp_new[slot[i] + 1] - a0;
       for (int64_t t = lane; t < la; t += 32) {
         MergeVal<VK> v;
         v.load(nv.v64, nv.vhi, nv.vlo, a0 + t);
@@ -1226,8 +1451,8 @@ __global__ void __launch_bounds__(256) k_merge_rows(const uint32_t* __restrict__
   }
 }
 
-void build_ham_csr(const Helpers& hp, const Det2* dets, const IntsView& ints, Csr& H, bool want64, bool want32,
-                   bool want_lo, size_t n_old, Prims& pr, cudaStream_t s) {
+void build_ham_csr(const Helpers& hp, const IntsView& ints, Csr& H, bool want64, bool want32, bool want_lo,
+                   size_t n_old, Prims& pr, cudaStream_t s) {
   const size_t N = hp.N;
   PhaseTimer pt(s);
   const bool incremental = !H.block && n_old > 0 && n_old < N && H.N == n_old && H.perm.n >= n_old &&
@@ -1237,21 +1462,33 @@ void build_ham_csr(const Helpers& hp, const Det2* dets, const IntsView& ints, Cs
   if (!incremental) {
     if (n_old == N && H.N == N && !H.block) return;  // nothing new
     H.clear_block();
-    storage_order(hp, H.perm, H.spos, pr, s);
-    pt.mark("ham storage order");
-    H.nnz = emit_rows(hp, 0, N, H.spos.p, H.spos.p, dets, ints, H.rowptr, H.col, H.v64, H.vhi, H.vlo, want64, want32,
-                      want_lo, pr, s, pt);
+    H.perm.resize(N > 0 ? N : 1);
+    H.spos.resize(N > 0 ? N : 1);
+    if (N) {
+      SHCI_CUDA(cudaMemcpyAsync(H.perm.p, hp.perm.p, N * sizeof(uint32_t), cudaMemcpyDeviceToDevice, s));
+      SHCI_CUDA(cudaMemcpyAsync(H.spos.p, hp.spos.p, N * sizeof(uint32_t), cudaMemcpyDeviceToDevice, s));
+    }
+    H.nnz = emit_rows(hp, nullptr, N, ints, H.rowptr, H.col, H.v64, H.vhi, H.vlo, want64, want32, want_lo, pr, s, pt);
     H.N = N;
     SHCI_CUDA(cudaStreamSynchronize(s));
     return;
   }
   const size_t nr = N - n_old;
-  DevBuf<uint32_t> perm, spos;
-  storage_order(hp, perm, spos, pr, s);
-  pt.mark("ham storage order");
-  Csr Hn;  // rows of the determinants n_old .. N-1
-  Hn.nnz = emit_rows(hp, n_old, N, nullptr, spos.p, dets, ints, Hn.rowptr, Hn.col, Hn.v64, Hn.vhi, Hn.vlo, want64,
-                     want32, want_lo, pr, s, pt);
+  const DevBuf<uint32_t>&perm = hp.perm, &spos = hp.spos;
+  // the new determinants' storage positions, ascending, and each one's row among them
+  DevBuf<int64_t> flag, slot;
+  DevBuf<uint32_t> rows;
+  flag.resize(N);
+  slot.resize(N);
+  rows.resize(nr);
+  k_range_flags<<<grid_for(N, 256), 256, 0, s>>>(perm.p, N, (uint32_t)n_old, (uint32_t)N, flag.p);
+  SHCI_LAUNCH_CHECK();
+  scan_exclusive_i64(flag.p, slot.p, N, nullptr, pr, s);
+  k_range_fill<<<grid_for(N, 256), 256, 0, s>>>(perm.p, N, (uint32_t)n_old, (uint32_t)N, slot.p, rows.p, nullptr);
+  SHCI_LAUNCH_CHECK();
+  Csr Hn;  // rows of the determinants n_old .. N-1, in storage order
+  Hn.nnz = emit_rows(hp, rows.p, nr, ints, Hn.rowptr, Hn.col, Hn.v64, Hn.vhi, Hn.vlo, want64, want32, want_lo, pr, s,
+                     pt);
   CsrVals nv{Hn.col.p, Hn.v64.p, Hn.vhi.p, Hn.vlo.p};
   // new columns of the old rows, indexed by the old row's new storage position
   DevBuf<uint32_t> oldbits;
@@ -1279,7 +1516,7 @@ void build_ham_csr(const Helpers& hp, const Det2* dets, const IntsView& ints, Cs
   if (want32) Hd.vhi.resize(dcap);
   if (want32 && want_lo) Hd.vlo.resize(dcap);
   CsrVals dv{Hd.col.p, Hd.v64.p, Hd.vhi.p, Hd.vlo.p};
-  k_delta_fill<<<wblocks, 256, 0, s>>>(Hn.rowptr.p, nr, nv, oldbits.p, spos.p, (int64_t)n_old, dptr.p, dfill.p, dv);
+  k_delta_fill<<<wblocks, 256, 0, s>>>(Hn.rowptr.p, nr, nv, oldbits.p, rows.p, dptr.p, dfill.p, dv);
   SHCI_LAUNCH_CHECK();
   sort_rows(dptr.p, N, dv, s);
   pt.mark("ham new columns");
@@ -1292,7 +1529,7 @@ void build_ham_csr(const Helpers& hp, const Det2* dets, const IntsView& ints, Cs
   len.resize(N);
   rp.resize(N + 1);
   k_merged_len<<<grid_for(N, 256), 256, 0, s>>>(perm.p, H.spos.p, H.rowptr.p, dptr.p, (int64_t)n_old, Hn.rowptr.p,
-                                                (int64_t)N, len.p);
+                                                slot.p, (int64_t)N, len.p);
   SHCI_LAUNCH_CHECK();
   int64_t total = 0;
   scan_exclusive_i64(len.p, rp.p, N, &total, pr, s);
@@ -1307,11 +1544,11 @@ void build_ham_csr(const Helpers& hp, const Det2* dets, const IntsView& ints, Cs
   CsrVals ov{H.col.p, H.v64.p, H.vhi.p, H.vlo.p}, mv{M.col.p, M.v64.p, M.vhi.p, M.vlo.p};
   if (want64)
     k_merge_rows<0><<<grid_for(N * 32, 256, 152 * 16), 256, 0, s>>>(perm.p, H.spos.p, H.rowptr.p, ov, rel.p,
-                                                                    dptr.p, dv, Hn.rowptr.p, nv, (int64_t)n_old,
+                                                                    dptr.p, dv, Hn.rowptr.p, nv, slot.p, (int64_t)n_old,
                                                                     (int64_t)N, rp.p, mv);
   else
     k_merge_rows<1><<<grid_for(N * 32, 256, 152 * 16), 256, 0, s>>>(perm.p, H.spos.p, H.rowptr.p, ov, rel.p,
-                                                                    dptr.p, dv, Hn.rowptr.p, nv, (int64_t)n_old,
+                                                                    dptr.p, dv, Hn.rowptr.p, nv, slot.p, (int64_t)n_old,
                                                                     (int64_t)N, rp.p, mv);
   SHCI_LAUNCH_CHECK();
   SHCI_CUDA(cudaStreamSynchronize(s));
@@ -1320,8 +1557,10 @@ void build_ham_csr(const Helpers& hp, const Det2* dets, const IntsView& ints, Cs
   H.v64.swap(M.v64);
   H.vhi.swap(M.vhi);
   H.vlo.swap(M.vlo);
-  H.perm.swap(perm);
-  H.spos.swap(spos);
+  H.perm.resize(N);
+  H.spos.resize(N);
+  SHCI_CUDA(cudaMemcpyAsync(H.perm.p, perm.p, N * sizeof(uint32_t), cudaMemcpyDeviceToDevice, s));
+  SHCI_CUDA(cudaMemcpyAsync(H.spos.p, spos.p, N * sizeof(uint32_t), cudaMemcpyDeviceToDevice, s));
   H.N = N;
   H.nnz = total;
   pt.mark("ham merge");
@@ -1337,58 +1576,33 @@ void build_ham_csr(const Helpers& hp, const Det2* dets, const IntsView& ints, Cs
 // are storage positions of the whole space. A row's entries and their order
 // are those of the same row in the whole matrix.
 // ---------------------------------------------------------------------------
-__global__ void k_block_flags(const uint32_t* __restrict__ perm, size_t n, uint32_t r0, uint32_t r1,
-                              int64_t* __restrict__ flag) {
-  for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
-    const uint32_t d = perm[i];
-    flag[i] = (d >= r0 && d < r1) ? 1 : 0;
-  }
-}
-__global__ void k_block_fill(const uint32_t* __restrict__ perm, size_t n, uint32_t r0, uint32_t r1,
-                             const int64_t* __restrict__ pos, uint32_t* __restrict__ rows, uint32_t* __restrict__ xpos,
-                             uint32_t* __restrict__ slot) {
-  for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
-    const uint32_t d = perm[i];
-    if (d >= r0 && d < r1) {
-      const int64_t q = pos[i];
-      rows[q] = d;
-      xpos[q] = (uint32_t)i;
-      slot[d] = (uint32_t)q;
-    }
-  }
-}
-
-void build_ham_block(const Helpers& hp, const Det2* dets, const IntsView& ints, Csr& H, bool want64, bool want32,
-                     bool want_lo, size_t r0, size_t r1, Prims& pr, cudaStream_t s) {
+void build_ham_block(const Helpers& hp, const IntsView& ints, Csr& H, bool want64, bool want32, bool want_lo,
+                     size_t r0, size_t r1, Prims& pr, cudaStream_t s) {
   const size_t N = hp.N;
   if (!(r0 < r1 && r1 <= N)) throw Error(kErrInvalid, "row block [r0, r1) must be a non-empty range of the space");
   const size_t nb = r1 - r0;
   PhaseTimer pt(s);
-  DevBuf<uint32_t> perm, spos;
-  storage_order(hp, perm, spos, pr, s);
   DevBuf<int64_t> flag, pos;
   flag.resize(N);
   pos.resize(N);
-  k_block_flags<<<grid_for(N, 256), 256, 0, s>>>(perm.p, N, (uint32_t)r0, (uint32_t)r1, flag.p);
+  k_range_flags<<<grid_for(N, 256), 256, 0, s>>>(hp.perm.p, N, (uint32_t)r0, (uint32_t)r1, flag.p);
   SHCI_LAUNCH_CHECK();
   int64_t nflag = 0;
   scan_exclusive_i64(flag.p, pos.p, N, &nflag, pr, s);
   if ((size_t)nflag != nb) throw Error(kErrState, "row block: storage order lost determinants");
-  DevBuf<uint32_t> rows, xpos, slot;
+  DevBuf<uint32_t> rows, xpos;
   rows.resize(nb);
   xpos.resize(nb);
-  slot.resize(N);
-  k_block_fill<<<grid_for(N, 256), 256, 0, s>>>(perm.p, N, (uint32_t)r0, (uint32_t)r1, pos.p, rows.p, xpos.p,
-                                                slot.p);
+  k_range_fill<<<grid_for(N, 256), 256, 0, s>>>(hp.perm.p, N, (uint32_t)r0, (uint32_t)r1, pos.p, xpos.p, rows.p);
   SHCI_LAUNCH_CHECK();
   pt.mark("ham block order");
   H.drop_compressed();
-  H.nnz = emit_rows(hp, r0, r1, slot.p, spos.p, dets, ints, H.rowptr, H.col, H.v64, H.vhi, H.vlo, want64, want32,
-                    want_lo, pr, s, pt);
+  H.nnz = emit_rows(hp, xpos.p, nb, ints, H.rowptr, H.col, H.v64, H.vhi, H.vlo, want64, want32, want_lo, pr, s, pt);
+  H.xperm.resize(N);
+  SHCI_CUDA(cudaMemcpyAsync(H.xperm.p, hp.perm.p, N * sizeof(uint32_t), cudaMemcpyDeviceToDevice, s));
   SHCI_CUDA(cudaStreamSynchronize(s));
   H.perm.swap(rows);
   H.xpos.swap(xpos);
-  H.xperm.swap(perm);
   H.spos.release();
   H.N = nb;
   H.nfull = N;
@@ -1422,152 +1636,186 @@ void compute_diag(const Det2* dets, size_t n, const IntsView& ints, double* diag
 }
 
 // ---------------------------------------------------------------------------
-// Matrix-free sigma: y[I] = diag[I] x[I] + sum_J H_IJ x[J] with H_IJ
-// recomputed for every connection. X and Y are row-interleaved [N][K].
+// Matrix-free sigma (HmultDirect, SHCI/Hmult.h:241-381): y[I] = diag[I] x[I] +
+// sum_J H_IJ x[J], row I's connections found by visit_row and H_IJ recomputed.
+// Hits wait per warp in three queues (singles, alpha-beta doubles, doubles of
+// one spin) and are evaluated 32 at a time, so a full warp runs one element
+// formula on strings it already holds. x is in storage order: the hits of a
+// scan are neighbours there. FP64: the reference's arithmetic. FP32 (the first
+// stage of the mixed matrix-free path): FP32 integrals, FP32 elements,
+// compensated FP32 accumulation of h * x.
 // ---------------------------------------------------------------------------
-// Matrix-free sigma (HmultDirect, SHCI/Hmult.h:241-381): row I's connections
-// are found by visit_row and H_IJ is recomputed (ket = max(I, J), so the
-// element is the same in both triangles). Hits are queued per warp, singles
-// and doubles apart, and evaluated 32 at a time on full warps, as in the H
-// build. FP64: the reference's arithmetic. FP32 (the first stage of the
-// mixed matrix-free path): FP32 integrals, FP32 elements, compensated FP32
-// accumulation of h * x.
 template <int K, bool F32>
 struct DirectQVisitor {
-  using T = typename std::conditional<F32, float, double>::type;
-  const Det2* dets;
-  IntsView ints;
-  Det2 dI;
-  uint32_t I;
+  using T = typename Elem<F32>::T;
+  const HelperView& h;
+  const IntsView& ints;
+  uint64_t A, B;
   const T* x;  // [N][K]
-  uint32_t* qs;
-  uint32_t* qd;
-  int ns, nd;
-  Acc a32[K];
-  double a64[K];
+  uint32_t* q;  // three queues of 64
+  int ns, nd, nm;
+  Acc a32[F32 ? K : 1];
+  double a64[F32 ? 1 : K];
 
-  __device__ void add(uint32_t J) {
-    const Det2 dJ = dets[J];
-    if constexpr (F32) {
-      const float hv = ham_element_f32(ints.I1f, ints.I2f, ints.V1f, ints.norb, dI, dJ, J < I);
-#pragma unroll
-      for (int r = 0; r < K; ++r) acc_add(a32[r], hv, x[(size_t)J * K + r]);
+  __device__ __forceinline__ void load(T (&v)[K], uint32_t p) const {
+    if constexpr (K == 1) {
+      v[0] = __ldg(x + p);
+    } else if constexpr (F32 && K == 2) {
+      const float2 t = __ldg(reinterpret_cast<const float2*>(x) + p);
+      v[0] = t.x;
+      v[1] = t.y;
+    } else if constexpr (F32) {
+      const float4 t = __ldg(reinterpret_cast<const float4*>(x) + p);
+      v[0] = t.x;
+      v[1] = t.y;
+      v[2] = t.z;
+      v[3] = t.w;
     } else {
-      const double hv = ham_element(ints.I1, ints.I2, ints.V1, ints.norb, dI, dJ, J < I);
 #pragma unroll
-      for (int r = 0; r < K; ++r) a64[r] += hv * x[(size_t)J * K + r];
-    }
-  }
-  __device__ int drain(uint32_t* q, int n, int cnt) {
-    const int lane = threadIdx.x & 31;
-    if (lane < cnt) add(q[lane]);
-    __syncwarp();
-    const int rest = n - cnt;
-    const uint32_t v = lane < rest ? q[cnt + lane] : 0u;
-    __syncwarp();
-    if (lane < rest) q[lane] = v;
-    __syncwarp();
-    return rest;
-  }
-  __device__ void step(bool hit, uint32_t J, bool single) {
-    const int lane = threadIdx.x & 31;
-    const unsigned lt = (1u << lane) - 1u;
-    const unsigned ms = __ballot_sync(kFull, hit && single);
-    const unsigned md = __ballot_sync(kFull, hit && !single);
-    if (hit && single) qs[ns + __popc(ms & lt)] = J;
-    if (hit && !single) qd[nd + __popc(md & lt)] = J;
-    ns += __popc(ms);
-    nd += __popc(md);
-    __syncwarp();
-    if (ns >= 32) ns = drain(qs, ns, 32);
-    if (nd >= 32) nd = drain(qd, nd, 32);
-  }
-  __device__ void flush() {
-    if (ns) ns = drain(qs, ns, ns);
-    if (nd) nd = drain(qd, nd, nd);
-  }
-};
-
-template <int K, bool F32>
-__global__ void __launch_bounds__(256, SHCI_DIRECT_MIN_BLOCKS) k_sigma_direct(HelperView h, const Det2* __restrict__ dets, IntsView ints,
-                                                      const double* __restrict__ diag,
-                                                      const typename DirectQVisitor<K, F32>::T* __restrict__ x,
-                                                      double* __restrict__ y) {
-  __shared__ uint32_t s_q[8][2][64];
-  const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-  const int64_t warps = (int64_t)gridDim.x * (blockDim.x >> 5);
-  // rows in alpha-major order (the alpha groups' determinant lists): rows of
-  // one alpha string run side by side and probe the same sections of the
-  // partial-string index, and largely the same connections, from cache
-  for (int64_t k = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; k < (int64_t)h.N; k += warps) {
-    const int64_t I = h.aDets[k];
-    DirectQVisitor<K, F32> v;
-    v.dets = dets;
-    v.ints = ints;
-    v.dI = dets[I];
-    v.I = (uint32_t)I;
-    v.x = x;
-    v.qs = s_q[wib][0];
-    v.qd = s_q[wib][1];
-    v.ns = v.nd = 0;
-#pragma unroll
-    for (int r = 0; r < K; ++r) {
-      v.a32[r] = Acc{0.f, 0.f};
-      v.a64[r] = 0.0;
-    }
-    visit_row(h, (uint32_t)I, v);
-    v.flush();
-#pragma unroll
-    for (int r = 0; r < K; ++r) {
-      if constexpr (F32) {
-        Acc a = v.a32[r];
-        // merge in lane order (a fixed tree); FP64 diagonal term
-#pragma unroll
-        for (int o = 16; o; o >>= 1) {
-          Acc other{__shfl_xor_sync(kFull, a.s, o), __shfl_xor_sync(kFull, a.c, o)};
-          if ((lane & o) == 0) {
-            acc_merge(a, other);
-          } else {
-            acc_merge(other, a);
-            a = other;
-          }
-        }
-        if (lane == 0) y[(size_t)I * K + r] = diag[I] * (double)x[(size_t)I * K + r] + ((double)a.s + (double)a.c);
-      } else {
-        double a = v.a64[r];
-#pragma unroll
-        for (int o = 16; o; o >>= 1) a += __shfl_xor_sync(kFull, a, o);
-        if (lane == 0) y[(size_t)I * K + r] = diag[I] * x[(size_t)I * K + r] + a;
+      for (int r = 0; r < K; r += 2) {
+        const double2 t = __ldg(reinterpret_cast<const double2*>(x + (size_t)p * K + r));
+        v[r] = t.x;
+        v[r + 1] = t.y;
       }
     }
   }
+  // which: 0 singles, 1 alpha-beta doubles, 2 doubles of one spin
+  template <int which>
+  __device__ __forceinline__ void add(uint32_t p) {
+    const ulonglong2 J = h.str[p];
+    T xv[K];
+    load(xv, p);
+    T hv;
+    if constexpr (which == 0) {
+      const bool beta = J.x == A;
+      hv = elem_single<F32>(ints.I1, ints.V1, ints.I1f, ints.V1f, ints.norb, A, B, beta ? B : A, beta ? J.y : J.x,
+                            beta);
+    } else if constexpr (which == 1) {
+      hv = elem_ab<F32>(ints, A, B, J.x, J.y);
+    } else {
+      hv = J.x == A ? elem_same<F32, 1>(ints, B, A, J.y) : elem_same<F32, 0>(ints, A, B, J.x);
+    }
+#pragma unroll
+    for (int r = 0; r < K; ++r) {
+      if constexpr (F32)
+        acc_add(a32[r], hv, xv[r]);
+      else
+        a64[r] += hv * xv[r];
+    }
+  }
+  template <int which>
+  __device__ __forceinline__ int drain(uint32_t* w, int n, int cnt) {
+    const int lane = threadIdx.x & 31;
+    if (lane < cnt) add<which>(w[lane]);
+    __syncwarp();
+    const int rest = n - cnt;
+    const uint32_t v = lane < rest ? w[cnt + lane] : 0u;
+    __syncwarp();
+    if (lane < rest) w[lane] = v;
+    __syncwarp();
+    return rest;
+  }
+  __device__ __forceinline__ void step(bool hit, uint32_t p, int cls) {
+    const unsigned lt = (1u << (threadIdx.x & 31)) - 1u;
+    if (cls == kAlpha) {  // the class is that of the scan, uniform but for singles
+      const bool single = hit && h.bstr[p] == B;
+      const unsigned ms = __ballot_sync(kFull, single), md = __ballot_sync(kFull, hit && !single);
+      if (single)
+        q[ns + __popc(ms & lt)] = p;
+      else if (hit)
+        q[64 + nd + __popc(md & lt)] = p;
+      ns += __popc(ms);
+      nd += __popc(md);
+    } else {
+      const bool single = hit && cls == kSingleB;
+      const unsigned ms = __ballot_sync(kFull, single), md = __ballot_sync(kFull, hit && !single);
+      if (single)
+        q[ns + __popc(ms & lt)] = p;
+      else if (hit)
+        q[128 + nm + __popc(md & lt)] = p;
+      ns += __popc(ms);
+      nm += __popc(md);
+    }
+    __syncwarp();
+    if (ns >= 32) ns = drain<0>(q, ns, 32);
+    if (nd >= 32) nd = drain<1>(q + 64, nd, 32);
+    if (nm >= 32) nm = drain<2>(q + 128, nm, 32);
+  }
+  __device__ __forceinline__ void flush() {
+    if (ns) drain<0>(q, ns, ns);
+    if (nd) drain<1>(q + 64, nd, nd);
+    if (nm) drain<2>(q + 128, nm, nm);
+  }
+};
+
+// A warp per row, four rows a block and as many blocks as rows need: the
+// rows' work differs by two orders of magnitude (the lowest determinant's row
+// holds 29,219 of 100,000 columns), and the block scheduler evens it out.
+constexpr int kDirThreads = 128;
+template <int K, bool F32>
+__global__ void __launch_bounds__(kDirThreads) k_sigma_direct(HelperView h, IntsView ints,
+                                                              const uint32_t* __restrict__ perm,
+                                                              const double* __restrict__ diag,
+                                                              const typename Elem<F32>::T* __restrict__ x, int kw,
+                                                              double* __restrict__ y, size_t ldy) {
+  __shared__ uint32_t s_q[kDirThreads / 32][192];
+  const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
+  const size_t p = (size_t)blockIdx.x * (kDirThreads / 32) + wib;
+  if (p >= h.N) return;
+  const ulonglong2 I = h.str[p];
+  DirectQVisitor<K, F32> v{h, ints, I.x, I.y, x, s_q[wib], 0, 0, 0, {}, {}};
+  visit_row(h, (uint32_t)p, I.x, I.y, v);
+  v.flush();
+  const size_t o = perm[p];
+  const double dg = diag[o];
+#pragma unroll
+  for (int r = 0; r < K; ++r) {
+    double t;
+    if constexpr (F32) {
+      Acc a = v.a32[r];
+      // merge in lane order (a fixed tree); FP64 diagonal term
+#pragma unroll
+      for (int b = 16; b; b >>= 1) {
+        Acc other{__shfl_xor_sync(kFull, a.s, b), __shfl_xor_sync(kFull, a.c, b)};
+        if ((lane & b) == 0) {
+          acc_merge(a, other);
+        } else {
+          acc_merge(other, a);
+          a = other;
+        }
+      }
+      t = (double)a.s + (double)a.c;
+    } else {
+      t = v.a64[r];
+#pragma unroll
+      for (int b = 16; b; b >>= 1) t += __shfl_xor_sync(kFull, t, b);
+    }
+    if (lane == 0 && r < kw) y[(size_t)r * ldy + o] = dg * (double)x[p * K + r] + t;
+  }
 }
 
-void sigma_direct(const Helpers& hp, const Det2* dets, const IntsView& ints, const double* diag, const double* x,
-                  double* y, int k, cudaStream_t s) {
+template <bool F32>
+static void launch_direct(const Helpers& hp, const IntsView& ints, const double* diag,
+                          const typename Elem<F32>::T* x, int k, int kw, double* y, size_t ldy, cudaStream_t s) {
+  if (hp.N == 0) return;
   HelperView hv = hp.view();
-  const unsigned blocks = grid_for(hp.N * 32, 256, 152 * 16);
+  const unsigned blocks = (unsigned)((hp.N + kDirThreads / 32 - 1) / (kDirThreads / 32));
   switch (k) {
-    case 1: k_sigma_direct<1, false><<<blocks, 256, 0, s>>>(hv, dets, ints, diag, x, y); break;
-    case 2: k_sigma_direct<2, false><<<blocks, 256, 0, s>>>(hv, dets, ints, diag, x, y); break;
-    case 4: k_sigma_direct<4, false><<<blocks, 256, 0, s>>>(hv, dets, ints, diag, x, y); break;
+    case 1: k_sigma_direct<1, F32><<<blocks, kDirThreads, 0, s>>>(hv, ints, hp.perm.p, diag, x, kw, y, ldy); break;
+    case 2: k_sigma_direct<2, F32><<<blocks, kDirThreads, 0, s>>>(hv, ints, hp.perm.p, diag, x, kw, y, ldy); break;
+    case 4: k_sigma_direct<4, F32><<<blocks, kDirThreads, 0, s>>>(hv, ints, hp.perm.p, diag, x, kw, y, ldy); break;
     default: throw Error(kErrInvalid, "direct sigma supports k in {1,2,4}");
   }
   SHCI_LAUNCH_CHECK();
 }
-
-void sigma_direct32(const Helpers& hp, const Det2* dets, const IntsView& ints, const double* diag, const float* x,
-                    double* y, int k, cudaStream_t s) {
+void sigma_direct(const Helpers& hp, const IntsView& ints, const double* diag, const double* x, int k, int kw,
+                  double* y, size_t ldy, cudaStream_t s) {
+  launch_direct<false>(hp, ints, diag, x, k, kw, y, ldy, s);
+}
+void sigma_direct32(const Helpers& hp, const IntsView& ints, const double* diag, const float* x, int k, int kw,
+                    double* y, size_t ldy, cudaStream_t s) {
   if (!ints.I1f || !ints.I2f) throw Error(kErrState, "FP32 integrals missing");
-  HelperView hv = hp.view();
-  const unsigned blocks = grid_for(hp.N * 32, 256, 152 * 16);
-  switch (k) {
-    case 1: k_sigma_direct<1, true><<<blocks, 256, 0, s>>>(hv, dets, ints, diag, x, y); break;
-    case 2: k_sigma_direct<2, true><<<blocks, 256, 0, s>>>(hv, dets, ints, diag, x, y); break;
-    case 4: k_sigma_direct<4, true><<<blocks, 256, 0, s>>>(hv, dets, ints, diag, x, y); break;
-    default: throw Error(kErrInvalid, "direct sigma supports k in {1,2,4}");
-  }
-  SHCI_LAUNCH_CHECK();
+  launch_direct<true>(hp, ints, diag, x, k, kw, y, ldy, s);
 }
 
 }  // namespace shci

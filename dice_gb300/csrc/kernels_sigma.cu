@@ -637,11 +637,6 @@ __global__ void k_pack_f64(const double* __restrict__ A, size_t lda, int c0, int
     for (int c = 0; c < kp; ++c) out[r * kp + c] = c < k ? A[(size_t)(c0 + c) * lda + src] : 0.0;
   }
 }
-__global__ void k_unpack_f64(const double* __restrict__ in, int kp, int k, size_t N, double* __restrict__ A,
-                             size_t lda, int c0) {
-  for (size_t r = (size_t)blockIdx.x * blockDim.x + threadIdx.x; r < N; r += (size_t)gridDim.x * blockDim.x)
-    for (int c = 0; c < k; ++c) A[(size_t)(c0 + c) * lda + r] = in[r * kp + c];
-}
 __global__ void k_pack_ff(const double* __restrict__ A, size_t lda, int c0, int k, int kp, size_t N,
                           float2* __restrict__ out, const uint32_t* __restrict__ perm) {
   for (size_t r = (size_t)blockIdx.x * blockDim.x + threadIdx.x; r < N; r += (size_t)gridDim.x * blockDim.x)
@@ -691,11 +686,6 @@ void gather_rows(const void* in, size_t bytes_per_row, const uint32_t* perm, siz
   }
   SHCI_LAUNCH_CHECK();
 }
-void unpack_f64(const double* in, int kp, int k, size_t N, double* A, size_t lda, int c0, cudaStream_t s) {
-  k_unpack_f64<<<grid_for(N, 256), 256, 0, s>>>(in, kp, k, N, A, lda, c0);
-  SHCI_LAUNCH_CHECK();
-}
-
 // ---------------------------------------------------------------------------
 // Tall-skinny Gram: G = A^T B. Blocks own contiguous row ranges and write
 // one partial per block; a second kernel adds the partials in block order, so
