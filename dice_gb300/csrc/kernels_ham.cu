@@ -266,7 +266,7 @@ __global__ void k_m1_insert(const uint4* __restrict__ ent, int64_t n, const uint
 // 4-vector matrix-free sigma: 60.7 ms probing every group, 49.7 / 48.8 / 47.5 /
 // 47.7 ms with factors 2 / 3 / 4 / 6.
 #ifndef SHCI_SCAN_FACTOR
-#define SHCI_SCAN_FACTOR 4
+#define SHCI_SCAN_FACTOR 8
 #endif
 constexpr int kScanFactor = SHCI_SCAN_FACTOR;
 // One warp per group; each part is put in ascending order by counting (a list
@@ -856,39 +856,13 @@ __device__ __forceinline__ int run_below(const uint32_t* run, int n, uint32_t c)
   return lo;
 }
 
-__device__ __forceinline__ void finish_row(const HelperView& h, const IntsView& ints, uint32_t p, const uint4& n,
-                                           const uint32_t* run, int64_t p0, int32_t* __restrict__ col,
-                                           double* __restrict__ v64, float* __restrict__ vhi, float* __restrict__ vlo) {
-  const ulonglong2 I = h.str[p];
-  const uint64_t A = I.x, B = I.y;
-  const int n1 = (int)n.x, n2 = (int)n.y, n3 = (int)n.z, n4 = (int)n.w;
-  const uint32_t *r2 = run + n1, *r3 = r2 + n2, *r4 = r3 + n3;
-  const int len = n1 + n2 + n3 + n4;
-  for (int e = threadIdx.x; e < len; e += blockDim.x) {
-    const uint32_t c = run[e];
-    const ulonglong2 J = h.str[c];
-    int rank;
-    double v;
-    if (e < n1) {
-      rank = e + run_below(r2, n2, c) + run_below(r3, n3, c) + run_below(r4, n4, c);
-      v = __popcll(B ^ J.y) == 4 ? elem_same<false, 1>(ints, B, A, J.y)
-                                 : elem_single<false>(ints.I1, ints.V1, nullptr, nullptr, ints.norb, A, B, B, J.y, 1);
-    } else {
-      rank = n1 > 0 && c > run[0] ? n1 : 0;
-      if (e >= n1 + n2 + n3) {
-        rank += e - (n1 + n2 + n3) + run_below(r2, n2, c) + run_below(r3, n3, c);
-        v = elem_same<false, 0>(ints, A, B, J.x);
-      } else {
-        if (e >= n1 + n2)
-          rank += e - (n1 + n2) + run_below(r2, n2, c) + run_below(r4, n4, c);
-        else
-          rank += e - n1 + run_below(r3, n3, c) + run_below(r4, n4, c);
-        v = J.y == B ? elem_single<false>(ints.I1, ints.V1, nullptr, nullptr, ints.norb, A, B, A, J.x, 0)
-                     : elem_ab<false>(ints, A, B, J.x, J.y);
-      }
-    }
-    const int64_t q = p0 + rank;
-    col[q] = (int32_t)c;
+// Where a row's entries go.
+struct FinishOut {
+  int32_t* __restrict__ col;
+  double* __restrict__ v64;
+  float* __restrict__ vhi;
+  float* __restrict__ vlo;
+  __device__ __forceinline__ void put(int64_t q, double v) const {
     if (v64) {
       v64[q] = v;
     } else {
@@ -896,6 +870,85 @@ __device__ __forceinline__ void finish_row(const HelperView& h, const IntsView& 
       vhi[q] = hi;
       if (vlo) vlo[q] = (float)(v - (double)hi);
     }
+  }
+};
+
+// Single excitations wait per warp, over rows, until 32 are there: their
+// elements are sums over every electron in FP64 (two lanes per clock and SM),
+// and one among a warp's 32 entries would make the whole warp run the sum.
+// Entry: place (64 bits), position of the row, of the column.
+struct SingleQueue {
+  uint4* q;  // 64 entries
+  int n = 0;
+  __device__ __forceinline__ void push(bool s, int64_t at, uint32_t p, uint32_t c, const HelperView& h,
+                                       const IntsView& ints, const FinishOut& out) {
+    const unsigned m = __ballot_sync(kFull, s);
+    if (!m) return;
+    if (s) q[n + __popc(m & ((1u << (threadIdx.x & 31)) - 1u))] = make_uint4((uint32_t)at, (uint32_t)(at >> 32), p, c);
+    n += __popc(m);
+    __syncwarp();
+    if (n >= 32) drain(32, h, ints, out);
+  }
+  __device__ __forceinline__ void drain(int cnt, const HelperView& h, const IntsView& ints, const FinishOut& out) {
+    const int lane = threadIdx.x & 31;
+    if (lane < cnt) {
+      const uint4 w = q[lane];
+      const ulonglong2 I = h.str[w.z], J = h.str[w.w];
+      const bool beta = I.x == J.x;
+      out.put((int64_t)(((uint64_t)w.y << 32) | w.x),
+              elem_single<false>(ints.I1, ints.V1, nullptr, nullptr, ints.norb, I.x, I.y, beta ? I.y : I.x,
+                                 beta ? J.y : J.x, beta));
+    }
+    __syncwarp();
+    const int rest = n - cnt;
+    const uint4 v = lane < rest ? q[cnt + lane] : make_uint4(0u, 0u, 0u, 0u);
+    __syncwarp();
+    if (lane < rest) q[lane] = v;
+    __syncwarp();
+    n = rest;
+  }
+};
+
+__device__ __forceinline__ void finish_row(const HelperView& h, const IntsView& ints, uint32_t p, const uint4& n,
+                                           const uint32_t* run, int64_t p0, const FinishOut& out, SingleQueue& sq) {
+  const ulonglong2 I = h.str[p];
+  const uint64_t A = I.x, B = I.y;
+  const int n1 = (int)n.x, n2 = (int)n.y, n3 = (int)n.z, n4 = (int)n.w;
+  const uint32_t *r2 = run + n1, *r3 = r2 + n2, *r4 = r3 + n3;
+  const int len = n1 + n2 + n3 + n4;
+  for (int e0 = 0; e0 < len; e0 += blockDim.x) {  // all lanes together: the queue's ballots
+    const int e = e0 + (int)threadIdx.x;
+    bool single = false;
+    uint32_t c = 0;
+    int64_t q = 0;
+    if (e < len) {
+      c = run[e];
+      const ulonglong2 J = h.str[c];
+      int rank;
+      double v = 0.0;
+      if (e < n1) {
+        rank = e + run_below(r2, n2, c) + run_below(r3, n3, c) + run_below(r4, n4, c);
+        single = __popcll(B ^ J.y) == 2;
+        if (!single) v = elem_same<false, 1>(ints, B, A, J.y);
+      } else {
+        rank = n1 > 0 && c > run[0] ? n1 : 0;
+        if (e >= n1 + n2 + n3) {
+          rank += e - (n1 + n2 + n3) + run_below(r2, n2, c) + run_below(r3, n3, c);
+          v = elem_same<false, 0>(ints, A, B, J.x);
+        } else {
+          if (e >= n1 + n2)
+            rank += e - (n1 + n2) + run_below(r2, n2, c) + run_below(r4, n4, c);
+          else
+            rank += e - n1 + run_below(r3, n3, c) + run_below(r4, n4, c);
+          single = J.y == B;
+          if (!single) v = elem_ab<false>(ints, A, B, J.x, J.y);
+        }
+      }
+      q = p0 + rank;
+      out.col[q] = (int32_t)c;
+      if (!single) out.put(q, v);
+    }
+    sq.push(single, q, p, c, h, ints, out);
   }
 }
 
@@ -906,15 +959,19 @@ __global__ void __launch_bounds__(kFinThreads) k_ham_finish(HelperView h, IntsVi
                                                             int32_t* __restrict__ col, double* __restrict__ v64,
                                                             float* __restrict__ vhi, float* __restrict__ vlo) {
   __shared__ uint32_t run[kRunCap];
+  __shared__ uint4 s_q[kFinThreads / 32][64];
+  const FinishOut out{col, v64, vhi, vlo};
+  SingleQueue sq{s_q[threadIdx.x >> 5]};
   for (int64_t k = blockIdx.x; k < nr; k += gridDim.x) {
     const int64_t p0 = rowptr[k];
     const int len = (int)(rowptr[k + 1] - p0);
     if (len == 0 || len > kRunCap) continue;  // uniform across the block
     for (int e = threadIdx.x; e < len; e += blockDim.x) run[e] = (uint32_t)col[p0 + e];
     __syncthreads();
-    finish_row(h, ints, rows ? rows[k] : (uint32_t)k, parts[k], run, p0, col, v64, vhi, vlo);
+    finish_row(h, ints, rows ? rows[k] : (uint32_t)k, parts[k], run, p0, out, sq);
     __syncthreads();
   }
+  if (sq.n) sq.drain(sq.n, h, ints, out);
 }
 
 // Rows past kRunCap: listed with their places in a scratch copy of their runs.
@@ -935,13 +992,17 @@ __global__ void __launch_bounds__(1024) k_ham_finish_long(HelperView h, IntsView
                                                           const int64_t* __restrict__ rowptr,
                                                           int32_t* __restrict__ col, double* __restrict__ v64,
                                                           float* __restrict__ vhi, float* __restrict__ vlo) {
+  __shared__ uint4 s_q[32][64];
+  const FinishOut out{col, v64, vhi, vlo};
+  SingleQueue sq{s_q[threadIdx.x >> 5]};
   const uint2 l = list[blockIdx.x];
   const int64_t p0 = rowptr[l.x];
   const int len = (int)(rowptr[l.x + 1] - p0);
   uint32_t* run = scratch + 32 * (size_t)l.y;
   for (int e = threadIdx.x; e < len; e += blockDim.x) run[e] = (uint32_t)col[p0 + e];
   __syncthreads();
-  finish_row(h, ints, rows ? rows[l.x] : l.x, parts[l.x], run, p0, col, v64, vhi, vlo);
+  finish_row(h, ints, rows ? rows[l.x] : l.x, parts[l.x], run, p0, out, sq);
+  if (sq.n) sq.drain(sq.n, h, ints, out);
 }
 
 __global__ void k_set_last(int64_t* rowptr, int64_t n, int64_t total) { rowptr[n] = total; }
@@ -1455,7 +1516,7 @@ void build_ham_csr(const Helpers& hp, const IntsView& ints, Csr& H, bool want64,
                    size_t n_old, Prims& pr, cudaStream_t s) {
   const size_t N = hp.N;
   PhaseTimer pt(s);
-  const bool incremental = !H.block && n_old > 0 && n_old < N && H.N == n_old && H.perm.n >= n_old &&
+  const bool incremental = !H.block && n_old > 0 && N - n_old < n_old && H.N == n_old && H.perm.n >= n_old &&
                            (want64 ? !want32 : (want32 && want_lo)) &&
                            (H.v64.p != nullptr) == want64 && (H.vhi.p != nullptr) == want32 &&
                            (H.vlo.p != nullptr) == (want32 && want_lo);
