@@ -767,21 +767,7 @@ __global__ void __launch_bounds__(256) k_ham_emit(HelperView h, const uint32_t* 
 // of the two determinants is the ket makes no difference: a double's integrals
 // are symmetric, and a single's sum differs only in where its zero terms
 // stand ((ai|ii) - (ai|ii) for the orbital left behind).
-//
-// Moving an electron of string S between orbitals lo < hi passes the
-// electrons of S strictly between, and in the interleaved order (alpha of an
-// orbital before beta) the other string O's in [lo, hi) for an alpha electron
-// and in (lo, hi] for a beta one.
 // ---------------------------------------------------------------------------
-__device__ __forceinline__ uint64_t bits_from(int lo, int hi) { return (1ull << hi) - (1ull << lo); }  // [lo, hi)
-template <int kSpin>
-__device__ __forceinline__ uint64_t passed(uint64_t S, uint64_t O, int i, int a) {
-  const int lo = i < a ? i : a, hi = i < a ? a : i;
-  const uint64_t m = bits_from(lo, hi), open = m ^ (1ull << lo);
-  return (S & open) ^ (O & (kSpin ? open ^ (1ull << hi) : m));
-}
-__device__ __forceinline__ int low_bit(uint64_t x) { return __ffsll((long long)x) - 1; }
-
 // Integral access in either precision (FP64: __dsub_rn, so never contracted).
 template <bool F32>
 struct Elem;

@@ -98,6 +98,18 @@ __device__ inline int occ_between(const Det2& d, int lo, int hi) {
   return c;
 }
 
+// Electrons passed (as a set whose population parity is the sign) when one of
+// string S moves between orbitals i and a: those of S strictly between, and in
+// the interleaved order (alpha of an orbital before beta) the other string O's
+// in [lo, hi) for an alpha electron (kSpin 0) and in (lo, hi] for a beta one.
+template <int kSpin>
+__device__ __forceinline__ uint64_t passed(uint64_t S, uint64_t O, int i, int a) {
+  const int lo = i < a ? i : a, hi = i < a ? a : i;
+  const uint64_t m = (1ull << hi) - (1ull << lo), open = m ^ (1ull << lo);
+  return (S & open) ^ (O & (kSpin ? open ^ (1ull << hi) : m));
+}
+__device__ __forceinline__ int low_bit(uint64_t x) { return __ffsll((long long)x) - 1; }
+
 // Device view of the integrals (SHCI/integral.h:47-101).
 struct IntsView {
   const double* I1;        // (2n)x(2n) spin-orbital matrix
