@@ -191,6 +191,7 @@ struct Context {
   DevBuf<float> dI1f, dI2f;  // FP32 copies for the FP32 matrix-free sigma
   DevBuf<double> dV1;        // terms of Hij_1Excite per (a, i, j) (IntsView::V1)
   DevBuf<float> dV1f;
+  DevBuf<float2> dI2ff;      // I2 as FP32 head and tail, for the mixed build
   DevBuf<float> dSameVal, dOppVal;
   DevBuf<int16_t> dSamePairs, dOppPairs;
   DevBuf<int64_t> dSameStart, dOppStart;
@@ -348,7 +349,7 @@ struct Context {
   }
 
   IntsView ints() const {
-    return IntsView{dI1.p, dI2.p, dDirect.p, dExchange.p, hints.norb, dI1f.p, dI2f.p, dV1.p, dV1f.p};
+    return IntsView{dI1.p, dI2.p, dDirect.p, dExchange.p, hints.norb, dI1f.p, dI2f.p, dV1.p, dV1f.p, dI2ff.p};
   }
   HeatBathView hb() const {
     return HeatBathView{dSameVal.p, dSamePairs.p, dSameStart.p, dOppVal.p, dOppPairs.p, dOppStart.p, dSingles.p, dHbCum.p};
@@ -380,6 +381,10 @@ struct Context {
       const std::vector<float> f1(hints.I1.begin(), hints.I1.end()), f2(hints.I2.begin(), hints.I2.end());
       upload(dI1f, f1);
       upload(dI2f, f2);
+      std::vector<float2> ff(hints.I2.size());
+      for (size_t t = 0; t < ff.size(); ++t)
+        ff[t] = make_float2(f2[t], (float)(hints.I2[t] - (double)f2[t]));
+      upload(dI2ff, ff);
       std::vector<double> v1;
       std::vector<float> v1f;
       single_terms(hints, v1, v1f);

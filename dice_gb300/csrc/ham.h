@@ -4,19 +4,33 @@
 
 namespace shci {
 
+// A determinant as its {alpha, beta} strings: 32-bit words up to 32 orbitals,
+// where every mask, population count and bit search is one instruction and a
+// string pair half the bytes, 64-bit words beyond.
+template <class S>
+struct StrPair;
+template <>
+struct StrPair<uint32_t> {
+  using T = uint2;
+};
+template <>
+struct StrPair<uint64_t> {
+  using T = ulonglong2;
+};
+
 // Plain-pointer view passed to kernels. Everything is indexed by storage
 // position: the determinants sorted by (alpha string, beta string).
+template <class S>
 struct HelperView {
   size_t N;
-  const ulonglong2* str;  // {alpha, beta} string of each position
-  const uint64_t* bstr;   // beta string of each position
+  const typename StrPair<S>::T* str;  // strings of each position
+  const S* bstr;          // beta string of each position
   const uint32_t* agrp;   // position -> alpha group
   const uint32_t* bgrp;   // position -> beta group
-  const uint64_t* ua;     // alpha string of each alpha group, ascending
   const int64_t* aStart;  // alpha group g is the positions [aStart[g], aStart[g+1])
   const int64_t* bStart;
   const uint32_t* bPos;    // positions grouped by beta string, ascending in each group
-  const uint64_t* bAlpha;  // alpha string of bPos[q]
+  const S* bAlpha;         // alpha string of bPos[q]
   const int64_t* aSingStart;  // single-excitation neighbours of each alpha group as CSR
   const uint32_t* aSing;
   // the list of alpha group g holds its small groups (a few times n_beta
@@ -41,10 +55,10 @@ struct HelperView {
 // (HamHelpers2, SHCI/SHCImakeHamiltonian.h:44-82).
 struct Helpers {
   size_t N = 0;
+  bool narrow = true;  // 32-bit strings (up to 32 orbitals)
   int64_t NA = 0, NB = 0, nsing = 0;
   DevBuf<uint32_t> perm, spos;  // storage position -> determinant index, and its inverse
-  DevBuf<ulonglong2> str;
-  DevBuf<uint64_t> bstr, ua, bAlpha;
+  DevBuf<uint64_t> str, bstr, ua, bAlpha;  // strings as the views' words, sized in bytes by `narrow`
   DevBuf<uint32_t> agrp, bgrp, bPos, aSing;
   DevBuf<int64_t> aStart, bStart, aSingStart, aSingMid;
   DevBuf<uint4> m1ent;
@@ -52,10 +66,23 @@ struct Helpers {
   DevBuf<uint64_t> m1dir;
   int64_t nm1 = 0;
   void build(const Det2* dets, size_t n, int norb, Prims& pr, cudaStream_t s);
-  HelperView view() const {
-    return HelperView{N,        str.p,   bstr.p,  agrp.p,       bgrp.p,  ua.p,       aStart.p, bStart.p,
-                      bPos.p,   bAlpha.p, aSingStart.p, aSing.p, aSingMid.p, nm1 > 0 ? m1ent.p : nullptr,
-                      m1tab.p,  m1dir.p};
+  template <class S>
+  HelperView<S> view() const {
+    return HelperView<S>{N,
+                         reinterpret_cast<const typename StrPair<S>::T*>(str.p),
+                         reinterpret_cast<const S*>(bstr.p),
+                         agrp.p,
+                         bgrp.p,
+                         aStart.p,
+                         bStart.p,
+                         bPos.p,
+                         reinterpret_cast<const S*>(bAlpha.p),
+                         aSingStart.p,
+                         aSing.p,
+                         aSingMid.p,
+                         nm1 > 0 ? m1ent.p : nullptr,
+                         m1tab.p,
+                         m1dir.p};
   }
   size_t bytes() const {
     return perm.bytes() + spos.bytes() + str.bytes() + bstr.bytes() + ua.bytes() + bAlpha.bytes() + agrp.bytes() +

@@ -73,18 +73,20 @@ __global__ void k_group_fill(const uint64_t* __restrict__ key, const uint32_t* _
     grp[pos ? pos[p] : (uint32_t)p] = (uint32_t)seg;
   }
 }
+template <class S>
 __global__ void k_pair_strings(const uint64_t* __restrict__ a, const uint64_t* __restrict__ b,
-                               const uint32_t* __restrict__ perm, size_t n, ulonglong2* __restrict__ str,
-                               uint32_t* __restrict__ spos, uint64_t* __restrict__ bkey, uint32_t* __restrict__ bpos) {
+                               const uint32_t* __restrict__ perm, size_t n, typename StrPair<S>::T* __restrict__ str,
+                               S* __restrict__ bstr, uint32_t* __restrict__ spos, uint32_t* __restrict__ bpos) {
   for (size_t p = (size_t)blockIdx.x * blockDim.x + threadIdx.x; p < n; p += (size_t)gridDim.x * blockDim.x) {
-    str[p] = make_ulonglong2(a[p], b[p]);
+    str[p] = {(S)a[p], (S)b[p]};
+    bstr[p] = (S)b[p];
     spos[perm[p]] = (uint32_t)p;
-    bkey[p] = b[p];
     bpos[p] = (uint32_t)p;
   }
 }
-__global__ void k_gather_alpha(const ulonglong2* __restrict__ str, const uint32_t* __restrict__ pos, size_t n,
-                               uint64_t* __restrict__ out) {
+template <class S>
+__global__ void k_gather_alpha(const typename StrPair<S>::T* __restrict__ str, const uint32_t* __restrict__ pos,
+                               size_t n, S* __restrict__ out) {
   for (size_t q = (size_t)blockIdx.x * blockDim.x + threadIdx.x; q < n; q += (size_t)gridDim.x * blockDim.x)
     out[q] = str[pos[q]].x;
 }
@@ -149,12 +151,14 @@ __global__ void k_iota_last(int64_t* start, int64_t n_groups, int64_t n_total) {
 // of rows of the same alpha string touch the same small regions.
 constexpr uint32_t kM1GroupBits = 26;
 
-__global__ void k_m1_count(const uint64_t* __restrict__ bstr, size_t n, int64_t* __restrict__ cnt) {
+template <class S>
+__global__ void k_m1_count(const S* __restrict__ bstr, size_t n, int64_t* __restrict__ cnt) {
   for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
-    cnt[i] = __popcll(bstr[i]);
+    cnt[i] = bit_count(bstr[i]);
 }
 // (index entries refer to their determinant by storage position)
-__global__ void k_m1_fill(const uint64_t* __restrict__ bstr, const uint32_t* __restrict__ agrp, size_t n,
+template <class S>
+__global__ void k_m1_fill(const S* __restrict__ bstr, const uint32_t* __restrict__ agrp, size_t n,
                           const int64_t* __restrict__ off, uint64_t* __restrict__ key, uint32_t* __restrict__ perm,
                           uint4* __restrict__ ent) {
   for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
@@ -190,12 +194,14 @@ __device__ __forceinline__ bool m1_same_key(const uint4& a, const uint4& b) {
 }
 // Fibonacci hashing: the top lg bits of the partial string times 2^64 / phi
 // pick the slot; 26 bits of a second product are the slot's fingerprint
-__device__ __forceinline__ uint64_t m1_slot(uint64_t bm, unsigned lg) {
-  return (bm * 0x9e3779b97f4a7c15ull) >> (64u - lg);
+__device__ __forceinline__ uint32_t m1_slot(uint64_t bm, unsigned lg) {
+  return (uint32_t)((bm * 0x9e3779b97f4a7c15ull) >> (64u - lg));
 }
+__device__ __forceinline__ uint32_t m1_slot(uint32_t bm, unsigned lg) { return (bm * 0x9e3779b9u) >> (32u - lg); }
 __device__ __forceinline__ uint32_t m1_fingerprint(uint64_t bm) {
   return (uint32_t)((bm * 0xc2b2ae3d27d4eb4full) >> 38);
 }
+__device__ __forceinline__ uint32_t m1_fingerprint(uint32_t bm) { return (bm * 0xc2b2ae3du) >> 6; }
 constexpr uint32_t kM1Empty = 0xffffffffu;
 // The entries of one group are contiguous, and the largest group holds a tenth
 // of them: a warp's heads of one group are added at once (400,000 determinants:
@@ -234,6 +240,7 @@ __global__ void k_m1_dir(const int64_t* __restrict__ slots, const int64_t* __res
 // One thread per run: measure the run (at most 64 entries: one per beta
 // orbital outside the partial string) and claim a slot of its group's table
 // by linear probing; a table more than half empty always has a free slot.
+template <class S>
 __global__ void k_m1_insert(const uint4* __restrict__ ent, int64_t n, const uint64_t* __restrict__ dir,
                             uint2* __restrict__ tab) {
   constexpr uint32_t gmask = (1u << kM1GroupBits) - 1u;
@@ -246,7 +253,7 @@ __global__ void k_m1_insert(const uint4* __restrict__ ent, int64_t n, const uint
     const unsigned lg = (unsigned)(d & 63);
     const uint64_t mask = (1ull << lg) - 1;
     uint2* t = tab + (d >> 6);
-    const uint64_t bm = ((uint64_t)e.y << 32) | e.x;
+    const S bm = (S)(((uint64_t)e.y << 32) | e.x);
     uint64_t q = m1_slot(bm, lg);
     for (uint64_t step = 0; step <= mask; ++step) {
       if (atomicCAS(&t[q].x, kM1Empty, (uint32_t)k) == kM1Empty) {
@@ -272,14 +279,15 @@ constexpr int kScanFactor = SHCI_SCAN_FACTOR;
 // One warp per group; each part is put in ascending order by counting (a list
 // has at most n_alpha x (norb - n_alpha) entries, some hundred), so that the
 // hits of a row's scans come in ascending order too.
+template <class S>
 __global__ void k_split_singles(const int64_t* __restrict__ sstart, const uint32_t* __restrict__ in,
-                                const int64_t* __restrict__ gstart, const uint64_t* __restrict__ bstr, int64_t na,
+                                const int64_t* __restrict__ gstart, const S* __restrict__ bstr, int64_t na,
                                 uint32_t* __restrict__ out, int64_t* __restrict__ mid) {
   const int lane = threadIdx.x & 31;
   const int64_t warps = (int64_t)gridDim.x * (blockDim.x >> 5);
   for (int64_t g = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; g < na; g += warps) {
     const int64_t s0 = sstart[g], s1 = sstart[g + 1];
-    const int64_t cap = (int64_t)kScanFactor * __popcll(bstr[gstart[g]]);
+    const int64_t cap = (int64_t)kScanFactor * bit_count(bstr[gstart[g]]);
     int64_t nsmall = 0;
     for (int64_t q = s0 + lane; q < s1; q += 32) nsmall += gstart[in[q] + 1] - gstart[in[q]] <= cap;
 #pragma unroll
@@ -305,28 +313,118 @@ __global__ void k_split_singles(const int64_t* __restrict__ sstart, const uint32
   }
 }
 
+// Single-excitation lists and partial-string index, from the strings by position.
+template <class S>
+static void build_singles_and_index(Helpers& hp, int norb, Prims& pr, cudaStream_t s) {
+  const size_t n = hp.N;
+  const S* bstr = reinterpret_cast<const S*>(hp.bstr.p);
+  // alpha single-excitation lists
+  DevBuf<int64_t> cnt;
+  cnt.resize(hp.NA);
+  hp.aSingStart.resize(hp.NA + 1);
+  k_alpha_singles<false><<<grid_for((size_t)hp.NA * 32, 256), 256, 0, s>>>(hp.ua.p, hp.NA, norb, cnt.p, nullptr, nullptr);
+  SHCI_LAUNCH_CHECK();
+  int64_t total = 0;
+  scan_exclusive_i64(cnt.p, hp.aSingStart.p, hp.NA, &total, pr, s);
+  k_iota_last<<<1, 1, 0, s>>>(hp.aSingStart.p, hp.NA, total);
+  SHCI_LAUNCH_CHECK();
+  hp.aSing.resize(total > 0 ? total : 1);
+  k_alpha_singles<true><<<grid_for((size_t)hp.NA * 32, 256), 256, 0, s>>>(hp.ua.p, hp.NA, norb, nullptr, hp.aSingStart.p,
+                                                                         hp.aSing.p);
+  SHCI_LAUNCH_CHECK();
+  hp.nsing = total;
+  {
+    DevBuf<uint32_t> split;
+    split.resize(total > 0 ? total : 1);
+    hp.aSingMid.resize(hp.NA);
+    k_split_singles<S><<<grid_for((size_t)hp.NA * 32, 256), 256, 0, s>>>(hp.aSingStart.p, hp.aSing.p, hp.aStart.p, bstr, hp.NA,
+                                                                   split.p, hp.aSingMid.p);
+    SHCI_LAUNCH_CHECK();
+    hp.aSing.swap(split);
+  }
+  // partial-string index (one entry per determinant and occupied beta orbital)
+  {
+    DevBuf<int64_t> c1, o1;
+    c1.resize(n);
+    o1.resize(n + 1);
+    k_m1_count<S><<<grid_for(n, 256), 256, 0, s>>>(bstr, n, c1.p);
+    SHCI_LAUNCH_CHECK();
+    int64_t ne = 0;
+    scan_exclusive_i64(c1.p, o1.p, n, &ne, pr, s);
+    if (ne >= ((int64_t)1 << 32)) throw Error(kErrInvalid, "partial-string index too large");
+    if (hp.NA >= ((int64_t)1 << kM1GroupBits)) throw Error(kErrInvalid, "too many alpha strings for the partial-string index");
+    hp.nm1 = ne;
+    if (ne > 0) {
+      DevBuf<uint64_t> key;
+      DevBuf<uint32_t> perm;
+      DevBuf<uint4> raw;
+      key.resize(ne);
+      perm.resize(ne);
+      raw.resize(ne);
+      hp.m1ent.resize(ne);
+      const unsigned eb = grid_for((size_t)ne, 256);
+      k_m1_fill<S><<<grid_for(n, 256), 256, 0, s>>>(bstr, hp.agrp.p, n, o1.p, key.p, perm.p, raw.p);
+      SHCI_LAUNCH_CHECK();
+      sort_u64(key.p, perm.p, (size_t)ne, pr, s);  // by partial string
+      k_m1_group_keys<<<eb, 256, 0, s>>>(raw.p, perm.p, ne, key.p);
+      SHCI_LAUNCH_CHECK();
+      sort_u64(key.p, perm.p, (size_t)ne, pr, s);  // then by alpha group (stable)
+      k_m1_permute<<<eb, 256, 0, s>>>(raw.p, perm.p, ne, hp.m1ent.p);
+      SHCI_LAUNCH_CHECK();
+      // the groups' hash tables
+      DevBuf<uint32_t> nkey;
+      DevBuf<int64_t> slots, first;
+      nkey.resize((size_t)hp.NA);
+      slots.resize((size_t)hp.NA);
+      first.resize((size_t)hp.NA + 1);
+      SHCI_CUDA(cudaMemsetAsync(nkey.p, 0, (size_t)hp.NA * sizeof(uint32_t), s));
+      k_m1_heads<<<eb, 256, 0, s>>>(hp.m1ent.p, ne, nkey.p);
+      SHCI_LAUNCH_CHECK();
+      k_m1_slots<<<grid_for((size_t)hp.NA, 256), 256, 0, s>>>(nkey.p, hp.NA, slots.p);
+      SHCI_LAUNCH_CHECK();
+      int64_t nslot = 0;
+      scan_exclusive_i64(slots.p, first.p, hp.NA, &nslot, pr, s);
+      hp.m1dir.resize((size_t)hp.NA);
+      k_m1_dir<<<grid_for((size_t)hp.NA, 256), 256, 0, s>>>(slots.p, first.p, hp.NA, hp.m1dir.p);
+      SHCI_LAUNCH_CHECK();
+      hp.m1tab.resize((size_t)nslot);
+      SHCI_CUDA(cudaMemsetAsync(hp.m1tab.p, 0xff, (size_t)nslot * sizeof(uint2), s));
+      k_m1_insert<S><<<eb, 256, 0, s>>>(hp.m1ent.p, ne, hp.m1dir.p, hp.m1tab.p);
+      SHCI_LAUNCH_CHECK();
+    }
+  }
+  SHCI_CUDA(cudaStreamSynchronize(s));
+}
+
 void Helpers::build(const Det2* dets, size_t n, int norb, Prims& pr, cudaStream_t s) {
   N = n;
   perm.resize(n);
   spos.resize(n);
-  str.resize(n);
-  bstr.resize(n);
+  narrow = norb <= 32;
+  str.resize(narrow ? n : 2 * n);
+  bstr.resize(narrow ? (n + 1) / 2 : n);
+  bAlpha.resize(narrow ? (n + 1) / 2 : n);
   agrp.resize(n);
   bgrp.resize(n);
   bPos.resize(n);
-  bAlpha.resize(n);
+  DevBuf<uint64_t> bkey;  // beta strings by position, then in beta order
   {
-    DevBuf<uint64_t> a, bkey;
+    DevBuf<uint64_t> a;
     DevBuf<int64_t> flag, excl;
     a.resize(n);
     bkey.resize(n);
     flag.resize(n);
     excl.resize(n);
     const unsigned g = grid_for(n, 256);
-    k_strings<<<g, 256, 0, s>>>(dets, n, a.p, bstr.p, perm.p);
+    k_strings<<<g, 256, 0, s>>>(dets, n, a.p, bkey.p, perm.p);
     SHCI_LAUNCH_CHECK();
-    sort_u128(bstr.p, a.p, perm.p, n, pr, s);  // by (alpha, beta): the storage order
-    k_pair_strings<<<g, 256, 0, s>>>(a.p, bstr.p, perm.p, n, str.p, spos.p, bkey.p, bPos.p);
+    sort_u128(bkey.p, a.p, perm.p, n, pr, s);  // by (alpha, beta): the storage order
+    if (narrow)
+      k_pair_strings<uint32_t><<<g, 256, 0, s>>>(a.p, bkey.p, perm.p, n, reinterpret_cast<uint2*>(str.p),
+                                                 reinterpret_cast<uint32_t*>(bstr.p), spos.p, bPos.p);
+    else
+      k_pair_strings<uint64_t><<<g, 256, 0, s>>>(a.p, bkey.p, perm.p, n, reinterpret_cast<ulonglong2*>(str.p), bstr.p,
+                                                 spos.p, bPos.p);
     SHCI_LAUNCH_CHECK();
     k_group_flags<<<g, 256, 0, s>>>(a.p, n, flag.p);
     SHCI_LAUNCH_CHECK();
@@ -346,109 +444,41 @@ void Helpers::build(const Det2* dets, size_t n, int norb, Prims& pr, cudaStream_
     SHCI_LAUNCH_CHECK();
     k_iota_last<<<1, 1, 0, s>>>(bStart.p, NB, (int64_t)n);
     SHCI_LAUNCH_CHECK();
-    k_gather_alpha<<<g, 256, 0, s>>>(str.p, bPos.p, n, bAlpha.p);
+    if (narrow)
+      k_gather_alpha<uint32_t><<<g, 256, 0, s>>>(reinterpret_cast<const uint2*>(str.p), bPos.p, n,
+                                                 reinterpret_cast<uint32_t*>(bAlpha.p));
+    else
+      k_gather_alpha<uint64_t><<<g, 256, 0, s>>>(reinterpret_cast<const ulonglong2*>(str.p), bPos.p, n, bAlpha.p);
     SHCI_LAUNCH_CHECK();
   }
-  // alpha single-excitation lists
-  DevBuf<int64_t> cnt;
-  cnt.resize(NA);
-  aSingStart.resize(NA + 1);
-  k_alpha_singles<false><<<grid_for((size_t)NA * 32, 256), 256, 0, s>>>(ua.p, NA, norb, cnt.p, nullptr, nullptr);
-  SHCI_LAUNCH_CHECK();
-  int64_t total = 0;
-  scan_exclusive_i64(cnt.p, aSingStart.p, NA, &total, pr, s);
-  k_iota_last<<<1, 1, 0, s>>>(aSingStart.p, NA, total);
-  SHCI_LAUNCH_CHECK();
-  aSing.resize(total > 0 ? total : 1);
-  k_alpha_singles<true><<<grid_for((size_t)NA * 32, 256), 256, 0, s>>>(ua.p, NA, norb, nullptr, aSingStart.p,
-                                                                         aSing.p);
-  SHCI_LAUNCH_CHECK();
-  nsing = total;
-  {
-    DevBuf<uint32_t> split;
-    split.resize(total > 0 ? total : 1);
-    aSingMid.resize(NA);
-    k_split_singles<<<grid_for((size_t)NA * 32, 256), 256, 0, s>>>(aSingStart.p, aSing.p, aStart.p, bstr.p, NA,
-                                                                   split.p, aSingMid.p);
-    SHCI_LAUNCH_CHECK();
-    aSing.swap(split);
-  }
-  // partial-string index (one entry per determinant and occupied beta orbital)
-  {
-    DevBuf<int64_t> c1, o1;
-    c1.resize(n);
-    o1.resize(n + 1);
-    k_m1_count<<<grid_for(n, 256), 256, 0, s>>>(bstr.p, n, c1.p);
-    SHCI_LAUNCH_CHECK();
-    int64_t ne = 0;
-    scan_exclusive_i64(c1.p, o1.p, n, &ne, pr, s);
-    if (ne >= ((int64_t)1 << 32)) throw Error(kErrInvalid, "partial-string index too large");
-    if (NA >= ((int64_t)1 << kM1GroupBits)) throw Error(kErrInvalid, "too many alpha strings for the partial-string index");
-    nm1 = ne;
-    if (ne > 0) {
-      DevBuf<uint64_t> key;
-      DevBuf<uint32_t> perm;
-      DevBuf<uint4> raw;
-      key.resize(ne);
-      perm.resize(ne);
-      raw.resize(ne);
-      m1ent.resize(ne);
-      const unsigned eb = grid_for((size_t)ne, 256);
-      k_m1_fill<<<grid_for(n, 256), 256, 0, s>>>(bstr.p, agrp.p, n, o1.p, key.p, perm.p, raw.p);
-      SHCI_LAUNCH_CHECK();
-      sort_u64(key.p, perm.p, (size_t)ne, pr, s);  // by partial string
-      k_m1_group_keys<<<eb, 256, 0, s>>>(raw.p, perm.p, ne, key.p);
-      SHCI_LAUNCH_CHECK();
-      sort_u64(key.p, perm.p, (size_t)ne, pr, s);  // then by alpha group (stable)
-      k_m1_permute<<<eb, 256, 0, s>>>(raw.p, perm.p, ne, m1ent.p);
-      SHCI_LAUNCH_CHECK();
-      // the groups' hash tables
-      DevBuf<uint32_t> nkey;
-      DevBuf<int64_t> slots, first;
-      nkey.resize((size_t)NA);
-      slots.resize((size_t)NA);
-      first.resize((size_t)NA + 1);
-      SHCI_CUDA(cudaMemsetAsync(nkey.p, 0, (size_t)NA * sizeof(uint32_t), s));
-      k_m1_heads<<<eb, 256, 0, s>>>(m1ent.p, ne, nkey.p);
-      SHCI_LAUNCH_CHECK();
-      k_m1_slots<<<grid_for((size_t)NA, 256), 256, 0, s>>>(nkey.p, NA, slots.p);
-      SHCI_LAUNCH_CHECK();
-      int64_t nslot = 0;
-      scan_exclusive_i64(slots.p, first.p, NA, &nslot, pr, s);
-      m1dir.resize((size_t)NA);
-      k_m1_dir<<<grid_for((size_t)NA, 256), 256, 0, s>>>(slots.p, first.p, NA, m1dir.p);
-      SHCI_LAUNCH_CHECK();
-      m1tab.resize((size_t)nslot);
-      SHCI_CUDA(cudaMemsetAsync(m1tab.p, 0xff, (size_t)nslot * sizeof(uint2), s));
-      k_m1_insert<<<eb, 256, 0, s>>>(m1ent.p, ne, m1dir.p, m1tab.p);
-      SHCI_LAUNCH_CHECK();
-    }
-  }
-  SHCI_CUDA(cudaStreamSynchronize(s));
+  if (narrow)
+    build_singles_and_index<uint32_t>(*this, norb, pr, s);
+  else
+    build_singles_and_index<uint64_t>(*this, norb, pr, s);
 }
-
 // ---------------------------------------------------------------------------
 // Row traversal shared by count, emit and the matrix-free sigma. The visitor's
-// v.step(hit, p, cls) is called by all 32 lanes together (p: storage position of
-// a connection), v.end_part(part) after each of the four parts.
+// v.step<part>(hit, single, p) is called by all 32 lanes together: p the storage
+// position of a connection, single whether it is a single excitation.
 // ---------------------------------------------------------------------------
-enum : int { kSingleB = 0, kDoubleBB = 1, kAlpha = 2, kDoubleAA = 3 };  // class of a hit; kAlpha: alpha moved once
+enum : int { kSameAlpha = 1, kAlphaMoved = 2, kSameBeta = 3 };
 
 // One lane's probe of the index: the run of entries of key (group As, bm).
-__device__ __forceinline__ void probe_index(const HelperView& h, uint32_t As, uint64_t bm, uint32_t& lo, int& len) {
+template <class S>
+__device__ __forceinline__ void probe_index(const HelperView<S>& h, uint32_t As, S bm, uint32_t& lo, int& len) {
   const uint64_t d = __ldg(h.m1dir + As);
   const unsigned lg = (unsigned)(d & 63);
   const uint32_t mask = (uint32_t)((1ull << lg) - 1);
   const uint2* tab = h.m1tab + (d >> 6);
   const uint32_t fp = m1_fingerprint(bm);
-  uint32_t q = (uint32_t)m1_slot(bm, lg);
+  uint32_t q = m1_slot(bm, lg);
   for (uint32_t step = 0; step <= mask; ++step) {
     const uint2 sl = __ldg(tab + q);
     if (sl.x == kM1Empty) return;
     if ((sl.y & ((1u << kM1GroupBits) - 1u)) == fp) {
       // a fingerprint match is confirmed on the run's first entry
       const uint2 k0 = __ldg(reinterpret_cast<const uint2*>(h.m1ent + sl.x));
-      if (k0.x == (uint32_t)bm && k0.y == (uint32_t)(bm >> 32)) {
+      if (k0.x == (uint32_t)bm && (sizeof(S) == 4 || k0.y == (uint32_t)((uint64_t)bm >> 32))) {
         lo = sl.x;
         len = (int)(sl.y >> kM1GroupBits) + 1;
         return;
@@ -458,10 +488,11 @@ __device__ __forceinline__ void probe_index(const HelperView& h, uint32_t As, ui
   }
 }
 
-// The k-th set bit of B (k < its population count).
-__device__ __forceinline__ int nth_bit(uint64_t B, int k) {
+// The k-th set bit of B (k < its population count), as a bit.
+template <class S>
+__device__ __forceinline__ S nth_bit(S B, int k) {
   for (int t = 0; t < k; ++t) B &= B - 1;
-  return __ffsll((long long)B) - 1;
+  return low_one(B);
 }
 
 // Owner of flat entry f among the lanes' ranges (excl: first flat entry of each
@@ -486,19 +517,23 @@ __device__ __forceinline__ int warp_incl_sum(int v) {
 }
 
 // Parts 1, 2a and 3: the scans. Each reports its hits in ascending position.
-template <class V>
-__device__ __forceinline__ void scan_same_alpha(const HelperView& h, uint32_t ga, uint64_t B, V& v) {
-  const int lane = threadIdx.x & 31;
+// The next round is loaded before this one is looked at: a round is a few
+// instructions behind an L2 latency. (Four rounds at a time put the visitor's
+// code in four places, and the matrix-free sigma waited for instructions.)
+template <class S, class V>
+__device__ __forceinline__ void scan_same_alpha(const HelperView<S>& h, uint32_t ga, S B, V& v) {
   const uint32_t p1 = (uint32_t)h.aStart[ga + 1];
-  for (uint32_t base = (uint32_t)h.aStart[ga]; base < p1; base += 32) {
-    const uint32_t p = base + lane;
-    int d = -1;
-    if (p < p1) d = __popcll(h.bstr[p] ^ B);
-    v.step(d == 2 || d == 4, p, d == 2 ? kSingleB : kDoubleBB);
+  uint32_t p = (uint32_t)h.aStart[ga] + (threadIdx.x & 31);
+  S b = p < p1 ? h.bstr[p] : B;  // B itself: distance 0, no hit
+  for (uint32_t base = p - (threadIdx.x & 31); base < p1; base += 32, p += 32) {
+    const S nb = p + 32 < p1 ? h.bstr[p + 32] : B;
+    const int d = bit_count((S)(b ^ B));
+    v.template step<kSameAlpha>(d == 2 || d == 4, d == 2, p);
+    b = nb;
   }
 }
-template <class V>
-__device__ __forceinline__ void scan_small_groups(const HelperView& h, int64_t s0, int64_t smid, uint64_t B, V& v) {
+template <class S, class V>
+__device__ __forceinline__ void scan_small_groups(const HelperView<S>& h, int64_t s0, int64_t smid, S B, V& v) {
   const int lane = threadIdx.x & 31;
   for (int64_t base = s0; base < smid; base += 32) {
     uint32_t g0 = 0;
@@ -512,49 +547,58 @@ __device__ __forceinline__ void scan_small_groups(const HelperView& h, int64_t s
     const int total = __shfl_sync(kFull, incl, 31);
     const int excl = incl - len;
     const uint32_t off = g0 - (uint32_t)excl;  // position of flat entry f: off of its owner + f
-    for (int f0 = 0; f0 < total; f0 += 32) {
-      const int f = f0 + lane;
-      const uint32_t p = __shfl_sync(kFull, off, flat_owner(excl, f)) + (uint32_t)f;
-      bool hit = false;
-      if (f < total) hit = __popcll(h.bstr[p] ^ B) <= 2;
-      v.step(hit, p, kAlpha);
+    uint32_t p = 0, np = 0;
+    S b = (S)~B, nb = (S)~B;  // ~B: no orbital in common, no hit
+    for (int f0 = -32; f0 < total; f0 += 32) {
+      const int f = f0 + 32 + lane;
+      nb = (S)~B;
+      if (f0 + 32 < total) {
+        np = __shfl_sync(kFull, off, flat_owner(excl, f)) + (uint32_t)f;
+        if (f < total) nb = h.bstr[np];
+      }
+      if (f0 >= 0) {
+        const int d = bit_count((S)(b ^ B));
+        v.template step<kAlphaMoved>(d <= 2, d == 0, p);
+      }
+      p = np;
+      b = nb;
     }
   }
 }
-template <class V>
-__device__ __forceinline__ void scan_same_beta(const HelperView& h, uint32_t gb, uint64_t A, V& v) {
-  const int lane = threadIdx.x & 31;
+template <class S, class V>
+__device__ __forceinline__ void scan_same_beta(const HelperView<S>& h, uint32_t gb, S A, V& v) {
   const uint32_t q1 = (uint32_t)h.bStart[gb + 1];
-  for (uint32_t base = (uint32_t)h.bStart[gb]; base < q1; base += 32) {
-    const uint32_t q = base + lane;
-    bool hit = false;
-    uint32_t p = 0;
-    if (q < q1) {
-      hit = __popcll(h.bAlpha[q] ^ A) == 4;
-      p = h.bPos[q];
-    }
-    v.step(hit, p, kDoubleAA);
+  uint32_t q = (uint32_t)h.bStart[gb] + (threadIdx.x & 31);
+  S a = q < q1 ? h.bAlpha[q] : A;
+  uint32_t p = q < q1 ? h.bPos[q] : 0u;
+  for (uint32_t base = q - (threadIdx.x & 31); base < q1; base += 32, q += 32) {
+    const bool more = q + 32 < q1;
+    const S na = more ? h.bAlpha[q + 32] : A;
+    const uint32_t np = more ? h.bPos[q + 32] : 0u;
+    v.template step<kSameBeta>(bit_count((S)(a ^ A)) == 4, false, p);
+    a = na;
+    p = np;
   }
 }
 
 // Part 2b in no particular order: probes t = (group, occupied beta orbital)
 // 32 at a time, each lane stepping its own pair (no division per probe).
-template <class V>
-__device__ __forceinline__ void probe_large_groups(const HelperView& h, int64_t smid, int64_t s1, uint64_t B, V& v) {
+template <class S, class V>
+__device__ __forceinline__ void probe_large_groups(const HelperView<S>& h, int64_t smid, int64_t s1, S B, V& v) {
   const int lane = threadIdx.x & 31;
-  const int nb = __popcll(B);
+  const int nb = bit_count(B);
   const int nprobe = (int)(s1 - smid) * nb;
   if (nprobe == 0) return;
-  const int occ_k = lane < nb ? nth_bit(B, lane) : 0;  // orbitals beyond the 32nd are found bit by bit
+  const int occ_k = lane < nb ? bit_index(nth_bit(B, lane)) : 0;  // orbitals beyond the 32nd are found bit by bit
   const int step_q = 32 / nb, step_r = 32 % nb;
   int sidx = lane / nb, which = lane % nb;
   for (int base = 0; base < nprobe; base += 32) {
     uint32_t lo = 0;
     int len = 0;  // at most 64: one entry per beta orbital outside the key
     int bq = __shfl_sync(kFull, occ_k, which & 31);  // the beta orbital removed by this probe
-    if (which >= 32) bq = nth_bit(B, which);
+    if (sizeof(S) == 8 && which >= 32) bq = bit_index(nth_bit(B, which));
     const uint32_t tag = (uint32_t)bq | (which == 0 ? 256u : 0u);
-    if (base + lane < nprobe) probe_index(h, h.aSing[smid + sidx], B ^ (1ull << bq), lo, len);
+    if (base + lane < nprobe) probe_index(h, h.aSing[smid + sidx], (S)(B ^ ((S)1 << bq)), lo, len);
     which += step_r;
     sidx += step_q;
     if (which >= nb) {
@@ -571,7 +615,7 @@ __device__ __forceinline__ void probe_large_groups(const HelperView& h, int64_t 
       const int src = flat_owner(excl, f);
       const uint32_t e = __shfl_sync(kFull, off, src) + (uint32_t)f;
       const uint32_t tg = __shfl_sync(kFull, tag, src);
-      bool hit = false;
+      bool hit = false, equal = false;
       uint32_t p = 0;
       if (f < total) {
         // the entry holds J and the orbital b' its beta string has beyond
@@ -579,15 +623,16 @@ __device__ __forceinline__ void probe_large_groups(const HelperView& h, int64_t 
         // for the first), otherwise a beta single excitation b -> b'
         const uint2 en = __ldg(reinterpret_cast<const uint2*>(h.m1ent + e) + 1);
         p = en.y;
-        hit = (en.x >> kM1GroupBits) != (tg & 255u) || (tg & 256u);
+        equal = (en.x >> kM1GroupBits) == (tg & 255u);
+        hit = !equal || (tg & 256u);
       }
-      v.step(hit, p, kAlpha);
+      v.template step<kAlphaMoved>(hit, equal, p);
     }
   }
 }
 
-template <class V>
-__device__ __forceinline__ void visit_row(const HelperView& h, uint32_t p, uint64_t A, uint64_t B, V& v) {
+template <class S, class V>
+__device__ __forceinline__ void visit_row(const HelperView<S>& h, uint32_t p, S A, S B, V& v) {
   const uint32_t ga = h.agrp[p];
   scan_same_alpha(h, ga, B, v);
   const int64_t s0 = h.aSingStart[ga], s1 = h.aSingStart[ga + 1];
@@ -599,7 +644,10 @@ __device__ __forceinline__ void visit_row(const HelperView& h, uint32_t p, uint6
 
 struct CountVisitor {
   int c = 0;
-  __device__ void step(bool hit, uint32_t, int) { c += hit; }
+  template <int part>
+  __device__ __forceinline__ void step(bool hit, bool, uint32_t) {
+    c += hit;
+  }
 };
 __device__ __forceinline__ int warp_total(int c) {
 #pragma unroll
@@ -611,14 +659,15 @@ __device__ __forceinline__ int warp_total(int c) {
 // The index is only probed: a key's run holds the determinants one beta
 // excitation away, and J with B itself (in every run of its group, to be
 // counted once), which the run of the first probe shows.
-__global__ void __launch_bounds__(256) k_ham_count(HelperView h, const uint32_t* __restrict__ rows, int64_t nr,
+template <class S>
+__global__ void __launch_bounds__(256) k_ham_count(HelperView<S> h, const uint32_t* __restrict__ rows, int64_t nr,
                                                    uint4* __restrict__ parts, int64_t* __restrict__ counts) {
   const int lane = threadIdx.x & 31;
   const int64_t warps = (int64_t)gridDim.x * (blockDim.x >> 5);
   for (int64_t k = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; k < nr; k += warps) {
     const uint32_t p = rows ? rows[k] : (uint32_t)k;
-    const ulonglong2 I = h.str[p];
-    const uint64_t A = I.x, B = I.y;
+    const auto I = h.str[p];
+    const S A = I.x, B = I.y;
     const uint32_t ga = h.agrp[p];
     CountVisitor v1, v2, v3;
     scan_same_alpha(h, ga, B, v1);
@@ -626,19 +675,19 @@ __global__ void __launch_bounds__(256) k_ham_count(HelperView h, const uint32_t*
     const int64_t smid = (h.m1ent != nullptr && B != 0) ? h.aSingMid[ga] : s1;
     scan_small_groups(h, s0, smid, B, v2);
     int c4 = 0;
-    const int nb = __popcll(B);
+    const int nb = bit_count(B);
     const int nprobe = (int)(s1 - smid) * nb;
     if (nprobe > 0) {
-      const int occ_k = lane < nb ? nth_bit(B, lane) : 0;
+      const int occ_k = lane < nb ? bit_index(nth_bit(B, lane)) : 0;
       const int step_q = 32 / nb, step_r = 32 % nb;
       int sidx = lane / nb, which = lane % nb;
       for (int base = 0; base < nprobe; base += 32) {
         int bq = __shfl_sync(kFull, occ_k, which & 31);
-        if (which >= 32) bq = nth_bit(B, which);
+        if (sizeof(S) == 8 && which >= 32) bq = bit_index(nth_bit(B, which));
         if (base + lane < nprobe) {
           uint32_t lo = 0;
           int len = 0;
-          probe_index(h, h.aSing[smid + sidx], B ^ (1ull << bq), lo, len);
+          probe_index(h, h.aSing[smid + sidx], (S)(B ^ ((S)1 << bq)), lo, len);
           c4 += len;
           if (which == 0)
             for (int e = 0; e < len; ++e)
@@ -667,51 +716,53 @@ __global__ void __launch_bounds__(256) k_ham_count(HelperView h, const uint32_t*
 // Writes the columns of each row as four ascending runs (the parts in the order
 // of k_ham_count). The scans' hits come in ascending order. The index's do
 // not: the hits of 32 / |B| groups are collected in shared memory and ranked
-// by counting (some 25 per collection); groups that hold more hits than fit
-// are scanned instead. Bound by instruction issue and the L2 latency of the
-// probes; no element is evaluated here, so 8 blocks fit an SM.
+// by counting (some 40 per collection); groups that hold more hits than fit
+// are scanned instead. Bound by instruction issue (68 %) and the L2 latency of
+// the probes.
 constexpr int kCollect = 256;
-__global__ void __launch_bounds__(256) k_ham_emit(HelperView h, const uint32_t* __restrict__ rows, int64_t nr,
+struct AppendVisitor {
+  int32_t* col;
+  int64_t pos;
+  unsigned lt;
+  template <int part>
+  __device__ __forceinline__ void step(bool hit, bool, uint32_t p) {
+    const unsigned m = __ballot_sync(kFull, hit);
+    if (hit) col[pos + __popc(m & lt)] = (int32_t)p;
+    pos += __popc(m);
+  }
+};
+template <class S>
+__global__ void __launch_bounds__(256) k_ham_emit(HelperView<S> h, const uint32_t* __restrict__ rows, int64_t nr,
                                                   const int64_t* __restrict__ rowptr, int32_t* __restrict__ col) {
   __shared__ __align__(16) uint32_t s_buf[8][kCollect];
   const int lane = threadIdx.x & 31;
   const unsigned lt = (1u << lane) - 1u;
   uint32_t* buf = s_buf[threadIdx.x >> 5];
   const int64_t warps = (int64_t)gridDim.x * (blockDim.x >> 5);
-  struct Append {
-    int32_t* col;
-    int64_t pos;
-    unsigned lt;
-    __device__ void step(bool hit, uint32_t p, int) {
-      const unsigned m = __ballot_sync(kFull, hit);
-      if (hit) col[pos + __popc(m & lt)] = (int32_t)p;
-      pos += __popc(m);
-    }
-  };
   for (int64_t k = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; k < nr; k += warps) {
     const uint32_t p = rows ? rows[k] : (uint32_t)k;
-    const ulonglong2 I = h.str[p];
-    const uint64_t A = I.x, B = I.y;
+    const auto I = h.str[p];
+    const S A = I.x, B = I.y;
     const uint32_t ga = h.agrp[p];
-    Append v{col, rowptr[k], lt};
+    AppendVisitor v{col, rowptr[k], lt};
     scan_same_alpha(h, ga, B, v);
     const int64_t s0 = h.aSingStart[ga], s1 = h.aSingStart[ga + 1];
     const int64_t smid = (h.m1ent != nullptr && B != 0) ? h.aSingMid[ga] : s1;
     scan_small_groups(h, s0, smid, B, v);
     if (smid < s1) {
-      const int nb = __popcll(B);
+      const int nb = bit_count(B);
       const int per = nb <= 32 ? 32 / nb : 1;  // groups per collection
       const int mine = nb <= 32 ? lane / nb : 0, which0 = nb <= 32 ? lane % nb : lane;
-      const int bq0 = which0 < nb ? nth_bit(B, which0) : 0;
+      const int bq0 = which0 < nb ? bit_index(nth_bit(B, which0)) : 0;
       for (int64_t s = smid; s < s1; s += per) {
         int n = 0;
         bool over = false;
         for (int w = 0; w < nb; w += 32) {  // more than one round only past 32 beta electrons
           const int which = which0 + w;
-          const int bq = w == 0 ? bq0 : (which < nb ? nth_bit(B, which) : 0);
+          const int bq = sizeof(S) == 4 || w == 0 ? bq0 : (which < nb ? bit_index(nth_bit(B, which)) : 0);
           uint32_t lo = 0;
           int len = 0;
-          if (mine < per && which < nb && s + mine < s1) probe_index(h, h.aSing[s + mine], B ^ (1ull << bq), lo, len);
+          if (mine < per && which < nb && s + mine < s1) probe_index(h, h.aSing[s + mine], (S)(B ^ ((S)1 << bq)), lo, len);
           const uint32_t tag = (uint32_t)bq | (which == 0 ? 256u : 0u);
           const int incl = warp_incl_sum(len);
           const int total = __shfl_sync(kFull, incl, 31);
@@ -769,52 +820,73 @@ __global__ void __launch_bounds__(256) k_ham_emit(HelperView h, const uint32_t* 
 // stand ((ai|ii) - (ai|ii) for the orbital left behind).
 // ---------------------------------------------------------------------------
 // Integral access in either precision (FP64: __dsub_rn, so never contracted).
+__device__ __forceinline__ int pair_of(int lo, int hi) { return hi * (hi + 1) / 2 + lo; }  // lo <= hi
 template <bool F32>
 struct Elem;
 template <>
 struct Elem<false> {
   using T = double;
-  __device__ static T i2(const IntsView& v, int i, int j, int k, int l) { return i2_spatial(v.I2, i, j, k, l); }
+  __device__ static T i2(const IntsView& v, int ij, int kl) {
+    const unsigned A = (unsigned)max(ij, kl), B = (unsigned)min(ij, kl);
+    return __ldg(v.I2 + (A * (A + 1) / 2 + B));
+  }
   __device__ static T sub(T a, T b) { return __dsub_rn(a, b); }
   __device__ static T signed_(T v, unsigned odd) {
-    return __longlong_as_double(__double_as_longlong(v) ^ ((long long)odd << 63));
+    return __hiloint2double(__double2hiint(v) ^ (int)(odd << 31), __double2loint(v));
   }
   __device__ static T single(const IntsView& v, const Det2& d, int a, int i) { return hij_single(v, d, a, i); }
 };
 template <>
 struct Elem<true> {
   using T = float;
-  __device__ static T i2(const IntsView& v, int i, int j, int k, int l) { return i2f_spatial(v.I2f, i, j, k, l); }
+  __device__ static T i2(const IntsView& v, int ij, int kl) {
+    const unsigned A = (unsigned)max(ij, kl), B = (unsigned)min(ij, kl);
+    return __ldg(v.I2f + (A * (A + 1) / 2 + B));
+  }
   __device__ static T sub(T a, T b) { return __fsub_rn(a, b); }
   __device__ static T signed_(T v, unsigned odd) { return __uint_as_float(__float_as_uint(v) ^ (odd << 31)); }
   __device__ static T single(const IntsView& v, const Det2& d, int a, int i) { return hij_single_f32(v, d, a, i); }
 };
 // alpha and beta moved once each
-template <bool F32>
-__device__ __forceinline__ typename Elem<F32>::T elem_ab(const IntsView& v, uint64_t A, uint64_t B, uint64_t A2,
-                                                         uint64_t B2) {
-  const uint64_t x = A ^ A2, y = B ^ B2;
-  const int i = low_bit(x & A), a = low_bit(x & A2), j = low_bit(y & B), b = low_bit(y & B2);
-  const unsigned odd = __popcll(passed<0>(A, B, i, a) ^ passed<1>(B, A2, j, b)) & 1;
-  return Elem<F32>::signed_(Elem<F32>::i2(v, a, i, b, j), odd);
+template <bool F32, class S>
+__device__ __forceinline__ typename Elem<F32>::T elem_ab(const IntsView& v, S A, S B, S A2, S B2) {
+  const S x = A ^ A2, y = B ^ B2;
+  const unsigned odd = bit_count((S)(passed(A, B, x, false) ^ passed(B, A2, y, true))) & 1;
+  const S xl = low_one(x), yl = low_one(y);  // a pair's index does not depend on which of the two was occupied
+  return Elem<F32>::signed_(Elem<F32>::i2(v, pair_of(bit_index(xl), bit_index((S)(x ^ xl))),
+                                          pair_of(bit_index(yl), bit_index((S)(y ^ yl)))),
+                            odd);
 }
-// two electrons of one spin moved: S -> S2, the other string O
-template <bool F32, int kSpin>
-__device__ __forceinline__ typename Elem<F32>::T elem_same(const IntsView& v, uint64_t S, uint64_t O, uint64_t S2) {
-  const uint64_t x = S ^ S2, d = x & S, c = x & S2;
-  const int i = low_bit(d), j = low_bit(d & (d - 1)), a = low_bit(c), b = low_bit(c & (c - 1));
-  const uint64_t S1 = S ^ (1ull << i) ^ (1ull << a);
-  const unsigned odd = __popcll(passed<kSpin>(S, O, i, a) ^ passed<kSpin>(S1, O, j, b)) & 1;
-  return Elem<F32>::signed_(Elem<F32>::sub(Elem<F32>::i2(v, a, i, b, j), Elem<F32>::i2(v, a, j, b, i)), odd);
+// the same as FP32 head and tail (exactly those of the FP64 value: the sign
+// changes neither rounding)
+template <class S>
+__device__ __forceinline__ float2 elem_ab_split(const IntsView& v, S A, S B, S A2, S B2) {
+  const S x = A ^ A2, y = B ^ B2;
+  const unsigned odd = bit_count((S)(passed(A, B, x, false) ^ passed(B, A2, y, true))) & 1;
+  const S xl = low_one(x), yl = low_one(y);
+  const int ij = pair_of(bit_index(xl), bit_index((S)(x ^ xl))), kl = pair_of(bit_index(yl), bit_index((S)(y ^ yl)));
+  const unsigned P = (unsigned)max(ij, kl), Q = (unsigned)min(ij, kl);
+  const float2 t = __ldg(v.I2ff + (P * (P + 1) / 2 + Q));
+  return make_float2(__uint_as_float(__float_as_uint(t.x) ^ (odd << 31)),
+                     __uint_as_float(__float_as_uint(t.y) ^ (odd << 31)));
 }
-// one electron moved: S -> S2 of spin sp
-template <bool F32>
-__device__ __noinline__ typename Elem<F32>::T elem_single(const double* I1, const double* V1, const float* I1f,
-                                                          const float* V1f, int norb, uint64_t A, uint64_t B,
-                                                          uint64_t S, uint64_t S2, int sp) {
-  const IntsView v{I1, nullptr, nullptr, nullptr, norb, I1f, nullptr, V1, V1f};
-  const uint64_t x = S ^ S2;
-  return Elem<F32>::single(v, det_from_strings(A, B), 2 * low_bit(x & S2) + sp, 2 * low_bit(x & S) + sp);
+// two electrons of one spin moved: s -> s2, the other string o
+template <bool F32, class S>
+__device__ __forceinline__ typename Elem<F32>::T elem_same(const IntsView& v, S s, S o, S s2, bool beta) {
+  const S x = s ^ s2, d = x & s, c = x ^ d;
+  const S di = low_one(d), dj = d ^ di, ca = low_one(c), cb = c ^ ca;
+  const unsigned odd = bit_count((S)(passed(s, o, (S)(di | ca), beta) ^ passed((S)(s ^ di ^ ca), o, (S)(dj | cb), beta))) & 1;
+  const int i = bit_index(di), j = bit_index(dj), a = bit_index(ca), b = bit_index(cb);
+  return Elem<F32>::signed_(Elem<F32>::sub(Elem<F32>::i2(v, pair_index(a, i), pair_index(b, j)),
+                                           Elem<F32>::i2(v, pair_index(a, j), pair_index(b, i))),
+                            odd);
+}
+// one electron moved: s -> s2 of a determinant with strings A and B
+template <bool F32, class S>
+__device__ __forceinline__ typename Elem<F32>::T elem_single(const IntsView& v, S A, S B, S s, S s2, bool beta) {
+  const S x = s ^ s2;
+  return Elem<F32>::single(v, det_from_strings((uint64_t)A, (uint64_t)B), 2 * bit_index((S)(x & s2)) + (beta ? 1 : 0),
+                           2 * bit_index((S)(x & s)) + (beta ? 1 : 0));
 }
 
 // ---------------------------------------------------------------------------
@@ -824,11 +896,12 @@ __device__ __noinline__ typename Elem<F32>::T elem_single(const double* I1, cons
 // alpha string) is one range of positions that no other run enters, so only
 // the other two runs are searched. Evaluating here, and not where a connection
 // is found, keeps the walk's registers free of the element code and puts
-// every lane on an element. 405,690 rows, 5.5e8 entries (mol24, mixed, full and
-// new rows): emitting with evaluation 27.9 ms and sorting each row 30.7 ms.
+// every lane on an element. 5.5e8 entries (mol24, mixed: the spaces of 81,233
+// and 405,690 determinants): emitting 12.7 ms, finishing 12.9 ms; emitting with
+// evaluation and sorting each row by a bitonic network took 58.6 ms for 3.6e8.
 // ---------------------------------------------------------------------------
 constexpr int kRunCap = 3072;  // entries of a row kept in shared memory
-constexpr int kFinThreads = 128;
+constexpr int kFinThreads = 128;  // 64: 15.4 ms, 96: 12.9 ms, 128: 11.4 ms for 5.5e8 entries
 
 __device__ __forceinline__ int run_below(const uint32_t* run, int n, uint32_t c) {  // entries of a run below c
   int lo = 0, hi = n;
@@ -842,7 +915,10 @@ __device__ __forceinline__ int run_below(const uint32_t* run, int n, uint32_t c)
   return lo;
 }
 
-// Where a row's entries go.
+// Where a row's entries go. Mixed values are an FP32 head and tail; an
+// alpha-beta double's come from a table of split integrals, since the two
+// conversions and the subtraction would take the FP64 pipe (two lanes per
+// clock and SM) 64 clocks per 32 entries.
 struct FinishOut {
   int32_t* __restrict__ col;
   double* __restrict__ v64;
@@ -857,16 +933,21 @@ struct FinishOut {
       if (vlo) vlo[q] = (float)(v - (double)hi);
     }
   }
+  __device__ __forceinline__ void put(int64_t q, float2 v) const {
+    vhi[q] = v.x;
+    if (vlo) vlo[q] = v.y;
+  }
 };
 
 // Single excitations wait per warp, over rows, until 32 are there: their
 // elements are sums over every electron in FP64 (two lanes per clock and SM),
 // and one among a warp's 32 entries would make the whole warp run the sum.
 // Entry: place (64 bits), position of the row, of the column.
+template <class S>
 struct SingleQueue {
   uint4* q;  // 64 entries
   int n = 0;
-  __device__ __forceinline__ void push(bool s, int64_t at, uint32_t p, uint32_t c, const HelperView& h,
+  __device__ __forceinline__ void push(bool s, int64_t at, uint32_t p, uint32_t c, const HelperView<S>& h,
                                        const IntsView& ints, const FinishOut& out) {
     const unsigned m = __ballot_sync(kFull, s);
     if (!m) return;
@@ -875,15 +956,14 @@ struct SingleQueue {
     __syncwarp();
     if (n >= 32) drain(32, h, ints, out);
   }
-  __device__ __forceinline__ void drain(int cnt, const HelperView& h, const IntsView& ints, const FinishOut& out) {
+  __device__ __forceinline__ void drain(int cnt, const HelperView<S>& h, const IntsView& ints, const FinishOut& out) {
     const int lane = threadIdx.x & 31;
     if (lane < cnt) {
       const uint4 w = q[lane];
-      const ulonglong2 I = h.str[w.z], J = h.str[w.w];
+      const auto I = h.str[w.z], J = h.str[w.w];
       const bool beta = I.x == J.x;
       out.put((int64_t)(((uint64_t)w.y << 32) | w.x),
-              elem_single<false>(ints.I1, ints.V1, nullptr, nullptr, ints.norb, I.x, I.y, beta ? I.y : I.x,
-                                 beta ? J.y : J.x, beta));
+              elem_single<false, S>(ints, I.x, I.y, beta ? I.y : I.x, beta ? J.y : J.x, beta));
     }
     __syncwarp();
     const int rest = n - cnt;
@@ -895,50 +975,65 @@ struct SingleQueue {
   }
 };
 
-__device__ __forceinline__ void finish_row(const HelperView& h, const IntsView& ints, uint32_t p, const uint4& n,
-                                           const uint32_t* run, int64_t p0, const FinishOut& out, SingleQueue& sq) {
-  const ulonglong2 I = h.str[p];
-  const uint64_t A = I.x, B = I.y;
+template <class S, bool kSplit>
+__device__ __forceinline__ void finish_row(const HelperView<S>& h, const IntsView& ints, uint32_t p, const uint4& n,
+                                           const uint32_t* run, int64_t p0, const FinishOut& out, SingleQueue<S>& sq) {
+  const auto I = h.str[p];
+  const S A = I.x, B = I.y;
   const int n1 = (int)n.x, n2 = (int)n.y, n3 = (int)n.z, n4 = (int)n.w;
   const uint32_t *r2 = run + n1, *r3 = r2 + n2, *r4 = r3 + n3;
   const int len = n1 + n2 + n3 + n4;
-  for (int e0 = 0; e0 < len; e0 += blockDim.x) {  // all lanes together: the queue's ballots
-    const int e = e0 + (int)threadIdx.x;
-    bool single = false;
-    uint32_t c = 0;
-    int64_t q = 0;
-    if (e < len) {
-      c = run[e];
-      const ulonglong2 J = h.str[c];
-      int rank;
-      double v = 0.0;
-      if (e < n1) {
-        rank = e + run_below(r2, n2, c) + run_below(r3, n3, c) + run_below(r4, n4, c);
-        single = __popcll(B ^ J.y) == 2;
-        if (!single) v = elem_same<false, 1>(ints, B, A, J.y);
+  // kTwo entries of a thread at a time: their strings and integrals are in
+  // flight together. All lanes together: the queue's ballots.
+  constexpr int kTwo = 2;
+  for (int e0 = 0; e0 < len; e0 += kTwo * blockDim.x) {
+    bool single[kTwo];
+    uint32_t c[kTwo];
+    int64_t q[kTwo];
+    typename StrPair<S>::T J[kTwo];
+#pragma unroll
+    for (int u = 0; u < kTwo; ++u) {
+      const int e = e0 + u * (int)blockDim.x + (int)threadIdx.x;
+      single[u] = false;
+      c[u] = e < len ? run[e] : p;
+      J[u] = h.str[c[u]];
+    }
+#pragma unroll
+    for (int u = 0; u < kTwo; ++u) {
+      const int e = e0 + u * (int)blockDim.x + (int)threadIdx.x;
+      if (e >= len) continue;
+      // the two other runs to be searched (run 1: all three)
+      const bool in1 = e < n1, in2 = !in1 && e < n1 + n2, in4 = e >= n1 + n2 + n3;
+      const bool first = !in2, last = in2 || (!in1 && !in4);  // run 2 is searched first; run 4 last (else run 3)
+      int rank = e + run_below(first ? r2 : r3, first ? n2 : n3, c[u]) + run_below(last ? r4 : r3, last ? n4 : n3, c[u]);
+      if (in1)
+        rank += run_below(r4, n4, c[u]);
+      else
+        rank -= (n1 > 0 && c[u] > run[0] ? 0 : n1) + (in2 ? 0 : in4 ? n2 + n3 : n2);
+      q[u] = p0 + rank;
+      out.col[q[u]] = (int32_t)c[u];
+      if (in1 || in4) {  // same alpha or same beta string
+        const bool beta = in1;
+        single[u] = beta && bit_count((S)(B ^ J[u].y)) == 2;
+        if (!single[u])
+          out.put(q[u], elem_same<false, S>(ints, beta ? B : A, beta ? A : B, beta ? J[u].y : J[u].x, beta));
       } else {
-        rank = n1 > 0 && c > run[0] ? n1 : 0;
-        if (e >= n1 + n2 + n3) {
-          rank += e - (n1 + n2 + n3) + run_below(r2, n2, c) + run_below(r3, n3, c);
-          v = elem_same<false, 0>(ints, A, B, J.x);
-        } else {
-          if (e >= n1 + n2)
-            rank += e - (n1 + n2) + run_below(r2, n2, c) + run_below(r4, n4, c);
+        single[u] = J[u].y == B;
+        if (!single[u]) {
+          if constexpr (kSplit)
+            out.put(q[u], elem_ab_split<S>(ints, A, B, J[u].x, J[u].y));
           else
-            rank += e - n1 + run_below(r3, n3, c) + run_below(r4, n4, c);
-          single = J.y == B;
-          if (!single) v = elem_ab<false>(ints, A, B, J.x, J.y);
+            out.put(q[u], elem_ab<false, S>(ints, A, B, J[u].x, J[u].y));
         }
       }
-      q = p0 + rank;
-      out.col[q] = (int32_t)c;
-      if (!single) out.put(q, v);
     }
-    sq.push(single, q, p, c, h, ints, out);
+#pragma unroll
+    for (int u = 0; u < kTwo; ++u) sq.push(single[u], q[u], p, c[u], h, ints, out);
   }
 }
 
-__global__ void __launch_bounds__(kFinThreads) k_ham_finish(HelperView h, IntsView ints,
+template <class S, bool kSplit>
+__global__ void __launch_bounds__(kFinThreads) k_ham_finish(HelperView<S> h, IntsView ints,
                                                             const uint32_t* __restrict__ rows, int64_t nr,
                                                             const uint4* __restrict__ parts,
                                                             const int64_t* __restrict__ rowptr,
@@ -947,14 +1042,14 @@ __global__ void __launch_bounds__(kFinThreads) k_ham_finish(HelperView h, IntsVi
   __shared__ uint32_t run[kRunCap];
   __shared__ uint4 s_q[kFinThreads / 32][64];
   const FinishOut out{col, v64, vhi, vlo};
-  SingleQueue sq{s_q[threadIdx.x >> 5]};
+  SingleQueue<S> sq{s_q[threadIdx.x >> 5]};
   for (int64_t k = blockIdx.x; k < nr; k += gridDim.x) {
     const int64_t p0 = rowptr[k];
     const int len = (int)(rowptr[k + 1] - p0);
     if (len == 0 || len > kRunCap) continue;  // uniform across the block
     for (int e = threadIdx.x; e < len; e += blockDim.x) run[e] = (uint32_t)col[p0 + e];
     __syncthreads();
-    finish_row(h, ints, rows ? rows[k] : (uint32_t)k, parts[k], run, p0, out, sq);
+    finish_row<S, kSplit>(h, ints, rows ? rows[k] : (uint32_t)k, parts[k], run, p0, out, sq);
     __syncthreads();
   }
   if (sq.n) sq.drain(sq.n, h, ints, out);
@@ -971,7 +1066,8 @@ __global__ void k_long_runs(const int64_t* __restrict__ rowptr, int64_t nr, uint
     if (i < cap) list[i] = make_uint2((uint32_t)k, (uint32_t)off);
   }
 }
-__global__ void __launch_bounds__(1024) k_ham_finish_long(HelperView h, IntsView ints,
+template <class S, bool kSplit>
+__global__ void __launch_bounds__(1024) k_ham_finish_long(HelperView<S> h, IntsView ints,
                                                           const uint32_t* __restrict__ rows,
                                                           const uint2* __restrict__ list, uint32_t* scratch,
                                                           const uint4* __restrict__ parts,
@@ -980,14 +1076,14 @@ __global__ void __launch_bounds__(1024) k_ham_finish_long(HelperView h, IntsView
                                                           float* __restrict__ vhi, float* __restrict__ vlo) {
   __shared__ uint4 s_q[32][64];
   const FinishOut out{col, v64, vhi, vlo};
-  SingleQueue sq{s_q[threadIdx.x >> 5]};
+  SingleQueue<S> sq{s_q[threadIdx.x >> 5]};
   const uint2 l = list[blockIdx.x];
   const int64_t p0 = rowptr[l.x];
   const int len = (int)(rowptr[l.x + 1] - p0);
   uint32_t* run = scratch + 32 * (size_t)l.y;
   for (int e = threadIdx.x; e < len; e += blockDim.x) run[e] = (uint32_t)col[p0 + e];
   __syncthreads();
-  finish_row(h, ints, rows ? rows[l.x] : l.x, parts[l.x], run, p0, out, sq);
+  finish_row<S, kSplit>(h, ints, rows ? rows[l.x] : l.x, parts[l.x], run, p0, out, sq);
   if (sq.n) sq.drain(sq.n, h, ints, out);
 }
 
@@ -1241,18 +1337,19 @@ static void sort_rows(const int64_t* rowptr, size_t n, const CsrVals& v, cudaStr
 
 // Full rows of nr positions (rows[k], or all when null) into (rowptr, vals),
 // columns ascending; returns nnz.
-static int64_t emit_rows(const Helpers& hp, const uint32_t* rows, size_t nr, const IntsView& ints,
+template <class S>
+static int64_t emit_rows_as(const Helpers& hp, const uint32_t* rows, size_t nr, const IntsView& ints,
                          DevBuf<int64_t>& rowptr, DevBuf<int32_t>& col, DevBuf<double>& v64, DevBuf<float>& vhi,
                          DevBuf<float>& vlo, bool want64, bool want32, bool want_lo, Prims& pr, cudaStream_t s,
                          PhaseTimer& pt) {
-  HelperView hv = hp.view();
+  HelperView<S> hv = hp.view<S>();
   DevBuf<int64_t> counts;
   DevBuf<uint4> parts;
   counts.resize(nr > 0 ? nr : 1);
   parts.resize(nr > 0 ? nr : 1);
   const unsigned blocks = grid_for(nr * 32, 256, 152 * 16);
   if (nr) {
-    k_ham_count<<<blocks, 256, 0, s>>>(hv, rows, (int64_t)nr, parts.p, counts.p);
+    k_ham_count<S><<<blocks, 256, 0, s>>>(hv, rows, (int64_t)nr, parts.p, counts.p);
     SHCI_LAUNCH_CHECK();
   }
   pt.mark("ham count");
@@ -1267,7 +1364,7 @@ static int64_t emit_rows(const Helpers& hp, const uint32_t* rows, size_t nr, con
   if (want32) vhi.resize(cap); else vhi.release();
   if (want32 && want_lo) vlo.resize(cap); else vlo.release();
   if (total == 0) return 0;
-  k_ham_emit<<<blocks, 256, 0, s>>>(hv, rows, (int64_t)nr, rowptr.p, col.p);
+  k_ham_emit<S><<<blocks, 256, 0, s>>>(hv, rows, (int64_t)nr, rowptr.p, col.p);
   SHCI_LAUNCH_CHECK();
   pt.mark("ham emit");
   double* d64 = want64 ? v64.p : nullptr;
@@ -1282,8 +1379,14 @@ static int64_t emit_rows(const Helpers& hp, const uint32_t* rows, size_t nr, con
   SHCI_CUDA(cudaMemsetAsync(tot.p, 0, 2 * sizeof(unsigned long long), s));
   k_long_runs<<<grid_for(nr, 256), 256, 0, s>>>(rowptr.p, (int64_t)nr, list.p, (uint32_t)ncap, tot.p);
   SHCI_LAUNCH_CHECK();
-  k_ham_finish<<<(unsigned)std::min<size_t>(nr, 152 * 16), kFinThreads, 0, s>>>(hv, ints, rows, (int64_t)nr, parts.p,
-                                                                               rowptr.p, col.p, d64, dhi, dlo);
+  const bool split = want32 && ints.I2ff != nullptr;
+  const unsigned fb = (unsigned)std::min<size_t>(nr, 152 * 16);
+  if (split)
+    k_ham_finish<S, true><<<fb, kFinThreads, 0, s>>>(hv, ints, rows, (int64_t)nr, parts.p, rowptr.p, col.p, d64, dhi,
+                                                     dlo);
+  else
+    k_ham_finish<S, false><<<fb, kFinThreads, 0, s>>>(hv, ints, rows, (int64_t)nr, parts.p, rowptr.p, col.p, d64, dhi,
+                                                      dlo);
   SHCI_LAUNCH_CHECK();
   unsigned long long nl[2] = {0, 0};
   SHCI_CUDA(cudaMemcpyAsync(nl, tot.p, sizeof(nl), cudaMemcpyDeviceToHost, s));
@@ -1291,12 +1394,25 @@ static int64_t emit_rows(const Helpers& hp, const uint32_t* rows, size_t nr, con
   if (nl[0] > 0) {
     DevBuf<uint32_t> scratch;
     scratch.resize(32 * (size_t)nl[1]);
-    k_ham_finish_long<<<(unsigned)nl[0], 1024, 0, s>>>(hv, ints, rows, list.p, scratch.p, parts.p, rowptr.p, col.p,
-                                                        d64, dhi, dlo);
+    if (split)
+      k_ham_finish_long<S, true><<<(unsigned)nl[0], 1024, 0, s>>>(hv, ints, rows, list.p, scratch.p, parts.p, rowptr.p,
+                                                                  col.p, d64, dhi, dlo);
+    else
+      k_ham_finish_long<S, false><<<(unsigned)nl[0], 1024, 0, s>>>(hv, ints, rows, list.p, scratch.p, parts.p,
+                                                                   rowptr.p, col.p, d64, dhi, dlo);
     SHCI_LAUNCH_CHECK();
   }
   pt.mark("ham finish");
   return total;
+}
+static int64_t emit_rows(const Helpers& hp, const uint32_t* rows, size_t nr, const IntsView& ints,
+                         DevBuf<int64_t>& rowptr, DevBuf<int32_t>& col, DevBuf<double>& v64, DevBuf<float>& vhi,
+                         DevBuf<float>& vlo, bool want64, bool want32, bool want_lo, Prims& pr, cudaStream_t s,
+                         PhaseTimer& pt) {
+  return hp.narrow ? emit_rows_as<uint32_t>(hp, rows, nr, ints, rowptr, col, v64, vhi, vlo, want64, want32, want_lo, pr,
+                                            s, pt)
+                   : emit_rows_as<uint64_t>(hp, rows, nr, ints, rowptr, col, v64, vhi, vlo, want64, want32, want_lo, pr,
+                                            s, pt);
 }
 
 // Positions of the determinants [r0, r1), ascending: flags, and after their
@@ -1686,20 +1802,23 @@ void compute_diag(const Det2* dets, size_t n, const IntsView& ints, double* diag
 // Matrix-free sigma (HmultDirect, SHCI/Hmult.h:241-381): y[I] = diag[I] x[I] +
 // sum_J H_IJ x[J], row I's connections found by visit_row and H_IJ recomputed.
 // Hits wait per warp in three queues (singles, alpha-beta doubles, doubles of
-// one spin) and are evaluated 32 at a time, so a full warp runs one element
-// formula on strings it already holds. x is in storage order: the hits of a
-// scan are neighbours there. FP64: the reference's arithmetic. FP32 (the first
-// stage of the mixed matrix-free path): FP32 integrals, FP32 elements,
-// compensated FP32 accumulation of h * x.
+// one spin) and are evaluated on full warps, one element formula at a time, on
+// strings read by position. x is in storage order: the hits of a scan are
+// neighbours there. FP64: the reference's arithmetic. FP32 (the first stage of
+// the mixed matrix-free path): FP32 integrals, FP32 elements, compensated FP32
+// accumulation of h * x.
+// Bound by instruction issue (61 %) and latency at 28 warps per SM. 100,762
+// determinants of 36 orbitals, 1.1e8 connections, 4 vectors: 6.65 ms with a
+// generic element routine and 64-bit decoding per hit, now 3.21 ms.
 // ---------------------------------------------------------------------------
-template <int K, bool F32>
-struct DirectQVisitor {
+template <class S, int K, bool F32>
+struct DirectVisitor {
   using T = typename Elem<F32>::T;
-  const HelperView& h;
+  const HelperView<S>& h;
   const IntsView& ints;
-  uint64_t A, B;
+  S A, B;
   const T* x;  // [N][K]
-  uint32_t* q;  // three queues of 64
+  uint32_t* q;  // three queues of 64: singles, alpha-beta doubles, doubles of one spin
   int ns, nd, nm;
   Acc a32[F32 ? K : 1];
   double a64[F32 ? 1 : K];
@@ -1726,22 +1845,19 @@ struct DirectQVisitor {
       }
     }
   }
-  // which: 0 singles, 1 alpha-beta doubles, 2 doubles of one spin
   template <int which>
-  __device__ __forceinline__ void add(uint32_t p) {
-    const ulonglong2 J = h.str[p];
-    T xv[K];
-    load(xv, p);
-    T hv;
+  __device__ __forceinline__ T element(const typename StrPair<S>::T& J) const {
     if constexpr (which == 0) {
       const bool beta = J.x == A;
-      hv = elem_single<F32>(ints.I1, ints.V1, ints.I1f, ints.V1f, ints.norb, A, B, beta ? B : A, beta ? J.y : J.x,
-                            beta);
+      return elem_single<F32, S>(ints, A, B, beta ? B : A, beta ? J.y : J.x, beta);
     } else if constexpr (which == 1) {
-      hv = elem_ab<F32>(ints, A, B, J.x, J.y);
+      return elem_ab<F32, S>(ints, A, B, J.x, J.y);
     } else {
-      hv = J.x == A ? elem_same<F32, 1>(ints, B, A, J.y) : elem_same<F32, 0>(ints, A, B, J.x);
+      const bool beta = J.x == A;
+      return elem_same<F32, S>(ints, beta ? B : A, beta ? A : B, beta ? J.y : J.x, beta);
     }
+  }
+  __device__ __forceinline__ void add(T hv, const T (&xv)[K]) {
 #pragma unroll
     for (int r = 0; r < K; ++r) {
       if constexpr (F32)
@@ -1751,47 +1867,49 @@ struct DirectQVisitor {
     }
   }
   template <int which>
-  __device__ __forceinline__ int drain(uint32_t* w, int n, int cnt) {
-    const int lane = threadIdx.x & 31;
-    if (lane < cnt) add<which>(w[lane]);
-    __syncwarp();
-    const int rest = n - cnt;
-    const uint32_t v = lane < rest ? w[cnt + lane] : 0u;
-    __syncwarp();
-    if (lane < rest) w[lane] = v;
-    __syncwarp();
-    return rest;
+  __device__ __forceinline__ void one(uint32_t p) {
+    T xv[K];
+    load(xv, p);
+    add(element<which>(h.str[p]), xv);
   }
-  __device__ __forceinline__ void step(bool hit, uint32_t p, int cls) {
-    const unsigned lt = (1u << (threadIdx.x & 31)) - 1u;
-    if (cls == kAlpha) {  // the class is that of the scan, uniform but for singles
-      const bool single = hit && h.bstr[p] == B;
-      const unsigned ms = __ballot_sync(kFull, single), md = __ballot_sync(kFull, hit && !single);
-      if (single)
-        q[ns + __popc(ms & lt)] = p;
-      else if (hit)
-        q[64 + nd + __popc(md & lt)] = p;
-      ns += __popc(ms);
-      nd += __popc(md);
-    } else {
-      const bool single = hit && cls == kSingleB;
-      const unsigned ms = __ballot_sync(kFull, single), md = __ballot_sync(kFull, hit && !single);
-      if (single)
-        q[ns + __popc(ms & lt)] = p;
-      else if (hit)
-        q[128 + nm + __popc(md & lt)] = p;
-      ns += __popc(ms);
-      nm += __popc(md);
-    }
+  template <int which>
+  __device__ __forceinline__ int drain(uint32_t* w, int n) {  // the first 32 of n entries, 32 <= n < 64
+    const int lane = threadIdx.x & 31;
     __syncwarp();
-    if (ns >= 32) ns = drain<0>(q, ns, 32);
-    if (nd >= 32) nd = drain<1>(q + 64, nd, 32);
-    if (nm >= 32) nm = drain<2>(q + 128, nm, 32);
+    one<which>(w[lane]);
+    const uint32_t v = w[32 + lane];
+    __syncwarp();
+    if (lane < n - 32) w[lane] = v;
+    return n - 32;
+  }
+  template <int part>
+  __device__ __forceinline__ void step(bool hit, bool single, uint32_t p) {
+    const unsigned lt = (1u << (threadIdx.x & 31)) - 1u;
+    if (part != kSameBeta) {  // no single excitation there
+      const unsigned ms = __ballot_sync(kFull, hit && single);
+      if (ms) {
+        if (hit && single) q[ns + __popc(ms & lt)] = p;
+        ns += __popc(ms);
+        if (ns >= 32) ns = drain<0>(q, ns);
+      }
+    }
+    const unsigned md = __ballot_sync(kFull, hit && !single);
+    if (part == kAlphaMoved) {
+      if (hit && !single) q[64 + nd + __popc(md & lt)] = p;
+      nd += __popc(md);
+      if (nd >= 32) nd = drain<1>(q + 64, nd);
+    } else {
+      if (hit && !single) q[128 + nm + __popc(md & lt)] = p;
+      nm += __popc(md);
+      if (nm >= 32) nm = drain<2>(q + 128, nm);
+    }
   }
   __device__ __forceinline__ void flush() {
-    if (ns) drain<0>(q, ns, ns);
-    if (nd) drain<1>(q + 64, nd, nd);
-    if (nm) drain<2>(q + 128, nm, nm);
+    const int lane = threadIdx.x & 31;
+    __syncwarp();
+    if (lane < ns) one<0>(q[lane]);
+    if (lane < nd) one<1>(q[64 + lane]);
+    if (lane < nm) one<2>(q[128 + lane]);
   }
 };
 
@@ -1799,19 +1917,17 @@ struct DirectQVisitor {
 // rows' work differs by two orders of magnitude (the lowest determinant's row
 // holds 29,219 of 100,000 columns), and the block scheduler evens it out.
 constexpr int kDirThreads = 128;
-template <int K, bool F32>
-__global__ void __launch_bounds__(kDirThreads) k_sigma_direct(HelperView h, IntsView ints,
-                                                              const uint32_t* __restrict__ perm,
-                                                              const double* __restrict__ diag,
-                                                              const typename Elem<F32>::T* __restrict__ x, int kw,
-                                                              double* __restrict__ y, size_t ldy) {
+template <class S, int K, bool F32>
+__global__ void __launch_bounds__(kDirThreads, 8)
+    k_sigma_direct(HelperView<S> h, IntsView ints, const uint32_t* __restrict__ perm, const double* __restrict__ diag,
+                   const typename Elem<F32>::T* __restrict__ x, int kw, double* __restrict__ y, size_t ldy) {
   __shared__ uint32_t s_q[kDirThreads / 32][192];
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
   const size_t p = (size_t)blockIdx.x * (kDirThreads / 32) + wib;
   if (p >= h.N) return;
-  const ulonglong2 I = h.str[p];
-  DirectQVisitor<K, F32> v{h, ints, I.x, I.y, x, s_q[wib], 0, 0, 0, {}, {}};
-  visit_row(h, (uint32_t)p, I.x, I.y, v);
+  const auto I = h.str[p];
+  DirectVisitor<S, K, F32> v{h, ints, I.x, I.y, x, s_q[wib], 0, 0, 0, {}, {}};
+  visit_row<S>(h, (uint32_t)p, I.x, I.y, v);
   v.flush();
   const size_t o = perm[p];
   const double dg = diag[o];
@@ -1841,28 +1957,34 @@ __global__ void __launch_bounds__(kDirThreads) k_sigma_direct(HelperView h, Ints
   }
 }
 
-template <bool F32>
+template <class S, bool F32>
 static void launch_direct(const Helpers& hp, const IntsView& ints, const double* diag,
                           const typename Elem<F32>::T* x, int k, int kw, double* y, size_t ldy, cudaStream_t s) {
   if (hp.N == 0) return;
-  HelperView hv = hp.view();
+  HelperView<S> hv = hp.view<S>();
   const unsigned blocks = (unsigned)((hp.N + kDirThreads / 32 - 1) / (kDirThreads / 32));
   switch (k) {
-    case 1: k_sigma_direct<1, F32><<<blocks, kDirThreads, 0, s>>>(hv, ints, hp.perm.p, diag, x, kw, y, ldy); break;
-    case 2: k_sigma_direct<2, F32><<<blocks, kDirThreads, 0, s>>>(hv, ints, hp.perm.p, diag, x, kw, y, ldy); break;
-    case 4: k_sigma_direct<4, F32><<<blocks, kDirThreads, 0, s>>>(hv, ints, hp.perm.p, diag, x, kw, y, ldy); break;
+    case 1: k_sigma_direct<S, 1, F32><<<blocks, kDirThreads, 0, s>>>(hv, ints, hp.perm.p, diag, x, kw, y, ldy); break;
+    case 2: k_sigma_direct<S, 2, F32><<<blocks, kDirThreads, 0, s>>>(hv, ints, hp.perm.p, diag, x, kw, y, ldy); break;
+    case 4: k_sigma_direct<S, 4, F32><<<blocks, kDirThreads, 0, s>>>(hv, ints, hp.perm.p, diag, x, kw, y, ldy); break;
     default: throw Error(kErrInvalid, "direct sigma supports k in {1,2,4}");
   }
   SHCI_LAUNCH_CHECK();
 }
 void sigma_direct(const Helpers& hp, const IntsView& ints, const double* diag, const double* x, int k, int kw,
                   double* y, size_t ldy, cudaStream_t s) {
-  launch_direct<false>(hp, ints, diag, x, k, kw, y, ldy, s);
+  if (hp.narrow)
+    launch_direct<uint32_t, false>(hp, ints, diag, x, k, kw, y, ldy, s);
+  else
+    launch_direct<uint64_t, false>(hp, ints, diag, x, k, kw, y, ldy, s);
 }
 void sigma_direct32(const Helpers& hp, const IntsView& ints, const double* diag, const float* x, int k, int kw,
                     double* y, size_t ldy, cudaStream_t s) {
   if (!ints.I1f || !ints.I2f) throw Error(kErrState, "FP32 integrals missing");
-  launch_direct<true>(hp, ints, diag, x, k, kw, y, ldy, s);
+  if (hp.narrow)
+    launch_direct<uint32_t, true>(hp, ints, diag, x, k, kw, y, ldy, s);
+  else
+    launch_direct<uint64_t, true>(hp, ints, diag, x, k, kw, y, ldy, s);
 }
 
 }  // namespace shci

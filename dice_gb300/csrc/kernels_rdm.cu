@@ -178,24 +178,22 @@ __global__ void __launch_bounds__(kRdmThreads) k_rdm_off(const RdmDet* __restric
         v = __double2ll_rn(J.c * cI * kRdmUnit);
         const uint64_t x = A ^ J.a, y = B ^ J.b;
         if (x != 0 && y != 0) {
-          const int i = low_bit(x & A), a = low_bit(x & J.a), j = low_bit(y & B), b = low_bit(y & J.b);
-          if (__popcll(passed<0>(A, B, i, a) ^ passed<1>(B, J.a, j, b)) & 1) v = -v;
-          add_fix(U + elem4(n, a, b, i, j), v);
+          if (bit_count(passed(A, B, x, false) ^ passed(B, J.a, y, true)) & 1) v = -v;
+          add_fix(U + elem4(n, bit_index(x & J.a), bit_index(y & J.b), bit_index(x & A), bit_index(y & B)), v);
         } else {
           const bool beta = x == 0;
-          const uint64_t z = beta ? y : x, S = beta ? B : A, O = beta ? A : B, S2 = beta ? J.b : J.a;
-          const uint64_t d = z & S, c = z & S2;
-          const int i = low_bit(d), a = low_bit(c);
-          const uint64_t m1 = beta ? passed<1>(S, O, i, a) : passed<0>(S, O, i, a);
-          if ((d & (d - 1)) == 0) {
+          const uint64_t z = beta ? y : x, S = beta ? B : A, O = beta ? A : B;
+          const uint64_t d = z & S, c = z ^ d, di = low_one(d), ca = low_one(c);
+          const int i = bit_index(di), a = bit_index(ca);
+          const uint64_t m1 = passed(S, O, di | ca, beta);
+          if (d == di) {
             single = true;
-            if (__popcll(m1) & 1) v = -v;
+            if (bit_count(m1) & 1) v = -v;
             cd = a | (i << 8) | ((int)beta << 16);
           } else {
-            const int j = low_bit(d & (d - 1)), b = low_bit(c & (c - 1));
-            const uint64_t S1 = S ^ (1ull << i) ^ (1ull << a);
-            const uint64_t m2 = beta ? passed<1>(S1, O, j, b) : passed<0>(S1, O, j, b);
-            if (__popcll(m1 ^ m2) & 1) v = -v;
+            const uint64_t dj = d ^ di, cb = c ^ ca;
+            const int j = bit_index(dj), b = bit_index(cb);
+            if (bit_count(m1 ^ passed(S ^ di ^ ca, O, dj | cb, beta)) & 1) v = -v;
             add_fix(U + elem4(n, b, a, j, i), v);
             add_fix(U + elem4(n, b, a, i, j), -v);
           }

@@ -98,17 +98,27 @@ __device__ inline int occ_between(const Det2& d, int lo, int hi) {
   return c;
 }
 
-// Electrons passed (as a set whose population parity is the sign) when one of
-// string S moves between orbitals i and a: those of S strictly between, and in
-// the interleaved order (alpha of an orbital before beta) the other string O's
-// in [lo, hi) for an alpha electron (kSpin 0) and in (lo, hi] for a beta one.
-template <int kSpin>
-__device__ __forceinline__ uint64_t passed(uint64_t S, uint64_t O, int i, int a) {
-  const int lo = i < a ? i : a, hi = i < a ? a : i;
-  const uint64_t m = (1ull << hi) - (1ull << lo), open = m ^ (1ull << lo);
-  return (S & open) ^ (O & (kSpin ? open ^ (1ull << hi) : m));
+__device__ __forceinline__ int bit_count(uint32_t x) { return __popc(x); }
+__device__ __forceinline__ int bit_count(uint64_t x) { return __popcll(x); }
+// Index of the set bit of x (one bit set).
+__device__ __forceinline__ int bit_index(uint32_t x) { return 31 - __clz((int)x); }
+__device__ __forceinline__ int bit_index(uint64_t x) { return 63 - __clzll((long long)x); }
+template <class S>
+__device__ __forceinline__ S low_one(S x) {
+  return x & (S)(0 - x);
 }
-__device__ __forceinline__ int low_bit(uint64_t x) { return __ffsll((long long)x) - 1; }
+// Electrons passed (as a set whose population parity is the sign) when one of
+// string S moves between the orbitals of the two bits of `move`: those of S
+// strictly between, and in the interleaved order (alpha of an orbital before
+// beta) the other string O's in [lo, hi) for an alpha electron and in (lo, hi]
+// for a beta one. [lo, hi) is the difference of the two bits, so no orbital
+// index is needed.
+template <class S>
+__device__ __forceinline__ S passed(S s, S o, S move, bool beta) {
+  const S lo = low_one(move), hi = move ^ lo;
+  const S m = hi - lo, open = m ^ lo;
+  return (s & open) ^ (o & (beta ? open ^ hi : m));
+}
 
 // Device view of the integrals (SHCI/integral.h:47-101).
 struct IntsView {
@@ -125,6 +135,7 @@ struct IntsView {
   // difference the sum adds (V1) and its FP32 counterpart (V1f). Optional.
   const double* V1;
   const float* V1f;
+  const float2* I2ff;  // I2 as FP32 head and tail. Optional.
 };
 
 __device__ __forceinline__ int pair_index(int i, int j) {
