@@ -2059,8 +2059,8 @@ int shci_sigma_bytes(shci_ctx* ctx, int mode, int k, int64_t* bytes) {
     if (!c.whole_ham()) throw Error(SHCI_ERR_STATE, "no stored Hamiltonian of the whole space");
     const int64_t N = (int64_t)c.H.N, nnz = c.H.nnz;
     int64_t b = 0;
-    if (mode == SHCI_MODE_MIXED && k == 1 && c.H.cvalid)  // 16-bit deltas + FP32 values, row bases
-      b = c.H.cnnz * 6 + 8 * (N + 1) + 4 * N + 8 * N + 4 * N + 8 * N;
+    if (mode == SHCI_MODE_MIXED && k == 1 && c.H.cvalid)  // 24-bit columns + FP32 values
+      b = c.H.cnnz * 7 + 8 * (N + 1) + 8 * N + 4 * N + 8 * N;
     else if (mode == SHCI_MODE_MIXED)
       b = nnz * 8 + 8 * (N + 1) + 8 * N + (int64_t)k * N * (4 + 8);
     else if (mode == SHCI_MODE_FP64 && c.H.v64.p)

@@ -113,15 +113,15 @@ struct Csr {
   DevBuf<double> v64;
   DevBuf<float> vhi, vlo;
   DevBuf<uint32_t> perm, spos;
-  // Copy for the single-vector FP32 sigma with 16-bit column deltas: row r's
-  // entries are [crow[r], crow[r+1]); the column of an entry is cbase[r] plus
-  // the deltas of the row up to and including it (the first delta is 0).
-  // Gaps of 65536 or more are bridged by zero-valued entries of delta 65535.
-  // 6 bytes per entry instead of 8.
+  // Copy for the single-vector FP32 sigma: row r's entries are [crow[r],
+  // crow[r+1]) (a multiple of four), 24-bit columns in two planes and FP32
+  // values, laid out for cvw lanes per row (MixedCompactBody in
+  // kernels_sigma.cu). 7 bytes per entry instead of 8.
   DevBuf<int64_t> crow;
-  DevBuf<int32_t> cbase;
-  DevBuf<uint16_t> cdel;
+  DevBuf<uint16_t> clo;
+  DevBuf<uint8_t> chi;
   DevBuf<float> cval;
+  int cvw = 32;
   int64_t cnnz = 0;
   bool cvalid = false;
   // Row block (build_ham_block): N local rows, the full rows of the
@@ -144,18 +144,18 @@ struct Csr {
   }
   size_t bytes() const {
     return rowptr.bytes() + col.bytes() + v64.bytes() + vhi.bytes() + vlo.bytes() + perm.bytes() + spos.bytes() +
-           crow.bytes() + cbase.bytes() + cdel.bytes() + cval.bytes() + xpos.bytes() + xperm.bytes();
+           crow.bytes() + clo.bytes() + chi.bytes() + cval.bytes() + xpos.bytes() + xperm.bytes();
   }
   void drop_compressed() {
     crow.release();
-    cbase.release();
-    cdel.release();
+    clo.release();
+    chi.release();
     cval.release();
     cnnz = 0;
     cvalid = false;
   }
 };
-// Builds the 16-bit-delta copy of a column-sorted FP32 (head) matrix.
+// Builds the compact copy of a column-sorted FP32 (head) matrix.
 void compress_csr(Csr& H, Prims& pr, cudaStream_t s);
 
 // Builds H for the space described by hp, in storage order. When H already
