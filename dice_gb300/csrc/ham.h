@@ -219,6 +219,21 @@ struct ParentSplit {
 void split_parents(const Det2* dets, const int32_t* plist, const double* c, size_t n, double eps, double maxEntry,
                    const HeatBathView& hb, int norb, ParentSplit& ps, cudaStream_t s);
 
+// Entries of a list sorted by |value| descending that are >= eps_f in magnitude.
+// Most lists hold none for most parents: the first entry is looked at first.
+__device__ __forceinline__ int prefix_length(const float* __restrict__ vals, int n, float eps_f) {
+  if (n == 0 || fabsf(__ldg(vals)) < eps_f) return 0;
+  int lo = 1, hi = n;
+  while (lo < hi) {
+    const int mid = (lo + hi) >> 1;
+    if (fabsf(__ldg(vals + mid)) < eps_f)
+      hi = mid;
+    else
+      lo = mid + 1;
+  }
+  return lo;
+}
+
 // The next unit for the calling warp; false when the queue is empty. Parent
 // 0xffffffff: an unused entry, to be skipped.
 __device__ __forceinline__ bool next_unit(const SplitView& v, size_t n, uint32_t nextra, uint32_t& parent, int& slice,

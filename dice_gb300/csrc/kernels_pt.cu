@@ -105,6 +105,38 @@ struct PtArgs {
   double2* n2p;
 };
 
+// Determinants of up to 32 orbitals are one word (W2 false): the second word
+// is a constant zero and every mask, count and hash below is half as long.
+template <bool W2>
+__device__ __forceinline__ bool occupied(const Det2& d, int p) {
+  return W2 ? det_getocc(d, p) : (d.w0 >> p) & 1ull;
+}
+template <bool W2>
+__device__ __forceinline__ void toggle(Det2& d, int p) {
+  if (W2)
+    det_flip(d, p);
+  else
+    d.w0 ^= 1ull << p;
+}
+template <bool W2>
+__device__ __forceinline__ int between(const Det2& d, int p, int q) {
+  const int lo = p < q ? p : q, hi = p < q ? q : p;
+  if (W2) return occ_between(d, lo, hi);
+  return __popcll(d.w0 & (((1ull << hi) - (1ull << lo)) ^ (1ull << lo)));
+}
+template <bool W2>
+__device__ __forceinline__ bool in_space(const PtArgs& a, const Det2& x) {
+  if (W2) return hash_contains(a.hslots, a.hmask, a.dets, x);
+  uint64_t h = det_hash(Det2{x.w0, 0}) & a.hmask;
+  for (uint64_t probe = 0; probe <= a.hmask; ++probe) {
+    const uint32_t s = __ldg(a.hslots + h);
+    if (s == 0xffffffffu) return false;
+    if (__ldg(&a.dets[s].w0) == x.w0) return true;
+    h = (h + 1) & a.hmask;
+  }
+  return false;
+}
+
 __device__ __forceinline__ bool in_part(const PtArgs& a, const Det2& d) {
   return a.nparts == 1 || (uint32_t)((det_hash(d) >> 32) % a.nparts) == a.part;
 }
@@ -113,12 +145,13 @@ __device__ __forceinline__ bool in_part(const PtArgs& a, const Det2& d) {
 // (SHCI/Determinants.cpp:332-357 as called at SHCIgetdeterminants.cpp:155-157):
 // the a<->i transposition counted on di, then b<->j on di with a emptied and
 // i refilled.
-__device__ __forceinline__ double pt_double_sign(Det2 di, int a, int b, int i, int j) {
-  int n1 = occ_between(di, a < i ? a : i, a < i ? i : a);
-  det_flip(di, a);
-  det_flip(di, i);
-  int n2 = occ_between(di, b < j ? b : j, b < j ? j : b);
-  return ((n1 + n2) & 1) ? -1.0 : 1.0;
+template <bool W2>
+__device__ __forceinline__ bool pt_double_odd(Det2 di, int a, int b, int i, int j) {
+  int n = between<W2>(di, a, i);
+  toggle<W2>(di, a);
+  toggle<W2>(di, i);
+  n += between<W2>(di, b, j);
+  return n & 1;
 }
 
 // ---- float pairs (hi + lo, |lo| <= ulp(hi)/2): the per-candidate arithmetic
@@ -296,14 +329,16 @@ __device__ __forceinline__ float2 vpair(const float2* sJ, const float2* sJK, int
   return ((p ^ q) & 1) ? sJ[o] : sJK[o];
 }
 
+template <bool W2>
 __global__ void __launch_bounds__(kPtThreads) k_pt_gen(PtArgs a) {
   extern __shared__ float2 smf[];
   __shared__ unsigned char s_closed[kPtWarps][kMaxSpin];
   __shared__ unsigned char s_open[kPtWarps][kMaxSpin];   // alpha holes, then beta holes
   __shared__ unsigned char s_cspin[kPtWarps][kMaxSpin];  // alpha electrons, then beta electrons
   __shared__ float2 s_F[kPtWarps][kMaxSpin];
-  __shared__ uint32_t s_qo[kPtWarps][64];
+  __shared__ uint32_t s_qo[kPtWarps][64], s_ro[kPtWarps][64];
   __shared__ float s_qv[kPtWarps][64];
+  __shared__ float2 s_rv[kPtWarps][64];
   const int n = a.ints.norb, nn = n * n;
   float2* sD = smf;            // J
   float2* sX = smf + nn;       // J - K
@@ -328,7 +363,8 @@ __global__ void __launch_bounds__(kPtThreads) k_pt_gen(PtArgs a) {
   while (next_unit(a.split, a.n, nextra, pp, slice, slices)) {
     if (pp == 0xffffffffu) continue;
     const size_t p = a.plist ? (size_t)a.plist[pp] : (size_t)pp;
-    const Det2 d = a.dets[p];
+    Det2 d = a.dets[p];
+    if (!W2) d.w1 = 0;
     const double cp = a.c[p];
     const double eps = fabs(a.eps2 / cp);
     if (!(eps < INFINITY)) continue;  // c_i = 0: nothing passes either threshold
@@ -351,7 +387,7 @@ __global__ void __launch_bounds__(kPtThreads) k_pt_gen(PtArgs a) {
       for (int base = 0; base < n2; base += 32) {
         const int q = base + lane;
         const bool valid = q < n2;
-        const bool occ = valid && det_getocc(d, q);
+        const bool occ = valid && occupied<W2>(d, q);
         const unsigned mo = __ballot_sync(kFull, occ), mv = __ballot_sync(kFull, valid);
         const unsigned mh = mv & ~mo;
         const unsigned evn = 0x55555555u, odd = 0xaaaaaaaau;  // alpha lanes, beta lanes
@@ -383,7 +419,7 @@ __global__ void __launch_bounds__(kPtThreads) k_pt_gen(PtArgs a) {
       for (int k = 0; k < nclosed; ++k) f = ff_add(f, vpair(sD, sX, n, q, closed[k]));
       const float2 hq = sH[q];
       F[q] = ff_add(hq, f);
-      if (det_getocc(d, q)) {
+      if (occupied<W2>(d, q)) {
         const float2 half = ff_add(hq, make_float2(0.5f * f.x, 0.5f * f.y));
         ed = ff_add(ed, half);
       }
@@ -395,14 +431,17 @@ __global__ void __launch_bounds__(kPtThreads) k_pt_gen(PtArgs a) {
     int cur[kMaxRestrict];
     for (int r = 0; r < sp.nrestrict; ++r) cur[r] = __popcll(d.w0 & sp.rmask0[r]) + __popcll(d.w1 & sp.rmask1[r]);
 
-    // Survivors of the cheap tests wait in a per-warp ring of 64 entries and
-    // are processed 32 at a time, so that the costly part (pair-arithmetic
-    // element or energy, hash probe, stores) runs on full warps. Entry: the
-    // orbitals i | j << 8 | a << 16 | b << 24 (j = b = 0xff for a single) and
-    // the heat-bath value of a double.
-    uint32_t* qo = s_qo[wib];
+    // Survivors of the cheap tests wait in a per-warp ring of 64 entries; 32 at
+    // a time are decided (a single's element, the probe of the variational
+    // space, which drops two of three), and those kept wait in a second ring
+    // for the costly part (sign, numerator, energy, stores), so that each part
+    // runs on full warps. Entry: the orbitals i | j << 8 | a << 16 | b << 24
+    // (j = b = 0xff for a single) and the heat-bath value of a double; in the
+    // second ring, a single's element.
+    uint32_t *qo = s_qo[wib], *ro = s_ro[wib];
     float* qv = s_qv[wib];
-    unsigned qh = 0, qn = 0;  // ring head and length (warp-uniform)
+    float2* rv = s_rv[wib];
+    unsigned qh = 0, qn = 0, rh = 0, rn = 0;  // ring heads and lengths (warp-uniform)
     auto push = [&](bool surv, uint32_t w, float val) {
       const unsigned m = __ballot_sync(kFull, surv);
       if (surv) {
@@ -413,70 +452,97 @@ __global__ void __launch_bounds__(kPtThreads) k_pt_gen(PtArgs a) {
       qn += __popc(m);
       __syncwarp();
     };
-    auto drain = [&](unsigned cnt) {  // the first cnt (<= 32) entries
-      bool keep = false, present = false;
+    auto excite = [&](uint32_t w) {
+      Det2 x = d;
+      toggle<W2>(x, w & 0xff);
+      toggle<W2>(x, (w >> 16) & 0xff);
+      if (((w >> 8) & 0xff) != 0xff) {
+        toggle<W2>(x, (w >> 8) & 0xff);
+        toggle<W2>(x, w >> 24);
+      }
+      return x;
+    };
+    auto write = [&](unsigned cnt) {  // the first cnt (<= 32) entries of the second ring
+      const bool keep = (unsigned)lane < cnt;
+      bool present = false;
       Det2 cand = d;
       float2 v = make_float2(0.0f, 0.0f), e = v;
       double2 vs = make_double2(0.0, 0.0);
-      if ((unsigned)lane < cnt) {
-        const unsigned slot = (qh + lane) & 63u;
-        const uint32_t w = qo[slot];
+      if (keep) {
+        const unsigned slot = (rh + lane) & 63u;
+        const uint32_t w = ro[slot];
+        const float2 val = rv[slot];
         const int oi = w & 0xff, oj = (w >> 8) & 0xff, oa = (w >> 16) & 0xff, ob = w >> 24;
+        cand = excite(w);
         if (oj == 0xff) {
-          // single i -> a: float pairs, then (rarely) the FP64 element
-          float2 H = make_float2(0.0f, 0.0f);
-          int dec = single_ff(a, d, oa, oi, eps_ff, H);
-          if (dec == 0) {
-            const double h = hij_single_rows(a, d, oa, oi);
-            dec = fabs(h) > eps ? 1 : -1;
-            H = ff_of(h);
+          v = ff_mul(val, cp_ff);
+          if (stoch) {
+            // numerators as the reference forms them, from the FP64 element
+            const double hd = hij_single_rows(a, d, oa, oi);
+            vs = make_double2(__dmul_rn(hd, ci1), __dmul_rn(__dmul_rn(__dmul_rn(hd, hd), ci1), kfac));
+            present = fabs(hd) > epsL;
           }
-          if (dec > 0) {
-            det_flip(cand, oa);
-            det_flip(cand, oi);
-            keep = in_part(a, cand) && !hash_contains(a.hslots, a.hmask, a.dets, cand);
-            if (keep) {
-              v = ff_mul(H, cp_ff);
-              if (stoch) {
-                // numerators as the reference forms them, from the FP64 element
-                const double hd = hij_single_rows(a, d, oa, oi);
-                vs = make_double2(__dmul_rn(hd, ci1), __dmul_rn(__dmul_rn(__dmul_rn(hd, hd), ci1), kfac));
-                present = fabs(hd) > epsL;
-              }
-              e = ff_sub(ff_add(ed, ff_sub(F[oa], F[oi])), vpair(sD, sX, n, oa, oi));
-            }
-          }
+          e = ff_sub(ff_add(ed, ff_sub(F[oa], F[oi])), vpair(sD, sX, n, oa, oi));
         } else {
-          // double i -> a, j -> b
-          det_flip(cand, oa);
-          det_flip(cand, ob);
-          det_flip(cand, oi);
-          det_flip(cand, oj);
-          keep = in_part(a, cand) && !hash_contains(a.hslots, a.hmask, a.dets, cand);
-          if (keep) {
-            const float vf = qv[slot];
-            v = ff_mul_f(pt_double_sign(cand, oa, ob, oi, oj) > 0.0 ? vf : -vf, cp_ff);
-            if (stoch) {
-              // integrals[index] * sgn * ci1 and integrals[index]^2 (a float
-              // product) * ci1 * kfac, as the reference forms them
-              const double sg = pt_double_sign(cand, oa, ob, oi, oj);
-              const float sq = __fmul_rn(vf, vf);
-              vs = make_double2(__dmul_rn(__dmul_rn((double)vf, sg), ci1),
-                                __dmul_rn(__dmul_rn((double)sq, ci1), kfac));
-              present = fabsf(vf) > epsL_f;  // (double)|v| > epsL exactly
-            }
-            const float2 fa = ff_add(F[oa], F[ob]), fi = ff_add(F[oi], F[oj]);
-            const float2 vin = ff_add(vpair(sD, sX, n, oi, oj), vpair(sD, sX, n, oa, ob));
-            const float2 vx = ff_add(ff_add(vpair(sD, sX, n, oa, oi), vpair(sD, sX, n, oa, oj)),
-                                     ff_add(vpair(sD, sX, n, ob, oi), vpair(sD, sX, n, ob, oj)));
-            e = ff_add(ed, ff_add(ff_sub(fa, fi), ff_sub(vin, vx)));
+          const float vf = val.x;
+          const bool odd = pt_double_odd<W2>(cand, oa, ob, oi, oj);
+          v = ff_mul_f(odd ? -vf : vf, cp_ff);
+          if (stoch) {
+            // integrals[index] * sgn * ci1 and integrals[index]^2 (a float
+            // product) * ci1 * kfac, as the reference forms them
+            const float sq = __fmul_rn(vf, vf);
+            vs = make_double2(__dmul_rn(odd ? -(double)vf : (double)vf, ci1),
+                              __dmul_rn(__dmul_rn((double)sq, ci1), kfac));
+            present = fabsf(vf) > epsL_f;  // (double)|v| > epsL exactly
           }
+          const float2 fa = ff_add(F[oa], F[ob]), fi = ff_add(F[oi], F[oj]);
+          const float2 vin = ff_add(vpair(sD, sX, n, oi, oj), vpair(sD, sX, n, oa, ob));
+          const float2 vx = ff_add(ff_add(vpair(sD, sX, n, oa, oi), vpair(sD, sX, n, oa, oj)),
+                                   ff_add(vpair(sD, sX, n, ob, oi), vpair(sD, sX, n, ob, oj)));
+          e = ff_add(ed, ff_add(ff_sub(fa, fi), ff_sub(vin, vx)));
         }
       }
       pt_put(a, keep, cand, v, e, vs, present);
+      rh = (rh + cnt) & 63u;
+      rn -= cnt;
+      __syncwarp();
+    };
+    auto drain = [&](unsigned cnt) {  // decides the first cnt (<= 32) entries of the first ring
+      bool keep = false;
+      uint32_t w = 0;
+      float2 val = make_float2(0.0f, 0.0f);
+      if ((unsigned)lane < cnt) {
+        const unsigned slot = (qh + lane) & 63u;
+        w = qo[slot];
+        val.x = qv[slot];
+        keep = true;
+        if (((w >> 8) & 0xff) == 0xff) {
+          // single i -> a: float pairs, then (rarely) the FP64 element
+          const int oi = w & 0xff, oa = (w >> 16) & 0xff;
+          int dec = single_ff(a, d, oa, oi, eps_ff, val);
+          if (dec == 0) {
+            const double h = hij_single_rows(a, d, oa, oi);
+            dec = fabs(h) > eps ? 1 : -1;
+            val = ff_of(h);
+          }
+          keep = dec > 0;
+        }
+        if (keep) {
+          const Det2 x = excite(w);
+          keep = in_part(a, x) && !in_space<W2>(a, x);
+        }
+      }
+      const unsigned m = __ballot_sync(kFull, keep);
+      if (keep) {
+        const unsigned slot = (rh + rn + __popc(m & lt)) & 63u;
+        ro[slot] = w;
+        rv[slot] = val;
+      }
+      rn += __popc(m);
       qh = (qh + cnt) & 63u;
       qn -= cnt;
       __syncwarp();
+      if (rn >= 32) write(32);
     };
 
     // ---- singles: every same-spin (i, a) (a spin flip has a zero element:
@@ -508,15 +574,18 @@ __global__ void __launch_bounds__(kPtThreads) k_pt_gen(PtArgs a) {
     while (qn > 0) drain(qn < 32 ? qn : 32);
 
     // ---- doubles: heat-bath list prefixes, flattened over the warp
-    if (fabs(a.maxEntry) < eps) continue;
+    if (fabs(a.maxEntry) < eps) {
+      if (rn > 0) write(rn);
+      continue;
+    }
     // for a float v, (double)|v| < eps exactly when |v| < eps rounded up to float
     const float eps_f = __double2float_ru(eps);
     const int npairs = nclosed * (nclosed - 1) / 2;
     // this slice's pairs: q = slice, slice + slices, ...
     for (int pb = slice; pb < npairs; pb += 32 * slices) {
       const int q = pb + lane * slices;
-      int ci = 0, cj = 0;
-      int64_t lstart = 0, len = 0;
+      int ci = 0, cj = 0, len = 0;
+      uint32_t lstart = 0;
       bool same = false;
       if (q < npairs) {
         // q -> (i, j), i > j, q = i(i-1)/2 + j
@@ -532,59 +601,47 @@ __global__ void __launch_bounds__(kPtThreads) k_pt_gen(PtArgs a) {
         same = (ci & 1) == (cj & 1);
         const int64_t* st = same ? a.hb.sameStart : a.hb.oppStart;
         const float* vals = same ? a.hb.sameVal : a.hb.oppVal;
-        const int64_t s0 = st[pair], s1 = st[pair + 1];
-        // first entry with |v| < eps (lists sorted by |v| descending)
-        int64_t lo = s0, hi = s1;
-        while (lo < hi) {
-          const int64_t mid = (lo + hi) >> 1;
-          if (fabsf(vals[mid]) < eps_f)
-            hi = mid;
-          else
-            lo = mid + 1;
-        }
-        lstart = s0;
-        len = lo - s0;
+        lstart = (uint32_t)st[pair];
+        len = prefix_length(vals + lstart, (int)((uint32_t)st[pair + 1] - lstart), eps_f);
       }
-      int64_t incl = len;
+      int incl = len;
 #pragma unroll
       for (int o = 1; o < 32; o <<= 1) {
-        const int64_t y = __shfl_up_sync(kFull, incl, o);
+        const int y = __shfl_up_sync(kFull, incl, o);
         if (lane >= o) incl += y;
       }
-      const int64_t total = __shfl_sync(kFull, incl, 31);
-      const int64_t excl = incl - len;
-      for (int64_t f0 = 0; f0 < total; f0 += 32) {
-        const int64_t f = f0 + lane;
-        // owner lane of flattened entry f: last lane with excl <= f
+      const int total = __shfl_sync(kFull, incl, 31);
+      const int excl = incl - len;
+      const uint32_t off = lstart - (uint32_t)excl;  // list index of flat entry f: off of its owner + f
+      const uint32_t who = (uint32_t)ci | ((uint32_t)cj << 8) | (same ? 0x10000u : 0u);
+      for (int f0 = 0; f0 < total; f0 += 32) {
+        const int f = f0 + lane;
+        // owner lane of flat entry f: last lane with excl <= f
         int lo = 0;
 #pragma unroll
         for (int st = 16; st >= 1; st >>= 1) {
-          const int c2 = lo + st;
-          const int64_t e2 = __shfl_sync(kFull, excl, c2 < 32 ? c2 : 31);
-          if (c2 < 32 && e2 <= f) lo = c2;
+          const int e2 = __shfl_sync(kFull, excl, lo + st);
+          if (e2 <= f) lo += st;
         }
-        const int64_t ls = __shfl_sync(kFull, lstart, lo);
-        const int64_t eo = __shfl_sync(kFull, excl, lo);
-        const int oci = __shfl_sync(kFull, ci, lo);
-        const int ocj = __shfl_sync(kFull, cj, lo);
-        const bool osame = __shfl_sync(kFull, (int)same, lo) != 0;
+        const uint32_t index = __shfl_sync(kFull, off, lo) + (uint32_t)f;
+        const uint32_t ow = __shfl_sync(kFull, who, lo);
         bool surv = false;
         uint32_t w = 0;
         float vf = 0.0f;
         if (f < total) {
-          const int64_t index = ls + (f - eo);
-          const int16_t* pr = osame ? a.hb.samePairs : a.hb.oppPairs;
-          const int av = 2 * pr[2 * index] + (oci & 1);
-          const int bv = 2 * pr[2 * index + 1] + (ocj & 1);
+          const bool osame = (ow & 0x10000u) != 0;
+          const int oci = ow & 0xff, ocj = (ow >> 8) & 0xff;
+          const short2 pr = __ldg(reinterpret_cast<const short2*>(osame ? a.hb.samePairs : a.hb.oppPairs) + index);
+          const int av = 2 * pr.x + (oci & 1), bv = 2 * pr.y + (ocj & 1);
           bool ok = true;
           for (int r = 0; ok && r < sp.nrestrict; ++r) {
             int c2 = cur[r] - in_mask(sp, r, oci) - in_mask(sp, r, ocj) + in_mask(sp, r, av) + in_mask(sp, r, bv);
             ok = c2 >= sp.rmin[r] && c2 <= sp.rmax[r];
           }
-          surv = ok && !(det_getocc(d, av) || det_getocc(d, bv));
+          surv = ok && !(occupied<W2>(d, av) || occupied<W2>(d, bv));
           if (surv) {
             w = (uint32_t)oci | ((uint32_t)ocj << 8) | ((uint32_t)av << 16) | ((uint32_t)bv << 24);
-            vf = (osame ? a.hb.sameVal : a.hb.oppVal)[index];
+            vf = __ldg((osame ? a.hb.sameVal : a.hb.oppVal) + index);
           }
         }
         push(surv, w, vf);
@@ -592,6 +649,7 @@ __global__ void __launch_bounds__(kPtThreads) k_pt_gen(PtArgs a) {
       }
     }
     while (qn > 0) drain(qn < 32 ? qn : 32);
+    if (rn > 0) write(rn);
   }
 }
 
@@ -937,8 +995,17 @@ size_t pt_prepare(PtArgs& a, const Det2* dets, size_t n, const double* c, double
     a.e0 = make_float2(h, (float)(E0 - (double)h));
   }
   const size_t gsmem = sizeof(float2) * (2 * ints.norb * ints.norb + 2 * ints.norb);
-  SHCI_CUDA(cudaFuncSetAttribute(k_pt_gen, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)gsmem));
+  if (ints.norb > 32)
+    SHCI_CUDA(cudaFuncSetAttribute(k_pt_gen<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)gsmem));
+  else
+    SHCI_CUDA(cudaFuncSetAttribute(k_pt_gen<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)gsmem));
   return gsmem;
+}
+void launch_gen(const PtArgs& a, size_t gsmem, cudaStream_t s) {
+  if (a.ints.norb > 32)
+    k_pt_gen<true><<<kPtGenBlocks, kPtThreads, gsmem, s>>>(a);
+  else
+    k_pt_gen<false><<<kPtGenBlocks, kPtThreads, gsmem, s>>>(a);
 }
 
 }  // namespace
@@ -983,7 +1050,7 @@ PtResult pt_deterministic(const Det2* dets, size_t n, const double* c, double E0
     a.ne = w.ne.p;
     SHCI_CUDA(cudaMemsetAsync(w.next.p, 0, sizeof(unsigned long long), s));
     ps.rewind(s);
-    k_pt_gen<<<kPtGenBlocks, kPtThreads, gsmem, s>>>(a);
+    launch_gen(a, gsmem, s);
     SHCI_LAUNCH_CHECK();
     unsigned long long total = 0;
     SHCI_CUDA(cudaMemcpyAsync(&total, w.next.p, sizeof(total), cudaMemcpyDeviceToHost, s));
@@ -1155,7 +1222,7 @@ PtStochResult pt_semistochastic(const Det2* dets, size_t n, const double* c_dev,
       a.n2p = w.n2p.p;
       SHCI_CUDA(cudaMemsetAsync(w.next.p, 0, sizeof(unsigned long long), s));
       ps.rewind(s);
-      k_pt_gen<<<kPtGenBlocks, kPtThreads, gsmem, s>>>(a);
+      launch_gen(a, gsmem, s);
       SHCI_LAUNCH_CHECK();
       unsigned long long total = 0;
       SHCI_CUDA(cudaMemcpyAsync(&total, w.next.p, sizeof(total), cudaMemcpyDeviceToHost, s));

@@ -182,8 +182,8 @@ __global__ void __launch_bounds__(kSelThreads) k_select(SelArgs a) {
     // this slice's pairs: q = slice, slice + slices, ...
     for (int pb = slice; pb < npairs; pb += 32 * slices) {
       const int q = pb + lane * slices;
-      int ci = 0, cj = 0;
-      int64_t lstart = 0, len = 0;
+      int ci = 0, cj = 0, len = 0;
+      uint32_t lstart = 0;
       bool same = false;
       if (q < npairs) {
         // q -> (i, j), i > j, q = i(i-1)/2 + j
@@ -200,49 +200,38 @@ __global__ void __launch_bounds__(kSelThreads) k_select(SelArgs a) {
           same = (ci & 1) == (cj & 1);
           const int64_t* st = same ? a.hb.sameStart : a.hb.oppStart;
           const float* vals = same ? a.hb.sameVal : a.hb.oppVal;
-          int64_t s0 = st[pair], s1 = st[pair + 1];
-          // first index with |v| < eps
-          int64_t lo = s0, hi = s1;
-          while (lo < hi) {
-            int64_t mid = (lo + hi) >> 1;
-            if (fabsf(vals[mid]) < eps_f)
-              hi = mid;
-            else
-              lo = mid + 1;
-          }
-          lstart = s0;
-          len = lo - s0;
+          lstart = (uint32_t)st[pair];
+          len = prefix_length(vals + lstart, (int)((uint32_t)st[pair + 1] - lstart), eps_f);
         }
       }
-      int64_t incl = len;
+      int incl = len;
 #pragma unroll
       for (int o = 1; o < 32; o <<= 1) {
-        int64_t y = __shfl_up_sync(kFull, incl, o);
+        int y = __shfl_up_sync(kFull, incl, o);
         if (lane >= o) incl += y;
       }
-      const int64_t total = __shfl_sync(kFull, incl, 31);
-      const int64_t excl = incl - len;
-      for (int64_t f0 = 0; f0 < total; f0 += 32) {
-        const int64_t f = f0 + lane;
+      const int total = __shfl_sync(kFull, incl, 31);
+      const int excl = incl - len;
+      const uint32_t off = lstart - (uint32_t)excl;  // list index of flat entry f: off of its owner + f
+      const uint32_t who = (uint32_t)ci | ((uint32_t)cj << 8) | (same ? 0x10000u : 0u);
+      for (int f0 = 0; f0 < total; f0 += 32) {
+        const int f = f0 + lane;
         int lo = 0;
 #pragma unroll
         for (int st = 16; st >= 1; st >>= 1) {
-          int c = lo + st;
-          int64_t e = __shfl_sync(kFull, excl, c < 32 ? c : 31);
-          if (c < 32 && e <= f) lo = c;
+          const int e = __shfl_sync(kFull, excl, lo + st);
+          if (e <= f) lo += st;
         }
-        const int64_t ls = __shfl_sync(kFull, lstart, lo);
-        const int64_t eo = __shfl_sync(kFull, excl, lo);
-        const int oci = __shfl_sync(kFull, ci, lo);
-        const int ocj = __shfl_sync(kFull, cj, lo);
-        const bool osame = __shfl_sync(kFull, (int)same, lo) != 0;
+        const uint32_t index = __shfl_sync(kFull, off, lo) + (uint32_t)f;
+        const uint32_t ow = __shfl_sync(kFull, who, lo);
+        const int oci = ow & 0xff, ocj = (ow >> 8) & 0xff;
         bool emit = false;
         Det2 cand = d;
         if (f < total) {
-          const int64_t index = ls + (f - eo);
-          const int16_t* pr = osame ? a.hb.samePairs : a.hb.oppPairs;
-          const int av = 2 * pr[2 * index] + (oci & 1);
-          const int bv = 2 * pr[2 * index + 1] + (ocj & 1);
+          const short2 pr =
+              __ldg(reinterpret_cast<const short2*>((ow & 0x10000u) ? a.hb.samePairs : a.hb.oppPairs) + index);
+          const int av = 2 * pr.x + (oci & 1);
+          const int bv = 2 * pr.y + (ocj & 1);
           bool ok = (av >> 1) < sp.ncore + sp.nact && (bv >> 1) < sp.ncore + sp.nact;
           for (int r = 0; ok && r < sp.nrestrict; ++r) {
             int e = cur[r] - in_mask(sp, r, oci) - in_mask(sp, r, ocj) + in_mask(sp, r, av) + in_mask(sp, r, bv);
