@@ -480,7 +480,7 @@ struct Context {
     size_t nnew = 0;
     if (n) {
       trev_buf.reserve(2 * n);
-      nnew = trev_new_dets(cand.p, n, hash, dets.p, trev_buf.p, trev_flag, trev_pos, prims, stream);
+      nnew = trev_new_dets(cand.p, n, hints.norb, hash, dets.p, trev_buf.p, trev_flag, trev_pos, prims, stream);
     }
     ncand = 0;
     if (nnew) {
@@ -517,7 +517,7 @@ struct Context {
     }
     size_t nnew = 0;
     if (total > 0) {
-      sort_dets(cand.p, nullptr, (size_t)total, prims, stream);
+      sort_dets(cand.p, nullptr, (size_t)total, hints.norb, prims, stream);
       nnew = unique_dets(cand.p, (size_t)total, prims, stream);
     }
     SHCI_CUDA(cudaStreamSynchronize(stream));

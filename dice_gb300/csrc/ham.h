@@ -298,7 +298,7 @@ int64_t select_candidates(const Det2* dets, const double* cmax, size_t n, double
 // returns how many.
 void trev_cmax(const Det2* dets, const double* ci, size_t ld, int nroots, size_t n, const int32_t* flip, double* out,
                cudaStream_t s);
-size_t trev_new_dets(Det2* cand, size_t n, const DetHash& present, const Det2* dets, Det2* out, DevBuf<int64_t>& flag,
+size_t trev_new_dets(Det2* cand, size_t n, int norb, const DetHash& present, const Det2* dets, Det2* out, DevBuf<int64_t>& flag,
                      DevBuf<int64_t>& pos, Prims& pr, cudaStream_t s);
 // Number of the n determinants q that the hash set `present` (over dets) holds.
 int64_t count_present(const Det2* q, size_t n, const DetHash& present, const Det2* dets, int64_t* d_counter,

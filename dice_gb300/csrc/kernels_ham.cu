@@ -365,10 +365,12 @@ static void build_singles_and_index(Helpers& hp, int norb, Prims& pr, cudaStream
       const unsigned eb = grid_for((size_t)ne, 256);
       k_m1_fill<S><<<grid_for(n, 256), 256, 0, s>>>(bstr, hp.agrp.p, n, o1.p, key.p, perm.p, raw.p);
       SHCI_LAUNCH_CHECK();
-      sort_u64(key.p, perm.p, (size_t)ne, pr, s);  // by partial string
+      sort_u64(key.p, perm.p, (size_t)ne, norb, pr, s);  // by partial string
       k_m1_group_keys<<<eb, 256, 0, s>>>(raw.p, perm.p, ne, key.p);
       SHCI_LAUNCH_CHECK();
-      sort_u64(key.p, perm.p, (size_t)ne, pr, s);  // then by alpha group (stable)
+      int gbits = 1;
+      while ((hp.NA >> gbits) != 0) ++gbits;
+      sort_u64(key.p, perm.p, (size_t)ne, gbits, pr, s);  // then by alpha group (stable)
       k_m1_permute<<<eb, 256, 0, s>>>(raw.p, perm.p, ne, hp.m1ent.p);
       SHCI_LAUNCH_CHECK();
       // the groups' hash tables
@@ -418,7 +420,7 @@ void Helpers::build(const Det2* dets, size_t n, int norb, Prims& pr, cudaStream_
     const unsigned g = grid_for(n, 256);
     k_strings<<<g, 256, 0, s>>>(dets, n, a.p, bkey.p, perm.p);
     SHCI_LAUNCH_CHECK();
-    sort_u128(bkey.p, a.p, perm.p, n, pr, s);  // by (alpha, beta): the storage order
+    sort_u128(bkey.p, a.p, perm.p, n, norb, norb, pr, s);  // by (alpha, beta): the storage order
     if (narrow)
       k_pair_strings<uint32_t><<<g, 256, 0, s>>>(a.p, bkey.p, perm.p, n, reinterpret_cast<uint2*>(str.p),
                                                  reinterpret_cast<uint32_t*>(bstr.p), spos.p, bPos.p);
@@ -435,7 +437,7 @@ void Helpers::build(const Det2* dets, size_t n, int norb, Prims& pr, cudaStream_
     SHCI_LAUNCH_CHECK();
     k_iota_last<<<1, 1, 0, s>>>(aStart.p, NA, (int64_t)n);
     SHCI_LAUNCH_CHECK();
-    sort_u64(bkey.p, bPos.p, n, pr, s);  // by beta string, stable: ascending positions within a group
+    sort_u64(bkey.p, bPos.p, n, norb, pr, s);  // by beta string, stable: ascending positions within a group
     k_group_flags<<<g, 256, 0, s>>>(bkey.p, n, flag.p);
     SHCI_LAUNCH_CHECK();
     scan_exclusive_i64(flag.p, excl.p, n, &NB, pr, s);

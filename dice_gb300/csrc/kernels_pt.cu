@@ -1057,12 +1057,13 @@ PtResult pt_deterministic(const Det2* dets, size_t n, const double* c, double E0
     SHCI_CUDA(cudaStreamSynchronize(s));
     return (int64_t)total;
   };
+  const int bits0 = std::min(64, 2 * ints.norb), bits1 = std::max(0, 2 * ints.norb - 64);
   PhaseTimer pt(s);
   auto reduce = [&](int64_t m, PtResult& r) {
     w.perm.resize((size_t)m);
     k_pt_iota<<<grid_for((size_t)m, 256), 256, 0, s>>>(w.perm.p, (size_t)m);
     SHCI_LAUNCH_CHECK();
-    sort_u128(w.key0.p, w.key1.p, w.perm.p, (size_t)m, pr, s);
+    sort_u128(w.key0.p, w.key1.p, w.perm.p, (size_t)m, bits0, bits1, pr, s);
     pt.mark("pt sort");
     k_pt_reduce<<<kPtRedBlocks, kPtRedThreads, 0, s>>>(w.key0.p, w.key1.p, w.perm.p, w.ne.p, (size_t)m,
                                                        w.part.p);
@@ -1238,7 +1239,8 @@ PtStochResult pt_semistochastic(const Det2* dets, size_t n, const double* c_dev,
       w.perm.resize((size_t)m);
       k_pt_iota<<<grid_for((size_t)m, 256), 256, 0, s>>>(w.perm.p, (size_t)m);
       SHCI_LAUNCH_CHECK();
-      sort_u128(w.key0.p, w.key1.p, w.perm.p, (size_t)m, pr, s);
+      sort_u128(w.key0.p, w.key1.p, w.perm.p, (size_t)m, std::min(64, 2 * ints.norb), std::max(0, 2 * ints.norb - 64),
+                pr, s);
       k_pt_reduce_stoch<<<kPtRedBlocks, kPtRedThreads, 0, s>>>(w.key0.p, w.key1.p, w.perm.p, w.ne.p, w.n2p.p,
                                                                (size_t)m, f, w.part.p);
       SHCI_LAUNCH_CHECK();

@@ -435,7 +435,7 @@ __global__ void k_trev_compact(const Det2* __restrict__ q, size_t n, const int64
     if (flag[i]) out[pos[i]] = flip_it ? det_flip_pair(q[i]) : q[i];
 }
 
-size_t trev_new_dets(Det2* cand, size_t n, const DetHash& present, const Det2* dets, Det2* out, DevBuf<int64_t>& flag,
+size_t trev_new_dets(Det2* cand, size_t n, int norb, const DetHash& present, const Det2* dets, Det2* out, DevBuf<int64_t>& flag,
                      DevBuf<int64_t>& pos, Prims& pr, cudaStream_t s) {
   if (n == 0) return 0;
   size_t blocks = std::min<size_t>((n + 255) / 256, 152 * 32);
@@ -443,7 +443,7 @@ size_t trev_new_dets(Det2* cand, size_t n, const DetHash& present, const Det2* d
   // sorted and unique (:992-994), without those already present (:996-997)
   k_make_standard<<<(unsigned)blocks, 256, 0, s>>>(cand, n);
   SHCI_LAUNCH_CHECK();
-  sort_dets(cand, nullptr, n, pr, s);
+  sort_dets(cand, nullptr, n, norb, pr, s);
   n = unique_dets(cand, n, pr, s);
   blocks = std::min<size_t>((n + 255) / 256, 152 * 32);
   flag.reserve(n);

@@ -1064,10 +1064,12 @@ __device__ __forceinline__ void grid_sums(double (&v)[M], int n, double* __restr
   if (threadIdx.x == 0) *count = 0u;
 }
 
-constexpr int kDavThreads = 512;
-constexpr unsigned kDavBlocks = 152;
+// Two rows a thread before more blocks: half the warps, so half the reductions
+// on an SM's FP64 pipe; large spaces fill the SMs with four blocks each.
+constexpr int kDavThreads = 256;
+constexpr unsigned kDavBlocks = 152 * 4;
 static unsigned dav_blocks(size_t N) {
-  const size_t b = (N + kDavThreads - 1) / kDavThreads;
+  const size_t b = (N + 2 * kDavThreads - 1) / (2 * kDavThreads);
   return (unsigned)(b < 1 ? 1 : (b > kDavBlocks ? kDavBlocks : b));
 }
 size_t dav_scratch() { return (size_t)kDavBlocks * kGramMax; }
@@ -1227,8 +1229,14 @@ void dav_correction(const double* V, size_t ld, int m, const double* X, const do
 // out = c / sqrt(g[0]) (unscaled when linearly dependent, for the host to drop)
 __global__ void k_append_unit(const double* __restrict__ c, size_t N, const double* __restrict__ g,
                               double* __restrict__ out) {
-  const double nrm = sqrt(g[0]);
-  const double sc = nrm > 1e-14 ? 1.0 / nrm : 1.0;
+  // one thread's square root and division, not every thread's
+  __shared__ double s_sc;
+  if (threadIdx.x == 0) {
+    const double nrm = sqrt(g[0]);
+    s_sc = nrm > 1e-14 ? 1.0 / nrm : 1.0;
+  }
+  __syncthreads();
+  const double sc = s_sc;
   for (size_t r = (size_t)blockIdx.x * blockDim.x + threadIdx.x; r < N; r += (size_t)gridDim.x * blockDim.x)
     out[r] = c[r] * sc;
 }
