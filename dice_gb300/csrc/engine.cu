@@ -1091,10 +1091,9 @@ struct Context {
       launch_body(((uint64_t)2 << 60) | ((uint64_t)m << 40) | ((uint64_t)keep << 20) | amask, [&]() {
         if (nact == 1) {
           const size_t c = (size_t)act[0] * N;
-          dav_correction(V.p, N, m, X.p + c, Y.p + c, pin + kPinAct, diag.p, shiftp, sector != 0 ? flipidx.p : nullptr,
-                         flipsgn.p, (double)sector, N, D.p, dw, dG.p, dG.p + 16, dnrm.p, pin + kPinNrm, stream);
-          if (collapse) dav_collapse(V.p, W.p, N, m, pin + kPinQ, keep, N, stream);
-          dav_append(D.p, N, dnrm.p, V.p + (size_t)m1 * N, stream);
+          dav_correction(V.p, W.p, N, m, X.p + c, Y.p + c, pin + kPinAct, diag.p, shiftp,
+                         sector != 0 ? flipidx.p : nullptr, flipsgn.p, (double)sector, N, D.p, dw, dG.p, dG.p + 16,
+                         collapse ? pin + kPinQ : nullptr, keep, m1, dnrm.p, pin + kPinNrm, stream);
           apply_sigma(mode, V.p, N, m1, 1, W.p, N, m1);
           // only the new column of G = V^T W
           dav_column(V.p, N, m1 + 1, W.p + (size_t)m1 * N, N, dw, pin + kPinG, stream);

@@ -428,12 +428,13 @@ void dav_ritz(const double* V, const double* W, size_t ld, int m, const double* 
               size_t N, double* X, double* Y, double* R, const DavWork& w, double* rr, cudaStream_t s);
 // D = preconditioned residual of one root (shift and flip may be null; p: the
 // flip sector), made orthogonal to the m columns of V by two classical
-// Gram-Schmidt passes; *nrm and *nrm_out = |D|^2. g1, g2: m doubles each.
-void dav_correction(const double* V, size_t ld, int m, const double* X, const double* Y, const double* lam,
+// Gram-Schmidt passes, normalised and written to V[:, at]; *nrm and *nrm_out =
+// its squared norm before. Q given: V and W are rotated to the keep columns V Q
+// and W Q in the same pass. g1: m, g2: m + 1 doubles.
+void dav_correction(double* V, double* W, size_t ld, int m, const double* X, const double* Y, const double* lam,
                     const double* diag, const double* shift, const int32_t* flip, const int8_t* sign, double p,
-                    size_t N, double* D, const DavWork& w, double* g1, double* g2, double* nrm, double* nrm_out,
-                    cudaStream_t s);
-void dav_append(const double* c, size_t N, const double* g, double* out, cudaStream_t s);
+                    size_t N, double* D, const DavWork& w, double* g1, double* g2, const double* Q, int keep, int at,
+                    double* nrm, double* nrm_out, cudaStream_t s);
 void dav_column(const double* V, size_t ld, int m, const double* w, size_t N, const DavWork& wk, double* out,
                 cudaStream_t s);
 void dav_collapse(double* V, double* W, size_t ld, int m, const double* Q, int keep, size_t N, cudaStream_t s);

@@ -1014,7 +1014,7 @@ void scale_inv_norm(double* c, size_t N, const double* g, cudaStream_t s) {
 // finish adds the blocks' partials, in block order, instead of a second launch.
 // 81,233 determinants, basis of at most 5: an iteration's vector work, 25
 // launches and 8 copies, took 180 us (gram sums 92, products 36, Gram parts 27);
-// now 7 launches.
+// now five launches, 55 us.
 //
 // The small matrices are read from and written to pinned host memory (Q, the
 // eigenvalues, the norms, the new column of the Rayleigh matrix): a few hundred
@@ -1041,7 +1041,7 @@ __device__ __forceinline__ void grid_sums(double (&v)[M], int n, double* __restr
     idx += up ? half : 0;
   }
   for (int q = o; q; q >>= 1) v[0] += __shfl_xor_sync(kFull, v[0], q);
-  if ((lane & (2 * o - 1)) == 0) s_w[w][idx] = v[0];
+  if ((lane & (o ? 2 * o - 1 : 0)) == 0) s_w[w][idx] = v[0];  // one lane of the group that holds value idx
   __syncthreads();
   if ((int)threadIdx.x < n) {
     double s = 0.0;
@@ -1072,7 +1072,7 @@ static unsigned dav_blocks(size_t N) {
   const size_t b = (N + 2 * kDavThreads - 1) / (2 * kDavThreads);
   return (unsigned)(b < 1 ? 1 : (b > kDavBlocks ? kDavBlocks : b));
 }
-size_t dav_scratch() { return (size_t)kDavBlocks * kGramMax; }
+size_t dav_scratch() { return (size_t)kDavBlocks * (kGramMax + 1); }
 
 // X = V Q, Y = W Q, R = Y - X diag(lam) (written where asked for), |R_c|^2.
 template <int M, int NR>
@@ -1172,19 +1172,18 @@ __global__ void __launch_bounds__(kDavThreads) k_dav_correct(const double* __res
   }
   grid_sums<M>(acc, m, part, count, nullptr, 0, G);
 }
-// D -= V g, then G = V^T D (kNorm false) or |D|^2 (kNorm true).
-template <int M, bool kNorm>
+// D -= V g, then G = V^T D and G[m] = |D|^2.
+template <int M>
 __global__ void __launch_bounds__(kDavThreads) k_dav_project(const double* __restrict__ V, size_t ld, int m,
                                                              const double* __restrict__ g, size_t N,
                                                              double* __restrict__ D, double* __restrict__ part,
-                                                             unsigned* __restrict__ count, double* __restrict__ G,
-                                                             double* out) {
+                                                             unsigned* __restrict__ count, double* __restrict__ G) {
   __shared__ double sg[M];
   if ((int)threadIdx.x < m) sg[threadIdx.x] = g[threadIdx.x];
   __syncthreads();
-  double acc[kNorm ? 1 : M];
+  double acc[2 * M];  // the reduction takes a power of two
 #pragma unroll
-  for (int i = 0; i < (kNorm ? 1 : M); ++i) acc[i] = 0.0;
+  for (int i = 0; i < 2 * M; ++i) acc[i] = 0.0;
   for (size_t r = (size_t)blockIdx.x * blockDim.x + threadIdx.x; r < N; r += (size_t)gridDim.x * blockDim.x) {
     double v[M], t = 0.0;
 #pragma unroll
@@ -1194,29 +1193,90 @@ __global__ void __launch_bounds__(kDavThreads) k_dav_project(const double* __res
       if (i < m) t += v[i] * sg[i];
     const double d = D[r] - t;
     D[r] = d;
-    if constexpr (kNorm) {
-      acc[0] += d * d;
-    } else {
 #pragma unroll
-      for (int i = 0; i < M; ++i)
-        if (i < m) acc[i] += v[i] * d;
+    for (int i = 0; i <= M; ++i)
+      if (i < m)
+        acc[i] += v[i] * d;
+      else if (i == m)
+        acc[i] += d * d;
+  }
+  if (m < M) {
+    double low[M];
+#pragma unroll
+    for (int i = 0; i < M; ++i) low[i] = acc[i];
+    grid_sums<M>(low, m + 1, part, count, nullptr, 0, G);
+  } else {
+    grid_sums<2 * M>(acc, m + 1, part, count, nullptr, 0, G);
+  }
+}
+// The second Gram-Schmidt projection, the normalisation and the append in one
+// pass, with the rotation of V and W when the basis collapses (Q given: keep
+// columns; in place, every thread owns its row): V[:, at] = (D - V g) / |D - V g|.
+// |D - V g|^2 = |D|^2 - |g|^2, V being orthonormal and g a rounding residue;
+// a dependent D (norm below 1e-14) is left for the host to drop.
+template <int M>
+__global__ void __launch_bounds__(256) k_dav_append(double* __restrict__ V, double* __restrict__ W, size_t ld, int m,
+                                                    const double* __restrict__ g, size_t N,
+                                                    const double* __restrict__ D, const double* Q, int keep, int at,
+                                                    double* nrm, double* nrm_out) {
+  __shared__ double sQ[kGramMax * kGramMax];
+  __shared__ double sg[M], s_sc;
+  if (Q)
+    for (int e = threadIdx.x; e < m * keep; e += blockDim.x) sQ[e] = Q[e];
+  if ((int)threadIdx.x < m) sg[threadIdx.x] = g[threadIdx.x];
+  __syncthreads();
+  if (threadIdx.x == 0) {  // one thread's square root and division, not every thread's
+    double n2 = g[m];
+    for (int i = 0; i < m; ++i) n2 -= sg[i] * sg[i];
+    const double n = sqrt(n2);
+    s_sc = n > 1e-14 ? 1.0 / n : 1.0;
+    if (blockIdx.x == 0) {
+      *nrm = n2;
+      *nrm_out = n2;
     }
   }
-  grid_sums<(kNorm ? 1 : M)>(acc, kNorm ? 1 : m, part, count, out, 1, G);
+  __syncthreads();
+  const double sc = s_sc;
+  for (size_t r = (size_t)blockIdx.x * blockDim.x + threadIdx.x; r < N; r += (size_t)gridDim.x * blockDim.x) {
+    double v[M], t = 0.0;
+#pragma unroll
+    for (int i = 0; i < M; ++i) v[i] = i < m ? V[(size_t)i * ld + r] : 0.0;
+#pragma unroll
+    for (int i = 0; i < M; ++i)
+      if (i < m) t += v[i] * sg[i];
+    const double d = (D[r] - t) * sc;
+    if (Q) {
+      double w[M];
+#pragma unroll
+      for (int i = 0; i < M; ++i) w[i] = i < m ? W[(size_t)i * ld + r] : 0.0;
+      for (int c = 0; c < keep; ++c) {
+        double x = 0.0, y = 0.0;
+#pragma unroll
+        for (int i = 0; i < M; ++i)
+          if (i < m) {
+            x += v[i] * sQ[c * m + i];
+            y += w[i] * sQ[c * m + i];
+          }
+        V[(size_t)c * ld + r] = x;
+        W[(size_t)c * ld + r] = y;
+      }
+    }
+    V[(size_t)at * ld + r] = d;
+  }
 }
-void dav_correction(const double* V, size_t ld, int m, const double* X, const double* Y, const double* lam,
+void dav_correction(double* V, double* W, size_t ld, int m, const double* X, const double* Y, const double* lam,
                     const double* diag, const double* shift, const int32_t* flip, const int8_t* sign, double p,
-                    size_t N, double* D, const DavWork& w, double* g1, double* g2, double* nrm, double* nrm_out,
-                    cudaStream_t s) {
-  if (m > kGramMax) throw Error(kErrInvalid, "Gram block too wide");
+                    size_t N, double* D, const DavWork& w, double* g1, double* g2, const double* Q, int keep, int at,
+                    double* nrm, double* nrm_out, cudaStream_t s) {
+  if (m > kGramMax || keep > m) throw Error(kErrInvalid, "Gram block too wide");
   const unsigned nb = dav_blocks(N);
 #define SHCI_CORR(M)                                                                                                 \
   k_dav_correct<M><<<nb, kDavThreads, 0, s>>>(V, ld, m, X, Y, lam, diag, shift, flip, sign, p, N, D, w.part, w.count, \
                                               g1);                                                                   \
   SHCI_LAUNCH_CHECK();                                                                                               \
-  k_dav_project<M, false><<<nb, kDavThreads, 0, s>>>(V, ld, m, g1, N, D, w.part, w.count, g2, nullptr);              \
+  k_dav_project<M><<<nb, kDavThreads, 0, s>>>(V, ld, m, g1, N, D, w.part, w.count, g2);                              \
   SHCI_LAUNCH_CHECK();                                                                                               \
-  k_dav_project<M, true><<<nb, kDavThreads, 0, s>>>(V, ld, m, g2, N, D, w.part, w.count, nrm, nrm_out);              \
+  k_dav_append<M><<<grid_for(N, 256), 256, 0, s>>>(V, W, ld, m, g2, N, D, Q, keep, at, nrm, nrm_out);                \
   SHCI_LAUNCH_CHECK()
   if (m <= 8) {
     SHCI_CORR(8);
@@ -1224,25 +1284,6 @@ void dav_correction(const double* V, size_t ld, int m, const double* X, const do
     SHCI_CORR(16);
   }
 #undef SHCI_CORR
-}
-
-// out = c / sqrt(g[0]) (unscaled when linearly dependent, for the host to drop)
-__global__ void k_append_unit(const double* __restrict__ c, size_t N, const double* __restrict__ g,
-                              double* __restrict__ out) {
-  // one thread's square root and division, not every thread's
-  __shared__ double s_sc;
-  if (threadIdx.x == 0) {
-    const double nrm = sqrt(g[0]);
-    s_sc = nrm > 1e-14 ? 1.0 / nrm : 1.0;
-  }
-  __syncthreads();
-  const double sc = s_sc;
-  for (size_t r = (size_t)blockIdx.x * blockDim.x + threadIdx.x; r < N; r += (size_t)gridDim.x * blockDim.x)
-    out[r] = c[r] * sc;
-}
-void dav_append(const double* c, size_t N, const double* g, double* out, cudaStream_t s) {
-  k_append_unit<<<grid_for(N, 256), 256, 0, s>>>(c, N, g, out);
-  SHCI_LAUNCH_CHECK();
 }
 
 // out[i] = V_i . w for the m columns of V (pinned host memory)
