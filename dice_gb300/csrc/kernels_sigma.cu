@@ -75,7 +75,7 @@ struct VecF<4> {
 // from a shared-memory counter. Consecutive rows of the determinant order are
 // close determinants with largely the same connections, so the rows one block
 // runs together gather the same parts of x and hit in L1 (launched as two
-// 1024-thread blocks per SM, one wave).
+// blocks per SM, one wave).
 // Several vectors: the grid strides over the rows (x is k times larger and
 // the band of rows the whole GPU works on at once is what stays in cache).
 //
@@ -83,7 +83,10 @@ struct VecF<4> {
 // determinants' rows hold tens of times the mean (19,739 of 80,730 columns
 // against 881), and one warp on such a row outlasts the rest of the launch: in
 // the balanced walk their pieces are put aside and shared by the block's warps
-// after its other rows. The sums are the same either way.
+// after its other rows (Body::kAside). The sums are the same either way. The FP32
+// bodies put nothing aside: the second phase's registers cost their first more
+// than the tail (k = 2, 16,068 rows 34 -> 32 us without, compact copy 30 -> 19 us,
+// and 2.47 -> 2.41 ms at 1.2 million).
 constexpr int kTasks = 96;  // pieces a block can put aside; further long rows stay with their warp
 
 // First index of the ascending a[0, n) with a[i] >= v, found by a warp: 32
@@ -150,9 +153,10 @@ __device__ __forceinline__ void walk_rows(const int64_t* __restrict__ rowptr, si
       uint32_t row;
       int piece;
     };
+    constexpr bool kAside = VW == 32 && Body::kAside;
     __shared__ unsigned s_next, s_end, s_tasks, s_task_next;  // rows are below 2^31
-    __shared__ Task s_task[VW == 32 ? kTasks : 1];
-    __shared__ A s_acc[VW == 32 ? kTasks : 1][Body::KP];
+    __shared__ Task s_task[kAside ? kTasks : 1];
+    __shared__ A s_acc[kAside ? kTasks : 1][Body::KP];
     const int warp = threadIdx.x >> 5;
     if (warp < 2) {
       const int64_t nnz = rowptr[N];
@@ -162,7 +166,7 @@ __device__ __forceinline__ void walk_rows(const int64_t* __restrict__ rowptr, si
       if (lane == 0) (warp ? s_end : s_next) = (unsigned)r;
     }
     if (threadIdx.x == 64) s_tasks = s_task_next = 0;
-    if (VW == 32 && threadIdx.x >= 128 && threadIdx.x < 128 + kTasks) s_task[threadIdx.x - 128].row = 0xffffffffu;
+    if (kAside && threadIdx.x >= 128 && threadIdx.x < 128 + kTasks) s_task[threadIdx.x - 128].row = 0xffffffffu;
     __syncthreads();
     const unsigned end = s_end;
     while (true) {
@@ -173,7 +177,7 @@ __device__ __forceinline__ void walk_rows(const int64_t* __restrict__ rowptr, si
       const size_t pos = wr + lane / VW;
       const bool live = pos < end;
       const int64_t p0 = live ? __ldg(rowptr + pos) : 0, p1 = live ? __ldg(rowptr + pos + 1) : 0;
-      if constexpr (VW == 32) {
+      if constexpr (kAside) {
         if (p1 - p0 > kPiece) {
           const int np = (int)((p1 - p0 + kPiece - 1) / kPiece);
           int at = kTasks;
@@ -189,7 +193,7 @@ __device__ __forceinline__ void walk_rows(const int64_t* __restrict__ rowptr, si
       }
       sum_row<VW, Body>(k, live ? pos : 0, live, p0, p1);
     }
-    if constexpr (VW == 32) {
+    if constexpr (kAside) {
       __syncthreads();
       const int nt = (int)(s_tasks < (unsigned)kTasks ? s_tasks : (unsigned)kTasks);
       if (nt == 0) return;
@@ -260,12 +264,16 @@ struct DoubleSum {
 };
 
 // FP32 sigma on int32 columns. One and two vectors walk balanced row ranges
-// (two 1024-thread blocks per SM); four vectors the grid-strided rows, which is
+// (two blocks per SM); four vectors the grid-strided rows, which is
 // faster there (mol24, 2.91 M determinants: k = 2 10.8 ms balanced against
 // 12.6 ms strided; k = 4 20.6 ms against 16.9 ms).
+// Four blocks per SM, 64 registers: the unrolled gathers stay in flight (202,439
+// determinants of 36 orbitals, k = 4: 808 us; 852 with the compiler's 71 registers,
+// 882 with five blocks, 900 with six, 1105 with eight).
 template <int KP_>
 struct MixedBody : AccSum {
   static constexpr int KP = KP_;
+  static constexpr bool kAside = false;
   static constexpr int kPiece = 4096;
   const int32_t* __restrict__ col;
   const float* __restrict__ val;
@@ -305,7 +313,7 @@ struct MixedBody : AccSum {
   }
 };
 template <int VW, int KP, bool kBalWalk = (KP <= 2)>
-__global__ void __launch_bounds__(kBalWalk ? 1024 : 256, kBalWalk ? 2 : 1)
+__global__ void __launch_bounds__(kBalWalk ? 1024 : 256, kBalWalk ? 2 : 4)
     k_sigma_mixed(const int64_t* __restrict__ rowptr, size_t N, const __grid_constant__ MixedBody<KP> k) {
   walk_rows<VW, kBalWalk>(rowptr, N, k);
 }
@@ -323,6 +331,7 @@ __global__ void __launch_bounds__(kBalWalk ? 1024 : 256, kBalWalk ? 2 : 1)
 // 2.52 ms, 83 % of the measured copy bandwidth.
 struct MixedCompactBody : AccSum {
   static constexpr int KP = 1;
+  static constexpr bool kAside = false;
   static constexpr int kPiece = 4096;
   const uint16_t* __restrict__ clo;
   const uint8_t* __restrict__ chi;
@@ -458,6 +467,7 @@ void compress_csr(Csr& H, Prims& pr, cudaStream_t s) {
 template <int KP_>
 struct F64Body : DoubleSum {
   static constexpr int KP = KP_;
+  static constexpr bool kAside = KP == 1;
   static constexpr int kPiece = 2048;  // 1024: 25.4 ms, 2048: 23.9 ms, 4096: 27.2 ms for 126 sigmas of 81,233 rows
   const int32_t* __restrict__ col;
   const double* __restrict__ v64;
@@ -496,8 +506,14 @@ struct F64Body : DoubleSum {
       if (c < k) y[(size_t)c * ldy + o] = dg * x[xr * KP + c] + acc[c];
   }
 };
+// One FP64 vector runs as two blocks of 768 threads per SM: 42 registers keep a
+// row's loads in flight that 1024 threads' 32 do not (16,068 rows 45.7 -> 40.3 us,
+// 82,090 rows 194.6 -> 190.1; 512 x 3 and x 4 slower at 250,000). The FP32 and
+// float-float bodies are faster with 1024 (refine at 200,836 rows 488 against
+// 517 us, compact copy at 1.2 million 2.50 against 2.69 ms).
+constexpr int kF64Threads = 768;
 template <int VW, int KP>
-__global__ void __launch_bounds__(KP == 1 ? 1024 : 256, KP == 1 ? 2 : 1)
+__global__ void __launch_bounds__(KP == 1 ? kF64Threads : 256, KP == 1 ? 2 : 1)
     k_sigma_f64(const int64_t* __restrict__ rowptr, size_t N, const __grid_constant__ F64Body<KP> k) {
   walk_rows<VW, KP == 1>(rowptr, N, k);
 }
@@ -554,6 +570,7 @@ struct VecFF<4> {
 template <int KP_>
 struct FFBody : AccSum {
   static constexpr int KP = KP_;
+  static constexpr bool kAside = KP == 1;
   static constexpr int kPiece = 4096;
   const int32_t* __restrict__ col;
   const float* __restrict__ vhi;
@@ -599,7 +616,7 @@ __global__ void __launch_bounds__(KP == 1 ? 1024 : 256, KP == 1 ? 2 : 1)
 }
 
 // Launch shape of the stored-matrix sigma kernels (see walk_rows): one vector
-// runs as two 1024-thread blocks per SM over nonzero-balanced row ranges;
+// runs as two blocks of `threads1` per SM over nonzero-balanced row ranges;
 // several vectors as a grid-strided launch of 256-thread blocks.
 struct SigmaLaunch {
   unsigned blocks;
@@ -614,8 +631,8 @@ static int sm_count() {
   }();
   return n;
 }
-static SigmaLaunch sigma_launch(size_t N, int vw, int kp) {
-  if (kp == 1) return SigmaLaunch{(unsigned)(2 * sm_count()), 1024};
+static SigmaLaunch sigma_launch(size_t N, int vw, int kp, int threads1 = 1024) {
+  if (kp == 1) return SigmaLaunch{(unsigned)(2 * sm_count()), threads1};
   return SigmaLaunch{grid_for(N * (size_t)vw, 256, (size_t)sm_count() * 16), 256};
 }
 
@@ -661,7 +678,7 @@ void sigma_csr_mixed(const Csr& H, const double* diag, const float* x32, int kp,
 template <int KP>
 static void launch_f64(int vw, const Csr& H, const double* diag, const double* x, int k, double* y, size_t ldy,
                        cudaStream_t s) {
-  const SigmaLaunch L = sigma_launch(H.N, vw, KP);
+  const SigmaLaunch L = sigma_launch(H.N, vw, KP, kF64Threads);
   const F64Body<KP> b{{}, H.col.p, H.v64.p, diag, x, k, y, ldy, H.perm.p, H.block ? H.xpos.p : nullptr};
   switch (vw) {
     case 32: k_sigma_f64<32, KP><<<L.blocks, L.threads, 0, s>>>(H.rowptr.p, H.N, b); break;
