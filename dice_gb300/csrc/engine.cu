@@ -294,6 +294,14 @@ struct Context {
   // captured Davidson iterations: graph per (phase, basis size, active roots)
   bool use_graphs = true;
   bool sigma_deferred = false;  // apply_sigma inside a capture: timing read later
+  bool sigma_untimed = false;   // apply_sigma before a synchronisation of the caller's: timing read then
+  // Host vectors of a small shci_sigma pass through this pinned memory: the
+  // pack kernel reads x from it, and the copy of y back does not stage. Up to
+  // 8,192 entries, where a copy engine's round trip costs more than the packing
+  // loses to the link (4,027 determinants 53 -> 41 us, 8,185 73 -> 58; with four
+  // vectors of 8,185 107 against 113).
+  static constexpr size_t kStage = 8192;  // doubles each way
+  double* stage = nullptr;
   std::unordered_map<uint64_t, std::pair<cudaGraphExec_t, int64_t>> gcache;
   double* pin = nullptr;  // pinned staging for the small matrices (kPin doubles)
   static constexpr int kPinQ = 0, kPinLam = 256, kPinAct = 272, kPinRR = 288, kPinG = 544, kPinNrm = 800,
@@ -343,6 +351,7 @@ struct Context {
   ~Context() {
     graphs_clear();
     if (pin) cudaFreeHost(pin);
+    if (stage) cudaFreeHost(stage);
     if (ev0) cudaEventDestroy(ev0);
     if (ev1) cudaEventDestroy(ev1);
     if (stream) cudaStreamDestroy(stream);
@@ -795,12 +804,41 @@ struct Context {
       done += kk;
     }
     SHCI_CUDA(cudaEventRecordWithFlags(ev1, stream, evflag));
-    if (sigma_deferred) return;  // captured: the caller reads the events after the replay
+    if (sigma_deferred || sigma_untimed) return;  // the caller reads the events after the replay / its synchronisation
     SHCI_CUDA(cudaEventSynchronize(ev1));
+    count_sigma();
+  }
+  void count_sigma() {
     float ms = 0.f;
     SHCI_CUDA(cudaEventElapsedTime(&ms, ev0, ev1));
     t_sigma += ms * 1e-3;
     n_sigma += 1;
+  }
+
+  // Y = H X on host vectors (column-major, ndet x k).
+  void sigma_host(int mode, const double* x, double* y, int k) {
+    const size_t n = ndet * (size_t)k;
+    struct Untimed {
+      bool& v;
+      explicit Untimed(bool& f) : v(f) { v = true; }
+      ~Untimed() { v = false; }
+    } untimed(sigma_untimed);
+    Y.reserve(n);
+    ensure_diag();
+    if (n <= kStage) {
+      std::memcpy(stage, x, n * sizeof(double));
+      apply_sigma(mode, stage, ndet, 0, k, Y.p, ndet, 0);
+      SHCI_CUDA(cudaMemcpyAsync(stage + kStage, Y.p, n * sizeof(double), cudaMemcpyDeviceToHost, stream));
+      SHCI_CUDA(cudaStreamSynchronize(stream));
+      std::memcpy(y, stage + kStage, n * sizeof(double));
+    } else {
+      X.reserve(n);
+      SHCI_CUDA(cudaMemcpyAsync(X.p, x, n * sizeof(double), cudaMemcpyHostToDevice, stream));
+      apply_sigma(mode, X.p, ndet, 0, k, Y.p, ndet, 0);
+      SHCI_CUDA(cudaMemcpyAsync(y, Y.p, n * sizeof(double), cudaMemcpyDeviceToHost, stream));
+      SHCI_CUDA(cudaStreamSynchronize(stream));
+    }
+    count_sigma();
   }
 
   // ---- Davidson -----------------------------------------------------------
@@ -1698,6 +1736,7 @@ int shci_ctx_create(int device, shci_ctx** out) {
     SHCI_CUDA(cudaEventCreate(&ctx->c.ev0));
     SHCI_CUDA(cudaEventCreate(&ctx->c.ev1));
     SHCI_CUDA(cudaMallocHost(&ctx->c.pin, Context::kPin * sizeof(double)));
+    SHCI_CUDA(cudaMallocHost(&ctx->c.stage, 2 * Context::kStage * sizeof(double)));
     *out = ctx.release();
     return SHCI_OK;
   } catch (const Error& e) {
@@ -1973,14 +2012,7 @@ int shci_sigma(shci_ctx* ctx, int mode, const double* x, double* y, int k) {
   return guarded(ctx, [&](Context& c) {
     if (k < 1 || k > 4) throw Error(SHCI_ERR_INVALID, "k must be in 1..4");
     if (!x || !y) throw Error(SHCI_ERR_INVALID, "null vector");
-    const size_t N = c.ndet;
-    c.X.reserve(N * k);
-    c.Y.reserve(N * k);
-    SHCI_CUDA(cudaMemcpyAsync(c.X.p, x, N * k * sizeof(double), cudaMemcpyHostToDevice, c.stream));
-    c.ensure_diag();
-    c.apply_sigma(mode, c.X.p, N, 0, k, c.Y.p, N, 0);
-    SHCI_CUDA(cudaMemcpyAsync(y, c.Y.p, N * k * sizeof(double), cudaMemcpyDeviceToHost, c.stream));
-    SHCI_CUDA(cudaStreamSynchronize(c.stream));
+    c.sigma_host(mode, x, y, k);
   });
 }
 
