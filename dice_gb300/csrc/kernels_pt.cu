@@ -881,46 +881,112 @@ __global__ void __launch_bounds__(kPtRedThreads) k_pt_reduce(const uint64_t* __r
 // thread per run of equal determinants: with S1, S2 the sums of the two
 // numerators (and S1B, S2B over the contributions flagged as already held by
 // the deterministic part), eA = sum (S1^2 f - S2) / (E_a - E0) and eB likewise
-// (SHCI/SHCIbasics.cpp:271-363). Sums in fixed point as in k_pt_reduce; block
-// partials {eA, eB, runs} in part[3 * block].
+// (SHCI/SHCIbasics.cpp:271-363). Block partials {eA, eB, runs} in
+// part[3 * block].
+//
+// Bound by the FP64 pipe, where a warp's operation takes 16 cycles whatever the
+// number of lanes that take part: the runs' first positions wait in two queues
+// of the warp, short runs (one or two elements) and longer ones apart, and are
+// evaluated 32 at a time. A run of one is taken as it is and a run of two by one
+// addition, which no order of the two changes; only the longer ones go through
+// the fixed-point sums of k_pt_reduce and their conversions (some 3 million candidates
+// 184 -> 120 us; one thread a run where it stands, with the same short sums, 155).
 __global__ void __launch_bounds__(kPtRedThreads) k_pt_reduce_stoch(const uint64_t* __restrict__ k0,
                                                                    const uint64_t* __restrict__ k1,
                                                                    const uint32_t* __restrict__ perm,
                                                                    const float4* __restrict__ ne,
                                                                    const double2* __restrict__ n2p, size_t m, double f,
                                                                    double* __restrict__ part) {
-  double eA = 0.0, eB = 0.0, cnt = 0.0;
-  for (size_t k = (size_t)blockIdx.x * blockDim.x + threadIdx.x; k < m; k += (size_t)gridDim.x * blockDim.x) {
-    const uint64_t d0 = k0[k], d1 = k1[k];
-    if (k > 0 && d0 == k0[k - 1] && d1 == k1[k - 1]) continue;
-    __int128 s1 = 0, s2 = 0, s1b = 0, s2b = 0;
-    bool flagged = false;
-    float2 e = make_float2(INFINITY, 0.0f);
-    for (size_t j = k; j < m; ++j) {
-      if (j > k && (k0[j] != d0 || k1[j] != d1)) break;
-      const uint32_t pk = perm[j];
-      const float4 x = ne[pk];
-      const double2 y = n2p[pk];
-      const __int128 f1 = to_fix(y.x), f2 = to_fix(y.y);
-      s1 += f1;
-      s2 += f2;
-      if (x.x != 0.0f) {
-        s1b += f1;
-        s2b += f2;
-        flagged = true;
+  __shared__ uint32_t s_run[kPtRedThreads / 32][2][64];
+  const int lane = threadIdx.x & 31;
+  const unsigned lt = (1u << lane) - 1u;
+  uint32_t(*run)[64] = s_run[threadIdx.x >> 5];
+  unsigned head[2] = {0, 0}, held[2] = {0, 0};  // warp-uniform
+  double eA = 0.0, eB = 0.0;
+  unsigned runs = 0;
+  auto same = [&](size_t i, size_t j) { return k0[i] == k0[j] && k1[i] == k1[j]; };
+  auto term = [&](double n1, double n2, float2 e) {
+    return (n1 * n1 * f - n2) / ((double)e.x + (double)e.y);  // over E_a - E0
+  };
+  auto flush = [&](auto longer, unsigned c) {
+    constexpr bool kLong = decltype(longer)::value;
+    if ((unsigned)lane < c) {
+      const size_t k = run[kLong][(head[kLong] + lane) & 63u];
+      double n1, n2, n1b, n2b;
+      bool flagged;
+      float2 e;
+      if constexpr (kLong) {
+        __int128 s1 = 0, s2 = 0, s1b = 0, s2b = 0;
+        flagged = false;
+        e = make_float2(INFINITY, 0.0f);
+        for (size_t j = k; j < m && (j < k + 3 || same(j, k)); ++j) {
+          const uint32_t pk = perm[j];
+          const float4 x = ne[pk];
+          const double2 y = n2p[pk];
+          const __int128 f1 = to_fix(y.x), f2 = to_fix(y.y);
+          s1 += f1;
+          s2 += f2;
+          if (x.x != 0.0f) {
+            s1b += f1;
+            s2b += f2;
+            flagged = true;
+          }
+          const float2 ej = make_float2(x.z, x.w);
+          if (ff_less(ej, e)) e = ej;
+        }
+        n1 = from_fix(s1);
+        n2 = from_fix(s2);
+        n1b = flagged ? from_fix(s1b) : 0.0;
+        n2b = flagged ? from_fix(s2b) : 0.0;
+      } else {
+        const uint32_t pk = perm[k];
+        const bool two = k + 1 < m && same(k + 1, k);
+        const uint32_t pl = perm[two ? k + 1 : k];
+        const float4 x = ne[pk], xl = ne[pl];
+        const double2 y = n2p[pk], yl = n2p[pl];
+        flagged = x.x != 0.0f;
+        n1 = y.x;
+        n2 = y.y;
+        n1b = flagged ? n1 : 0.0;
+        n2b = flagged ? n2 : 0.0;
+        e = make_float2(x.z, x.w);
+        if (two) {
+          n1 += yl.x;
+          n2 += yl.y;
+          if (xl.x != 0.0f) {
+            n1b += yl.x;
+            n2b += yl.y;
+            flagged = true;
+          }
+          const float2 el = make_float2(xl.z, xl.w);
+          if (ff_less(el, e)) e = el;
+        }
       }
-      const float2 ej = make_float2(x.z, x.w);
-      if (ff_less(ej, e)) e = ej;
+      eA += term(n1, n2, e);
+      if (flagged) eB += term(n1b, n2b, e);  // without a deterministic part none is
+      runs += 1;
     }
-    const double de = (double)e.x + (double)e.y;  // E_a - E0
-    const double n1 = from_fix(s1);
-    eA += (n1 * n1 * f - from_fix(s2)) / de;
-    if (flagged) {  // without a deterministic part nothing is: its FP64 work is half of the kernel's
-      const double n1b = from_fix(s1b);
-      eB += (n1b * n1b * f - from_fix(s2b)) / de;
-    }
-    cnt += 1.0;
+    head[kLong] += c;
+    held[kLong] -= c;
+    __syncwarp();
+  };
+  const size_t step = (size_t)gridDim.x * blockDim.x;
+  for (size_t b = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) & ~(size_t)31; b < m; b += step) {
+    const size_t q = b + lane;
+    const bool first = q < m && (q == 0 || !same(q, q - 1));
+    const bool longer = first && q + 2 < m && same(q + 2, q);  // the keys ascend
+    const unsigned ml = __ballot_sync(kFull, longer), ms = __ballot_sync(kFull, first && !longer);
+    if (first)
+      run[longer][(head[longer] + held[longer] + __popc((longer ? ml : ms) & lt)) & 63u] = (uint32_t)q;
+    held[0] += __popc(ms);
+    held[1] += __popc(ml);
+    __syncwarp();
+    if (held[0] >= 32) flush(std::false_type{}, 32);
+    if (held[1] >= 32) flush(std::true_type{}, 32);
   }
+  if (held[0]) flush(std::false_type{}, held[0]);
+  if (held[1]) flush(std::true_type{}, held[1]);
+  double cnt = (double)runs;
   __shared__ double r0[kPtRedThreads / 32], r1[kPtRedThreads / 32], r2[kPtRedThreads / 32];
   for (int o = 16; o; o >>= 1) {
     eA += __shfl_xor_sync(kFull, eA, o);
