@@ -542,114 +542,122 @@ __global__ void __launch_bounds__(kPtThreads) k_pt_gen(PtArgs a) {
       qh = (qh + cnt) & 63u;
       qn -= cnt;
       __syncwarp();
-      if (rn >= 32) write(32);
     };
 
-    // ---- singles: every same-spin (i, a) (a spin flip has a zero element:
-    // I1 has no alpha-beta block); FP32 screen here, the rest when drained
     const int ncB = nclosed - ncA, nhB = n - ncB;
     const int nsA = ncA * nhA, ns = nsA + ncB * nhB;
-    for (int b0 = 32 * slice; b0 < ns; b0 += 32 * slices) {
-      const int q = b0 + lane;
-      bool surv = false;
-      int ci = 0, oa = 0;
-      if (q < ns) {
-        if (q < nsA) {
-          ci = cspin[q / nhA];
-          oa = open[q % nhA];
-        } else {
-          ci = cspin[ncA + (q - nsA) / nhB];
-          oa = open[nhA + (q - nsA) % nhB];
-        }
-        bool ok = true;
-        for (int r = 0; ok && r < sp.nrestrict; ++r) {
-          int c2 = cur[r] - in_mask(sp, r, ci) + in_mask(sp, r, oa);
-          ok = c2 >= sp.rmin[r] && c2 <= sp.rmax[r];
-        }
-        surv = ok && single_screen(a, d, oa, ci, eps_lo, eps_hi) >= 0;
-      }
-      push(surv, (uint32_t)ci | 0xff00u | ((uint32_t)oa << 16) | 0xff000000u, 0.0f);
-      if (qn >= 32) drain(32);
-    }
-    while (qn > 0) drain(qn < 32 ? qn : 32);
-
-    // ---- doubles: heat-bath list prefixes, flattened over the warp
-    if (fabs(a.maxEntry) < eps) {
-      if (rn > 0) write(rn);
-      continue;
-    }
     // for a float v, (double)|v| < eps exactly when |v| < eps rounded up to float
     const float eps_f = __double2float_ru(eps);
-    const int npairs = nclosed * (nclosed - 1) / 2;
-    // this slice's pairs: q = slice, slice + slices, ...
-    for (int pb = slice; pb < npairs; pb += 32 * slices) {
-      const int q = pb + lane * slices;
-      int ci = 0, cj = 0, len = 0;
-      uint32_t lstart = 0;
-      bool same = false;
-      if (q < npairs) {
-        // q -> (i, j), i > j, q = i(i-1)/2 + j
-        int i = (int)((1.0f + sqrtf(1.0f + 8.0f * (float)q)) * 0.5f);  // corrected below
-        while (i * (i - 1) / 2 > q) --i;
-        while ((i + 1) * i / 2 <= q) ++i;
-        const int j = q - i * (i - 1) / 2;
-        ci = closed[i];
-        cj = closed[j];
-        const int I = ci >> 1, J = cj >> 1;
-        const int X = I > J ? I : J, Y = I > J ? J : I;
-        const int pair = X * (X + 1) / 2 + Y;
-        same = (ci & 1) == (cj & 1);
-        const int64_t* st = same ? a.hb.sameStart : a.hb.oppStart;
-        const float* vals = same ? a.hb.sameVal : a.hb.oppVal;
-        lstart = (uint32_t)st[pair];
-        len = prefix_length(vals + lstart, (int)((uint32_t)st[pair + 1] - lstart), eps_f);
-      }
-      int incl = len;
-#pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        const int y = __shfl_up_sync(kFull, incl, o);
-        if (lane >= o) incl += y;
-      }
-      const int total = __shfl_sync(kFull, incl, 31);
-      const int excl = incl - len;
-      const uint32_t off = lstart - (uint32_t)excl;  // list index of flat entry f: off of its owner + f
-      const uint32_t who = (uint32_t)ci | ((uint32_t)cj << 8) | (same ? 0x10000u : 0u);
-      for (int f0 = 0; f0 < total; f0 += 32) {
-        const int f = f0 + lane;
-        // owner lane of flat entry f: last lane with excl <= f
-        int lo = 0;
-#pragma unroll
-        for (int st = 16; st >= 1; st >>= 1) {
-          const int e2 = __shfl_sync(kFull, excl, lo + st);
-          if (e2 <= f) lo += st;
-        }
-        const uint32_t index = __shfl_sync(kFull, off, lo) + (uint32_t)f;
-        const uint32_t ow = __shfl_sync(kFull, who, lo);
-        bool surv = false;
-        uint32_t w = 0;
-        float vf = 0.0f;
-        if (f < total) {
-          const bool osame = (ow & 0x10000u) != 0;
-          const int oci = ow & 0xff, ocj = (ow >> 8) & 0xff;
-          const short2 pr = __ldg(reinterpret_cast<const short2*>(osame ? a.hb.samePairs : a.hb.oppPairs) + index);
-          const int av = 2 * pr.x + (oci & 1), bv = 2 * pr.y + (ocj & 1);
+    const int npairs = fabs(a.maxEntry) < eps ? 0 : nclosed * (nclosed - 1) / 2;
+    int b0 = 32 * slice;          // next single excitation
+    int pb = slice;               // next pair of electrons: slice, slice + slices, ...
+    int f0 = 0, total = 0;        // entries of the lists of 32 pairs
+    int excl = 0;                 // a lane's list: first flat entry,
+    uint32_t off = 0, who = 0;    // list index of flat entry f: off of its owner + f; the electrons
+    // One loop over all of a unit's excitations, with one place where either ring
+    // is emptied: with a copy of drain and write behind the singles, the doubles
+    // and each one's end the code outgrew the instruction cache (half of a warp's
+    // wait was for instructions; 39.5 million candidates 6.93 -> 5.40 ms).
+    while (true) {
+      bool surv = false, more = true;
+      uint32_t w = 0;
+      float vf = 0.0f;
+      if (b0 < ns) {
+        // singles: every same-spin (i, a) (a spin flip has a zero element: I1 has
+        // no alpha-beta block); FP32 screen here, the rest when drained
+        const int q = b0 + lane;
+        if (q < ns) {
+          int ci, oa;
+          if (q < nsA) {
+            ci = cspin[q / nhA];
+            oa = open[q % nhA];
+          } else {
+            ci = cspin[ncA + (q - nsA) / nhB];
+            oa = open[nhA + (q - nsA) % nhB];
+          }
           bool ok = true;
           for (int r = 0; ok && r < sp.nrestrict; ++r) {
-            int c2 = cur[r] - in_mask(sp, r, oci) - in_mask(sp, r, ocj) + in_mask(sp, r, av) + in_mask(sp, r, bv);
+            int c2 = cur[r] - in_mask(sp, r, ci) + in_mask(sp, r, oa);
             ok = c2 >= sp.rmin[r] && c2 <= sp.rmax[r];
           }
-          surv = ok && !(occupied<W2>(d, av) || occupied<W2>(d, bv));
-          if (surv) {
-            w = (uint32_t)oci | ((uint32_t)ocj << 8) | ((uint32_t)av << 16) | ((uint32_t)bv << 24);
-            vf = __ldg((osame ? a.hb.sameVal : a.hb.oppVal) + index);
-          }
+          surv = ok && single_screen(a, d, oa, ci, eps_lo, eps_hi) >= 0;
+          w = (uint32_t)ci | 0xff00u | ((uint32_t)oa << 16) | 0xff000000u;
         }
-        push(surv, w, vf);
-        if (qn >= 32) drain(32);
+        b0 += 32 * slices;
+      } else {
+        // doubles: heat-bath list prefixes, flattened over the warp
+        while (f0 >= total && pb < npairs) {
+          const int q = pb + lane * slices;
+          int ci = 0, cj = 0, len = 0;
+          uint32_t lstart = 0;
+          bool same = false;
+          if (q < npairs) {
+            // q -> (i, j), i > j, q = i(i-1)/2 + j
+            int i = (int)((1.0f + sqrtf(1.0f + 8.0f * (float)q)) * 0.5f);  // corrected below
+            while (i * (i - 1) / 2 > q) --i;
+            while ((i + 1) * i / 2 <= q) ++i;
+            const int j = q - i * (i - 1) / 2;
+            ci = closed[i];
+            cj = closed[j];
+            const int I = ci >> 1, J = cj >> 1;
+            const int X = I > J ? I : J, Y = I > J ? J : I;
+            const int pair = X * (X + 1) / 2 + Y;
+            same = (ci & 1) == (cj & 1);
+            const int64_t* st = same ? a.hb.sameStart : a.hb.oppStart;
+            const float* vals = same ? a.hb.sameVal : a.hb.oppVal;
+            lstart = (uint32_t)st[pair];
+            len = prefix_length(vals + lstart, (int)((uint32_t)st[pair + 1] - lstart), eps_f);
+          }
+          int incl = len;
+#pragma unroll
+          for (int o = 1; o < 32; o <<= 1) {
+            const int y = __shfl_up_sync(kFull, incl, o);
+            if (lane >= o) incl += y;
+          }
+          total = __shfl_sync(kFull, incl, 31);
+          excl = incl - len;
+          off = lstart - (uint32_t)excl;
+          who = (uint32_t)ci | ((uint32_t)cj << 8) | (same ? 0x10000u : 0u);
+          f0 = 0;
+          pb += 32 * slices;
+        }
+        if (f0 < total) {
+          const int f = f0 + lane;
+          // owner lane of flat entry f: last lane with excl <= f
+          int lo = 0;
+#pragma unroll
+          for (int st = 16; st >= 1; st >>= 1) {
+            const int e2 = __shfl_sync(kFull, excl, lo + st);
+            if (e2 <= f) lo += st;
+          }
+          const uint32_t index = __shfl_sync(kFull, off, lo) + (uint32_t)f;
+          const uint32_t ow = __shfl_sync(kFull, who, lo);
+          if (f < total) {
+            const bool osame = (ow & 0x10000u) != 0;
+            const int oci = ow & 0xff, ocj = (ow >> 8) & 0xff;
+            const short2 pr = __ldg(reinterpret_cast<const short2*>(osame ? a.hb.samePairs : a.hb.oppPairs) + index);
+            const int av = 2 * pr.x + (oci & 1), bv = 2 * pr.y + (ocj & 1);
+            bool ok = true;
+            for (int r = 0; ok && r < sp.nrestrict; ++r) {
+              int c2 = cur[r] - in_mask(sp, r, oci) - in_mask(sp, r, ocj) + in_mask(sp, r, av) + in_mask(sp, r, bv);
+              ok = c2 >= sp.rmin[r] && c2 <= sp.rmax[r];
+            }
+            surv = ok && !(occupied<W2>(d, av) || occupied<W2>(d, bv));
+            if (surv) {
+              w = (uint32_t)oci | ((uint32_t)ocj << 8) | ((uint32_t)av << 16) | ((uint32_t)bv << 24);
+              vf = __ldg((osame ? a.hb.sameVal : a.hb.oppVal) + index);
+            }
+          }
+          f0 += 32;
+        } else {
+          more = false;
+        }
       }
+      if (more) push(surv, w, vf);
+      if (qn >= 32 || (!more && qn > 0)) drain(qn < 32 ? qn : 32);
+      if (rn >= 32 || (!more && qn == 0 && rn > 0)) write(rn < 32 ? rn : 32);
+      if (!more && qn == 0 && rn == 0) break;
     }
-    while (qn > 0) drain(qn < 32 ? qn : 32);
-    if (rn > 0) write(rn);
   }
 }
 
