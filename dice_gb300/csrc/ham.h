@@ -194,7 +194,7 @@ struct HeatBathView {
 // lists (selection, perturbation theory). A parent's work goes with the list
 // entries above its threshold eps / |c|, which spans five orders of magnitude
 // over a space: one warp per parent leaves the GPU waiting for the few warps
-// that hold the largest coefficients. A parent estimated above kSplitEntries
+// that hold the largest coefficients. A parent estimated above a slice's
 // entries is cut into nsl[p] slices; `extra` lists its slices 1.. (in no
 // particular order, 0xffffffff = unused), and slice 0 of every parent follows
 // them implicitly: unit u < count is extra[u], then parent u - count.

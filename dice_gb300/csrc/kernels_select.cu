@@ -40,36 +40,55 @@ constexpr int kSelThreads = 256;
 constexpr int kSelWarps = kSelThreads / 32;
 
 // ---- work units -------------------------------------------------------------
-// Thread per parent: entries above its threshold in the lists of its occupied
-// pairs, taken as the mean list of each kind (entries above the threshold over
-// all lists / lists), and one slice per kSplitEntries of them. 2048 entries
-// are 64 rounds of a warp, a few times what a slice's set-up costs.
-constexpr float kSplitEntries = 2048.0f;
+// Entries above a parent's threshold in the lists of its occupied pairs, taken
+// as the mean list of each kind (entries above the threshold over all lists /
+// lists).
+__device__ __forceinline__ float parent_entries(const Det2& d, double e, double maxEntry,
+                                                const uint32_t* __restrict__ cum, int norb) {
+  if (!(e < INFINITY) || fabs(maxEntry) < e) return 0.0f;
+  const uint64_t ev = 0x5555555555555555ull;
+  const float na = (float)(__popcll(d.w0 & ev) + __popcll(d.w1 & ev));
+  const float nb = (float)(__popcll(d.w0 & ~ev) + __popcll(d.w1 & ~ev));
+  const unsigned bin = __float_as_uint(__double2float_rd(e)) >> 20;
+  const float lists = 0.5f * (float)norb * (float)(norb + 1);
+  return ((float)cum[bin] * 0.5f * (na * (na - 1.0f) + nb * (nb - 1.0f)) + (float)cum[kHbBins + bin] * na * nb) / lists;
+}
+// Entries of a slice: what all parents hold over ten units for each warp that
+// is resident (152 SMs x 40), within 2,048 (64 rounds of a warp, a few times
+// what a slice's set-up costs; a selection of 60,000 parents 631 us, with 4,096
+// 680) and 8,192 (507 million entries of 80,730 parents: 5.40 ms with 2,048, 5.01
+// with 4,096, 4.92 with 8,192, 5.01 with 16,384; an iteration of 200 parents
+// 0.30 ms with 2,048, 0.48 with 8,192). Fewer than kSplitCount parents are not
+// added up: the smallest slice is theirs.
+constexpr float kSplitMin = 2048.0f, kSplitCap = 8192.0f, kSplitUnits = 152.0f * 40.0f * 10.0f;
+constexpr size_t kSplitCount = 16384;
 constexpr int kSplitMax = 64;
+__global__ void k_split_total(const Det2* __restrict__ dets, const double* __restrict__ c, size_t n, double eps,
+                              double maxEntry, const uint32_t* __restrict__ cum, int norb,
+                              unsigned long long* __restrict__ total) {
+  unsigned long long t = 0;  // whole numbers: the same sum in any order
+  for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
+    t += (unsigned long long)parent_entries(dets[i], fabs(eps / c[i]), maxEntry, cum, norb);
+  for (int o = 16; o; o >>= 1) t += __shfl_xor_sync(kFull, t, o);
+  if ((threadIdx.x & 31) == 0 && t) atomicAdd(total, t);
+}
+// Thread per parent: one slice per so many of its entries.
 __global__ void k_split_parents(const Det2* __restrict__ dets, const int32_t* __restrict__ plist,
                                 const double* __restrict__ c, size_t n, double eps, double maxEntry,
-                                const uint32_t* __restrict__ cum, int norb, uint2* __restrict__ extra, uint32_t cap,
+                                const uint32_t* __restrict__ cum, int norb,
+                                const unsigned long long* __restrict__ total, uint2* __restrict__ extra, uint32_t cap,
                                 uint32_t* __restrict__ count, unsigned char* __restrict__ nsl) {
+  const float per = fminf(fmaxf((float)*total / kSplitUnits, kSplitMin), kSplitCap);
   for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
     const size_t p = plist ? (size_t)plist[i] : i;
-    const double e = fabs(eps / c[p]);
+    const float est = parent_entries(dets[p], fabs(eps / c[p]), maxEntry, cum, norb);
     int ns = 1;
-    if (e < INFINITY && !(fabs(maxEntry) < e)) {
-      const Det2 d = dets[p];
-      const uint64_t ev = 0x5555555555555555ull;
-      const float na = (float)(__popcll(d.w0 & ev) + __popcll(d.w1 & ev));
-      const float nb = (float)(__popcll(d.w0 & ~ev) + __popcll(d.w1 & ~ev));
-      const unsigned bin = __float_as_uint(__double2float_rd(e)) >> 20;
-      const float lists = 0.5f * (float)norb * (float)(norb + 1);
-      const float est = ((float)cum[bin] * 0.5f * (na * (na - 1.0f) + nb * (nb - 1.0f)) +
-                         (float)cum[kHbBins + bin] * na * nb) / lists;
-      const int want = 1 + (int)fminf(est / kSplitEntries, (float)(kSplitMax - 1));
-      if (want > 1) {
-        const uint32_t base = atomicAdd(count, (uint32_t)(want - 1));
-        if (base + (uint32_t)(want - 1) <= cap) {
-          for (int k = 1; k < want; ++k) extra[base + k - 1] = make_uint2((uint32_t)i, (uint32_t)k);
-          ns = want;
-        }
+    const int want = 1 + (int)fminf(est / per, (float)(kSplitMax - 1));
+    if (want > 1) {
+      const uint32_t base = atomicAdd(count, (uint32_t)(want - 1));
+      if (base + (uint32_t)(want - 1) <= cap) {
+        for (int k = 1; k < want; ++k) extra[base + k - 1] = make_uint2((uint32_t)i, (uint32_t)k);
+        ns = want;
       }
     }
     nsl[i] = (unsigned char)ns;
@@ -84,13 +103,17 @@ void split_parents(const Det2* dets, const int32_t* plist, const double* c, size
   ps.extra.reserve(cap);
   ps.nsl.reserve(n);
   ps.count.reserve(1);
-  ps.next.reserve(1);
+  ps.next.reserve(2);  // the queue, and the entries of all parents
   SHCI_CUDA(cudaMemsetAsync(ps.extra.p, 0xff, cap * sizeof(uint2), s));
   SHCI_CUDA(cudaMemsetAsync(ps.count.p, 0, sizeof(uint32_t), s));
-  ps.rewind(s);
+  SHCI_CUDA(cudaMemsetAsync(ps.next.p, 0, 2 * sizeof(unsigned long long), s));
   size_t blocks = std::max<size_t>(1, std::min<size_t>((n + 127) / 128, 152 * 16));
-  k_split_parents<<<(unsigned)blocks, 128, 0, s>>>(dets, plist, c, n, eps, maxEntry, hb.cum, norb, ps.extra.p, ps.cap,
-                                                   ps.count.p, ps.nsl.p);
+  if (!plist && n >= kSplitCount) {
+    k_split_total<<<(unsigned)blocks, 128, 0, s>>>(dets, c, n, eps, maxEntry, hb.cum, norb, ps.next.p + 1);
+    SHCI_LAUNCH_CHECK();
+  }
+  k_split_parents<<<(unsigned)blocks, 128, 0, s>>>(dets, plist, c, n, eps, maxEntry, hb.cum, norb, ps.next.p + 1,
+                                                   ps.extra.p, ps.cap, ps.count.p, ps.nsl.p);
   SHCI_LAUNCH_CHECK();
 }
 

@@ -80,3 +80,19 @@ def test_more_slices_than_the_list_holds(mol24):
     ref = np.unique(np.concatenate(parts), axis=0)
     e.set_selection_params()
     assert len(whole) == len(ref) and np.array_equal(np.unique(whole, axis=0), ref)
+
+
+@pytest.mark.parametrize("n", [16383, 16384, 30000])
+def test_slice_size_follows_the_total(mol24, n):
+    """From 16,384 parents on a slice's size goes with the entries of all of them: three quarters of the
+    coefficients at zero give smaller slices, and the same determinants."""
+    e, _ = mol24
+    dets = _dets(n, 4, orbs=15)
+    e.set_selection_params(0, 15)
+    e.set_dets(dets)
+    c = np.ones(n)
+    whole = e.select_candidates(c, 1e-7)
+    parts = [e.select_candidates(np.where(np.arange(n) % 4 == k, c, 0.0), 1e-7) for k in range(4)]
+    ref = np.unique(np.concatenate(parts), axis=0)
+    e.set_selection_params()
+    assert len(whole) == len(ref) and np.array_equal(np.unique(whole, axis=0), ref)
