@@ -384,6 +384,7 @@ struct Context {
     build_heatbath(hi, hb);
     hints = std::move(hi);
     hhb = std::move(hb);
+    ptw.tables_ok = false;
     upload(dI1, hints.I1);
     upload(dI2, hints.I2);
     {

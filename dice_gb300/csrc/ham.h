@@ -336,8 +336,7 @@ struct PtWork {
   DevBuf<double> coul, exch;        // dense (AI|JJ), (AJ|JI) of the integrals below
   DevBuf<float> coul32, exch32;     // and their FP32 roundings
   DevBuf<float2> coulff, exchff;    // and as float pairs
-  const double* tables_of = nullptr;
-  int tables_n = 0;
+  bool tables_ok = false;  // made again after integrals are read (their address says nothing: it comes back)
 };
 // E2 of the space `dets` (hash set `present` over it) with coefficients c
 // (device, n) for threshold eps2: candidates with |H_ai c_i| criteria of the

@@ -1044,7 +1044,7 @@ size_t pt_prepare(PtArgs& a, const Det2* dets, size_t n, const double* c, double
   a.hmask = present.mask;
   a.counter = w.next.p;
   a.nparts = 1;
-  if (w.tables_of != ints.I2 || w.tables_n != ints.norb) {
+  if (!w.tables_ok) {
     const size_t nt = (size_t)ints.norb * ints.norb * ints.norb;
     w.coul.resize(nt);
     w.exch.resize(nt);
@@ -1055,8 +1055,7 @@ size_t pt_prepare(PtArgs& a, const Det2* dets, size_t n, const double* c, double
     k_pt_tables<<<grid_for(nt, 256), 256, 0, s>>>(ints.I2, ints.norb, w.coul.p, w.exch.p, w.coul32.p, w.exch32.p,
                                                    w.coulff.p, w.exchff.p);
     SHCI_LAUNCH_CHECK();
-    w.tables_of = ints.I2;
-    w.tables_n = ints.norb;
+    w.tables_ok = true;
   }
   a.coul = w.coul.p;
   a.exch = w.exch.p;

@@ -96,3 +96,24 @@ def test_slice_size_follows_the_total(mol24, n):
     ref = np.unique(np.concatenate(parts), axis=0)
     e.set_selection_params()
     assert len(whole) == len(ref) and np.array_equal(np.unique(whole, axis=0), ref)
+
+
+def test_pt_tables_follow_the_integrals(tmp_path):
+    """Two FCIDUMPs of the same size in turn in one context: each correction is the oracle's for its own
+    integrals (the generator's tables are made again when integrals are read)."""
+    e = eng.Engine(0)
+    got, ref = [], []
+    for seed in (1, 2, 1):
+        path = str(tmp_path / ("F%d" % seed))
+        h, eri = synthetic.molecular_integrals(8, 8, seed)
+        synthetic.write_fcidump(path, h, eri, 8)
+        e.read_fcidump(path)
+        dets = np.array([(0b11111111, 0), (0b110111111, 0)], dtype=np.uint64)
+        c = np.array([0.9, 0.4])
+        e.set_dets(dets)
+        E0 = float(e.diag().min()) - 5.0
+        got.append(e.pt_deterministic(c, E0, 1e-6))
+        ref.append(orc.Oracle(path).pt_det(dets, c, E0, 1e-6)[0])
+    e.close()
+    assert abs(ref[0] - ref[1]) > 1e-3 * abs(ref[0])
+    assert np.allclose(got, ref, rtol=1e-10, atol=0)
