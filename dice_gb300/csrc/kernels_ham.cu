@@ -899,11 +899,17 @@ __device__ __forceinline__ typename Elem<F32>::T elem_single(const IntsView& v, 
 // the other two runs are searched. Evaluating here, and not where a connection
 // is found, keeps the walk's registers free of the element code and puts
 // every lane on an element. 5.5e8 entries (mol24, mixed: the spaces of 81,233
-// and 405,690 determinants): emitting 12.7 ms, finishing 12.9 ms; emitting with
+// and 405,690 determinants): emitting 11.3 ms, finishing 8.3 ms; emitting with
 // evaluation and sorting each row by a bitonic network took 58.6 ms for 3.6e8.
 // ---------------------------------------------------------------------------
 constexpr int kRunCap = 3072;  // entries of a row kept in shared memory
-constexpr int kFinThreads = 128;  // 64: 15.4 ms, 96: 12.9 ms, 128: 11.4 ms for 5.5e8 entries
+constexpr int kFinThreads = 128;  // 64: 15.4 ms, 96: 12.9 ms, 128: 11.4 ms for 5.5e8 entries (16 blocks per SM)
+// Blocks per SM of the launches that go over rows: many times what is resident
+// (5 and 12 blocks per SM), so that blocks that end early make room for others.
+// 5.5e8 entries, 16 per SM before (3.2 and 1.3 waves): counting 3.88 -> 3.46 ms and
+// emitting 12.84 -> 11.30 (5: 4.45 and 13.07; 40: 3.56 and 11.93), finishing 11.42 ->
+// 8.31 (12: 9.98; 96: 9.20; 4,000: 8.38).
+constexpr size_t kRowBlocks = 160, kFinBlocks = 1536;
 
 __device__ __forceinline__ int run_below(const uint32_t* run, int n, uint32_t c) {  // entries of a run below c
   int lo = 0, hi = n;
@@ -1349,7 +1355,7 @@ static int64_t emit_rows_as(const Helpers& hp, const uint32_t* rows, size_t nr, 
   DevBuf<uint4> parts;
   counts.resize(nr > 0 ? nr : 1);
   parts.resize(nr > 0 ? nr : 1);
-  const unsigned blocks = grid_for(nr * 32, 256, 152 * 16);
+  const unsigned blocks = grid_for(nr * 32, 256, 152 * kRowBlocks);
   if (nr) {
     k_ham_count<S><<<blocks, 256, 0, s>>>(hv, rows, (int64_t)nr, parts.p, counts.p);
     SHCI_LAUNCH_CHECK();
@@ -1382,7 +1388,7 @@ static int64_t emit_rows_as(const Helpers& hp, const uint32_t* rows, size_t nr, 
   k_long_runs<<<grid_for(nr, 256), 256, 0, s>>>(rowptr.p, (int64_t)nr, list.p, (uint32_t)ncap, tot.p);
   SHCI_LAUNCH_CHECK();
   const bool split = want32 && ints.I2ff != nullptr;
-  const unsigned fb = (unsigned)std::min<size_t>(nr, 152 * 16);
+  const unsigned fb = (unsigned)std::min<size_t>(nr, 152 * kFinBlocks);
   if (split)
     k_ham_finish<S, true><<<fb, kFinThreads, 0, s>>>(hv, ints, rows, (int64_t)nr, parts.p, rowptr.p, col.p, d64, dhi,
                                                      dlo);
