@@ -56,7 +56,7 @@ __device__ __forceinline__ float parent_entries(const Det2& d, double e, double 
 // Entries of a slice: what all parents hold over ten units for each warp that
 // is resident (152 SMs x 40), within 2,048 (64 rounds of a warp, a few times
 // what a slice's set-up costs; a selection of 60,000 parents 631 us, with 4,096
-// 680) and 8,192 (507 million entries of 80,730 parents: 5.40 ms with 2,048, 5.01
+// 680, before its queue) and 8,192 (507 million entries of 80,730 parents: 5.40 ms with 2,048, 5.01
 // with 4,096, 4.92 with 8,192, 5.01 with 16,384; an iteration of 200 parents
 // 0.30 ms with 2,048, 0.48 with 8,192). Fewer than kSplitCount parents are not
 // added up: the smallest slice is theirs.
@@ -132,9 +132,12 @@ __device__ __forceinline__ void append(const SelArgs& a, bool emit, const Det2& 
   }
 }
 
-__global__ void __launch_bounds__(kSelThreads) k_select(SelArgs a) {
+// Five blocks per SM: 4 (59 registers) 476 us, 5 (48) 438, 6 (40, spilled) 470 for
+// 60,000 parents of 36 orbitals; 614 with every entry's search where it stands.
+__global__ void __launch_bounds__(kSelThreads, 5) k_select(SelArgs a) {
   __shared__ unsigned char s_closed[kSelWarps][kMaxSpin];
   __shared__ unsigned char s_open[kSelWarps][kMaxSpin];
+  __shared__ uint2 s_q[kSelWarps][64];
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
   unsigned char* closed = s_closed[wib];
   unsigned char* open = s_open[wib];
@@ -142,6 +145,36 @@ __global__ void __launch_bounds__(kSelThreads) k_select(SelArgs a) {
   const unsigned lt = (1u << lane) - 1u;
   const uint32_t nextra = min(*a.split.count, a.split.cap);
   const SelectParams& sp = a.sp;
+  // Excitations that pass the cheap tests (one list entry in ten) wait in a ring
+  // of the warp, over units, for the element of a single and the search in the
+  // hash table, 32 at a time. Entry: the orbitals i | j << 8 | a << 16 | b << 24
+  // (j = b = 0xff for a single) and the parent.
+  uint2* ring = s_q[wib];
+  unsigned qh = 0, qn = 0;  // warp-uniform
+  auto drain = [&](unsigned cnt) {
+    bool emit = false;
+    Det2 cand{0, 0};
+    if ((unsigned)lane < cnt) {
+      const uint2 e = ring[(qh + lane) & 63u];
+      const int oi = e.x & 0xff, oj = (e.x >> 8) & 0xff, oa = (e.x >> 16) & 0xff, ob = e.x >> 24;
+      cand = a.dets[e.y];
+      emit = true;
+      if (oj == 0xff) {
+        if ((oi & 1) == (oa & 1))
+          emit = fabs(hij_single(a.ints, cand, oa, oi)) > a.eps1 / fabs(a.cmax[e.y]);
+      } else {
+        det_flip(cand, oj);
+        det_flip(cand, ob);
+      }
+      det_flip(cand, oi);
+      det_flip(cand, oa);
+      if (emit) emit = !hash_contains(a.hslots, a.hmask, a.dets, cand);
+    }
+    append(a, emit, cand);
+    qh = (qh + cnt) & 63u;
+    qn -= cnt;
+    __syncwarp();
+  };
   uint32_t p;
   int slice, slices;
   while (next_unit(a.split, a.n, nextra, p, slice, slices)) {
@@ -170,74 +203,70 @@ __global__ void __launch_bounds__(kSelThreads) k_select(SelArgs a) {
     int cur[kMaxRestrict];
     for (int r = 0; r < sp.nrestrict; ++r) cur[r] = __popcll(d.w0 & sp.rmask0[r]) + __popcll(d.w1 & sp.rmask1[r]);
 
-    // ---- singles
-    const int ns = nclosed * nopen;
-    for (int base = 32 * slice; base < ns; base += 32 * slices) {
-      const int q = base + lane;
-      bool emit = false;
-      Det2 cand = d;
-      if (q < ns) {
-        const int ci = closed[q / nopen], oa = open[q % nopen];
-        bool ok = (ci >> 1) >= sp.ncore && (oa >> 1) < sp.ncore + sp.nact;
-        for (int r = 0; ok && r < sp.nrestrict; ++r) {
-          int e = cur[r] - in_mask(sp, r, ci) + in_mask(sp, r, oa);
-          ok = e >= sp.rmin[r] && e <= sp.rmax[r];
-        }
-        if (ok) {
-          double integral = a.hb.singles[(size_t)oa * n2 + ci];
-          if (fabs(integral) > eps)
-            if ((ci & 1) == (oa & 1)) integral = hij_single(a.ints, d, oa, ci);
-          if (fabs(integral) > eps) {
-            det_flip(cand, oa);
-            det_flip(cand, ci);
-            emit = !hash_contains(a.hslots, a.hmask, a.dets, cand);
-          }
-        }
-      }
-      append(a, emit, cand);
-    }
-
-    // ---- doubles
-    if (fabs(a.maxEntry) < eps) continue;
     // for a float v, (double)|v| < eps exactly when |v| < eps rounded up to float
     const float eps_f = __double2float_ru(eps);
-    const int npairs = nclosed * (nclosed - 1) / 2;
-    // this slice's pairs: q = slice, slice + slices, ...
-    for (int pb = slice; pb < npairs; pb += 32 * slices) {
-      const int q = pb + lane * slices;
-      int ci = 0, cj = 0, len = 0;
-      uint32_t lstart = 0;
-      bool same = false;
-      if (q < npairs) {
-        // q -> (i, j), i > j, q = i(i-1)/2 + j
-        int i = (int)((1.0f + sqrtf(1.0f + 8.0f * (float)q)) * 0.5f);  // corrected below
-        while (i * (i - 1) / 2 > q) --i;
-        while ((i + 1) * i / 2 <= q) ++i;
-        int j = q - i * (i - 1) / 2;
-        ci = closed[i];
-        cj = closed[j];
-        if ((ci >> 1) >= sp.ncore && (cj >> 1) >= sp.ncore) {
-          int I = ci >> 1, J = cj >> 1;
-          int X = I > J ? I : J, Y = I > J ? J : I;
-          int pair = X * (X + 1) / 2 + Y;
-          same = (ci & 1) == (cj & 1);
-          const int64_t* st = same ? a.hb.sameStart : a.hb.oppStart;
-          const float* vals = same ? a.hb.sameVal : a.hb.oppVal;
-          lstart = (uint32_t)st[pair];
-          len = prefix_length(vals + lstart, (int)((uint32_t)st[pair + 1] - lstart), eps_f);
+    const int ns = nclosed * nopen;
+    const int npairs = fabs(a.maxEntry) < eps ? 0 : nclosed * (nclosed - 1) / 2;
+    int b0 = 32 * slice;        // next single excitation
+    int pb = slice;             // next pair of electrons: slice, slice + slices, ...
+    int f0 = 0, total = 0;      // entries of the lists of 32 pairs
+    int excl = 0;               // a lane's list: first flat entry,
+    uint32_t off = 0, who = 0;  // list index of flat entry f: off of its owner + f; the electrons
+    while (true) {
+      bool surv = false;
+      uint32_t w = 0;
+      if (b0 < ns) {
+        const int q = b0 + lane;
+        if (q < ns) {
+          const int ci = closed[q / nopen], oa = open[q % nopen];
+          bool ok = (ci >> 1) >= sp.ncore && (oa >> 1) < sp.ncore + sp.nact;
+          for (int r = 0; ok && r < sp.nrestrict; ++r) {
+            int e = cur[r] - in_mask(sp, r, ci) + in_mask(sp, r, oa);
+            ok = e >= sp.rmin[r] && e <= sp.rmax[r];
+          }
+          surv = ok && fabs(a.hb.singles[(size_t)oa * n2 + ci]) > eps;
+          w = (uint32_t)ci | 0xff00u | ((uint32_t)oa << 16) | 0xff000000u;
         }
-      }
-      int incl = len;
+        b0 += 32 * slices;
+      } else {
+        while (f0 >= total && pb < npairs) {
+          const int q = pb + lane * slices;
+          int ci = 0, cj = 0, len = 0;
+          uint32_t lstart = 0;
+          bool same = false;
+          if (q < npairs) {
+            // q -> (i, j), i > j, q = i(i-1)/2 + j
+            int i = (int)((1.0f + sqrtf(1.0f + 8.0f * (float)q)) * 0.5f);  // corrected below
+            while (i * (i - 1) / 2 > q) --i;
+            while ((i + 1) * i / 2 <= q) ++i;
+            int j = q - i * (i - 1) / 2;
+            ci = closed[i];
+            cj = closed[j];
+            if ((ci >> 1) >= sp.ncore && (cj >> 1) >= sp.ncore) {
+              int I = ci >> 1, J = cj >> 1;
+              int X = I > J ? I : J, Y = I > J ? J : I;
+              int pair = X * (X + 1) / 2 + Y;
+              same = (ci & 1) == (cj & 1);
+              const int64_t* st = same ? a.hb.sameStart : a.hb.oppStart;
+              const float* vals = same ? a.hb.sameVal : a.hb.oppVal;
+              lstart = (uint32_t)st[pair];
+              len = prefix_length(vals + lstart, (int)((uint32_t)st[pair + 1] - lstart), eps_f);
+            }
+          }
+          int incl = len;
 #pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        int y = __shfl_up_sync(kFull, incl, o);
-        if (lane >= o) incl += y;
-      }
-      const int total = __shfl_sync(kFull, incl, 31);
-      const int excl = incl - len;
-      const uint32_t off = lstart - (uint32_t)excl;  // list index of flat entry f: off of its owner + f
-      const uint32_t who = (uint32_t)ci | ((uint32_t)cj << 8) | (same ? 0x10000u : 0u);
-      for (int f0 = 0; f0 < total; f0 += 32) {
+          for (int o = 1; o < 32; o <<= 1) {
+            int y = __shfl_up_sync(kFull, incl, o);
+            if (lane >= o) incl += y;
+          }
+          total = __shfl_sync(kFull, incl, 31);
+          excl = incl - len;
+          off = lstart - (uint32_t)excl;
+          who = (uint32_t)ci | ((uint32_t)cj << 8) | (same ? 0x10000u : 0u);
+          f0 = 0;
+          pb += 32 * slices;
+        }
+        if (f0 >= total) break;
         const int f = f0 + lane;
         int lo = 0;
 #pragma unroll
@@ -247,10 +276,8 @@ __global__ void __launch_bounds__(kSelThreads) k_select(SelArgs a) {
         }
         const uint32_t index = __shfl_sync(kFull, off, lo) + (uint32_t)f;
         const uint32_t ow = __shfl_sync(kFull, who, lo);
-        const int oci = ow & 0xff, ocj = (ow >> 8) & 0xff;
-        bool emit = false;
-        Det2 cand = d;
         if (f < total) {
+          const int oci = ow & 0xff, ocj = (ow >> 8) & 0xff;
           const short2 pr =
               __ldg(reinterpret_cast<const short2*>((ow & 0x10000u) ? a.hb.samePairs : a.hb.oppPairs) + index);
           const int av = 2 * pr.x + (oci & 1);
@@ -260,18 +287,19 @@ __global__ void __launch_bounds__(kSelThreads) k_select(SelArgs a) {
             int e = cur[r] - in_mask(sp, r, oci) - in_mask(sp, r, ocj) + in_mask(sp, r, av) + in_mask(sp, r, bv);
             ok = e >= sp.rmin[r] && e <= sp.rmax[r];
           }
-          if (ok && !(det_getocc(d, av) || det_getocc(d, bv))) {
-            det_flip(cand, av);
-            det_flip(cand, bv);
-            det_flip(cand, oci);
-            det_flip(cand, ocj);
-            emit = !hash_contains(a.hslots, a.hmask, a.dets, cand);
-          }
+          surv = ok && !(det_getocc(d, av) || det_getocc(d, bv));
+          w = (uint32_t)oci | ((uint32_t)ocj << 8) | ((uint32_t)av << 16) | ((uint32_t)bv << 24);
         }
-        append(a, emit, cand);
+        f0 += 32;
       }
+      const unsigned m = __ballot_sync(kFull, surv);
+      if (surv) ring[(qh + qn + __popc(m & lt)) & 63u] = make_uint2(w, p);
+      qn += __popc(m);
+      __syncwarp();
+      if (qn >= 32) drain(32);
     }
   }
+  if (qn > 0) drain(qn);
 }
 
 // ---------------------------------------------------------------------------
