@@ -728,6 +728,11 @@ __device__ __forceinline__ double from_fix(__int128 v) {
 // inclusive scan over the lanes sums the fixed-point numerators and takes
 // the minimum energy per run; the lane at a run's end adds its term. Block
 // partials {E2, |psi1|^2, count} go to part[3 * block].
+// Bound by the latency of the gathers: they are issued a round before they are
+// used (39.5 million candidates 1.07 -> 0.93 ms), and the scan takes only the
+// steps that the round's longest run needs, run starts from one ballot (1.13 ->
+// 1.07). Tiles of 512 0.92 ms, 1,024 0.94, 2,048 0.97; 256 keeps the warps busy
+// down to a million candidates.
 constexpr int kPtRedTile = 256;
 
 __device__ __forceinline__ __int128 shfl_up_i128(__int128 v, int o) {
@@ -741,7 +746,7 @@ __device__ __forceinline__ __int128 shfl_i128(__int128 v, int src) {
   return (__int128)(((unsigned __int128)(unsigned long long)hi << 64) | lo);
 }
 
-__global__ void __launch_bounds__(kPtRedThreads) k_pt_reduce(const uint64_t* __restrict__ k0,
+__global__ void __launch_bounds__(kPtRedThreads, 4) k_pt_reduce(const uint64_t* __restrict__ k0,
                                                              const uint64_t* __restrict__ k1,
                                                              const uint32_t* __restrict__ perm,
                                                              const float4* __restrict__ ne, size_t m,
@@ -797,17 +802,23 @@ __global__ void __launch_bounds__(kPtRedThreads) k_pt_reduce(const uint64_t* __r
     float2 ce = make_float2(INFINITY, 0.0f);
     size_t chead = b;
     bool open = false;
+    // numerators and energies are gathered a round ahead, their places two
+    size_t q = b + lane;
+    uint32_t pk = q < m ? perm[q] : 0;
+    float4 xn = ne[pk];
+    pk = q + 32 < m ? perm[q + 32] : 0;
     for (; b < m; b += 32) {
       if (b >= t1 && !(open && chead < t1)) break;
-      const size_t q = b + lane;
+      q = b + lane;
       const bool valid = q < m;
+      const float4 x = xn;
+      xn = ne[pk];
+      pk = q + 64 < m ? perm[q + 64] : 0;
       bool head = false;
       __int128 v = 0;
       float2 e = make_float2(INFINITY, 0.0f);
       if (valid) {
         head = (lane == 0) ? !open : is_head(q);
-        const uint32_t pk = perm[q];
-        const float4 x = ne[pk];
         v = to_fix(make_float2(x.x, x.y));
         e = make_float2(x.z, x.w);
       }
@@ -816,26 +827,24 @@ __global__ void __launch_bounds__(kPtRedThreads) k_pt_reduce(const uint64_t* __r
         v += cs;
         if (ff_less(ce, e)) e = ce;
       }
-      size_t hp = head ? q : 0;
-      bool f = head;
+      // the lane's run starts at the last head up to it; before the round's first
+      // head the open run continues from lane 0. Steps of the scan that no run of
+      // the round reaches back for are left out.
+      const unsigned heads = __ballot_sync(kFull, head), upto = heads & (lt << 1 | 1u);
+      const int start = 31 - __clz(upto | 1u), dist = lane - start;
+      const size_t hp = upto ? b + start : chead;
 #pragma unroll
       for (int o = 1; o < 32; o <<= 1) {
+        if (!__any_sync(kFull, dist >= o)) break;
         const __int128 nv = shfl_up_i128(v, o);
         const float2 ne = make_float2(__shfl_up_sync(kFull, e.x, o), __shfl_up_sync(kFull, e.y, o));
-        const bool nf = __shfl_up_sync(kFull, (int)f, o) != 0;
-        const size_t nh = __shfl_up_sync(kFull, (unsigned long long)hp, o);
-        if (lane >= o) {
-          if (!f) {
-            v += nv;
-            if (ff_less(ne, e)) e = ne;
-          }
-          f = f || nf;
-          hp = hp > nh ? hp : nh;
+        if (dist >= o) {
+          v += nv;
+          if (ff_less(ne, e)) e = ne;
         }
       }
-      if (!f) hp = chead;  // lanes before the first head of the round
       // does the run of this lane end here? (next position is a head or past the end)
-      bool next_head = __shfl_down_sync(kFull, (int)head, 1) != 0;
+      bool next_head = (heads >> lane >> 1) & 1u;
       if (lane == 31) next_head = (q + 1 >= m) || is_head(q + 1);
       // a finished run waits in the warp's queue, evaluated 32 at a time
       // (the FP64 tail costs a full-warp issue however few lanes take part)
