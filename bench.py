@@ -65,11 +65,11 @@ PARITY_TOL = 1e-8
 # deterministic PT2 on the final mixed-precision space of the workload
 PT_EPS2 = 1e-5
 # DRAM bytes per mixed-sigma launch divided by its algorithmic bytes, from one
-# ncu capture of the medium case (4.4983 GB measured read + write / 4.4633 GB
+# ncu capture of the medium case (5.2686 GB measured read + write / 5.2002 GB
 # algorithmic, profiles/sigma_mol24_medium.md); the full-size launch is too
 # large to capture with all sections, and its traffic scales with the
 # nonzeros it streams.
-TRAFFIC_RATIO = 4.4983 / 4.4633
+TRAFFIC_RATIO = 5.2686 / 5.2002
 
 
 def dist_info():
@@ -579,7 +579,7 @@ def run_ours(args):
 
     peak, peak_kind = measured_peak_gbs()
     # algorithmic bytes of each launch as the library lays the matrix out
-    # (k = 1 mixed: 16-bit column deltas + FP32 values, 6 B per stored entry)
+    # (k = 1 mixed: 24-bit columns + FP32 values, 7 B per stored entry)
     achieved = alg_bytes / t_max / 1e9
     ach64 = alg64 / statistics.mean(ts64) / 1e9
 
@@ -688,7 +688,7 @@ def run_ham_only(args):
     """--section ham: the plain FP64 variational run of the chosen case, then
     the Hamiltonian of its final space built from scratch (string tables,
     partial-string index, diagonal, count, emit, row sort; for the mixed form
-    also the 16-bit-delta copy), FP64 and mixed, each timed build inside its
+    also the compact copy), FP64 and mixed, each timed build inside its
     own NVTX range (bench_ham_<mode>). Reloading the determinants before each
     build drops every table and the stored matrix."""
     import torch

@@ -223,7 +223,7 @@ void scan_exclusive_u32(const uint32_t* in, uint32_t* out, size_t n, Prims& pr, 
 // scatter ranks a tile's keys warp by warp without block barriers, exchanges
 // them through shared memory into digit order and writes runs of equal digits:
 // coalesced, where writing each key straight to its place touched a sector per
-// key. 39.5 M keys with payload (pt): 307 -> see below per pass.
+// key. 39.5 million keys with payload: 307 -> 288 us per pass.
 // ---------------------------------------------------------------------------
 constexpr int kRsThreads = 512;
 constexpr int kRsItems = 8;

@@ -14,8 +14,8 @@
 // variational space removed, and E2 = sum_a N_a^2 / (E0 - E_a).
 //
 // GPU form (one launch sequence per hash partition):
-//   k_pt_gen     one warp per parent (dynamic queue); candidates outside the
-//                variational space (hash probe) in this partition are
+//   k_pt_gen     one warp per parent or slice of one (dynamic queue); candidates
+//                outside the variational space (hash probe) in this partition are
 //                appended (warp-aggregated atomics) with their numerator and
 //                energy. The energy is updated from the parent's in O(1):
 //                with orbital energies F_p = h_pp + sum_{q occupied} V(p, q)
@@ -28,7 +28,7 @@
 //                element) only where the screen cannot decide or keeps them;
 //   radix sort   of the determinants (two key words, written apart by the
 //                generator) with the candidate index as payload;
-//   k_pt_reduce  one thread per run of equal determinants: the numerators are
+//   k_pt_reduce  runs of equal determinants, reduced by warps: the numerators are
 //                summed exactly in 128-bit fixed point (2^-80 units), so the
 //                sum does not depend on the order the atomics left the run in,
 //                E_a is the minimum over the run (the copies differ only by

@@ -35,7 +35,7 @@
 //               in the two determinants, so the order does not change the
 //               sums);
 //   k_rdm_fin   images and tables summed, fixed point -> FP64.
-// 151,842 determinants, 8e7 pairs (mol24): off-diagonal 8.19 -> 1.38 ms (before,
+// 151,842 determinants, 8e7 pairs (mol24): off-diagonal 8.19 -> 1.20 ms (before,
 // every element was added on its own, a spectator loop in one lane), diagonal
 // 1.98 -> 0.17 ms (before, atomics in shared memory).
 #include "ham.h"

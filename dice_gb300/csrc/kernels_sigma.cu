@@ -328,7 +328,7 @@ __global__ void __launch_bounds__(kBalWalk ? 1024 : 256, kBalWalk ? 2 : 4)
 // order, 6 bytes, bridged across wide gaps; a lane's four entries were
 // neighbours, so each gather spread over four times as many lines, and L1's
 // tag rate bound it at 90 %.) 1.2 million determinants, 2.03e9 entries: 2.75 ->
-// 2.52 ms, 83 % of the measured copy bandwidth.
+// 2.43 ms, 86 % of the measured copy bandwidth.
 struct MixedCompactBody : AccSum {
   static constexpr int KP = 1;
   static constexpr bool kAside = false;
