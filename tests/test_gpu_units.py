@@ -117,3 +117,25 @@ def test_pt_tables_follow_the_integrals(tmp_path):
     e.close()
     assert abs(ref[0] - ref[1]) > 1e-3 * abs(ref[0])
     assert np.allclose(got, ref, rtol=1e-10, atol=0)
+
+
+# keys per sort: 256 counts per 4,096 keys, scanned in chunks of 4,096; to 256 chunks (16.8 million keys)
+# in two launches, beyond in three. Parents of 29,436 connections each (12 + 12 electrons in 24 orbitals).
+@pytest.mark.parametrize("n", [2, 3, 570, 600])
+def test_sorts_to_either_side_of_a_scans_levels(mol24, n):
+    e, _ = mol24
+    dets = _dets(n, 31)
+    c = np.full(n, n ** -0.5)
+    e.set_selection_params()
+    e.set_dets(dets)
+    E0 = float(e.diag().min()) - 30.0
+    e2 = e.pt_deterministic(c, E0, 1e-12)
+    whole = e.pt_stats()
+    e.set_pt_batch(max(1000, whole["candidates"] // 5))  # parts of a fifth: small sorts
+    p2 = e.pt_deterministic(c, E0, 1e-12)
+    parts = e.pt_stats()
+    e.set_pt_batch(0)
+    assert parts["partitions"] > 1
+    assert (whole["candidates"], whole["unique"]) == (parts["candidates"], parts["unique"])
+    # the same terms, summed in parts: some 1e7 terms of one sign
+    assert abs(e2 - p2) <= 1e-11 * abs(e2)
