@@ -662,7 +662,7 @@ __device__ __forceinline__ int warp_total(int c) {
 // excitation away, and J with B itself (in every run of its group, to be
 // counted once), which the run of the first probe shows.
 template <class S>
-__global__ void __launch_bounds__(256) k_ham_count(HelperView<S> h, const uint32_t* __restrict__ rows, int64_t nr,
+__global__ void __launch_bounds__(256, 8) k_ham_count(HelperView<S> h, const uint32_t* __restrict__ rows, int64_t nr,
                                                    uint4* __restrict__ parts, int64_t* __restrict__ counts) {
   const int lane = threadIdx.x & 31;
   const int64_t warps = (int64_t)gridDim.x * (blockDim.x >> 5);
@@ -734,7 +734,7 @@ struct AppendVisitor {
   }
 };
 template <class S>
-__global__ void __launch_bounds__(256) k_ham_emit(HelperView<S> h, const uint32_t* __restrict__ rows, int64_t nr,
+__global__ void __launch_bounds__(256, 6) k_ham_emit(HelperView<S> h, const uint32_t* __restrict__ rows, int64_t nr,
                                                   const int64_t* __restrict__ rowptr, int32_t* __restrict__ col) {
   __shared__ __align__(16) uint32_t s_buf[8][kCollect];
   const int lane = threadIdx.x & 31;
@@ -899,16 +899,23 @@ __device__ __forceinline__ typename Elem<F32>::T elem_single(const IntsView& v, 
 // the other two runs are searched. Evaluating here, and not where a connection
 // is found, keeps the walk's registers free of the element code and puts
 // every lane on an element. 5.5e8 entries (mol24, mixed: the spaces of 81,233
-// and 405,690 determinants): emitting 11.3 ms, finishing 8.3 ms; emitting with
+// and 405,690 determinants): emitting 10.5 ms, finishing 6.9 + 1.3 ms; emitting with
 // evaluation and sorting each row by a bitonic network took 58.6 ms for 3.6e8.
 // ---------------------------------------------------------------------------
-constexpr int kRunCap = 3072;  // entries of a row kept in shared memory
+// Entries of a row kept in a small block's shared memory; longer rows go to
+// blocks of their own size, with up to kLongShared entries in shared memory and
+// the few beyond in a scratch copy. 5.5e8 entries, both kernels: 3,072 and blocks
+// of 1,024 that search in the scratch copy 8.31 + 1.53 ms; 3,072 8.31 + 0.94; 2,560
+// 6.86 + 1.32 (16 blocks per SM instead of 13); 2,048 6.29 + 2.08; 1,536 5.28 + 3.92.
+constexpr int kRunCap = 2560;
+constexpr int kLongThreads = 512, kLongShared = 7168;
 constexpr int kFinThreads = 128;  // 64: 15.4 ms, 96: 12.9 ms, 128: 11.4 ms for 5.5e8 entries (16 blocks per SM)
 // Blocks per SM of the launches that go over rows: many times what is resident
-// (5 and 12 blocks per SM), so that blocks that end early make room for others.
+// (5 to 16 blocks per SM), so that blocks that end early make room for others.
 // 5.5e8 entries, 16 per SM before (3.2 and 1.3 waves): counting 3.88 -> 3.46 ms and
 // emitting 12.84 -> 11.30 (5: 4.45 and 13.07; 40: 3.56 and 11.93), finishing 11.42 ->
-// 8.31 (12: 9.98; 96: 9.20; 4,000: 8.38).
+// 8.31 (12: 9.98; 96: 9.20; 4,000: 8.38). Counting with 8 resident blocks (32
+// registers) 3.46 -> 3.12, emitting with 6 (40) 11.32 -> 10.47.
 constexpr size_t kRowBlocks = 160, kFinBlocks = 1536;
 
 __device__ __forceinline__ int run_below(const uint32_t* run, int n, uint32_t c) {  // entries of a run below c
@@ -1063,35 +1070,43 @@ __global__ void __launch_bounds__(kFinThreads) k_ham_finish(HelperView<S> h, Int
   if (sq.n) sq.drain(sq.n, h, ints, out);
 }
 
-// Rows past kRunCap: listed with their places in a scratch copy of their runs.
+// Rows past kRunCap: listed, and with their places in a scratch copy past kLongShared.
 __global__ void k_long_runs(const int64_t* __restrict__ rowptr, int64_t nr, uint2* __restrict__ list, uint32_t cap,
                             unsigned long long* __restrict__ tot) {
   for (int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; k < nr; k += (int64_t)gridDim.x * blockDim.x) {
     const int64_t len = rowptr[k + 1] - rowptr[k];
     if (len <= kRunCap) continue;
     const unsigned long long i = atomicAdd(tot, 1ull);
-    const unsigned long long off = atomicAdd(tot + 1, (unsigned long long)((len + 31) / 32));
+    const unsigned long long off = len > kLongShared ? atomicAdd(tot + 1, (unsigned long long)((len + 31) / 32)) : 0;
     if (i < cap) list[i] = make_uint2((uint32_t)k, (uint32_t)off);
   }
 }
 template <class S, bool kSplit>
-__global__ void __launch_bounds__(1024) k_ham_finish_long(HelperView<S> h, IntsView ints,
+__global__ void __launch_bounds__(kLongThreads) k_ham_finish_long(HelperView<S> h, IntsView ints,
                                                           const uint32_t* __restrict__ rows,
                                                           const uint2* __restrict__ list, uint32_t* scratch,
                                                           const uint4* __restrict__ parts,
                                                           const int64_t* __restrict__ rowptr,
                                                           int32_t* __restrict__ col, double* __restrict__ v64,
                                                           float* __restrict__ vhi, float* __restrict__ vlo) {
-  __shared__ uint4 s_q[32][64];
+  __shared__ uint4 s_q[kLongThreads / 32][64];
+  __shared__ uint32_t s_run[kLongShared];
   const FinishOut out{col, v64, vhi, vlo};
   SingleQueue<S> sq{s_q[threadIdx.x >> 5]};
   const uint2 l = list[blockIdx.x];
   const int64_t p0 = rowptr[l.x];
   const int len = (int)(rowptr[l.x + 1] - p0);
-  uint32_t* run = scratch + 32 * (size_t)l.y;
-  for (int e = threadIdx.x; e < len; e += blockDim.x) run[e] = (uint32_t)col[p0 + e];
-  __syncthreads();
-  finish_row<S, kSplit>(h, ints, rows ? rows[l.x] : l.x, parts[l.x], run, p0, out, sq);
+  const uint32_t p = rows ? rows[l.x] : l.x;
+  if (len <= kLongShared) {
+    for (int e = threadIdx.x; e < len; e += blockDim.x) s_run[e] = (uint32_t)col[p0 + e];
+    __syncthreads();
+    finish_row<S, kSplit>(h, ints, p, parts[l.x], s_run, p0, out, sq);
+  } else {
+    uint32_t* run = scratch + 32 * (size_t)l.y;
+    for (int e = threadIdx.x; e < len; e += blockDim.x) run[e] = (uint32_t)col[p0 + e];
+    __syncthreads();
+    finish_row<S, kSplit>(h, ints, p, parts[l.x], run, p0, out, sq);
+  }
   if (sq.n) sq.drain(sq.n, h, ints, out);
 }
 
@@ -1401,12 +1416,12 @@ static int64_t emit_rows_as(const Helpers& hp, const uint32_t* rows, size_t nr, 
   SHCI_CUDA(cudaStreamSynchronize(s));
   if (nl[0] > 0) {
     DevBuf<uint32_t> scratch;
-    scratch.resize(32 * (size_t)nl[1]);
+    scratch.resize(nl[1] ? 32 * (size_t)nl[1] : 1);
     if (split)
-      k_ham_finish_long<S, true><<<(unsigned)nl[0], 1024, 0, s>>>(hv, ints, rows, list.p, scratch.p, parts.p, rowptr.p,
+      k_ham_finish_long<S, true><<<(unsigned)nl[0], kLongThreads, 0, s>>>(hv, ints, rows, list.p, scratch.p, parts.p, rowptr.p,
                                                                   col.p, d64, dhi, dlo);
     else
-      k_ham_finish_long<S, false><<<(unsigned)nl[0], 1024, 0, s>>>(hv, ints, rows, list.p, scratch.p, parts.p,
+      k_ham_finish_long<S, false><<<(unsigned)nl[0], kLongThreads, 0, s>>>(hv, ints, rows, list.p, scratch.p, parts.p,
                                                                    rowptr.p, col.p, d64, dhi, dlo);
     SHCI_LAUNCH_CHECK();
   }

@@ -114,8 +114,9 @@ def _check(e, o, dets, modes=("fp64", "mixed"), ks=(1, 2, 3, 4)):
 
 
 # the lowest determinant's row holds n - 1 entries: one piece of the FP64 walk (2,048), of the FP32 walk
-# (4,096), the merge in shared memory (3,072) and a sort tile (4,096), each to the entry, and several pieces
-@pytest.mark.parametrize("n", [2049, 2050, 3073, 3074, 4096, 4097, 4098, 8194])
+# (4,096), the merges in shared memory (2,560 and 7,168) and a sort tile (4,096), each to the entry, and several
+# pieces
+@pytest.mark.parametrize("n", [2049, 2050, 2561, 2562, 3073, 3074, 4096, 4097, 4098, 7169, 7170, 8194])
 def test_long_rows(system, n):
     e, o = system(20, 20)
     assert _check(e, o, _star(20, 10, 10, n, n)) == n - 1
