@@ -237,18 +237,21 @@ __global__ void k_m1_dir(const int64_t* __restrict__ slots, const int64_t* __res
   for (int64_t g = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; g < ng; g += (int64_t)gridDim.x * blockDim.x)
     dir[g] = ((uint64_t)first[g] << 6) | (uint64_t)(63 - __clzll((long long)slots[g]));
 }
-// One thread per run: measure the run (at most 64 entries: one per beta
-// orbital outside the partial string) and claim a slot of its group's table
-// by linear probing; a table more than half empty always has a free slot.
+// One thread per run: measure the run and claim a slot of its group's table
+// by linear probing; a table more than half empty always has a free slot. A
+// run of distinct determinants has at most 64 entries, one per beta orbital
+// outside the partial string. *too_long is set where repeated determinants make
+// one longer than a slot can say.
 template <class S>
 __global__ void k_m1_insert(const uint4* __restrict__ ent, int64_t n, const uint64_t* __restrict__ dir,
-                            uint2* __restrict__ tab) {
+                            uint2* __restrict__ tab, uint32_t* __restrict__ too_long) {
   constexpr uint32_t gmask = (1u << kM1GroupBits) - 1u;
   for (int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; k < n; k += (int64_t)gridDim.x * blockDim.x) {
     const uint4 e = ent[k];
     if (k > 0 && m1_same_key(e, ent[k - 1])) continue;
     int64_t f = k + 1;
     while (f < n && m1_same_key(ent[f], e)) ++f;
+    if (f - k > 64) *too_long = 1u;
     const uint64_t d = dir[e.z & gmask];
     const unsigned lg = (unsigned)(d & 63);
     const uint64_t mask = (1ull << lg) - 1;
@@ -391,8 +394,15 @@ static void build_singles_and_index(Helpers& hp, int norb, Prims& pr, cudaStream
       SHCI_LAUNCH_CHECK();
       hp.m1tab.resize((size_t)nslot);
       SHCI_CUDA(cudaMemsetAsync(hp.m1tab.p, 0xff, (size_t)nslot * sizeof(uint2), s));
-      k_m1_insert<S><<<eb, 256, 0, s>>>(hp.m1ent.p, ne, hp.m1dir.p, hp.m1tab.p);
+      DevBuf<uint32_t> flag;
+      flag.resize(1);
+      SHCI_CUDA(cudaMemsetAsync(flag.p, 0, sizeof(uint32_t), s));
+      k_m1_insert<S><<<eb, 256, 0, s>>>(hp.m1ent.p, ne, hp.m1dir.p, hp.m1tab.p, flag.p);
       SHCI_LAUNCH_CHECK();
+      uint32_t too_long = 0;
+      SHCI_CUDA(cudaMemcpyAsync(&too_long, flag.p, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
+      SHCI_CUDA(cudaStreamSynchronize(s));
+      if (too_long) hp.nm1 = 0;  // the views show no index: every group is scanned
     }
   }
   SHCI_CUDA(cudaStreamSynchronize(s));
@@ -660,7 +670,9 @@ __device__ __forceinline__ int warp_total(int c) {
 // Connections of row k (position rows[k], or k) by part, and their sum.
 // The index is only probed: a key's run holds the determinants one beta
 // excitation away, and J with B itself (in every run of its group, to be
-// counted once), which the run of the first probe shows.
+// counted once), which the run of the first probe shows. The space may hold a
+// determinant more than once; every copy of that J is counted, as k_ham_emit
+// writes each. A run ascends in its extra orbital, J's position being its order.
 template <class S>
 __global__ void __launch_bounds__(256, 8) k_ham_count(HelperView<S> h, const uint32_t* __restrict__ rows, int64_t nr,
                                                    uint4* __restrict__ parts, int64_t* __restrict__ counts) {
@@ -692,11 +704,11 @@ __global__ void __launch_bounds__(256, 8) k_ham_count(HelperView<S> h, const uin
           probe_index(h, h.aSing[smid + sidx], (S)(B ^ ((S)1 << bq)), lo, len);
           c4 += len;
           if (which == 0)
-            for (int e = 0; e < len; ++e)
-              if ((int)(__ldg(reinterpret_cast<const uint32_t*>(h.m1ent + lo + e) + 2) >> kM1GroupBits) == bq) {
-                c4 -= nb - 1;
-                break;
-              }
+            for (int e = 0; e < len; ++e) {
+              const int b = (int)(__ldg(reinterpret_cast<const uint32_t*>(h.m1ent + lo + e) + 2) >> kM1GroupBits);
+              if (b > bq) break;
+              c4 -= b == bq ? nb - 1 : 0;
+            }
         }
         which += step_r;
         sidx += step_q;

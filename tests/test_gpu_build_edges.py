@@ -1,0 +1,75 @@
+"""The Hamiltonian build on lists of determinants at the edge of what the calls
+take: determinants given more than once."""
+import itertools
+
+import numpy as np
+import pytest
+from scipy import sparse
+
+from dice_gb300.shard import ref_order
+from test_gpu_stored_edges import U64, _lower, _words, system  # noqa: F401  (fixture)
+
+pytestmark = pytest.mark.gpu
+
+
+def _grouped(alphas):
+    """All 1,716 beta strings of 6 electrons in 13 orbitals on each alpha string: groups that are looked up in the
+    index (more than 48 determinants)."""
+    bs = [sum(1 << k for k in c) for c in itertools.combinations(range(13), 6)]
+    return np.array([_words(a, b) for a in alphas for b in bs], dtype=np.uint64)
+
+
+def _expanded(o, dets):
+    """Lower triangle of the list's matrix: that of its distinct determinants, copied (two copies of one
+    determinant are not connected)."""
+    u, at = np.unique(dets, axis=0, return_inverse=True)
+    at = at.reshape(-1)
+    r, c, v = _lower(len(u), *o.ham(u))
+    # entries by their place, so that elements of exactly zero stay entries
+    k = np.arange(1, len(r) + 1, dtype=np.float64)
+    H = sparse.coo_matrix((np.r_[k, k], (np.r_[r, c], np.r_[c, r])), shape=(len(u),) * 2).tocsr()
+    H = sparse.tril(H[at][:, at], -1).tocoo()
+    s = np.lexsort((H.col, H.row))
+    return H.row[s].astype(np.int64), H.col[s].astype(np.int64), v[H.data[s].astype(np.int64) - 1]
+
+
+# copies of a few determinants, of the lowest one, and more than 64 of one (a run of the index longer than a
+# slot's length field)
+@pytest.mark.parametrize("copies", [(1,), (2, 1, 1, 3), (70,)])
+@pytest.mark.parametrize("norb", [13, 33])
+def test_repeated_determinants(system, norb, copies):  # noqa: F811
+    e, o = system(norb, 12)
+    dets = _grouped([0b111111, 0b1011111, 0b1101111])
+    rng = np.random.default_rng(len(copies))
+    twice = np.concatenate([[0], rng.choice(np.arange(1, len(dets)), len(copies) - 1, replace=False)])
+    dets = np.concatenate([dets] + [np.repeat(dets[i:i + 1], m, 0) for i, m in zip(twice, copies)])
+    dets = dets[rng.permutation(len(dets))]
+    n = len(dets)
+    ref = _expanded(o, dets)
+    x = rng.standard_normal(n)
+    for mode in ("fp64", "mixed"):
+        e.set_dets(dets)
+        nnz = e.ham_build(mode)
+        assert nnz == 2 * len(ref[0])
+        rp, col, val = e.ham_export(nnz)
+        got = _lower(n, rp, col, val)
+        assert np.array_equal(got[0], ref[0]) and np.array_equal(got[1], ref[1]), mode
+        assert np.all(np.abs(got[2] - ref[2]) <= (0.0 if mode == "fp64" else 2.0 ** -48) * np.abs(ref[2]))
+        if mode == "fp64":
+            diag = e.diag()
+            row = np.repeat(np.arange(n), np.diff(rp))
+            y = diag * x + np.bincount(row, val * x[col], n)
+            A = np.abs(diag * x) + np.bincount(row, np.abs(val * x[col]), n)
+            for m in ("fp64", "direct"):
+                assert np.all(np.abs(e.sigma(x, m) - y) <= 2 * (np.diff(rp) + 4) * U64 * A), m
+        # the same list reached by extending stored rows
+        tail = np.unique(dets, axis=0)
+        tail = tail[ref_order(tail)][-40:]
+        old = np.array([d for d in dets if not (tail == d).all(1).any()], dtype=np.uint64)
+        e.set_dets(np.concatenate([old, tail]))
+        full = e.ham_export(e.ham_build(mode))
+        e.set_dets(old)
+        e.ham_build(mode)
+        e.append_dets(tail)
+        for a, b in zip(e.ham_export(e.ham_build(mode)), full):
+            assert np.array_equal(a, b), mode
