@@ -1653,8 +1653,9 @@ void build_ham_csr(const Helpers& hp, const IntsView& ints, Csr& H, bool want64,
                    size_t n_old, Prims& pr, cudaStream_t s) {
   const size_t N = hp.N;
   PhaseTimer pt(s);
-  const bool incremental = !H.block && n_old > 0 && N - n_old < n_old && H.N == n_old && H.perm.n >= n_old &&
-                           (want64 ? !want32 : (want32 && want_lo)) &&
+  // a step that at least doubles the space is rebuilt; one that adds nothing is left as it is (below)
+  const bool incremental = !H.block && n_old > 0 && n_old < N && N - n_old < n_old && H.N == n_old &&
+                           H.perm.n >= n_old && (want64 ? !want32 : (want32 && want_lo)) &&
                            (H.v64.p != nullptr) == want64 && (H.vhi.p != nullptr) == want32 &&
                            (H.vlo.p != nullptr) == (want32 && want_lo);
   if (!incremental) {

@@ -1,5 +1,5 @@
 """The Hamiltonian build on lists of determinants at the edge of what the calls
-take: determinants given more than once."""
+take: determinants given more than once, spaces that have not changed."""
 import itertools
 
 import numpy as np
@@ -7,7 +7,7 @@ import pytest
 from scipy import sparse
 
 from dice_gb300.shard import ref_order
-from test_gpu_stored_edges import U64, _lower, _words, system  # noqa: F401  (fixture)
+from test_gpu_stored_edges import U64, _lower, _star, _words, system  # noqa: F401  (fixture)
 
 pytestmark = pytest.mark.gpu
 
@@ -73,3 +73,18 @@ def test_repeated_determinants(system, norb, copies):  # noqa: F811
         e.append_dets(tail)
         for a, b in zip(e.ham_export(e.ham_build(mode)), full):
             assert np.array_equal(a, b), mode
+
+
+@pytest.mark.parametrize("mode", ["fp64", "mixed"])
+def test_unchanged_space_is_not_built_again(system, mode):  # noqa: F811
+    """A repeated build of the same space keeps the stored rows: nothing is launched but the mixed form's compact
+    copy (lengths, their scan, the copy)."""
+    e, _ = system(20, 20)
+    e.set_dets(_star(20, 10, 10, 3000, 5))
+    nnz = e.ham_build(mode)
+    first = e.ham_export(nnz)
+    before = e.launch_count()
+    assert e.ham_build(mode) == nnz
+    assert e.launch_count() - before <= (0 if mode == "fp64" else 5)
+    for a, b in zip(e.ham_export(nnz), first):
+        assert np.array_equal(a, b)
