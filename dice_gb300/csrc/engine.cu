@@ -1216,17 +1216,26 @@ struct Context {
         G.swap(Gn);
         continue;
       }
-      // Some correction was linearly dependent on the basis (rare: tiny or
-      // exhausted spaces). Drop it, as the reference does, and redo the
+      // Some correction was linearly dependent on the basis, or nearly (rare:
+      // tiny or exhausted spaces). Drop it, as the reference does, and redo the
       // append and sigma for the others on the stream directly; the rotated
       // basis (if collapsed) is kept.
       int kept = 0;
-      for (int a = 0; a < nact; ++a) {
-        if (!(std::sqrt(pin[kPinNrm + a]) > 1e-14)) continue;
-        if (kept != a)
-          SHCI_CUDA(cudaMemcpyAsync(D.p + (size_t)kept * N, D.p + (size_t)a * N, N * sizeof(double),
-                                    cudaMemcpyDeviceToDevice, stream));
-        ++kept;
+      if (nact == 1) {  // appended as it was left, its norm not known
+        double* v = V.p + (size_t)m1 * N;
+        const double nv = norm_host(v);
+        if (nv > 1e-14) {
+          scale_col(v, 1.0 / nv);
+          kept = 1;
+        }
+      } else {
+        for (int a = 0; a < nact; ++a) {
+          if (!(std::sqrt(pin[kPinNrm + a]) > 1e-14)) continue;
+          if (kept != a)
+            SHCI_CUDA(cudaMemcpyAsync(D.p + (size_t)kept * N, D.p + (size_t)a * N, N * sizeof(double),
+                                      cudaMemcpyDeviceToDevice, stream));
+          ++kept;
+        }
       }
       m = m1;
       if (kept == 0) {  // nothing new to add: the subspace is exhausted
@@ -1241,8 +1250,9 @@ struct Context {
         finish();
         return;
       }
-      SHCI_CUDA(cudaMemcpyAsync(V.p + (size_t)m * N, D.p, (size_t)kept * N * sizeof(double),
-                                cudaMemcpyDeviceToDevice, stream));
+      if (nact > 1)
+        SHCI_CUDA(cudaMemcpyAsync(V.p + (size_t)m * N, D.p, (size_t)kept * N * sizeof(double),
+                                  cudaMemcpyDeviceToDevice, stream));
       apply_sigma(mode, V.p, N, m, kept, W.p, N, m);
       m += kept;
       G = gram_host(V.p, N, m, W.p, N, m);

@@ -428,7 +428,8 @@ void dav_ritz(const double* V, const double* W, size_t ld, int m, const double* 
 // D = preconditioned residual of one root (shift and flip may be null; p: the
 // flip sector), made orthogonal to the m columns of V by two classical
 // Gram-Schmidt passes, normalised and written to V[:, at]; *nrm and *nrm_out =
-// its squared norm before. Q given: V and W are rotated to the keep columns V Q
+// its squared norm before, or -1 where that has to be measured (V[:, at] is then
+// not normalised). Q given: V and W are rotated to the keep columns V Q
 // and W Q in the same pass. g1: m, g2: m + 1 doubles.
 void dav_correction(double* V, double* W, size_t ld, int m, const double* X, const double* Y, const double* lam,
                     const double* diag, const double* shift, const int32_t* flip, const int8_t* sign, double p,

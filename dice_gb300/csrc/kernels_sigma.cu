@@ -1229,8 +1229,12 @@ __global__ void __launch_bounds__(kDavThreads) k_dav_project(const double* __res
 // The second Gram-Schmidt projection, the normalisation and the append in one
 // pass, with the rotation of V and W when the basis collapses (Q given: keep
 // columns; in place, every thread owns its row): V[:, at] = (D - V g) / |D - V g|.
-// |D - V g|^2 = |D|^2 - |g|^2, V being orthonormal and g a rounding residue;
-// a dependent D (norm below 1e-14) is left for the host to drop.
+// |D - V g|^2 = |D|^2 - |g|^2, V being orthonormal, while g is small beside D
+// (a rounding residue, as a rule; a hundredth of D leaves the difference 15
+// digits). Where it is not, the first projection left little but rounding: the
+// difference has no digits, so D - V g is appended as it is and the norm given as
+// -1, for the host to measure it. A dependent D (norm below 1e-14) is left for the
+// host to drop.
 template <int M>
 __global__ void __launch_bounds__(256) k_dav_append(double* __restrict__ V, double* __restrict__ W, size_t ld, int m,
                                                     const double* __restrict__ g, size_t N,
@@ -1243,8 +1247,12 @@ __global__ void __launch_bounds__(256) k_dav_append(double* __restrict__ V, doub
   if ((int)threadIdx.x < m) sg[threadIdx.x] = g[threadIdx.x];
   __syncthreads();
   if (threadIdx.x == 0) {  // one thread's square root and division, not every thread's
-    double n2 = g[m];
-    for (int i = 0; i < m; ++i) n2 -= sg[i] * sg[i];
+    double n2 = g[m], gg = 0.0;
+    for (int i = 0; i < m; ++i) {
+      n2 -= sg[i] * sg[i];
+      gg += sg[i] * sg[i];
+    }
+    if (!(gg <= 1e-4 * g[m])) n2 = -1.0;
     const double n = sqrt(n2);
     s_sc = n > 1e-14 ? 1.0 / n : 1.0;
     if (blockIdx.x == 0) {
