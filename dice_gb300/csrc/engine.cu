@@ -730,8 +730,14 @@ struct Context {
       // (selection only appends), so only new rows and columns are built
       const size_t n_old = (ham_mode == mode && !H.block) ? H.N : 0;
       H.drop_compressed();  // stale; rebuilt below (frees its memory before the build)
-      build_ham_csr(helpers, ints(), H, mode == SHCI_MODE_FP64, mode == SHCI_MODE_MIXED,
-                    mode == SHCI_MODE_MIXED, n_old, prims, stream);
+      const size_t held = H.N;
+      try {
+        build_ham_csr(helpers, ints(), H, mode == SHCI_MODE_FP64, mode == SHCI_MODE_MIXED,
+                      mode == SHCI_MODE_MIXED, n_old, prims, stream);
+      } catch (...) {
+        if (H.N != held) ham_ok = false;  // the matrix that was there is gone
+        throw;
+      }
       if (mode == SHCI_MODE_MIXED) compress_csr(H, prims, stream);
       pt.mark("ham compress");
       noalloc_ptr = noalloc_scratch_address();

@@ -1370,13 +1370,17 @@ static void sort_rows(const int64_t* rowptr, size_t n, const CsrVals& v, cudaStr
   SHCI_CUDA(cudaStreamSynchronize(s));  // the scratch is freed on return
 }
 
-// Full rows of nr positions (rows[k], or all when null) into (rowptr, vals),
-// columns ascending; returns nnz.
+// Full rows of nr positions (rows[k], or all when null) into out's row pointers
+// and values, columns ascending; returns nnz. out holds no rows (N = 0) from where
+// its arrays are first touched, so that an allocation that fails half way leaves
+// nothing that looks like a matrix; the caller sets N.
 template <class S>
-static int64_t emit_rows_as(const Helpers& hp, const uint32_t* rows, size_t nr, const IntsView& ints,
-                         DevBuf<int64_t>& rowptr, DevBuf<int32_t>& col, DevBuf<double>& v64, DevBuf<float>& vhi,
-                         DevBuf<float>& vlo, bool want64, bool want32, bool want_lo, Prims& pr, cudaStream_t s,
-                         PhaseTimer& pt) {
+static int64_t emit_rows_as(const Helpers& hp, const uint32_t* rows, size_t nr, const IntsView& ints, Csr& out,
+                            bool want64, bool want32, bool want_lo, Prims& pr, cudaStream_t s, PhaseTimer& pt) {
+  DevBuf<int64_t>& rowptr = out.rowptr;
+  DevBuf<int32_t>& col = out.col;
+  DevBuf<double>& v64 = out.v64;
+  DevBuf<float>&vhi = out.vhi, &vlo = out.vlo;
   HelperView<S> hv = hp.view<S>();
   DevBuf<int64_t> counts;
   DevBuf<uint4> parts;
@@ -1388,6 +1392,8 @@ static int64_t emit_rows_as(const Helpers& hp, const uint32_t* rows, size_t nr, 
     SHCI_LAUNCH_CHECK();
   }
   pt.mark("ham count");
+  out.N = 0;
+  out.nnz = 0;
   rowptr.resize(nr + 1);
   int64_t total = 0;
   scan_exclusive_i64(counts.p, rowptr.p, nr, &total, pr, s);
@@ -1440,14 +1446,10 @@ static int64_t emit_rows_as(const Helpers& hp, const uint32_t* rows, size_t nr, 
   pt.mark("ham finish");
   return total;
 }
-static int64_t emit_rows(const Helpers& hp, const uint32_t* rows, size_t nr, const IntsView& ints,
-                         DevBuf<int64_t>& rowptr, DevBuf<int32_t>& col, DevBuf<double>& v64, DevBuf<float>& vhi,
-                         DevBuf<float>& vlo, bool want64, bool want32, bool want_lo, Prims& pr, cudaStream_t s,
-                         PhaseTimer& pt) {
-  return hp.narrow ? emit_rows_as<uint32_t>(hp, rows, nr, ints, rowptr, col, v64, vhi, vlo, want64, want32, want_lo, pr,
-                                            s, pt)
-                   : emit_rows_as<uint64_t>(hp, rows, nr, ints, rowptr, col, v64, vhi, vlo, want64, want32, want_lo, pr,
-                                            s, pt);
+static int64_t emit_rows(const Helpers& hp, const uint32_t* rows, size_t nr, const IntsView& ints, Csr& out, bool want64,
+                         bool want32, bool want_lo, Prims& pr, cudaStream_t s, PhaseTimer& pt) {
+  return hp.narrow ? emit_rows_as<uint32_t>(hp, rows, nr, ints, out, want64, want32, want_lo, pr, s, pt)
+                   : emit_rows_as<uint64_t>(hp, rows, nr, ints, out, want64, want32, want_lo, pr, s, pt);
 }
 
 // Positions of the determinants [r0, r1), ascending: flags, and after their
@@ -1660,6 +1662,7 @@ void build_ham_csr(const Helpers& hp, const IntsView& ints, Csr& H, bool want64,
                            (H.vlo.p != nullptr) == (want32 && want_lo);
   if (!incremental) {
     if (n_old == N && H.N == N && !H.block) return;  // nothing new
+    const int64_t nnz = emit_rows(hp, nullptr, N, ints, H, want64, want32, want_lo, pr, s, pt);
     H.clear_block();
     H.perm.resize(N > 0 ? N : 1);
     H.spos.resize(N > 0 ? N : 1);
@@ -1667,7 +1670,7 @@ void build_ham_csr(const Helpers& hp, const IntsView& ints, Csr& H, bool want64,
       SHCI_CUDA(cudaMemcpyAsync(H.perm.p, hp.perm.p, N * sizeof(uint32_t), cudaMemcpyDeviceToDevice, s));
       SHCI_CUDA(cudaMemcpyAsync(H.spos.p, hp.spos.p, N * sizeof(uint32_t), cudaMemcpyDeviceToDevice, s));
     }
-    H.nnz = emit_rows(hp, nullptr, N, ints, H.rowptr, H.col, H.v64, H.vhi, H.vlo, want64, want32, want_lo, pr, s, pt);
+    H.nnz = nnz;
     H.N = N;
     SHCI_CUDA(cudaStreamSynchronize(s));
     return;
@@ -1686,8 +1689,7 @@ void build_ham_csr(const Helpers& hp, const IntsView& ints, Csr& H, bool want64,
   k_range_fill<<<grid_for(N, 256), 256, 0, s>>>(perm.p, N, (uint32_t)n_old, (uint32_t)N, slot.p, rows.p, nullptr);
   SHCI_LAUNCH_CHECK();
   Csr Hn;  // rows of the determinants n_old .. N-1, in storage order
-  Hn.nnz = emit_rows(hp, rows.p, nr, ints, Hn.rowptr, Hn.col, Hn.v64, Hn.vhi, Hn.vlo, want64, want32, want_lo, pr, s,
-                     pt);
+  Hn.nnz = emit_rows(hp, rows.p, nr, ints, Hn, want64, want32, want_lo, pr, s, pt);
   CsrVals nv{Hn.col.p, Hn.v64.p, Hn.vhi.p, Hn.vlo.p};
   // new columns of the old rows, indexed by the old row's new storage position
   DevBuf<uint32_t> oldbits;
@@ -1750,16 +1752,19 @@ void build_ham_csr(const Helpers& hp, const IntsView& ints, Csr& H, bool want64,
                                                                     dptr.p, dv, Hn.rowptr.p, nv, slot.p, (int64_t)n_old,
                                                                     (int64_t)N, rp.p, mv);
   SHCI_LAUNCH_CHECK();
+  DevBuf<uint32_t> nperm, nspos;
+  nperm.resize(N);
+  nspos.resize(N);
+  SHCI_CUDA(cudaMemcpyAsync(nperm.p, perm.p, N * sizeof(uint32_t), cudaMemcpyDeviceToDevice, s));
+  SHCI_CUDA(cudaMemcpyAsync(nspos.p, spos.p, N * sizeof(uint32_t), cudaMemcpyDeviceToDevice, s));
   SHCI_CUDA(cudaStreamSynchronize(s));
   H.rowptr.swap(rp);
   H.col.swap(M.col);
   H.v64.swap(M.v64);
   H.vhi.swap(M.vhi);
   H.vlo.swap(M.vlo);
-  H.perm.resize(N);
-  H.spos.resize(N);
-  SHCI_CUDA(cudaMemcpyAsync(H.perm.p, perm.p, N * sizeof(uint32_t), cudaMemcpyDeviceToDevice, s));
-  SHCI_CUDA(cudaMemcpyAsync(H.spos.p, spos.p, N * sizeof(uint32_t), cudaMemcpyDeviceToDevice, s));
+  H.perm.swap(nperm);
+  H.spos.swap(nspos);
   H.N = N;
   H.nnz = total;
   pt.mark("ham merge");
@@ -1796,7 +1801,7 @@ void build_ham_block(const Helpers& hp, const IntsView& ints, Csr& H, bool want6
   SHCI_LAUNCH_CHECK();
   pt.mark("ham block order");
   H.drop_compressed();
-  H.nnz = emit_rows(hp, xpos.p, nb, ints, H.rowptr, H.col, H.v64, H.vhi, H.vlo, want64, want32, want_lo, pr, s, pt);
+  H.nnz = emit_rows(hp, xpos.p, nb, ints, H, want64, want32, want_lo, pr, s, pt);
   H.xperm.resize(N);
   SHCI_CUDA(cudaMemcpyAsync(H.xperm.p, hp.perm.p, N * sizeof(uint32_t), cudaMemcpyDeviceToDevice, s));
   SHCI_CUDA(cudaStreamSynchronize(s));

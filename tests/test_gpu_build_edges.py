@@ -1,11 +1,13 @@
 """The Hamiltonian build on lists of determinants at the edge of what the calls
-take: determinants given more than once, spaces that have not changed."""
+take: determinants given more than once, spaces that have not changed, builds that
+run out of memory half way."""
 import itertools
 
 import numpy as np
 import pytest
 from scipy import sparse
 
+from dice_gb300 import engine as eng
 from dice_gb300.shard import ref_order
 from test_gpu_stored_edges import U64, _lower, _star, _words, system  # noqa: F401  (fixture)
 
@@ -88,3 +90,65 @@ def test_unchanged_space_is_not_built_again(system, mode):  # noqa: F811
     assert e.launch_count() - before <= (0 if mode == "fp64" else 5)
     for a, b in zip(e.ham_export(nnz), first):
         assert np.array_equal(a, b)
+
+
+@pytest.mark.parametrize("build", ["mixed", "rows", "grown"])
+def test_build_that_runs_out_of_memory(system, build):  # noqa: F811
+    """Wherever a build stops for want of memory, the matrix that was there is either still there or refused,
+    and the next build is complete."""
+    e, _ = system(20, 20)
+    dets = _star(20, 10, 10, 4000, 11)
+    tail = dets[1500:][ref_order(dets[1500:])]
+    full = np.concatenate([dets[:1500], tail])
+    rng = np.random.default_rng(1)
+    x, xf = rng.standard_normal(1500 if build == "grown" else 4000), rng.standard_normal(4000)
+
+    def prepare():
+        e.set_dets(full[:1500] if build == "grown" else full)
+        e.ham_build("fp64")
+
+    def attempt():
+        if build == "grown":
+            e.append_dets(tail)
+            return e.ham_build("fp64")
+        return e.ham_build("mixed") if build == "mixed" else e.ham_build_rows(100, 3900, "fp64")
+
+    prepare()
+    y = e.sigma(x, "fp64")
+    e.set_dets(full)
+    nnz = e.ham_build("fp64")
+    yf = e.sigma(xf, "fp64")
+    refused = held = 0
+    cap, step = 2.0 ** 20, 2.0
+    while True:  # the smallest sufficient cap from below, then in small steps
+        prepare()
+        e.set_alloc_cap(int(cap))
+        try:
+            attempt()
+            ok = True
+        except eng.ShciError as err:
+            assert err.code == 4
+            ok = False
+        finally:
+            e.set_alloc_cap(0)
+        if ok:
+            if step < 1.01:
+                break
+            cap, step = cap / step, 1.0 + (step - 1.0) / 8.0  # back to the last cap that was too small
+            continue
+        if e.ndets() == len(x):
+            try:
+                assert np.array_equal(e.sigma(x, "fp64"), y)
+                held += 1
+            except eng.ShciError as err:
+                assert err.code == 7
+                refused += 1
+        if build == "grown":
+            try:
+                e.append_dets(tail)  # the append itself may have been what failed
+            except eng.ShciError as err:
+                assert err.code == 1
+        assert e.ham_build("fp64") == nnz
+        assert np.array_equal(e.sigma(xf, "fp64"), yf)
+        cap *= step
+    assert build == "grown" or refused > 0
