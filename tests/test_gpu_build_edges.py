@@ -92,7 +92,7 @@ def test_unchanged_space_is_not_built_again(system, mode):  # noqa: F811
         assert np.array_equal(a, b)
 
 
-@pytest.mark.parametrize("build", ["mixed", "rows", "grown"])
+@pytest.mark.parametrize("build", ["fp64", "rows", "grown"])
 def test_build_that_runs_out_of_memory(system, build):  # noqa: F811
     """Wherever a build stops for want of memory, the matrix that was there is either still there or refused,
     and the next build is complete."""
@@ -105,19 +105,19 @@ def test_build_that_runs_out_of_memory(system, build):  # noqa: F811
 
     def prepare():
         e.set_dets(full[:1500] if build == "grown" else full)
-        e.ham_build("fp64")
+        e.ham_build("mixed")
 
     def attempt():
         if build == "grown":
             e.append_dets(tail)
-            return e.ham_build("fp64")
-        return e.ham_build("mixed") if build == "mixed" else e.ham_build_rows(100, 3900, "fp64")
+            return e.ham_build("mixed")
+        return e.ham_build("fp64") if build == "fp64" else e.ham_build_rows(100, 3900, "mixed")
 
     prepare()
-    y = e.sigma(x, "fp64")
+    y = e.sigma(x, "mixed")
     e.set_dets(full)
-    nnz = e.ham_build("fp64")
-    yf = e.sigma(xf, "fp64")
+    nnz = e.ham_build("mixed")
+    yf = e.sigma(xf, "mixed")
     refused = held = 0
     cap, step = 2.0 ** 20, 2.0
     while True:  # the smallest sufficient cap from below, then in small steps
@@ -138,7 +138,7 @@ def test_build_that_runs_out_of_memory(system, build):  # noqa: F811
             continue
         if e.ndets() == len(x):
             try:
-                assert np.array_equal(e.sigma(x, "fp64"), y)
+                assert np.array_equal(e.sigma(x, "mixed"), y)
                 held += 1
             except eng.ShciError as err:
                 assert err.code == 7
@@ -148,7 +148,7 @@ def test_build_that_runs_out_of_memory(system, build):  # noqa: F811
                 e.append_dets(tail)  # the append itself may have been what failed
             except eng.ShciError as err:
                 assert err.code == 1
-        assert e.ham_build("fp64") == nnz
-        assert np.array_equal(e.sigma(xf, "fp64"), yf)
+        assert e.ham_build("mixed") == nnz
+        assert np.array_equal(e.sigma(xf, "mixed"), yf)
         cap *= step
     assert build == "grown" or refused > 0
