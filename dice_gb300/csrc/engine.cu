@@ -449,23 +449,23 @@ struct Context {
     flip_project(c, ndet, flipidx.p, flipsgn.p, p, ftmp.p, stream);
   }
 
+  // A determinant handed in (number i of a list): NELEC electrons, none beyond NORB.
+  void require_det(const uint64_t* w, int64_t i) const {
+    if (__builtin_popcountll(w[0]) + __builtin_popcountll(w[1]) != hints.nelec)
+      throw Error(kErrInvalid, "determinant " + std::to_string(i) + " has wrong electron count");
+    const int n2 = 2 * hints.norb;
+    const uint64_t lim0 = n2 >= 64 ? ~0ull : (1ull << n2) - 1ull;
+    const uint64_t lim1 = n2 >= 128 ? ~0ull : (n2 > 64 ? (1ull << (n2 - 64)) - 1ull : 0ull);
+    if ((w[0] & ~lim0) || (w[1] & ~lim1))
+      throw Error(kErrInvalid, "determinant " + std::to_string(i) + " occupies orbitals beyond NORB");
+  }
+
   void set_dets(const uint64_t* h, int64_t n) {
     require_ints();
     H.N = 0;  // the stored Hamiltonian no longer describes a prefix of the space
     H.nnz = 0;
     if (n < 0) throw Error(kErrInvalid, "negative determinant count");
-    const int n2 = 2 * hints.norb;
-    for (int64_t i = 0; i < n; ++i) {
-      uint64_t w0 = h[2 * i], w1 = h[2 * i + 1];
-      int ne = __builtin_popcountll(w0) + __builtin_popcountll(w1);
-      if (ne != hints.nelec) throw Error(kErrInvalid, "determinant " + std::to_string(i) + " has wrong electron count");
-      if (n2 < 128) {
-        uint64_t lim0 = n2 >= 64 ? ~0ull : ((1ull << n2) - 1ull);
-        uint64_t lim1 = n2 > 64 ? ((1ull << (n2 - 64)) - 1ull) : 0ull;
-        if ((w0 & ~lim0) || (w1 & ~lim1))
-          throw Error(kErrInvalid, "determinant " + std::to_string(i) + " occupies orbitals beyond NORB");
-      }
-    }
+    for (int64_t i = 0; i < n; ++i) require_det(h + 2 * i, i);
     dets.resize(n > 0 ? (size_t)n : 1);
     if (n) SHCI_CUDA(cudaMemcpyAsync(dets.p, h, (size_t)n * sizeof(Det2), cudaMemcpyHostToDevice, stream));
     ndet = (size_t)n;
@@ -552,7 +552,7 @@ struct Context {
 
   // Appends host determinants (the merged new determinants of a sharded
   // selection): they must follow the reference's order strictly, carry the
-  // right electron count and be absent from the space.
+  // right electron count, in orbitals that there are, and be absent from the space.
   void append_dets(const uint64_t* h, int64_t n) {
     require_ints();
     require_dets();
@@ -560,8 +560,7 @@ struct Context {
     if (n == 0) return;
     for (int64_t i = 0; i < n; ++i) {
       const uint64_t w0 = h[2 * i], w1 = h[2 * i + 1];
-      if (__builtin_popcountll(w0) + __builtin_popcountll(w1) != hints.nelec)
-        throw Error(kErrInvalid, "appended determinant " + std::to_string(i) + " has the wrong electron count");
+      require_det(h + 2 * i, i);
       if (i > 0) {  // Determinant::operator<: signed words from the top (SHCI/Determinants.h:490-498)
         const int64_t a1 = (int64_t)h[2 * i - 1], b1 = (int64_t)w1;
         const int64_t a0 = (int64_t)h[2 * i - 2], b0 = (int64_t)w0;

@@ -118,8 +118,8 @@ int shci_select(shci_ctx* ctx, const double* cmax, double eps1, int64_t* n_new);
  * shci_candidates_get: copies them out (cap >= *n_new, 2 words each).
  * shci_dets_append: appends determinants to the space in the given order; they
  *   must be strictly increasing in the reference's order (Determinant::operator<,
- *   SHCI/Determinants.h:490-498), carry NELEC electrons and be absent from the
- *   space (SHCI_ERR_INVALID otherwise), as the reference appends the merged
+ *   SHCI/Determinants.h:490-498), carry NELEC electrons in NORB orbitals and be
+ *   absent from the space (SHCI_ERR_INVALID otherwise), as the reference appends the merged
  *   new determinants at SHCI/SHCIbasics.cpp:1059-1077. */
 int shci_select_candidates(shci_ctx* ctx, const double* cmax, double eps1, int rank, int world, int64_t* n_new);
 int shci_candidates_get(shci_ctx* ctx, uint64_t* out, int64_t cap);

@@ -152,3 +152,19 @@ def test_build_that_runs_out_of_memory(system, build):  # noqa: F811
         assert np.array_equal(e.sigma(xf, "mixed"), yf)
         cap *= step
     assert build == "grown" or refused > 0
+
+
+@pytest.mark.parametrize("norb", [20, 32, 33, 64])
+def test_appended_determinants_lie_within_the_orbitals(system, norb):  # noqa: F811
+    """An electron past the last orbital, or one electron too many, is refused and the space stays as it was."""
+    e, _ = system(norb, 6)
+    dets = _star(norb, 3, 3, 20, 2)
+    e.set_dets(dets)
+    beyond = [(1 << (2 * norb)) | 0b11111] if norb < 64 else []
+    for w in beyond + [(1 << (2 * norb - 1)) | 0b111111]:
+        with pytest.raises(eng.ShciError) as err:
+            e.append_dets(np.array([(w & (2 ** 64 - 1), w >> 64)], dtype=np.uint64))
+        assert err.value.code == 1
+    w = (3 << (2 * norb - 2)) | (15 << (2 * norb - 6))  # the last three orbitals, doubly occupied
+    e.append_dets(np.array([(w & (2 ** 64 - 1), w >> 64)], dtype=np.uint64))
+    assert np.array_equal(e.dets(), np.concatenate([dets, [[w & (2 ** 64 - 1), w >> 64]]]))
