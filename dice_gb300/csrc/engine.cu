@@ -462,15 +462,16 @@ struct Context {
 
   void set_dets(const uint64_t* h, int64_t n) {
     require_ints();
-    H.N = 0;  // the stored Hamiltonian no longer describes a prefix of the space
-    H.nnz = 0;
     if (n < 0) throw Error(kErrInvalid, "negative determinant count");
     for (int64_t i = 0; i < n; ++i) require_det(h + 2 * i, i);
+    H.N = 0;  // the stored Hamiltonian no longer describes a prefix of the space
+    H.nnz = 0;
+    ndet = 0;
+    ndiag = 0;
+    invalidate_space();
     dets.resize(n > 0 ? (size_t)n : 1);
     if (n) SHCI_CUDA(cudaMemcpyAsync(dets.p, h, (size_t)n * sizeof(Det2), cudaMemcpyHostToDevice, stream));
     ndet = (size_t)n;
-    ndiag = 0;
-    invalidate_space();
     SHCI_CUDA(cudaStreamSynchronize(stream));
   }
 

@@ -168,3 +168,21 @@ def test_appended_determinants_lie_within_the_orbitals(system, norb):  # noqa: F
     w = (3 << (2 * norb - 2)) | (15 << (2 * norb - 6))  # the last three orbitals, doubly occupied
     e.append_dets(np.array([(w & (2 ** 64 - 1), w >> 64)], dtype=np.uint64))
     assert np.array_equal(e.dets(), np.concatenate([dets, [[w & (2 ** 64 - 1), w >> 64]]]))
+
+
+@pytest.mark.parametrize("mode", ["fp64", "mixed", "direct"])
+def test_refused_space_leaves_the_old_one(system, mode):  # noqa: F811
+    """A list with a wrong determinant is refused; the space and its matrix are still there."""
+    e, _ = system(20, 20)
+    dets = _star(20, 10, 10, 300, 4)
+    e.set_dets(dets)
+    e.ham_build(mode)
+    x = np.random.default_rng(0).standard_normal(300)
+    y = e.sigma(x, mode)
+    e.sigma(x + 1.0, mode)  # y is no longer in the context's buffers
+    bad = dets[:200].copy()
+    bad[150, 0] ^= np.uint64(1)  # an electron too few or too many
+    with pytest.raises(eng.ShciError) as err:
+        e.set_dets(bad)
+    assert err.value.code == 1
+    assert np.array_equal(e.dets(), dets) and np.array_equal(e.sigma(x, mode), y)
