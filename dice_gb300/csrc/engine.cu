@@ -201,6 +201,9 @@ struct Context {
 
   DevBuf<Det2> dets;
   size_t ndet = 0;
+  // the first determinant of the list set last, and the bits in which some
+  // determinant of the space, or of the candidates in cand, differs from it
+  Det2 ref{0, 0}, diff{0, 0}, cand_diff{0, 0};
   DetHash hash;
   Helpers helpers;
   bool helpers_ok = false;
@@ -449,30 +452,53 @@ struct Context {
     flip_project(c, ndet, flipidx.p, flipsgn.p, p, ftmp.p, stream);
   }
 
-  // A determinant handed in (number i of a list): NELEC electrons, none beyond NORB.
-  void require_det(const uint64_t* w, int64_t i) const {
-    if (__builtin_popcountll(w[0]) + __builtin_popcountll(w[1]) != hints.nelec)
-      throw Error(kErrInvalid, "determinant " + std::to_string(i) + " has wrong electron count");
+  // A list of determinants handed in: NELEC electrons each, none beyond NORB.
+  // Returns the bits in which some differ from r.
+  Det2 require_list(const uint64_t* h, int64_t n, const Det2& r) const {
     const int n2 = 2 * hints.norb;
     const uint64_t lim0 = n2 >= 64 ? ~0ull : (1ull << n2) - 1ull;
     const uint64_t lim1 = n2 >= 128 ? ~0ull : (n2 > 64 ? (1ull << (n2 - 64)) - 1ull : 0ull);
-    if ((w[0] & ~lim0) || (w[1] & ~lim1))
-      throw Error(kErrInvalid, "determinant " + std::to_string(i) + " occupies orbitals beyond NORB");
+    auto wrong = [&](const uint64_t* w) { return __builtin_popcountll(w[0]) + __builtin_popcountll(w[1]) != hints.nelec; };
+    Det2 d{0, 0}, any{0, 0};
+    bool bad = false;
+    for (int64_t i = 0; i < n; ++i) {
+      const uint64_t* w = h + 2 * i;
+      any.w0 |= w[0];
+      any.w1 |= w[1];
+      d.w0 |= w[0] ^ r.w0;
+      d.w1 |= w[1] ^ r.w1;
+      bad |= wrong(w);
+    }
+    if (bad || (any.w0 & ~lim0) || (any.w1 & ~lim1))
+      for (int64_t i = 0; i < n; ++i) {
+        const uint64_t* w = h + 2 * i;
+        if (wrong(w)) throw Error(kErrInvalid, "determinant " + std::to_string(i) + " has wrong electron count");
+        if ((w[0] & ~lim0) || (w[1] & ~lim1))
+          throw Error(kErrInvalid, "determinant " + std::to_string(i) + " occupies orbitals beyond NORB");
+      }
+    return d;
   }
 
   void set_dets(const uint64_t* h, int64_t n) {
     require_ints();
     if (n < 0) throw Error(kErrInvalid, "negative determinant count");
-    for (int64_t i = 0; i < n; ++i) require_det(h + 2 * i, i);
+    const Det2 r = n ? Det2{h[0], h[1]} : Det2{0, 0}, d = require_list(h, n, r);
     H.N = 0;  // the stored Hamiltonian no longer describes a prefix of the space
     H.nnz = 0;
     ndet = 0;
     ndiag = 0;
+    ref = r;
+    diff = d;
     invalidate_space();
     dets.resize(n > 0 ? (size_t)n : 1);
     if (n) SHCI_CUDA(cudaMemcpyAsync(dets.p, h, (size_t)n * sizeof(Det2), cudaMemcpyHostToDevice, stream));
     ndet = (size_t)n;
     SHCI_CUDA(cudaStreamSynchronize(stream));
+  }
+
+  void widen() {  // the candidates have become part of the space
+    diff.w0 |= cand_diff.w0;
+    diff.w1 |= cand_diff.w1;
   }
 
   // Heat-bath selection from every current determinant; appends new ones.
@@ -491,7 +517,10 @@ struct Context {
     size_t nnew = 0;
     if (n) {
       trev_buf.reserve(2 * n);
-      nnew = trev_new_dets(cand.p, n, hints.norb, hash, dets.p, trev_buf.p, trev_flag, trev_pos, prims, stream);
+      // flipped, a candidate differs from ref where it differed from ref's flip
+      const Det2 f = det_flip_pair(cand_diff), r = det_flip_pair(ref);
+      cand_diff = Det2{cand_diff.w0 | f.w0 | (ref.w0 ^ r.w0), cand_diff.w1 | f.w1 | (ref.w1 ^ r.w1)};
+      nnew = trev_new_dets(cand.p, n, cand_diff, hash, dets.p, trev_buf.p, trev_flag, trev_pos, prims, stream);
     }
     ncand = 0;
     if (nnew) {
@@ -500,6 +529,7 @@ struct Context {
       k_append<<<grid_for(nnew, 256), 256, 0, stream>>>(trev_buf.p, nnew, dets.p + ndet);
       SHCI_LAUNCH_CHECK();
       ndet += nnew;
+      widen();
       invalidate_space();
     }
     SHCI_CUDA(cudaStreamSynchronize(stream));
@@ -512,23 +542,23 @@ struct Context {
     require_ints();
     require_dets();
     hash.build(dets.p, ndet, stream);
-    counter.resize(1);
+    counter.resize(3);
     int64_t cap = (int64_t)std::max<size_t>(cand.cap, std::max<size_t>((size_t)1 << 20, 4 * ndet));
     cand.reserve((size_t)cap);
     cap = (int64_t)cand.cap;
     int64_t total = select_candidates(dets.p, cmax_dev, ndet, eps1, ints(), hb(), hints.maxEntry, sp, hash, cand.p,
-                                      cap, counter.p, psplit, stream);
+                                      cap, counter.p, ref, &cand_diff, psplit, stream);
     if (total > cap) {
       cand.release();
       cand.reserve((size_t)total + total / 8);
       cap = (int64_t)cand.cap;
       total = select_candidates(dets.p, cmax_dev, ndet, eps1, ints(), hb(), hints.maxEntry, sp, hash, cand.p, cap,
-                                counter.p, psplit, stream);
+                                counter.p, ref, &cand_diff, psplit, stream);
       if (total > cap) throw Error(kErrState, "candidate count changed between passes");
     }
     size_t nnew = 0;
     if (total > 0) {
-      sort_dets(cand.p, nullptr, (size_t)total, hints.norb, prims, stream);
+      sort_dets(cand.p, nullptr, (size_t)total, cand_diff, prims, stream);
       nnew = unique_dets(cand.p, (size_t)total, prims, stream);
     }
     SHCI_CUDA(cudaStreamSynchronize(stream));
@@ -545,6 +575,7 @@ struct Context {
       k_append<<<grid_for(nnew, 256), 256, 0, stream>>>(cand.p, nnew, dets.p + ndet);
       SHCI_LAUNCH_CHECK();
       ndet += nnew;
+      widen();
       invalidate_space();
     }
     ncand = 0;
@@ -559,15 +590,13 @@ struct Context {
     require_dets();
     if (n < 0) throw Error(kErrInvalid, "negative determinant count");
     if (n == 0) return;
-    for (int64_t i = 0; i < n; ++i) {
-      const uint64_t w0 = h[2 * i], w1 = h[2 * i + 1];
-      require_det(h + 2 * i, i);
-      if (i > 0) {  // Determinant::operator<: signed words from the top (SHCI/Determinants.h:490-498)
-        const int64_t a1 = (int64_t)h[2 * i - 1], b1 = (int64_t)w1;
-        const int64_t a0 = (int64_t)h[2 * i - 2], b0 = (int64_t)w0;
-        if (!(a1 < b1 || (a1 == b1 && a0 < b0)))
-          throw Error(kErrInvalid, "appended determinants must be sorted and unique");
-      }
+    const Det2 d = require_list(h, n, ref);
+    for (int64_t i = 1; i < n; ++i) {
+      // Determinant::operator<: signed words from the top (SHCI/Determinants.h:490-498)
+      const int64_t a1 = (int64_t)h[2 * i - 1], b1 = (int64_t)h[2 * i + 1];
+      const int64_t a0 = (int64_t)h[2 * i - 2], b0 = (int64_t)h[2 * i];
+      if (!(a1 < b1 || (a1 == b1 && a0 < b0)))
+        throw Error(kErrInvalid, "appended determinants must be sorted and unique");
     }
     hash.build(dets.p, ndet, stream);
     cand.reserve((size_t)n);
@@ -575,6 +604,7 @@ struct Context {
     counter.resize(1);
     if (count_present(cand.p, (size_t)n, hash, dets.p, counter.p, stream) != 0)
       throw Error(kErrInvalid, "appended determinants must be absent from the space");
+    cand_diff = d;
     append_candidates((size_t)n);
   }
 
@@ -621,7 +651,7 @@ struct Context {
     SelectParams psp = sp;
     psp.ncore = 0;
     psp.nact = 1 << 30;
-    pt_last = pt_deterministic(dets.p, ndet, c, E0 - hints.coreE, eps2, ints(), hb(), hints.maxEntry, psp, hash,
+    pt_last = pt_deterministic(dets.p, ndet, ref, c, E0 - hints.coreE, eps2, ints(), hb(), hints.maxEntry, psp, hash,
                                pt_max_cand, ptw, psplit, prims, stream);
     t_pt = now_s() - t0;
     pts_last = PtStochResult();
@@ -695,7 +725,7 @@ struct Context {
     SelectParams psp = sp;
     psp.ncore = 0;
     psp.nact = 1 << 30;
-    pts_last = pt_semistochastic(dets.p, ndet, c, ch, E0 - hints.coreE, eps2, eps2L, nsample, max_iter, target, seed,
+    pts_last = pt_semistochastic(dets.p, ndet, ref, c, ch, E0 - hints.coreE, eps2, eps2L, nsample, max_iter, target, seed,
                                  ints(), hb(), hints.maxEntry, psp, hash, ptw, psplit, prims, stream);
     pt_last = PtResult();
     pt_last.candidates = pts_last.candidates;
@@ -709,7 +739,7 @@ struct Context {
     if (mode < 0 || mode > 3) throw Error(kErrInvalid, "unknown Hamiltonian mode");
     PhaseTimer pt(stream);
     if (!helpers_ok) {
-      helpers.build(dets.p, ndet, hints.norb, prims, stream);
+      helpers.build(dets.p, ndet, hints.norb, ref, diff, prims, stream);
       helpers_ok = true;
     }
     pt.mark("string tables");
@@ -756,7 +786,7 @@ struct Context {
       throw Error(kErrInvalid, "a row block is stored: mode must be SHCI_MODE_FP64 or SHCI_MODE_MIXED");
     if (!(r0 < r1 && r1 <= ndet)) throw Error(kErrInvalid, "row block [r0, r1) must be a non-empty range of the space");
     if (!helpers_ok) {
-      helpers.build(dets.p, ndet, hints.norb, prims, stream);
+      helpers.build(dets.p, ndet, hints.norb, ref, diff, prims, stream);
       helpers_ok = true;
     }
     ensure_diag();

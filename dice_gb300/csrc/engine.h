@@ -134,16 +134,16 @@ struct Prims {
 void scan_exclusive_i64(const int64_t* in, int64_t* out, size_t n, int64_t* total_host, Prims& pr,
                         cudaStream_t s);
 void scan_exclusive_u32(const uint32_t* in, uint32_t* out, size_t n, Prims& pr, cudaStream_t s);
-// Stable sort of determinants of norb orbitals in Dice's order (signed words,
-// top word first), optionally carrying a uint32 payload (vals may be null).
-// Sorted in place.
-void sort_dets(Det2* keys, uint32_t* vals, size_t n, int norb, Prims& pr, cudaStream_t s);
-// Stable sort of uint64 keys (unsigned order) whose low `bits` bits may
-// differ, with a uint32 payload, in place.
-void sort_u64(uint64_t* keys, uint32_t* vals, size_t n, int bits, Prims& pr, cudaStream_t s);
+// The sorts take the bits in which keys may differ; the others are constant and
+// cost no pass.
+// Stable sort of determinants in Dice's order (signed words, top word first),
+// optionally carrying a uint32 payload (vals may be null). Sorted in place.
+void sort_dets(Det2* keys, uint32_t* vals, size_t n, const Det2& diff, Prims& pr, cudaStream_t s);
+// Stable sort of uint64 keys (unsigned order) with a uint32 payload, in place.
+void sort_u64(uint64_t* keys, uint32_t* vals, size_t n, uint64_t diff, Prims& pr, cudaStream_t s);
 // Stable sort of 128-bit keys (k1 high word, k0 low word; unsigned order)
-// with a uint32 payload, in place. bits1 0: a constant high word, not moved.
-void sort_u128(uint64_t* k0, uint64_t* k1, uint32_t* vals, size_t n, int bits0, int bits1, Prims& pr,
+// with a uint32 payload, in place. diff1 0: a constant high word, not moved.
+void sort_u128(uint64_t* k0, uint64_t* k1, uint32_t* vals, size_t n, uint64_t diff0, uint64_t diff1, Prims& pr,
                cudaStream_t s);
 // Remove adjacent duplicates of sorted determinants; returns the new count.
 size_t unique_dets(Det2* keys, size_t n, Prims& pr, cudaStream_t s);

@@ -65,7 +65,8 @@ struct Helpers {
   DevBuf<uint2> m1tab;
   DevBuf<uint64_t> m1dir;
   int64_t nm1 = 0;
-  void build(const Det2* dets, size_t n, int norb, Prims& pr, cudaStream_t s);
+  // ref: one of the determinants, diff: the bits in which some differ from it
+  void build(const Det2* dets, size_t n, int norb, const Det2& ref, const Det2& diff, Prims& pr, cudaStream_t s);
   template <class S>
   HelperView<S> view() const {
     return HelperView<S>{N,
@@ -286,19 +287,21 @@ __device__ __forceinline__ int in_mask(const SelectParams& sp, int r, int p) {
 
 // Candidates from every parent, dropping those already present (hash set);
 // returns the number of candidates written (may exceed cap: then nothing past
-// cap is written and the caller retries with a larger buffer).
+// cap is written and the caller retries with a larger buffer). *diff: the bits in
+// which some candidate differs from ref. d_counter: three words.
 int64_t select_candidates(const Det2* dets, const double* cmax, size_t n, double eps1, const IntsView& ints,
                           const HeatBathView& hb, double maxEntry, const SelectParams& sp, const DetHash& present,
-                          Det2* out, int64_t cap, int64_t* d_counter, ParentSplit& ps, cudaStream_t s);
+                          Det2* out, int64_t cap, int64_t* d_counter, const Det2& ref, Det2* diff, ParentSplit& ps,
+                          cudaStream_t s);
 // Time reversal (kernels_select.cu): cMax of the reference's symmetrized
 // basis for every determinant (0 for the non-standard member of a pair), and
 // the new determinants of a selection: the standard members of the
 // candidates' pairs, sorted, unique and absent from the space, followed by
 // the flipped partners of the open-shell ones, written to out (room for 2n);
-// returns how many.
+// returns how many. diff: the bits in which the standard members may differ.
 void trev_cmax(const Det2* dets, const double* ci, size_t ld, int nroots, size_t n, const int32_t* flip, double* out,
                cudaStream_t s);
-size_t trev_new_dets(Det2* cand, size_t n, int norb, const DetHash& present, const Det2* dets, Det2* out, DevBuf<int64_t>& flag,
+size_t trev_new_dets(Det2* cand, size_t n, const Det2& diff, const DetHash& present, const Det2* dets, Det2* out, DevBuf<int64_t>& flag,
                      DevBuf<int64_t>& pos, Prims& pr, cudaStream_t s);
 // Number of the n determinants q that the hash set `present` (over dets) holds.
 int64_t count_present(const Det2* q, size_t n, const DetHash& present, const Det2* dets, int64_t* d_counter,
@@ -343,7 +346,8 @@ struct PtWork {
 // reference, numerators merged per determinant. E0 without the core energy.
 // sp supplies the occupation restrictions (its ncore/nact are not applied).
 // max_candidates > 0 caps one partition (default: from free device memory).
-PtResult pt_deterministic(const Det2* dets, size_t n, const double* c, double E0, double eps2, const IntsView& ints,
+// ref: any determinant (the bits in which candidates differ are taken against it).
+PtResult pt_deterministic(const Det2* dets, size_t n, const Det2& ref, const double* c, double E0, double eps2, const IntsView& ints,
                           const HeatBathView& hb, double maxEntry, const SelectParams& sp, const DetHash& present,
                           int64_t max_candidates, PtWork& w, ParentSplit& ps, Prims& pr, cudaStream_t s);
 
@@ -364,7 +368,7 @@ struct PtStochResult {
 // Semistochastic PT2 (SHCIbasics::DoPerturbativeStochastic2SingleListDoubleEpsilon2AllTogether,
 // SHCI/SHCIbasics.cpp:55-451): c on the device and on the host (the alias
 // table and the draws are made on the host), E0 without the core energy.
-PtStochResult pt_semistochastic(const Det2* dets, size_t n, const double* c_dev, const std::vector<double>& c_host,
+PtStochResult pt_semistochastic(const Det2* dets, size_t n, const Det2& ref, const double* c_dev, const std::vector<double>& c_host,
                                 double E0, double eps2, double eps2L, int nsample, int max_iter, double target,
                                 uint64_t seed, const IntsView& ints, const HeatBathView& hb, double maxEntry,
                                 const SelectParams& sp, const DetHash& present, PtWork& w, ParentSplit& ps,

@@ -234,8 +234,11 @@ void scan_exclusive_u32(const uint32_t* in, uint32_t* out, size_t n, Prims& pr, 
 // ---------------------------------------------------------------------------
 // LSD radix sort, 8-bit digits, stable. Keys are unsigned 64-bit words (the
 // caller maps signed order onto unsigned order by flipping the sign bit); the
-// caller says how many low bits of each word can differ, so no pass over the
-// keys and no round trip to the host is needed to find the digits that do.
+// caller says in which bits of each word keys can differ (the space's from its
+// determinants as they come in, the candidates' from the kernels that write
+// them), so no pass over the keys and no round trip to the host is needed to find
+// them. A digit is the eight bits from the lowest differing bit that no earlier
+// digit holds: a frozen core and empty upper orbitals cost no pass.
 //
 // A pass counts the digits of each tile, scans the counts and scatters. The
 // scatter ranks a tile's keys warp by warp without block barriers, exchanges
@@ -370,39 +373,42 @@ static void rs_scatter(unsigned ntiles, const uint64_t* a0, const uint64_t* a1, 
   SHCI_LAUNCH_CHECK();
 }
 
-// Sorts (k0[, k1][, v]) in place by (k1, k0) unsigned lexicographic order; only
-// the low bits0 / bits1 bits of the words differ between keys.
-static void radix_sort_soa(uint64_t* k0, uint64_t* k1, uint32_t* v, size_t n, int bits0, int bits1, Prims& pr,
-                           cudaStream_t s) {
+// Sorts (k0[, k1][, v]) in place by (k1, k0) unsigned lexicographic order; keys
+// differ only in the bits diff0 / diff1 of the words.
+static void radix_sort_soa(uint64_t* k0, uint64_t* k1, uint32_t* v, size_t n, uint64_t diff0, uint64_t diff1,
+                           Prims& pr, cudaStream_t s) {
   if (n <= 1) return;
   if (n >= (size_t)0xffffffffu) throw Error(kErrInvalid, "sort size exceeds 2^32");
   const unsigned ntiles = (unsigned)((n + kRsTile - 1) / kRsTile);
-  if (bits1 <= 0) k1 = nullptr;  // a constant high word needs no moving: every permutation leaves it as is
+  if (diff1 == 0) k1 = nullptr;  // a constant high word needs no moving: every permutation leaves it as is
   pr.sort_hist.reserve((size_t)256 * ntiles);
   pr.sort_k0.reserve(n);
   if (k1) pr.sort_k1.reserve(n);
   if (v) pr.sort_v.reserve(n);
   uint64_t *a0 = k0, *a1 = k1, *b0 = pr.sort_k0.p, *b1 = k1 ? pr.sort_k1.p : nullptr;
   uint32_t *av = v, *bv = v ? pr.sort_v.p : nullptr;
-  const int pass0 = (bits0 + 7) / 8, pass1 = k1 ? (bits1 + 7) / 8 : 0;
-  for (int d = 0; d < pass0 + pass1; ++d) {
-    const int word = d >= pass0, shift = 8 * (word ? d - pass0 : d);
-    k_rs_tile_hist<<<ntiles, kRsThreads, 0, s>>>(word ? a1 : a0, n, shift, pr.sort_hist.p, ntiles);
-    SHCI_LAUNCH_CHECK();
-    scan_exclusive_u32(pr.sort_hist.p, pr.sort_hist.p, (size_t)256 * ntiles, pr, s);
-    if (k1 && v)
-      rs_scatter<true, true>(ntiles, a0, a1, av, b0, b1, bv, n, word, shift, pr.sort_hist.p, s);
-    else if (k1)
-      rs_scatter<true, false>(ntiles, a0, a1, av, b0, b1, bv, n, word, shift, pr.sort_hist.p, s);
-    else if (v)
-      rs_scatter<false, true>(ntiles, a0, a1, av, b0, b1, bv, n, word, shift, pr.sort_hist.p, s);
-    else
-      rs_scatter<false, false>(ntiles, a0, a1, av, b0, b1, bv, n, word, shift, pr.sort_hist.p, s);
-    std::swap(a0, b0);
-    std::swap(a1, b1);
-    std::swap(av, bv);
-  }
-  if ((pass0 + pass1) & 1) {
+  const uint64_t diff[2] = {diff0, diff1};
+  int npass = 0;
+  for (int word = 0; word < 2; ++word)
+    for (uint64_t left = diff[word]; left; ++npass) {
+      const int shift = __builtin_ctzll(left);
+      left &= ~(0xffull << shift);
+      k_rs_tile_hist<<<ntiles, kRsThreads, 0, s>>>(word ? a1 : a0, n, shift, pr.sort_hist.p, ntiles);
+      SHCI_LAUNCH_CHECK();
+      scan_exclusive_u32(pr.sort_hist.p, pr.sort_hist.p, (size_t)256 * ntiles, pr, s);
+      if (k1 && v)
+        rs_scatter<true, true>(ntiles, a0, a1, av, b0, b1, bv, n, word, shift, pr.sort_hist.p, s);
+      else if (k1)
+        rs_scatter<true, false>(ntiles, a0, a1, av, b0, b1, bv, n, word, shift, pr.sort_hist.p, s);
+      else if (v)
+        rs_scatter<false, true>(ntiles, a0, a1, av, b0, b1, bv, n, word, shift, pr.sort_hist.p, s);
+      else
+        rs_scatter<false, false>(ntiles, a0, a1, av, b0, b1, bv, n, word, shift, pr.sort_hist.p, s);
+      std::swap(a0, b0);
+      std::swap(a1, b1);
+      std::swap(av, bv);
+    }
+  if (npass & 1) {
     SHCI_CUDA(cudaMemcpyAsync(k0, a0, n * sizeof(uint64_t), cudaMemcpyDeviceToDevice, s));
     if (k1) SHCI_CUDA(cudaMemcpyAsync(k1, a1, n * sizeof(uint64_t), cudaMemcpyDeviceToDevice, s));
     if (v) SHCI_CUDA(cudaMemcpyAsync(v, av, n * sizeof(uint32_t), cudaMemcpyDeviceToDevice, s));
@@ -424,7 +430,7 @@ __global__ void k_dets_join(const uint64_t* __restrict__ k0, const uint64_t* __r
   }
 }
 
-void sort_dets(Det2* keys, uint32_t* vals, size_t n, int norb, Prims& pr, cudaStream_t s) {
+void sort_dets(Det2* keys, uint32_t* vals, size_t n, const Det2& diff, Prims& pr, cudaStream_t s) {
   if (n <= 1) return;
   // Split into two word arrays; the split copies live in temporaries owned by
   // this call so the radix passes can use the Prims buffers.
@@ -433,19 +439,19 @@ void sort_dets(Det2* keys, uint32_t* vals, size_t n, int norb, Prims& pr, cudaSt
   k1.resize(n);
   k_dets_split<<<grid_for(n, 256), 256, 0, s>>>(keys, n, k0.p, k1.p);
   SHCI_LAUNCH_CHECK();
-  // spin orbitals 0 .. 2 norb - 1; the flipped sign bits are constant below 64
-  radix_sort_soa(k0.p, k1.p, vals, n, std::min(64, 2 * norb), std::max(0, 2 * norb - 64), pr, s);
+  radix_sort_soa(k0.p, k1.p, vals, n, diff.w0, diff.w1, pr, s);
   k_dets_join<<<grid_for(n, 256), 256, 0, s>>>(k0.p, k1.p, n, keys);
   SHCI_LAUNCH_CHECK();
   SHCI_CUDA(cudaStreamSynchronize(s));
 }
 
-void sort_u64(uint64_t* keys, uint32_t* vals, size_t n, int bits, Prims& pr, cudaStream_t s) {
-  radix_sort_soa(keys, nullptr, vals, n, bits, 0, pr, s);
+void sort_u64(uint64_t* keys, uint32_t* vals, size_t n, uint64_t diff, Prims& pr, cudaStream_t s) {
+  radix_sort_soa(keys, nullptr, vals, n, diff, 0, pr, s);
 }
 
-void sort_u128(uint64_t* k0, uint64_t* k1, uint32_t* vals, size_t n, int bits0, int bits1, Prims& pr, cudaStream_t s) {
-  radix_sort_soa(k0, k1, vals, n, bits0, bits1, pr, s);
+void sort_u128(uint64_t* k0, uint64_t* k1, uint32_t* vals, size_t n, uint64_t diff0, uint64_t diff1, Prims& pr,
+               cudaStream_t s) {
+  radix_sort_soa(k0, k1, vals, n, diff0, diff1, pr, s);
 }
 
 __global__ void k_unique_flags(const Det2* __restrict__ k, size_t n, int64_t* __restrict__ flag) {

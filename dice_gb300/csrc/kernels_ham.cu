@@ -317,8 +317,9 @@ __global__ void k_split_singles(const int64_t* __restrict__ sstart, const uint32
 }
 
 // Single-excitation lists and partial-string index, from the strings by position.
+// bits: those in which partial beta strings may differ.
 template <class S>
-static void build_singles_and_index(Helpers& hp, int norb, Prims& pr, cudaStream_t s) {
+static void build_singles_and_index(Helpers& hp, int norb, uint64_t bits, Prims& pr, cudaStream_t s) {
   const size_t n = hp.N;
   const S* bstr = reinterpret_cast<const S*>(hp.bstr.p);
   // alpha single-excitation lists
@@ -368,11 +369,11 @@ static void build_singles_and_index(Helpers& hp, int norb, Prims& pr, cudaStream
       const unsigned eb = grid_for((size_t)ne, 256);
       k_m1_fill<S><<<grid_for(n, 256), 256, 0, s>>>(bstr, hp.agrp.p, n, o1.p, key.p, perm.p, raw.p);
       SHCI_LAUNCH_CHECK();
-      sort_u64(key.p, perm.p, (size_t)ne, norb, pr, s);  // by partial string
+      sort_u64(key.p, perm.p, (size_t)ne, bits, pr, s);  // by partial string
       k_m1_group_keys<<<eb, 256, 0, s>>>(raw.p, perm.p, ne, key.p);
       SHCI_LAUNCH_CHECK();
-      int gbits = 1;
-      while ((hp.NA >> gbits) != 0) ++gbits;
+      uint64_t gbits = 1;
+      while (((uint64_t)hp.NA & ~gbits) != 0) gbits = 2 * gbits + 1;
       sort_u64(key.p, perm.p, (size_t)ne, gbits, pr, s);  // then by alpha group (stable)
       k_m1_permute<<<eb, 256, 0, s>>>(raw.p, perm.p, ne, hp.m1ent.p);
       SHCI_LAUNCH_CHECK();
@@ -408,8 +409,10 @@ static void build_singles_and_index(Helpers& hp, int norb, Prims& pr, cudaStream
   SHCI_CUDA(cudaStreamSynchronize(s));
 }
 
-void Helpers::build(const Det2* dets, size_t n, int norb, Prims& pr, cudaStream_t s) {
+void Helpers::build(const Det2* dets, size_t n, int norb, const Det2& ref, const Det2& diff, Prims& pr,
+                    cudaStream_t s) {
   N = n;
+  const uint64_t abits = det_alpha(diff), bbits = det_beta(diff);
   perm.resize(n);
   spos.resize(n);
   narrow = norb <= 32;
@@ -430,7 +433,7 @@ void Helpers::build(const Det2* dets, size_t n, int norb, Prims& pr, cudaStream_
     const unsigned g = grid_for(n, 256);
     k_strings<<<g, 256, 0, s>>>(dets, n, a.p, bkey.p, perm.p);
     SHCI_LAUNCH_CHECK();
-    sort_u128(bkey.p, a.p, perm.p, n, norb, norb, pr, s);  // by (alpha, beta): the storage order
+    sort_u128(bkey.p, a.p, perm.p, n, bbits, abits, pr, s);  // by (alpha, beta): the storage order
     if (narrow)
       k_pair_strings<uint32_t><<<g, 256, 0, s>>>(a.p, bkey.p, perm.p, n, reinterpret_cast<uint2*>(str.p),
                                                  reinterpret_cast<uint32_t*>(bstr.p), spos.p, bPos.p);
@@ -447,7 +450,7 @@ void Helpers::build(const Det2* dets, size_t n, int norb, Prims& pr, cudaStream_
     SHCI_LAUNCH_CHECK();
     k_iota_last<<<1, 1, 0, s>>>(aStart.p, NA, (int64_t)n);
     SHCI_LAUNCH_CHECK();
-    sort_u64(bkey.p, bPos.p, n, norb, pr, s);  // by beta string, stable: ascending positions within a group
+    sort_u64(bkey.p, bPos.p, n, bbits, pr, s);  // by beta string, stable: ascending positions within a group
     k_group_flags<<<g, 256, 0, s>>>(bkey.p, n, flag.p);
     SHCI_LAUNCH_CHECK();
     scan_exclusive_i64(flag.p, excl.p, n, &NB, pr, s);
@@ -463,10 +466,12 @@ void Helpers::build(const Det2* dets, size_t n, int norb, Prims& pr, cudaStream_
       k_gather_alpha<uint64_t><<<g, 256, 0, s>>>(reinterpret_cast<const ulonglong2*>(str.p), bPos.p, n, bAlpha.p);
     SHCI_LAUNCH_CHECK();
   }
+  // a partial string lacks one electron, so an orbital that all strings hold varies too
+  const uint64_t mbits = bbits | det_beta(ref);
   if (narrow)
-    build_singles_and_index<uint32_t>(*this, norb, pr, s);
+    build_singles_and_index<uint32_t>(*this, norb, mbits, pr, s);
   else
-    build_singles_and_index<uint64_t>(*this, norb, pr, s);
+    build_singles_and_index<uint64_t>(*this, norb, mbits, pr, s);
 }
 // ---------------------------------------------------------------------------
 // Row traversal shared by count, emit and the matrix-free sigma. The visitor's

@@ -87,7 +87,8 @@ struct PtArgs {
   const float2* coulff;  // and as float pairs
   const float2* exchff;
   SplitView split;              // work units
-  unsigned long long* counter;  // candidates appended (counts past cap too)
+  unsigned long long* counter;  // candidates appended (counts past cap too), then the bits in which they differ from ref
+  Det2 ref;
   int64_t cap;
   uint64_t* key0;  // candidate determinant, low word
   uint64_t* key1;  // high word
@@ -194,11 +195,13 @@ __device__ __forceinline__ float2 shfl_ff(float2 v, int src) {
 
 // Warp-aggregated append of the lanes with `keep`; slots past cap are counted
 // but not written.
-__device__ __forceinline__ void pt_put(const PtArgs& a, bool keep, const Det2& cand, float2 v, float2 e,
-                                       double2 vs = make_double2(0.0, 0.0), bool present = false) {
+template <bool W2>
+__device__ __forceinline__ void pt_put(const PtArgs& a, bool keep, const Det2& cand, float2 v, float2 e, double2 vs,
+                                       bool present, unsigned long long* diff) {
   const int lane = threadIdx.x & 31;
   const unsigned m = __ballot_sync(kFull, keep);
   if (!m) return;
+  note_diff(diff, keep, cand, a.ref, W2);
   const int leader = __ffs(m) - 1;
   unsigned long long base = 0;
   if (lane == leader) base = atomicAdd(a.counter, (unsigned long long)__popc(m));
@@ -339,6 +342,7 @@ __global__ void __launch_bounds__(kPtThreads) k_pt_gen(PtArgs a) {
   __shared__ uint32_t s_qo[kPtWarps][64], s_ro[kPtWarps][64];
   __shared__ float s_qv[kPtWarps][64];
   __shared__ float2 s_rv[kPtWarps][64];
+  __shared__ unsigned long long s_diff[kPtWarps][2];
   const int n = a.ints.norb, nn = n * n;
   float2* sD = smf;            // J
   float2* sX = smf + nn;       // J - K
@@ -348,6 +352,7 @@ __global__ void __launch_bounds__(kPtThreads) k_pt_gen(PtArgs a) {
     sX[j] = ff_of(__dsub_rn(a.ints.Direct[j], a.ints.Exchange[j]));
   }
   for (int j = threadIdx.x; j < 2 * n; j += blockDim.x) sH[j] = ff_of(a.ints.I1[(size_t)j * (2 * n + 1)]);
+  if (threadIdx.x < 2 * kPtWarps) s_diff[threadIdx.x >> 1][threadIdx.x & 1] = 0ull;
   __syncthreads();
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
   unsigned char* closed = s_closed[wib];
@@ -502,7 +507,7 @@ __global__ void __launch_bounds__(kPtThreads) k_pt_gen(PtArgs a) {
           e = ff_add(ed, ff_add(ff_sub(fa, fi), ff_sub(vin, vx)));
         }
       }
-      pt_put(a, keep, cand, v, e, vs, present);
+      pt_put<W2>(a, keep, cand, v, e, vs, present, s_diff[wib]);
       rh = (rh + cnt) & 63u;
       rn -= cnt;
       __syncwarp();
@@ -659,6 +664,7 @@ __global__ void __launch_bounds__(kPtThreads) k_pt_gen(PtArgs a) {
       if (!more && qn == 0 && rn == 0) break;
     }
   }
+  add_diff<kPtWarps>(s_diff, a.counter + 1);
 }
 
 __global__ void k_pt_tables(const double* __restrict__ I2, int n, double* __restrict__ coul,
@@ -1035,10 +1041,10 @@ namespace {
 
 // Fields of PtArgs shared by both modes; builds the dense integral tables on
 // first use. Returns the generator's dynamic shared memory size.
-size_t pt_prepare(PtArgs& a, const Det2* dets, size_t n, const double* c, double E0, double eps2,
+size_t pt_prepare(PtArgs& a, const Det2* dets, size_t n, const Det2& ref, const double* c, double E0, double eps2,
                   const IntsView& ints, const HeatBathView& hb, double maxEntry, const SelectParams& sp,
                   const DetHash& present, PtWork& w, cudaStream_t s) {
-  w.next.resize(1);
+  w.next.resize(3);
   w.part.resize(3 * kPtRedBlocks);
   a = PtArgs{};
   a.dets = dets;
@@ -1052,6 +1058,7 @@ size_t pt_prepare(PtArgs& a, const Det2* dets, size_t n, const double* c, double
   a.hslots = present.slots.p;
   a.hmask = present.mask;
   a.counter = w.next.p;
+  a.ref = ref;
   a.nparts = 1;
   if (!w.tables_ok) {
     const size_t nt = (size_t)ints.norb * ints.norb * ints.norb;
@@ -1092,7 +1099,7 @@ void launch_gen(const PtArgs& a, size_t gsmem, cudaStream_t s) {
 
 }  // namespace
 
-PtResult pt_deterministic(const Det2* dets, size_t n, const double* c, double E0, double eps2, const IntsView& ints,
+PtResult pt_deterministic(const Det2* dets, size_t n, const Det2& ref, const double* c, double E0, double eps2, const IntsView& ints,
                           const HeatBathView& hb, double maxEntry, const SelectParams& sp, const DetHash& present,
                           int64_t max_candidates, PtWork& w, ParentSplit& ps, Prims& pr, cudaStream_t s) {
   PtResult res;
@@ -1100,7 +1107,7 @@ PtResult pt_deterministic(const Det2* dets, size_t n, const double* c, double E0
   if (!(eps2 >= 0.0)) throw Error(kErrInvalid, "epsilon2 must be >= 0");
   PtArgs a;
   split_parents(dets, nullptr, c, n, eps2, maxEntry, hb, ints.norb, ps, s);
-  const size_t gsmem = pt_prepare(a, dets, n, c, E0, eps2, ints, hb, maxEntry, sp, present, w, s);
+  const size_t gsmem = pt_prepare(a, dets, n, ref, c, E0, eps2, ints, hb, maxEntry, sp, present, w, s);
   a.split = ps.view();
 
   // capacity of one partition
@@ -1120,6 +1127,7 @@ PtResult pt_deterministic(const Det2* dets, size_t n, const double* c, double E0
   if (cap < 1) throw Error(kErrOOM, "no device memory left for perturbation candidates");
 
   // one generation pass into buffers of `room` candidates; returns the count
+  unsigned long long got[3] = {0, 0, 0};  // and the bits in which the candidates differ
   auto gen = [&](uint32_t nparts, uint32_t part, int64_t room) -> int64_t {
     w.key0.reserve((size_t)room);
     w.key1.reserve((size_t)room);
@@ -1130,22 +1138,20 @@ PtResult pt_deterministic(const Det2* dets, size_t n, const double* c, double E0
     a.key0 = w.key0.p;
     a.key1 = w.key1.p;
     a.ne = w.ne.p;
-    SHCI_CUDA(cudaMemsetAsync(w.next.p, 0, sizeof(unsigned long long), s));
+    SHCI_CUDA(cudaMemsetAsync(w.next.p, 0, sizeof(got), s));
     ps.rewind(s);
     launch_gen(a, gsmem, s);
     SHCI_LAUNCH_CHECK();
-    unsigned long long total = 0;
-    SHCI_CUDA(cudaMemcpyAsync(&total, w.next.p, sizeof(total), cudaMemcpyDeviceToHost, s));
+    SHCI_CUDA(cudaMemcpyAsync(got, w.next.p, sizeof(got), cudaMemcpyDeviceToHost, s));
     SHCI_CUDA(cudaStreamSynchronize(s));
-    return (int64_t)total;
+    return (int64_t)got[0];
   };
-  const int bits0 = std::min(64, 2 * ints.norb), bits1 = std::max(0, 2 * ints.norb - 64);
   PhaseTimer pt(s);
   auto reduce = [&](int64_t m, PtResult& r) {
     w.perm.resize((size_t)m);
     k_pt_iota<<<grid_for((size_t)m, 256), 256, 0, s>>>(w.perm.p, (size_t)m);
     SHCI_LAUNCH_CHECK();
-    sort_u128(w.key0.p, w.key1.p, w.perm.p, (size_t)m, bits0, bits1, pr, s);
+    sort_u128(w.key0.p, w.key1.p, w.perm.p, (size_t)m, got[1], got[2], pr, s);
     pt.mark("pt sort");
     k_pt_reduce<<<kPtRedBlocks, kPtRedThreads, 0, s>>>(w.key0.p, w.key1.p, w.perm.p, w.ne.p, (size_t)m,
                                                        w.part.p);
@@ -1226,7 +1232,7 @@ static void alias_setup(const std::vector<double>& ci, double cumulative, std::v
   }
 }
 
-PtStochResult pt_semistochastic(const Det2* dets, size_t n, const double* c_dev, const std::vector<double>& c_host,
+PtStochResult pt_semistochastic(const Det2* dets, size_t n, const Det2& ref, const double* c_dev, const std::vector<double>& c_host,
                                 double E0, double eps2, double eps2L, int nsample, int max_iter, double target,
                                 uint64_t seed, const IntsView& ints, const HeatBathView& hb, double maxEntry,
                                 const SelectParams& sp, const DetHash& present, PtWork& w, ParentSplit& ps,
@@ -1236,7 +1242,7 @@ PtStochResult pt_semistochastic(const Det2* dets, size_t n, const double* c_dev,
   if (!(eps2 >= 0.0)) throw Error(kErrInvalid, "epsilon2 must be >= 0");
   if (nsample < 2) throw Error(kErrInvalid, "sampleN must be at least 2");
   if (max_iter < 1) throw Error(kErrInvalid, "nPTiter must be at least 1");
-  if (eps2L < 999) res.e_large = pt_deterministic(dets, n, c_dev, E0, eps2L, ints, hb, maxEntry, sp, present, 0, w,
+  if (eps2L < 999) res.e_large = pt_deterministic(dets, n, ref, c_dev, E0, eps2L, ints, hb, maxEntry, sp, present, 0, w,
                                                   ps, pr, s).e2;
   double cumulative = 0.0;
   for (size_t i = 0; i < n; i++) cumulative += fabs(c_host[i]);
@@ -1244,7 +1250,7 @@ PtStochResult pt_semistochastic(const Det2* dets, size_t n, const double* c_dev,
   std::vector<double> prob;
   alias_setup(c_host, cumulative, alias, prob);
   PtArgs a;
-  const size_t gsmem = pt_prepare(a, dets, n, c_dev, E0, eps2, ints, hb, maxEntry, sp, present, w, s);
+  const size_t gsmem = pt_prepare(a, dets, n, ref, c_dev, E0, eps2, ints, hb, maxEntry, sp, present, w, s);
   a.eps2L = eps2L;
   a.nmc = (double)nsample;
   DevBuf<int32_t> dlist;
@@ -1293,6 +1299,7 @@ PtStochResult pt_semistochastic(const Det2* dets, size_t n, const double* c_dev,
     a.split = ps.view();
     // generate (twice when the buffers turn out too small)
     int64_t room = std::max<int64_t>((int64_t)w.key0.cap, (int64_t)1 << 20), m = 0;
+    unsigned long long got[3] = {0, 0, 0};  // candidates, and the bits in which they differ
     for (int pass = 0; pass < 2; ++pass) {
       w.key0.reserve((size_t)room);
       w.key1.reserve((size_t)room);
@@ -1303,14 +1310,13 @@ PtStochResult pt_semistochastic(const Det2* dets, size_t n, const double* c_dev,
       a.key1 = w.key1.p;
       a.ne = w.ne.p;
       a.n2p = w.n2p.p;
-      SHCI_CUDA(cudaMemsetAsync(w.next.p, 0, sizeof(unsigned long long), s));
+      SHCI_CUDA(cudaMemsetAsync(w.next.p, 0, sizeof(got), s));
       ps.rewind(s);
       launch_gen(a, gsmem, s);
       SHCI_LAUNCH_CHECK();
-      unsigned long long total = 0;
-      SHCI_CUDA(cudaMemcpyAsync(&total, w.next.p, sizeof(total), cudaMemcpyDeviceToHost, s));
+      SHCI_CUDA(cudaMemcpyAsync(got, w.next.p, sizeof(got), cudaMemcpyDeviceToHost, s));
       SHCI_CUDA(cudaStreamSynchronize(s));
-      m = (int64_t)total;
+      m = (int64_t)got[0];
       if (m <= room) break;
       if (m >= (int64_t)0xfffffff0u) throw Error(kErrOOM, "semistochastic sample exceeds 2^32 candidates");
       room = m;
@@ -1321,8 +1327,7 @@ PtStochResult pt_semistochastic(const Det2* dets, size_t n, const double* c_dev,
       w.perm.resize((size_t)m);
       k_pt_iota<<<grid_for((size_t)m, 256), 256, 0, s>>>(w.perm.p, (size_t)m);
       SHCI_LAUNCH_CHECK();
-      sort_u128(w.key0.p, w.key1.p, w.perm.p, (size_t)m, std::min(64, 2 * ints.norb), std::max(0, 2 * ints.norb - 64),
-                pr, s);
+      sort_u128(w.key0.p, w.key1.p, w.perm.p, (size_t)m, got[1], got[2], pr, s);
       k_pt_reduce_stoch<<<kPtRedBlocks, kPtRedThreads, 0, s>>>(w.key0.p, w.key1.p, w.perm.p, w.ne.p, w.n2p.p,
                                                                (size_t)m, f, w.part.p);
       SHCI_LAUNCH_CHECK();

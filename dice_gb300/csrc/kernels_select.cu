@@ -34,8 +34,9 @@ struct SelArgs {
   uint64_t hmask;
   Det2* out;
   int64_t cap;
-  int64_t* counter;
+  int64_t* counter;  // candidates, then two words: the bits in which they differ from ref
   SplitView split;
+  Det2 ref;
 };
 
 constexpr int kSelThreads = 256;
@@ -120,10 +121,11 @@ void split_parents(const Det2* dets, const int32_t* plist, const double* c, size
 }
 
 // Warp-aggregated append of one candidate per lane with `emit` set.
-__device__ __forceinline__ void append(const SelArgs& a, bool emit, const Det2& cand) {
+__device__ __forceinline__ void append(const SelArgs& a, bool emit, const Det2& cand, unsigned long long* diff) {
   const int lane = threadIdx.x & 31;
   unsigned m = __ballot_sync(kFull, emit);
   if (!m) return;
+  note_diff(diff, emit, cand, a.ref, a.ints.norb > 32);
   int leader = __ffs(m) - 1;
   int64_t base = 0;
   if (lane == leader) base = atomicAdd((unsigned long long*)a.counter, (unsigned long long)__popc(m));
@@ -140,7 +142,10 @@ __global__ void __launch_bounds__(kSelThreads, 5) k_select(SelArgs a) {
   __shared__ unsigned char s_closed[kSelWarps][kMaxSpin];
   __shared__ unsigned char s_open[kSelWarps][kMaxSpin];
   __shared__ uint2 s_q[kSelWarps][64];
+  __shared__ unsigned long long s_diff[kSelWarps][2];
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
+  if (lane < 2) s_diff[wib][lane] = 0ull;
+  __syncwarp();
   unsigned char* closed = s_closed[wib];
   unsigned char* open = s_open[wib];
   const int n2 = 2 * a.ints.norb;
@@ -172,7 +177,7 @@ __global__ void __launch_bounds__(kSelThreads, 5) k_select(SelArgs a) {
       det_flip(cand, oa);
       if (emit) emit = !hash_contains(a.hslots, a.hmask, a.dets, cand);
     }
-    append(a, emit, cand);
+    append(a, emit, cand, s_diff[wib]);
     qh = (qh + cnt) & 63u;
     qn -= cnt;
     __syncwarp();
@@ -302,6 +307,7 @@ __global__ void __launch_bounds__(kSelThreads, 5) k_select(SelArgs a) {
     }
   }
   if (qn > 0) drain(qn);
+  add_diff<kSelWarps>(s_diff, reinterpret_cast<unsigned long long*>(a.counter) + 1);
 }
 
 // ---------------------------------------------------------------------------
@@ -488,7 +494,7 @@ __global__ void k_trev_compact(const Det2* __restrict__ q, size_t n, const int64
     if (flag[i]) out[pos[i]] = flip_it ? det_flip_pair(q[i]) : q[i];
 }
 
-size_t trev_new_dets(Det2* cand, size_t n, int norb, const DetHash& present, const Det2* dets, Det2* out, DevBuf<int64_t>& flag,
+size_t trev_new_dets(Det2* cand, size_t n, const Det2& diff, const DetHash& present, const Det2* dets, Det2* out, DevBuf<int64_t>& flag,
                      DevBuf<int64_t>& pos, Prims& pr, cudaStream_t s) {
   if (n == 0) return 0;
   size_t blocks = std::min<size_t>((n + 255) / 256, 152 * 32);
@@ -496,7 +502,7 @@ size_t trev_new_dets(Det2* cand, size_t n, int norb, const DetHash& present, con
   // sorted and unique (:992-994), without those already present (:996-997)
   k_make_standard<<<(unsigned)blocks, 256, 0, s>>>(cand, n);
   SHCI_LAUNCH_CHECK();
-  sort_dets(cand, nullptr, n, norb, pr, s);
+  sort_dets(cand, nullptr, n, diff, pr, s);
   n = unique_dets(cand, n, pr, s);
   blocks = std::min<size_t>((n + 255) / 256, 152 * 32);
   flag.reserve(n);
@@ -546,20 +552,22 @@ int64_t count_present(const Det2* q, size_t n, const DetHash& present, const Det
 
 int64_t select_candidates(const Det2* dets, const double* cmax, size_t n, double eps1, const IntsView& ints,
                           const HeatBathView& hb, double maxEntry, const SelectParams& sp, const DetHash& present,
-                          Det2* out, int64_t cap, int64_t* d_counter, ParentSplit& ps, cudaStream_t s) {
-  SHCI_CUDA(cudaMemsetAsync(d_counter, 0, sizeof(int64_t), s));
+                          Det2* out, int64_t cap, int64_t* d_counter, const Det2& ref, Det2* diff, ParentSplit& ps,
+                          cudaStream_t s) {
+  SHCI_CUDA(cudaMemsetAsync(d_counter, 0, 3 * sizeof(int64_t), s));
   split_parents(dets, nullptr, cmax, n, eps1, maxEntry, hb, ints.norb, ps, s);
   SelArgs a{dets, cmax,   n,  eps1, ints,      hb, maxEntry, sp, present.slots.p, present.mask, out,
-            cap,  d_counter, ps.view()};
+            cap,  d_counter, ps.view(), ref};
   size_t blocks = n <= 8192 ? 8 * n : n / kSelWarps + 1;  // 64 slices a parent at most
   if (blocks > 152 * 6) blocks = 152 * 6;
   if (blocks < 1) blocks = 1;
   k_select<<<(unsigned)blocks, kSelThreads, 0, s>>>(a);
   SHCI_LAUNCH_CHECK();
-  int64_t total = 0;
-  SHCI_CUDA(cudaMemcpyAsync(&total, d_counter, sizeof(int64_t), cudaMemcpyDeviceToHost, s));
+  int64_t got[3] = {0, 0, 0};
+  SHCI_CUDA(cudaMemcpyAsync(got, d_counter, sizeof(got), cudaMemcpyDeviceToHost, s));
   SHCI_CUDA(cudaStreamSynchronize(s));
-  return total;
+  *diff = Det2{(uint64_t)got[1], (uint64_t)got[2]};
+  return got[0];
 }
 
 }  // namespace shci

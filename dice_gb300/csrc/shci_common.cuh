@@ -120,6 +120,31 @@ __device__ __forceinline__ S passed(S s, S o, S move, bool beta) {
   return (s & open) ^ (o & (beta ? open ^ hi : m));
 }
 
+// Adds to a warp's words acc (shared memory) the bits in which its lanes'
+// determinants x (where `on`) differ from ref; two: x and ref have a second word.
+// All lanes together. What the radix sort of these determinants needs to know.
+__device__ __forceinline__ void note_diff(unsigned long long* acc, bool on, const Det2& x, const Det2& ref, bool two) {
+  const uint64_t a = on ? x.w0 ^ ref.w0 : 0;
+  const uint32_t lo = __reduce_or_sync(kFull, (uint32_t)a), hi = __reduce_or_sync(kFull, (uint32_t)(a >> 32));
+  if ((threadIdx.x & 31) == 0) acc[0] |= (uint64_t)hi << 32 | lo;
+  if (two) {
+    const uint64_t b = on ? x.w1 ^ ref.w1 : 0;
+    const uint32_t l1 = __reduce_or_sync(kFull, (uint32_t)b), h1 = __reduce_or_sync(kFull, (uint32_t)(b >> 32));
+    if ((threadIdx.x & 31) == 0) acc[1] |= (uint64_t)h1 << 32 | l1;
+  }
+}
+// The words of a block's warps added to the launch's, at the end of the block
+// (one atomic a block and word: warps that end together queue at the address).
+template <int kWarps>
+__device__ __forceinline__ void add_diff(const unsigned long long (*acc)[2], unsigned long long* total) {
+  __syncthreads();
+  if (threadIdx.x >= 2) return;
+  unsigned long long v = 0;
+#pragma unroll
+  for (int w = 0; w < kWarps; ++w) v |= acc[w][threadIdx.x];
+  if (v & ~__ldcg(total + threadIdx.x)) atomicOr(total + threadIdx.x, v);
+}
+
 // Device view of the integrals (SHCI/integral.h:47-101).
 struct IntsView {
   const double* I1;        // (2n)x(2n) spin-orbital matrix
