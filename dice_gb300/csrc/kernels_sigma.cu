@@ -426,7 +426,11 @@ static int pick_vw(const Csr& H) {
 }
 
 // The copy is left out where columns need more than 24 bits and where the
-// device has no room for it; the sigma then reads the int32 columns.
+// device has no room for it (SHCI_TRACE says so; shci_sigma_bytes counts what is
+// read); the sigma then reads the int32 columns. Past 24 bits those are the better
+// form: at 17.5 million columns differences of 16 bits, bridged across wide gaps,
+// took 10.8 ms for 34 entries a row where int32 columns take 3.3, and 0.94 ms for
+// 400,000 rows of 750 entries against 0.89.
 void compress_csr(Csr& H, Prims& pr, cudaStream_t s) {
   H.drop_compressed();
   if (!H.vhi.p || H.N == 0 || H.ncols() > ((size_t)1 << 24)) return;
@@ -448,6 +452,8 @@ void compress_csr(Csr& H, Prims& pr, cudaStream_t s) {
   } catch (const Error& e) {
     H.drop_compressed();
     if (e.code != kErrOOM) throw;
+    if (trace_level() > 0)
+      std::fprintf(stderr, "[ham] no device memory for the compact copy: FP32 sigma on int32 columns\n");
     return;
   }
   const int vw = pick_vw(H);

@@ -186,3 +186,25 @@ def test_refused_space_leaves_the_old_one(system, mode):  # noqa: F811
         e.set_dets(bad)
     assert err.value.code == 1
     assert np.array_equal(e.dets(), dets) and np.array_equal(e.sigma(x, mode), y)
+
+
+def test_no_room_for_the_compact_copy(system):  # noqa: F811
+    """A mixed build whose compact copy finds no memory keeps its int32 columns, says so in the bytes of a sigma, and
+    gives the same products."""
+    e, _ = system(20, 20)
+    n = 4000
+    e.set_dets(_star(20, 10, 10, n, 12))
+    nnz = e.ham_build("mixed")
+    rp, col, val = e.ham_export(nnz)
+    x = np.random.default_rng(2).standard_normal(n)
+    y, small = e.sigma(x, "mixed"), e.sigma_bytes("mixed", 1)
+
+    e.set_alloc_cap(1)  # the unchanged space: only the copy is made again
+    try:
+        assert e.ham_build("mixed") == nnz
+    finally:
+        e.set_alloc_cap(0)
+    assert e.sigma_bytes("mixed", 1) > small
+    # compensated sums of the same products in another order: 2^-40 of their absolute values
+    A = np.bincount(np.repeat(np.arange(n), np.diff(rp)), np.abs(val * x[col]), n) + np.abs(e.diag() * x)
+    assert np.all(np.abs(e.sigma(x, "mixed") - y) <= 2.0 ** -40 * A)
