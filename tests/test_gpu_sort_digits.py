@@ -8,6 +8,7 @@ import pytest
 
 from dice_gb300.shard import ref_order
 from test_gpu_stored_edges import _check, _words, system  # noqa: F401  (fixture)
+from test_gpu_units import _dets, mol24  # noqa: F401  (fixture)
 
 pytestmark = pytest.mark.gpu
 
@@ -70,3 +71,28 @@ def test_space_grown_from_one_determinant(system):  # noqa: F811
     assert len(cand) > 100 and np.array_equal(e.select_candidates(c, 1e-2), cand)
     assert e.pt_deterministic(c, float(e.diag().min()) - 30.0, 1e-3) == e2
     assert e.pt_stats()["unique"] == st["unique"] > 100
+
+
+# 256 counts per tile of 4,096 keys, scanned in chunks of 4,096 counts: up to 256 chunks (16,777,216 keys) in two
+# launches, beyond in three. A parent of 12 + 12 electrons in 24 orbitals has 288 + 8,712 + 20,736 = 29,736
+# connections: 564 parents stay below, 565 do not.
+@pytest.mark.parametrize("n", [564, 565])
+def test_scan_at_its_chunk_limit(mol24, n):  # noqa: F811
+    e, _ = mol24
+    dets = _dets(n, 31)
+    c = np.full(n, n ** -0.5)
+    e.set_selection_params()
+    e.set_dets(dets)
+    E0 = float(e.diag().min()) - 30.0
+    e2 = e.pt_deterministic(c, E0, 1e-12)
+    whole = e.pt_stats()
+    assert whole["partitions"] == 1 and (whole["candidates"] <= 16777216) == (n == 564)
+    assert abs(whole["candidates"] - 16777216) < 30000
+    e.set_pt_batch(whole["candidates"] // 5)
+    p2 = e.pt_deterministic(c, E0, 1e-12)
+    parts = e.pt_stats()
+    e.set_pt_batch(0)
+    assert parts["partitions"] > 1
+    assert (whole["candidates"], whole["unique"]) == (parts["candidates"], parts["unique"])
+    # the same terms, summed in parts: some 1e7 terms of one sign
+    assert abs(e2 - p2) <= 1e-11 * abs(e2)
