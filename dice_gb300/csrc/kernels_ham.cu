@@ -271,17 +271,14 @@ __global__ void k_m1_insert(const uint4* __restrict__ ent, int64_t n, const uint
 // Orders each alpha group's single-excitation list: groups A_s of at most
 // kScanFactor x n_beta determinants first (cheaper to scan, one coalesced
 // load and popcount per determinant, than to probe the index n_beta times),
-// then the rest, each part in its original order; mid[g] is where the large
-// groups start. One thread per group. mol36 (498,028 determinants), FP64
-// 4-vector matrix-free sigma: 60.7 ms probing every group, 49.7 / 48.8 / 47.5 /
-// 47.7 ms with factors 2 / 3 / 4 / 6.
-#ifndef SHCI_SCAN_FACTOR
-#define SHCI_SCAN_FACTOR 8
-#endif
-constexpr int kScanFactor = SHCI_SCAN_FACTOR;
-// One warp per group; each part is put in ascending order by counting (a list
-// has at most n_alpha x (norb - n_alpha) entries, some hundred), so that the
-// hits of a row's scans come in ascending order too.
+// then the rest; mid[g] is where the large groups start. Each part is in
+// ascending order, so that the hits of a row's scans are too: the merge of a
+// row's runs rests on it. One warp per group, by counting (a list has at most
+// n_alpha x (norb - n_alpha) entries, some hundred). With factors 2 / 4 / 6 / 8 /
+// 12 / 16 / 32, FP64 4-vector matrix-free sigma of 100,762 determinants of 36
+// orbitals: 3.35 / 3.23 / 3.22 / 3.23 / 3.33 / 3.43 / 3.89 ms, FP64 build of the
+// same 7.37 / 7.25 / 7.11 / 7.09 / 7.19 / 7.31 / 7.81 ms.
+constexpr int kScanFactor = 8;
 template <class S>
 __global__ void k_split_singles(const int64_t* __restrict__ sstart, const uint32_t* __restrict__ in,
                                 const int64_t* __restrict__ gstart, const S* __restrict__ bstr, int64_t na,
@@ -1129,15 +1126,14 @@ __global__ void __launch_bounds__(kLongThreads) k_ham_finish_long(HelperView<S> 
 
 __global__ void k_set_last(int64_t* rowptr, int64_t n, int64_t total) { rowptr[n] = total; }
 
-// Sort of one row by column, one block per row. The row's columns become
-// 64-bit keys (column << 12 | position in the row) sorted by a bitonic network
-// in which each of the 256 threads keeps E consecutive keys in registers: the
-// compare-exchange steps between keys of one thread run in registers, only
-// the longer-distance steps go through shared memory (36 of the 66 steps for
-// a 2048-key row). The values are then gathered from their old positions
-// (read into registers before any write, the row is sorted in place). Rows
-// longer than kRowSortCap are left in emission order (still correct, only
-// with less gather locality in sigma).
+// Sort of one row's new columns (extended builds), one block per row. The
+// columns become 64-bit keys (column << 12 | position in the row) sorted by a
+// bitonic network in which each of the 256 threads keeps E consecutive keys in
+// registers: the compare-exchange steps between keys of one thread run in
+// registers, only the longer-distance steps go through shared memory (36 of the
+// 66 steps for a 2048-key row). The values are then gathered from their old
+// positions (read into registers before any write, the row is sorted in place).
+// Rows longer than kRowSortCap are sorted by k_long_row_sort.
 constexpr int kRowSortCap = 4096;
 constexpr int kSortThreads = 256;
 
@@ -1481,8 +1477,8 @@ __global__ void k_range_fill(const uint32_t* __restrict__ perm, size_t n, uint32
 // Incremental build helpers. The rows of the new determinants R >= n_old are
 // emitted in full (in storage order, columns in the new storage order);
 // their entries whose column is an old determinant C < n_old are the new
-// columns of old row C (same value: H_CR is evaluated with R, the higher
-// index, as the ket in both places).
+// columns of old row C: an element is bit for bit the same with either of its
+// determinants as the ket.
 // Bit x of `old` = storage position x holds an old determinant (index < n_old).
 __global__ void k_old_bits(const uint32_t* __restrict__ perm, int64_t N, int64_t n_old, uint32_t* __restrict__ old) {
   const int64_t nw = (N + 31) >> 5;
@@ -1660,7 +1656,11 @@ void build_ham_csr(const Helpers& hp, const IntsView& ints, Csr& H, bool want64,
                    size_t n_old, Prims& pr, cudaStream_t s) {
   const size_t N = hp.N;
   PhaseTimer pt(s);
-  // a step that at least doubles the space is rebuilt; one that adds nothing is left as it is (below)
+  // A step that at least doubles the space is rebuilt; one that adds nothing is left as it is (below). Extended /
+  // rebuilt by new per old determinant, mixed form: to 402,058 determinants 0.25 19.4 / 24.1 ms, 0.5 25.3 / 24.1,
+  // 0.95 27.3 / 24.1, 1.2 31.0 / 24.1; to 150,924 of 36 orbitals 0.25 10.3 / 12.0, 0.5 12.4 / 12.0; to 30,666
+  // 0.25 2.45 / 1.98. From the line on a rebuild is the faster at every size; below it an extension is up to a fifth
+  // faster (large spaces, to 0.4) and costs up to a sixth more (0.5 to 1), or 0.9 ms (small spaces).
   const bool incremental = !H.block && n_old > 0 && n_old < N && N - n_old < n_old && H.N == n_old &&
                            H.perm.n >= n_old && (want64 ? !want32 : (want32 && want_lo)) &&
                            (H.v64.p != nullptr) == want64 && (H.vhi.p != nullptr) == want32 &&

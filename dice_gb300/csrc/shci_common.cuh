@@ -173,11 +173,6 @@ __device__ __forceinline__ double i2_spatial(const double* __restrict__ I2, int 
   size_t A = ij > kl ? ij : kl, B = ij > kl ? kl : ij;
   return __ldg(I2 + A * (A + 1) / 2 + B);
 }
-// twoInt::operator() on spin orbitals: zero unless both pairs are same-spin
-__device__ __forceinline__ double i2_spin(const double* __restrict__ I2, int i, int j, int k, int l) {
-  if (((i ^ j) & 1) || ((k ^ l) & 1)) return 0.0;
-  return i2_spatial(I2, i >> 1, j >> 1, k >> 1, l >> 1);
-}
 
 // Hij_1Excite (SHCI/Determinants.cpp:437-505): `a` created, `i` destroyed,
 // the sum running over the ket's occupied spin orbitals in ascending order.
@@ -221,38 +216,10 @@ __device__ inline double hij_single(const IntsView& I, const Det2& ket, int a, i
   return (occ_between(ket, lo, hi) & 1) ? -energy : energy;
 }
 
-// Hij_2Excite (SHCI/Determinants.cpp:406-434): i<j destroyed, a<b created.
-__device__ inline double hij_double(const IntsView& I, const Det2& ket, int i, int j, int a, int b) {
-  int c = occ_between(ket, i < a ? i : a, i < a ? a : i) + occ_between(ket, j < b ? j : b, j < b ? b : j);
-  double sgn = (c & 1) ? -1.0 : 1.0;
-  if (a > j || b < i) sgn = -sgn;
-  double v = __dsub_rn(i2_spin(I.I2, a, i, b, j), i2_spin(I.I2, a, j, b, i));
-  return sgn * v;
-}
-
-// Hij(bra, ket) for determinants at excitation distance 1 or 2
-// (SHCI/Determinants.cpp:564-631).
-__device__ inline double hij_any(const IntsView& I, const Det2& bra, const Det2& ket) {
-  uint64_t u0 = bra.w0 ^ ket.w0, u1 = bra.w1 ^ ket.w1;
-  uint64_t c0 = u0 & bra.w0, c1 = u1 & bra.w1;  // created
-  uint64_t d0 = u0 & ket.w0, d1 = u1 & ket.w1;  // destroyed
-  int ncre = __popcll(c0) + __popcll(c1);
-  int cre[2], des[2];
-  int k = 0;
-  while (c0 && k < 2) { cre[k++] = __ffsll((long long)c0) - 1; c0 &= c0 - 1; }
-  while (c1 && k < 2) { cre[k++] = __ffsll((long long)c1) - 1 + 64; c1 &= c1 - 1; }
-  k = 0;
-  while (d0 && k < 2) { des[k++] = __ffsll((long long)d0) - 1; d0 &= d0 - 1; }
-  while (d1 && k < 2) { des[k++] = __ffsll((long long)d1) - 1 + 64; d1 &= d1 - 1; }
-  if (ncre == 1) return hij_single(I, ket, cre[0], des[0]);
-  if (ncre == 2) return hij_double(I, ket, des[0], des[1], cre[0], cre[1]);
-  return 0.0;
-}
-
-// FP32 counterparts of hij_single / hij_double / hij_any on the FP32 integral
-// copies, for the FP32 matrix-free sigma: same excitation and sign logic,
-// FP32 arithmetic (about 1e-7 relative error per element: the rounding of
-// the integrals to FP32 plus the FP32 sum of a single excitation's terms).
+// FP32 counterpart of hij_single on the FP32 integral copies, for the FP32
+// matrix-free sigma: same excitation and sign logic, FP32 arithmetic (about 1e-7
+// relative error per element: the rounding of the integrals to FP32 plus the
+// FP32 sum of the terms).
 __device__ __forceinline__ float i2f_spatial(const float* __restrict__ I2f, int i, int j, int k, int l) {
   int ij = pair_index(i, j), kl = pair_index(k, l);
   size_t A = ij > kl ? ij : kl, B = ij > kl ? kl : ij;
@@ -292,31 +259,6 @@ __device__ inline float hij_single_f32(const IntsView& I, const Det2& ket, int a
   }
   const int lo = a < i ? a : i, hi = a < i ? i : a;
   return (occ_between(ket, lo, hi) & 1) ? -energy : energy;
-}
-__device__ inline float hij_double_f32(const IntsView& I, const Det2& ket, int i, int j, int a, int b) {
-  int c = occ_between(ket, i < a ? i : a, i < a ? a : i) + occ_between(ket, j < b ? j : b, j < b ? b : j);
-  bool neg = (c & 1) != 0;
-  if (a > j || b < i) neg = !neg;
-  float v = 0.f;
-  if (!(((a ^ i) & 1) || ((b ^ j) & 1))) v = i2f_spatial(I.I2f, a >> 1, i >> 1, b >> 1, j >> 1);
-  if (!(((a ^ j) & 1) || ((b ^ i) & 1))) v -= i2f_spatial(I.I2f, a >> 1, j >> 1, b >> 1, i >> 1);
-  return neg ? -v : v;
-}
-__device__ inline float hij_any_f32(const IntsView& I, const Det2& bra, const Det2& ket) {
-  uint64_t u0 = bra.w0 ^ ket.w0, u1 = bra.w1 ^ ket.w1;
-  uint64_t c0 = u0 & bra.w0, c1 = u1 & bra.w1;
-  uint64_t d0 = u0 & ket.w0, d1 = u1 & ket.w1;
-  int ncre = __popcll(c0) + __popcll(c1);
-  int cre[2], des[2];
-  int k = 0;
-  while (c0 && k < 2) { cre[k++] = __ffsll((long long)c0) - 1; c0 &= c0 - 1; }
-  while (c1 && k < 2) { cre[k++] = __ffsll((long long)c1) - 1 + 64; c1 &= c1 - 1; }
-  k = 0;
-  while (d0 && k < 2) { des[k++] = __ffsll((long long)d0) - 1; d0 &= d0 - 1; }
-  while (d1 && k < 2) { des[k++] = __ffsll((long long)d1) - 1 + 64; d1 &= d1 - 1; }
-  if (ncre == 1) return hij_single_f32(I, ket, cre[0], des[0]);
-  if (ncre == 2) return hij_double_f32(I, ket, des[0], des[1], cre[0], cre[1]);
-  return 0.f;
 }
 
 // Compensated FP32 accumulator (s + c): TwoSum of every addition and the FMA
