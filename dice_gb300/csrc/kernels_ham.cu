@@ -403,7 +403,6 @@ static void build_singles_and_index(Helpers& hp, int norb, uint64_t bits, Prims&
       if (too_long) hp.nm1 = 0;  // the views show no index: every group is scanned
     }
   }
-  SHCI_CUDA(cudaStreamSynchronize(s));
 }
 
 void Helpers::build(const Det2* dets, size_t n, int norb, const Det2& ref, const Det2& diff, Prims& pr,

@@ -1254,12 +1254,10 @@ __global__ void __launch_bounds__(256) k_dav_append(double* __restrict__ V, doub
   if ((int)threadIdx.x < m) sg[threadIdx.x] = g[threadIdx.x];
   __syncthreads();
   if (threadIdx.x == 0) {  // one thread's square root and division, not every thread's
-    double n2 = g[m], gg = 0.0;
-    for (int i = 0; i < m; ++i) {
-      n2 -= sg[i] * sg[i];
-      gg += sg[i] * sg[i];
-    }
-    if (!(gg <= 1e-4 * g[m])) n2 = -1.0;
+    const double d2 = g[m];
+    double n2 = d2;
+    for (int i = 0; i < m; ++i) n2 -= sg[i] * sg[i];
+    if (!(n2 >= 0.9999 * d2)) n2 = -1.0;
     const double n = sqrt(n2);
     s_sc = n > 1e-14 ? 1.0 / n : 1.0;
     if (blockIdx.x == 0) {
