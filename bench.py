@@ -687,7 +687,7 @@ def run_sigma_only(args):
 def run_ham_only(args):
     """--section ham: the plain FP64 variational run of the chosen case, then
     the Hamiltonian of its final space built from scratch (string tables,
-    partial-string index, diagonal, count, emit, row sort; for the mixed form
+    partial-string index, diagonal, count, emit, finish; for the mixed form
     also the compact copy), FP64 and mixed, each timed build inside its
     own NVTX range (bench_ham_<mode>). Reloading the determinants before each
     build drops every table and the stored matrix."""

@@ -93,7 +93,10 @@ int shci_set_selection_params(shci_ctx* ctx, int ncore, int nact, int nrestrict,
 
 /* Determinant space. set replaces the space; get copies it out in index
  * order (new determinants are appended in sorted order, as the reference
- * does at SHCI/SHCIbasics.cpp:1059-1077). */
+ * does at SHCI/SHCIbasics.cpp:1059-1077). A list may hold a determinant more
+ * than once (copies are not connected to each other); one with a wrong electron
+ * count or an orbital beyond NORB is refused (SHCI_ERR_INVALID) and the space
+ * stays as it was. */
 int shci_dets_set(shci_ctx* ctx, const uint64_t* dets, int64_t n);
 int shci_dets_count(shci_ctx* ctx, int64_t* n);
 int shci_dets_get(shci_ctx* ctx, uint64_t* out, int64_t cap);
